@@ -285,6 +285,41 @@ def test_gemm_simt_row_does_not_depend_on_the_batch(ops):
         assert torch.equal(part, full[rows])
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9, 16, 17, 32, 33, 64, 65, 200])
+@pytest.mark.parametrize("N,K", [(1, 4), (31, 60), (32, 64), (33, 68), (130, 260), (65, 1028), (70, 2300), (1024, 3072), (40, 12800)])
+def test_gemm_f32_sizes(ops, M, N, K):
+    """float32 rows of whole 16-byte vectors: tiles' edges, K below, at and beyond a slice of 64 and four of them, strided operands,
+    accumulation.  Bound: 64 terms a chain, four chains a group, the groups' sum, every rounding 2^-24 of a partial sum of |a| |w|:
+    (68 + groups of 256) 2^-24 sum |a w|."""
+    torch.manual_seed(7)
+    a = torch.randn(M, K + 8)[:, 4:4 + K]
+    w = torch.randn(N, K) * 0.2
+    ad = dev(torch.zeros(M, K + 8))[:, 4:4 + K]
+    ad.copy_(a)
+    big = torch.zeros(M, N + 6, device="cuda")
+    view = big[:, 3:3 + N]
+    ops.gemm_simt(view, ad, dev(w))
+    ref, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    bound = (68 + (K + 255) // 256) * 2.0 ** -24 * size
+    assert bool(((view.double().cpu() - ref).abs() <= bound).all())
+    once = view.clone()
+    ops.gemm_simt(view, ad, dev(w), accumulate=True)
+    assert torch.equal(view, once + once)
+    assert float(big[:, :3].abs().sum()) == 0.0 and float(big[:, 3 + N:].abs().sum()) == 0.0
+
+
+@pytest.mark.parametrize("N,K", [(1024, 2048), (4096, 1024), (200, 700)])
+def test_gemm_f32_row_does_not_depend_on_the_batch(ops, N, K):
+    torch.manual_seed(8)
+    a, w = dev(torch.randn(300, K)), dev(torch.randn(N, K))
+    full = torch.empty(300, N, device="cuda")
+    ops.gemm_simt(full, a, w)
+    for rows in ([0], [1, 299], [5, 6, 7], list(range(7)), list(range(20, 36)), list(range(100, 131)), list(range(40, 110))):
+        part = torch.empty(len(rows), N, device="cuda")
+        ops.gemm_simt(part, a[rows].contiguous(), w)
+        assert torch.equal(part, full[rows])
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (5, 72, 136), (33, 384, 512), (128, 128, 64), (200, 1000, 1032),
                                    (257, 4096, 1024), (64, 130, 2048), (2048, 1024, 3072), (300, 50, 40)])
 @pytest.mark.parametrize("out_dtype", DTYPES)
