@@ -1,0 +1,569 @@
+// Matrix memories with one decay per head and token, over prompts, on the tensor cores:
+//
+//   S_t = a_t S_(t-1) + b_t k_t v_t^T      o_t = S_t^T q_t
+//
+// with a per-head constant a and b = 1 (CM_CONST: the linear attention of linear_attention.cu), or with the gates of a memory under a
+// running maximum (CM_MAX: memory_scan.cu's mlstm, a = exp(f + m_before - m), b = exp(i - m), and a vector n that decays with S and takes b k).
+//
+// A sequence's tokens are taken in chunks of 64.  With A(i, j) the weight of token j in the output of token i >= j (the decays between
+// them times b_j), g_i the decays from the chunk's start through i, w_j the weight of token j in the state after the chunk:
+//   chunk_memory_local   dS = K^T diag(w) V of every chunk by itself, and the chunk's whole decay
+//   chunk_memory_scan    the state before each chunk, S <- decay S + dS, a thread per entry; the request's state afterwards
+//   chunk_memory_out     o_i = g_i S_before^T q_i + sum_(j <= i) A(i, j) (q_i . k_j) v_j
+// so nothing but the scan's one multiply-add per entry and chunk runs along the sequence.
+//
+// Everything is 32-bit arithmetic although the products run on `mma.sync.m16n8k16`: a float32 operand enters as THREE bfloat16 terms
+// x = x1 + x2 + x3 (24 bits of mantissa), a product of two such operands as the six products of terms whose places add up to at
+// most the third (what is left out is 2^-25 of the product), an operand that is bfloat16 to begin with as itself; the sums are
+// float32, rounded.  What bounds it: a third of the time the tensor cores (for 2,048 tokens on 16 heads of 128 x 128, whose float32 operands take
+// six products, 4 M of them), the rest the conversion of what is staged, and the latency of one block an SM.
+//
+// Measured (us, one sequence, 16 heads of 128 x 128, bfloat16 rows, before -> now), and the error against float64 of the rows:
+//   linear attention   2,048 tokens 352 -> 108 (segments of 256 tokens walked 32 at a time on the CUDA cores), 1.9e-7 -> 0.9e-7;  512: 203 -> 43;  96: 50 -> 38
+//   running maximum    2,048 tokens 798 -> 82 (a walk token by token), 7.4e-7 -> 6.5e-7;  512: 202 -> 34;  96: 41 -> 31
+// Steps of up to 64 tokens keep the walks: one launch, and no state but the request's own to write.
+// A value that is no number reaches the outputs of its sequence from the sixteen tokens it lies in on, not only from its own token on.
+#pragma once
+#include "common.cuh"
+
+namespace chunk_memory {
+
+constexpr int C = 64;           // tokens a chunk
+constexpr int EB = 64;          // value columns at a time
+constexpr int THREADS = 256;
+constexpr int LDE = EB + 8, LDP = C + 8;      // rows of 144 bytes: eight rows' 16 bytes lie in different banks
+enum { CM_CONST = 0, CM_MAX = 1 };
+
+struct Params {
+    const void *q, *k, *v;      // storage type, rows ldq / ldk / ldv apart, heads side by side
+    long long ldq, ldk, ldv;
+    float* out;                 // [tokens, H E]
+    float* state;               // CM_CONST [slots, H, D, E]; CM_MAX rows `state_ld` apart: S [H, D, E], then n [H, D]
+    long long state_ld;
+    const float* decay;         // CM_CONST: [H]
+    const float4* gates;        // CM_MAX: [tokens, H] = (i, f, -, m before the token)
+    const int *cu_q, *state_slots;
+    float* scratch;             // [chunks][H][D E (+ D)], then the chunks' decays [chunks][H]
+    int H, D, E, n_seqs, chunks, silu;      // chunks: the most that the step can have
+    float q_scale, den_eps;
+};
+
+inline bool sizes_usable(int D, int E) { return (D == 64 || D == 128) && E % EB == 0; }
+inline long long scratch_floats(int form, int n_tokens, int n_seqs, int H, int D, int E) {
+    return (long long)(n_tokens / C + n_seqs) * H * ((long long)D * E + (form == CM_MAX ? D : 0) + 1);
+}
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const bf16* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const bf16* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// (x, y) as NT pairs of bfloat16, the most significant first.
+template <int NT>
+__device__ __forceinline__ void terms(uint32_t (&t)[NT], float x, float y) {
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+        t[i] = *reinterpret_cast<const uint32_t*>(&v);
+        if (i + 1 < NT) {
+            const float2 f = __bfloat1622float2(v);
+            x -= f.x;
+            y -= f.y;
+        }
+    }
+}
+// Sums of products: `main` takes the products of the first terms, one MMA after the other added in rounded float32 arithmetic (the tensor cores
+// cut off what an accumulator cannot hold, and always towards zero: 48 products of a sum on one accumulator were 6 times further off), `rest` the
+// products of the other terms, which are 2^-8 of them and below, on an accumulator.
+template <int N8>
+struct Sums {
+    float main[N8][4], rest[N8][4];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int i = 0; i < N8; ++i)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) main[i][u] = rest[i][u] = 0.f;
+    }
+    __device__ __forceinline__ float at(int i, int u) const { return main[i][u] + rest[i][u]; }
+};
+// The products of term ta of A and term tb of B that count: places that add up to at most the last, smallest first.
+template <int NA, int NB, int N8>
+__device__ __forceinline__ void mma_terms(Sums<N8>& s, int n, const uint32_t (&a)[NA][4], const uint32_t (&b)[NB][4]) {
+    constexpr int LAST = (NA > NB ? NA : NB) - 1;
+#pragma unroll
+    for (int sum = LAST; sum >= 1; --sum)
+#pragma unroll
+        for (int ta = 0; ta < NA; ++ta) {
+            const int tb = sum - ta;
+            if (tb < 0 || tb >= NB) continue;
+            mma(s.rest[n], a[ta], b[tb][0], b[tb][1]);
+            mma(s.rest[n + 1], a[ta], b[tb][2], b[tb][3]);
+        }
+    float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+    mma(x, a[0], b[0][0], b[0][1]);
+    mma(y, a[0], b[0][2], b[0][3]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        s.main[n][u] += x[u];
+        s.main[n + 1][u] += y[u];
+    }
+}
+
+__device__ __forceinline__ float act(float x, int silu) { return silu ? __fdividef(x, 1.0f + __expf(-x)) : x; }
+
+// Which sequence and which of its chunks chunk number `c` of the step is (s = -1: the step has fewer).  All threads of a warp.
+struct Place {
+    int s, chunk, base;         // base: number of the sequence's first chunk
+};
+__device__ __forceinline__ Place place_of(const int* __restrict__ cu_q, int n_seqs, int c) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;
+    for (int s0 = 0; s0 < n_seqs; s0 += 32) {
+        const int s = s0 + lane;
+        const int n = s < n_seqs ? ceil_div(max(0, cu_q[s + 1] - cu_q[s]), C) : 0;
+        int upto = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += x;
+        }
+        const unsigned holds = __ballot_sync(0xffffffffu, before + upto > c);
+        if (holds) {
+            const int at = __ffs(holds) - 1;
+            const int base = before + __shfl_sync(0xffffffffu, upto - n, at);
+            return {s0 + at, c - base, base};
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return {-1, 0, 0};
+}
+
+// What the weights of a chunk follow from, per token i: CM_MAX the sums F_i = f_1 + .. + f_i as two floats, i and m; CM_CONST powers of the decay.
+struct Weights {
+    float hi[C], lo[C], gate[C], top[C];    // CM_MAX
+    float pw[C + 1];                        // CM_CONST
+    float m_before;
+};
+template <int FORM>
+__device__ __forceinline__ void make_weights(Weights& w, const Params& p, int h, int t0, int n) {
+    const int tid = threadIdx.x;
+    if (FORM == CM_CONST) {
+        if (tid <= C) w.pw[tid] = powf(p.decay[h], (float)tid);
+        return;
+    }
+    if (tid >= 32) return;
+    double f[2], sum = 0.0;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int i = 2 * tid + u;
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n) g = p.gates[(size_t)(t0 + i) * p.H + h];
+        if (i == 0) w.m_before = g.w;
+        w.gate[i] = i < n ? g.x : 0.f;
+        w.top[i] = i < n ? fmaxf(g.y + g.w, g.x) : 0.f;
+        sum += (double)g.y;
+        f[u] = sum;
+    }
+    double upto = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double x = __shfl_up_sync(0xffffffffu, upto, o);
+        if (tid >= o) upto += x;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const double F = upto - sum + f[u];
+        w.hi[2 * tid + u] = (float)F;
+        w.lo[2 * tid + u] = (float)(F - (double)(float)F);
+    }
+}
+// The weight of token j in what token i (or the state after it) holds, i >= j.
+template <int FORM>
+__device__ __forceinline__ float weight(const Weights& w, int i, int j) {
+    if (FORM == CM_CONST) return w.pw[i - j];
+    return expf((w.hi[i] - w.hi[j]) + (w.lo[i] - w.lo[j]) + (w.gate[j] - w.top[i]));
+}
+// The decays from the chunk's start through token i.
+template <int FORM>
+__device__ __forceinline__ float from_start(const Weights& w, int i) {
+    if (FORM == CM_CONST) return w.pw[i + 1];
+    return expf((w.hi[i] + (w.m_before - w.top[i])) + w.lo[i]);
+}
+
+// COLS columns of a chunk's rows on their way into shared memory: `ask` sends for a thread's 16-byte vectors, all at once, and `put` writes them
+// as NT terms, times `scale` per row (null: 1), zeros beyond the chunk's n tokens.
+template <typename T, int NT, int COLS>
+struct Rows {
+    static constexpr int VN = Vec16<T>::N, LD = COLS + 8, EACH = C * COLS / VN / THREADS;
+    Vec16<T> held[EACH];
+    __device__ __forceinline__ void ask(const T* src, long long ld, int n) {
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            const int idx = threadIdx.x + i * THREADS, r = idx / (COLS / VN), c = idx % (COLS / VN) * VN;
+            if (r < n) held[i].raw = *reinterpret_cast<const decltype(held[i].raw)*>(src + (size_t)r * ld + c);
+        }
+    }
+    __device__ __forceinline__ void put(bf16* dst, int n, int silu, const float* scale) {
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            const int idx = threadIdx.x + i * THREADS, r = idx / (COLS / VN), c = idx % (COLS / VN) * VN;
+            float f[VN];
+            if (r < n) {
+                if constexpr (NT == 1) {        // (bfloat16 as it is)
+                    *reinterpret_cast<decltype(held[i].raw)*>(dst + r * LD + c) = held[i].raw;
+                    continue;
+                }
+                held[i].unpack(f);
+                const float s = scale ? scale[r] : 1.f;
+#pragma unroll
+                for (int u = 0; u < VN; ++u) f[u] = act(f[u], silu) * s;
+            } else {
+#pragma unroll
+                for (int u = 0; u < VN; ++u) f[u] = 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < VN; u += 4) {
+                uint32_t a[NT], b[NT];
+                terms<NT>(a, f[u], f[u + 1]);
+                terms<NT>(b, f[u + 2], f[u + 3]);
+#pragma unroll
+                for (int t = 0; t < NT; ++t) *reinterpret_cast<uint2*>(dst + (t * C + r) * LD + c + u) = make_uint2(a[t], b[t]);
+            }
+        }
+    }
+};
+
+// Terms of q, k and v: one where they are bfloat16 values as they are stored.
+template <typename T, int FORM> constexpr int input_terms() { return sizeof(T) == 2 && FORM == CM_MAX ? 1 : 3; }
+
+// ---------------------------------------------------------------------------------------------------------------- local
+// Block (chunk, head): dS [D, E], 64 columns at a time; warp w has rows 16 (w % (D / 16)) of D and, with D = 64, half of the columns.
+template <typename T, int FORM, int D>
+__global__ void __launch_bounds__(THREADS, 2) chunk_memory_local_kernel(Params p) {
+    constexpr int NT = input_terms<T, FORM>(), LDD = D + 8;
+    constexpr int ROW_WARPS = D / 16, COL_WARPS = 8 / ROW_WARPS, N8 = EB / 8 / COL_WARPS;
+    extern __shared__ __align__(16) bf16 smem[];
+    bf16* Ks = smem;                            // [NT][C][LDD]
+    bf16* Vs = Ks + NT * C * LDD;               // [3][C][LDE]: the values times their weights
+    __shared__ Weights w;
+    __shared__ float wj[C];
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
+    const Place at = place_of(p.cu_q, p.n_seqs, blockIdx.x);
+    if (at.s < 0 || (FORM == CM_CONST && p.state_slots[at.s] < 0)) return;
+    const int q_beg = p.cu_q[at.s], t0 = q_beg + at.chunk * C, n = min(C, p.cu_q[at.s + 1] - t0);
+    Rows<T, NT, D> keys;
+    Rows<T, 3, EB> values;
+    const T* vp = static_cast<const T*>(p.v) + (size_t)t0 * p.ldv + (size_t)h * p.E;
+    keys.ask(static_cast<const T*>(p.k) + (size_t)t0 * p.ldk + (size_t)h * D, p.ldk, n);
+    values.ask(vp, p.ldv, n);
+    make_weights<FORM>(w, p, h, t0, n);
+    keys.put(Ks, n, p.silu, nullptr);
+    __syncthreads();
+    if (tid < C) wj[tid] = tid < n ? weight<FORM>(w, n - 1, tid) : 0.f;
+    float* dst = p.scratch + ((size_t)blockIdx.x * p.H + h) * ((size_t)D * p.E + (FORM == CM_MAX ? D : 0));
+    if (tid == 0) {
+        float* gains = p.scratch + (size_t)p.chunks * p.H * ((size_t)D * p.E + (FORM == CM_MAX ? D : 0));
+        gains[(size_t)blockIdx.x * p.H + h] = from_start<FORM>(w, n - 1);
+    }
+    __syncthreads();
+    const int d0 = 16 * (warp % ROW_WARPS), e_warp = (warp / ROW_WARPS) * (N8 * 8);
+    for (int e0 = 0; e0 < p.E; e0 += EB) {
+        if (e0 > 0) __syncthreads();            // the columns before are used
+        values.put(Vs, n, p.silu, wj);
+        __syncthreads();
+        if (e0 + EB < p.E) values.ask(vp + e0 + EB, p.ldv, n);
+        Sums<N8> acc;
+        acc.clear();
+        for (int j0 = 0; j0 < n; j0 += 16) {
+            uint32_t a[NT][4];
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+                ldsm4t(a[t], Ks + (t * C + j0 + (lane & 7) + (lane >> 4) * 8) * LDD + d0 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+            for (int n8 = 0; n8 < N8; n8 += 2) {
+                uint32_t b[3][4];
+#pragma unroll
+                for (int t = 0; t < 3; ++t)
+                    ldsm4t(b[t], Vs + (t * C + j0 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDE + e_warp + n8 * 8 + (lane >> 4) * 8);
+                mma_terms(acc, n8, a, b);
+            }
+        }
+#pragma unroll
+        for (int n8 = 0; n8 < N8; ++n8) {
+            float* o = dst + (size_t)(d0 + lane / 4) * p.E + e0 + e_warp + n8 * 8 + 2 * (lane & 3);
+            *reinterpret_cast<float2*>(o) = make_float2(acc.at(n8, 0), acc.at(n8, 1));
+            *reinterpret_cast<float2*>(o + (size_t)8 * p.E) = make_float2(acc.at(n8, 2), acc.at(n8, 3));
+        }
+    }
+    if (FORM == CM_MAX && tid < D) {            // n's own sum
+        float s = 0.f;
+        for (int j = 0; j < n; ++j) {
+            float k = 0.f;
+#pragma unroll
+            for (int t = NT - 1; t >= 0; --t) k += to_float(Ks[(t * C + j) * LDD + tid]);
+            s = fmaf(wj[j], k, s);
+        }
+        dst[(size_t)D * p.E + tid] = s;
+    }
+}
+
+// ----------------------------------------------------------------------------------------------------------------- scan
+// A thread per entry of the state (CM_MAX: of n too): a chunk's sum is replaced by the state before it, eight chunks' values asked for at once.
+template <int FORM>
+__global__ void __launch_bounds__(THREADS) chunk_memory_scan_kernel(Params p) {
+    const int s = blockIdx.x, h = blockIdx.y, entry = blockIdx.z * THREADS + threadIdx.x;
+    const int entries = p.D * p.E + (FORM == CM_MAX ? p.D : 0);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int slot = p.state_slots[s], n_tok = p.cu_q[s + 1] - p.cu_q[s];
+    if (n_tok <= 0 || (slot < 0 && FORM == CM_CONST)) return;
+    int base = 0;
+    for (int i = 0; i < s; ++i) base += ceil_div(max(0, p.cu_q[i + 1] - p.cu_q[i]), C);
+    if (entry >= entries) return;
+    const int count = ceil_div(n_tok, C);
+    float* Sg = nullptr;
+    if (slot >= 0) {
+        const int DE = p.D * p.E;
+        Sg = p.state + (size_t)slot * p.state_ld + (entry < DE ? (size_t)h * DE + entry : (size_t)p.H * DE + (size_t)h * p.D + (entry - DE));
+    }
+    const size_t stride = (size_t)p.H * entries;
+    float* at = p.scratch + ((size_t)base * p.H + h) * entries + entry;
+    const float* gain = p.scratch + (size_t)p.chunks * p.H * entries + (size_t)base * p.H + h;
+    float S = Sg ? *Sg : 0.f;
+    for (int c0 = 0; c0 < count; c0 += 8) {
+        float add[8], g[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            add[u] = c0 + u < count ? at[(size_t)(c0 + u) * stride] : 0.f;
+            g[u] = c0 + u < count ? gain[(size_t)(c0 + u) * p.H] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (c0 + u >= count) break;
+            at[(size_t)(c0 + u) * stride] = S;
+            S = fmaf(g[u], S, add[u]);
+        }
+    }
+    if (Sg) *Sg = S;
+}
+
+// ------------------------------------------------------------------------------------------------------------------ out
+// Block (chunk, head): warp w has rows 16 (w % 4) of the chunk and half of the keys (scores) or of 64 value columns (outputs).
+template <typename T, int FORM, int D>
+struct OutLayout {
+    static constexpr int NT = input_terms<T, FORM>(), LDD = D + 8;
+    static constexpr int Q = NT * C * LDD, KS = (NT * C * LDD > 3 * D * LDE ? NT * C * LDD : 3 * D * LDE), P = 3 * C * LDP, V = NT * C * LDE;
+    static constexpr size_t bytes() { return (size_t)(Q + KS + P + V) * sizeof(bf16); }
+};
+template <typename T, int FORM, int D>
+__global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) {
+    using L = OutLayout<T, FORM, D>;
+    constexpr int NT = L::NT, LDD = L::LDD;
+    extern __shared__ __align__(16) bf16 smem[];
+    bf16* Qs = smem;                            // [NT][C][LDD]
+    bf16* Ks = Qs + L::Q;                       // [NT][C][LDD], then the state's columns [3][D][LDE]
+    bf16* Ps = Ks + L::KS;                      // [3][C][LDP]: the weighted scores
+    bf16* Vs = Ps + L::P;                       // [NT][C][LDE]
+    __shared__ Weights w;
+    __shared__ float start[C], sums[2][C], n_dot[C];
+    const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
+    const Place at = place_of(p.cu_q, p.n_seqs, blockIdx.x);
+    if (at.s < 0 || (FORM == CM_CONST && p.state_slots[at.s] < 0)) return;
+    const int q_beg = p.cu_q[at.s], t0 = q_beg + at.chunk * C, n = min(C, p.cu_q[at.s + 1] - t0);
+    const float* before = p.scratch + ((size_t)blockIdx.x * p.H + h) * ((size_t)D * p.E + (FORM == CM_MAX ? D : 0));
+    // the state's entries of 64 columns, float4 a thread and turn: asked for early, put down where the keys were
+    constexpr int SV = D * EB / 4 / THREADS;
+    float4 held[SV];
+    auto ask = [&](int e0) {
+#pragma unroll
+        for (int i = 0; i < SV; ++i) {
+            const int idx = tid + i * THREADS, d = idx / (EB / 4), c = idx % (EB / 4) * 4;
+            held[i] = *reinterpret_cast<const float4*>(before + (size_t)d * p.E + e0 + c);
+        }
+    };
+    const T* vp = static_cast<const T*>(p.v) + (size_t)t0 * p.ldv + (size_t)h * p.E;
+    Rows<T, NT, EB> values;
+    {
+        Rows<T, NT, D> queries, keys;
+        queries.ask(static_cast<const T*>(p.q) + (size_t)t0 * p.ldq + (size_t)h * D, p.ldq, n);
+        keys.ask(static_cast<const T*>(p.k) + (size_t)t0 * p.ldk + (size_t)h * D, p.ldk, n);
+        values.ask(vp, p.ldv, n);
+        ask(0);
+        make_weights<FORM>(w, p, h, t0, n);
+        queries.put(Qs, n, p.silu, nullptr);
+        keys.put(Ks, n, p.silu, nullptr);
+    }
+    __syncthreads();
+    if (tid < C) start[tid] = tid < n ? from_start<FORM>(w, tid) * p.q_scale : 0.f;
+    const int r0 = 16 * (warp & 3), half = warp >> 2;
+    // scores of 16 rows and 32 keys, those of keys behind all rows left out
+    {
+        Sums<4> s;
+        s.clear();
+        const int j0 = 32 * half;
+        if (j0 <= r0 + 15) {
+#pragma unroll 2
+            for (int d = 0; d < D; d += 16) {
+                uint32_t a[NT][4];
+#pragma unroll
+                for (int t = 0; t < NT; ++t) ldsm4(a[t], Qs + (t * C + r0 + (lane & 15)) * LDD + d + (lane >> 4) * 8);
+#pragma unroll
+                for (int n8 = 0; n8 < 4; n8 += 2) {
+                    if (j0 + 8 * n8 > r0 + 15) continue;
+                    uint32_t b[NT][4];
+#pragma unroll
+                    for (int t = 0; t < NT; ++t)
+                        ldsm4(b[t], Ks + (t * C + j0 + 8 * n8 + (lane & 7) + (lane >> 4) * 8) * LDD + d + ((lane >> 3) & 1) * 8);
+                    mma_terms(s, n8, a, b);
+                }
+            }
+        }
+        float row_sum[2] = {0.f, 0.f};
+#pragma unroll
+        for (int n8 = 0; n8 < 4; ++n8)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = r0 + lane / 4 + 8 * u, j = j0 + 8 * n8 + 2 * (lane & 3);
+                float x = 0.f, y = 0.f;
+                if (j <= i && i < n) x = s.at(n8, 2 * u) * (weight<FORM>(w, i, j) * p.q_scale);
+                if (j + 1 <= i && i < n) y = s.at(n8, 2 * u + 1) * (weight<FORM>(w, i, j + 1) * p.q_scale);
+                row_sum[u] += x + y;
+                uint32_t t[3];
+                terms<3>(t, x, y);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t*>(Ps + (k * C + i) * LDP + j) = t[k];
+            }
+        if (FORM == CM_MAX) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                row_sum[u] += __shfl_xor_sync(0xffffffffu, row_sum[u], 1);
+                row_sum[u] += __shfl_xor_sync(0xffffffffu, row_sum[u], 2);
+                if ((lane & 3) == 0) sums[half][r0 + lane / 4 + 8 * u] = row_sum[u];
+            }
+            // q . n of 8 rows a warp
+            const float* nb = before + (size_t)D * p.E;
+            for (int i = warp; i < n; i += 8) {
+                float x = 0.f;
+#pragma unroll
+                for (int d = lane; d < D; d += 32) {
+                    float q = 0.f;
+#pragma unroll
+                    for (int t = NT - 1; t >= 0; --t) q += to_float(Qs[(t * C + i) * LDD + d]);
+                    x = fmaf(q, nb[d], x);
+                }
+                x = warp_sum(x);
+                if (lane == 0) n_dot[i] = x;
+            }
+        }
+    }
+    for (int e0 = 0; e0 < p.E; e0 += EB) {
+        __syncthreads();                        // the keys, or the columns before, are used
+#pragma unroll
+        for (int i = 0; i < SV; ++i) {
+            const int idx = tid + i * THREADS, d = idx / (EB / 4), c = idx % (EB / 4) * 4;
+            uint32_t a[3], b[3];
+            terms<3>(a, held[i].x, held[i].y);
+            terms<3>(b, held[i].z, held[i].w);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) *reinterpret_cast<uint2*>(Ks + (t * D + d) * LDE + c) = make_uint2(a[t], b[t]);
+        }
+        values.put(Vs, n, p.silu, nullptr);
+        __syncthreads();
+        if (e0 + EB < p.E) {
+            ask(e0 + EB);
+            values.ask(vp + e0 + EB, p.ldv, n);
+        }
+        Sums<4> o;
+        o.clear();
+#pragma unroll 2
+        for (int d = 0; d < D; d += 16) {
+            uint32_t a[NT][4];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) ldsm4(a[t], Qs + (t * C + r0 + (lane & 15)) * LDD + d + (lane >> 4) * 8);
+#pragma unroll
+            for (int n8 = 0; n8 < 4; n8 += 2) {
+                uint32_t b[3][4];
+#pragma unroll
+                for (int t = 0; t < 3; ++t)
+                    ldsm4t(b[t], Ks + (t * D + d + (lane & 7) + ((lane >> 3) & 1) * 8) * LDE + 32 * half + 8 * n8 + (lane >> 4) * 8);
+                mma_terms(o, n8, a, b);
+            }
+        }
+        const float g[2] = {start[r0 + lane / 4], start[r0 + lane / 4 + 8]};
+#pragma unroll
+        for (int n8 = 0; n8 < 4; ++n8)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                o.main[n8][u] *= g[u / 2];
+                o.rest[n8][u] *= g[u / 2];
+            }
+        for (int j = 0; j <= r0; j += 16) {      // keys behind the rows weigh nothing
+            uint32_t a[3][4];
+#pragma unroll
+            for (int t = 0; t < 3; ++t) ldsm4(a[t], Ps + (t * C + r0 + (lane & 15)) * LDP + j + (lane >> 4) * 8);
+#pragma unroll
+            for (int n8 = 0; n8 < 4; n8 += 2) {
+                uint32_t b[NT][4];
+#pragma unroll
+                for (int t = 0; t < NT; ++t)
+                    ldsm4t(b[t], Vs + (t * C + j + (lane & 7) + ((lane >> 3) & 1) * 8) * LDE + 32 * half + 8 * n8 + (lane >> 4) * 8);
+                mma_terms(o, n8, a, b);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = r0 + lane / 4 + 8 * u;
+            if (i >= n) continue;
+            float inv = 1.f;
+            if (FORM == CM_MAX) {
+                const float dot = fmaf(start[i], n_dot[i], sums[0][i] + sums[1][i]);
+                inv = 1.0f / (fmaxf(fabsf(dot), expf(-w.top[i])) + p.den_eps);
+            }
+            float* to = p.out + (size_t)(t0 + i) * ((size_t)p.H * p.E) + (size_t)h * p.E + e0 + 32 * half + 2 * (lane & 3);
+#pragma unroll
+            for (int n8 = 0; n8 < 4; ++n8) *reinterpret_cast<float2*>(to + 8 * n8) = make_float2(o.at(n8, 2 * u) * inv, o.at(n8, 2 * u + 1) * inv);
+        }
+    }
+}
+
+// Whether the kernels above take these sizes and addresses: key widths of 64 and 128, value widths in whole runs of 64 columns, rows of 16-byte vectors.
+inline bool usable(const Params& p, int elem) {
+    const int v = 16 / elem;
+    return sizes_usable(p.D, p.E) && p.ldq % v == 0 && p.ldk % v == 0 && p.ldv % v == 0 && host_aligned16(p.q) && host_aligned16(p.k) &&
+           host_aligned16(p.v) && host_aligned16(p.out) && host_aligned16(p.scratch);
+}
+
+template <typename T, int FORM, int D>
+int launch_width(const Params& p, cudaStream_t s) {
+    constexpr int NT = input_terms<T, FORM>();
+    const size_t local = (size_t)(NT * C * (D + 8) + 3 * C * LDE) * sizeof(bf16), out = OutLayout<T, FORM, D>::bytes();
+    auto k1 = chunk_memory_local_kernel<T, FORM, D>;
+    auto k3 = chunk_memory_out_kernel<T, FORM, D>;
+    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)local);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
+    if (e != cudaSuccess) LLMK_FAIL("chunk_memory: cannot raise shared memory: %s", cudaGetErrorString(e));
+    const dim3 grid(p.chunks, p.H);
+    const int entries = p.D * p.E + (FORM == CM_MAX ? p.D : 0);
+    LLMK_CHECK_LAUNCH_RC("chunk_memory_local", llmk_launch(k1, grid, dim3(THREADS), local, s, true, p));
+    LLMK_CHECK_LAUNCH_RC("chunk_memory_scan", llmk_launch(chunk_memory_scan_kernel<FORM>, dim3(p.n_seqs, p.H, ceil_div(entries, THREADS)), dim3(THREADS), 0, s, true, p));
+    LLMK_CHECK_LAUNCH_RC("chunk_memory_out", llmk_launch(k3, grid, dim3(THREADS), out, s, true, p));
+    return LLMK_OK;
+}
+template <typename T, int FORM>
+int launch(const Params& p, cudaStream_t s) {
+    return p.D == 64 ? launch_width<T, FORM, 64>(p, s) : launch_width<T, FORM, 128>(p, s);
+}
+
+}  // namespace chunk_memory

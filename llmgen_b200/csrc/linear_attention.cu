@@ -22,10 +22,15 @@
 // state), and a third launch adds that state's share, lambda^(i+1) S_before^T q_i, to the segment's outputs.  A
 // prompt's chunks then no longer form one chain of dependent steps on a handful of SMs.
 //
+// Steps of more than 64 tokens with key widths of 64 or 128, value widths in runs of 64 and rows of 16-byte vectors take the
+// chunks of 64 tokens of chunk_memory.cuh instead, whose products run on the tensor cores at 32-bit precision.
+//
 // A sequence whose state slot is negative or that brings no tokens (the padding of a step laid out for replay) is
 // skipped.
 #define LLMK_MODULE_NAME "linear_attention"
 #include "common.cuh"
+#include "chunk_memory.cuh"
+#include <algorithm>
 
 LLMK_DEFINE_LAST_ERROR()
 
@@ -51,6 +56,7 @@ struct LinAttnParams {
 };
 
 constexpr int LA_SEG = 256;     // tokens per segment (a multiple of the chunk)
+constexpr int LA_CHUNKS_FROM = 64;      // steps of more tokens take the chunks of chunk_memory.cuh where it takes the sizes
 
 // Index of sequence s's first segment among all segments of the step, and how many it has.
 __device__ __forceinline__ int la_segment_base(const int* cu_q, int s, int& count) {
@@ -411,8 +417,11 @@ static int dispatch_linear_attention(const LinAttnParams& p, dim3 grid, size_t s
 // Floats of scratch that a step of `n_tokens` tokens in `n_seqs` sequences needs for its segments' states (0: the step
 // runs without segments).
 LLMK_EXPORT long long llmk_linear_attention_scratch_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim) {
-    if (n_tokens <= LA_SEG) return 0;
-    return (long long)(n_tokens / LA_SEG + n_seqs) * heads * dim * vdim;
+    long long need = 0;
+    if (n_tokens > LA_SEG) need = (long long)(n_tokens / LA_SEG + n_seqs) * heads * dim * vdim;
+    if (n_tokens > LA_CHUNKS_FROM && chunk_memory::sizes_usable(dim, vdim))
+        need = std::max(need, chunk_memory::scratch_floats(chunk_memory::CM_CONST, n_tokens, n_seqs, heads, dim, vdim));
+    return need;
 }
 
 // n_tokens: rows of `out` (all tokens of the step).  With more than LA_SEG of them a sequence's tokens are cut into
@@ -435,6 +444,15 @@ LLMK_EXPORT int llmk_linear_attention(float* out, const void* q, const void* k, 
     if (dtype != LLMK_F32 && dtype != LLMK_BF16) LLMK_FAIL("linear_attention: unknown dtype %d", dtype);
     const int vsplits = ceil_div(vdim, LA_EV);
     if ((long long)vsplits * p.segments > 65535) LLMK_FAIL("linear_attention: too many segments");
+    if (n_tokens > LA_CHUNKS_FROM && seg_state) {
+        chunk_memory::Params c = {};
+        c.q = q; c.k = k; c.v = v; c.ldq = c.ldk = c.ldv = ld; c.out = out; c.state = state; c.state_ld = (long long)heads * dim * vdim;
+        c.decay = decay; c.cu_q = cu_q; c.state_slots = state_slots; c.scratch = seg_state; c.H = heads; c.D = dim; c.E = vdim;
+        c.n_seqs = n_seqs; c.chunks = n_tokens / chunk_memory::C + n_seqs; c.silu = silu; c.q_scale = 1.f;
+        if (chunk_memory::usable(c, dtype == LLMK_F32 ? 4 : 2))
+            return dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_CONST>(c, (cudaStream_t)stream)
+                                     : chunk_memory::launch<bf16, chunk_memory::CM_CONST>(c, (cudaStream_t)stream);
+    }
     const size_t smem = ((size_t)LA_C * (((dim + 3) & ~3) + dim + 1) + (size_t)dim * LA_C + LA_C * LA_EV + LA_C * (LA_C + 1) +
                          (size_t)dim * LA_EV + LA_C + 1) * sizeof(float);
     dim3 grid(n_seqs, heads, vsplits * p.segments);

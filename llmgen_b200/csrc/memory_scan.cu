@@ -20,10 +20,13 @@
 // A step's sequences are given as everywhere else: sequence s owns token rows [cu_q[s], cu_q[s+1]), its state lies in
 // slot state_slots[s] (-1: none; the sequence then starts from zeros and leaves nothing).  Rows beyond cu_q[n_seqs]
 // belong to no sequence and are skipped, sequences without tokens too, so every launch here follows from a step's shape.
+// Prompts through the mlstm form with key widths of 64 or 128 and value widths in runs of 64 take the chunks of chunk_memory.cuh.
 // States, gates, decays, their logarithms and exponentials, unit norms and the recurrences are float32 arithmetic in both
-// storage dtypes.  The arithmetic of a token does not depend on where a step was cut.
+// storage dtypes.  The arithmetic of a token of a walk does not depend on where a step was cut;
+// in chunks its sums are grouped by the chunks of its step.
 #define LLMK_MODULE_NAME "memory_scan"
 #include "common.cuh"
+#include "chunk_memory.cuh"
 
 LLMK_DEFINE_LAST_ERROR()
 
@@ -191,6 +194,60 @@ __global__ void mlstm_maxima_kernel(float* __restrict__ gates, float* __restrict
         m = __shfl_sync(0xffffffffu, after, nt - 1);
     }
     if (slot >= 0 && lane == 0) m_state[(size_t)slot * state_ld + h] = m;
+}
+
+// The same for steps of many tokens: a block per (sequence, head) takes 2,048 tokens at a time, eight in a row a thread, whose steps compose
+// in the thread, over the warp's lanes and over the warps (48 us a warp, 2,048 tokens on 16 heads; nearly all of it the wait for gates).
+constexpr int MX_THREADS = 256, MX_EACH = 8;
+__global__ void __launch_bounds__(MX_THREADS) mlstm_maxima_block_kernel(float* __restrict__ gates, float* __restrict__ m_state, long long state_ld,
+                                                                        const int* __restrict__ cu_q, const int* __restrict__ state_slots, int H) {
+    __shared__ float2 warps[MX_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int s = blockIdx.y, h = blockIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int q_beg = cu_q[s], n = cu_q[s + 1] - q_beg;
+    if (n <= 0) return;
+    const int slot = state_slots[s];
+    float m = slot >= 0 ? m_state[(size_t)slot * state_ld + h] : 0.f;
+    float4* g = reinterpret_cast<float4*>(gates) + (size_t)q_beg * H + h;
+    for (int t0 = 0; t0 < n; t0 += MX_THREADS * MX_EACH) {
+        const int t = t0 + (int)threadIdx.x * MX_EACH;
+        float2 own[MX_EACH];
+#pragma unroll
+        for (int u = 0; u < MX_EACH; ++u)      // beyond the sequence: the step that changes nothing
+            own[u] = t + u < n ? *reinterpret_cast<const float2*>(g + (size_t)(t + u) * H) : make_float2(-INFINITY, 0.f);
+        float f = 0.f, i = -INFINITY;
+#pragma unroll
+        for (int u = 0; u < MX_EACH; ++u) {
+            i = fmaxf(i + own[u].y, own[u].x);
+            f += own[u].y;
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float pf = __shfl_up_sync(0xffffffffu, f, o), pi = __shfl_up_sync(0xffffffffu, i, o);
+            if (lane >= o) {
+                i = fmaxf(pi + f, i);
+                f += pf;
+            }
+        }
+        if (lane == 31) warps[warp] = make_float2(f, i);
+        __syncthreads();
+        float before = m;                       // ... the maximum before this warp's tokens, and after all of this turn's
+        for (int w = 0; w < MX_THREADS / 32; ++w) {
+            if (w == warp) before = m;
+            m = fmaxf(warps[w].x + m, warps[w].y);
+        }
+        const float pf = __shfl_up_sync(0xffffffffu, f, 1), pi = __shfl_up_sync(0xffffffffu, i, 1);
+        float x = lane > 0 ? fmaxf(pf + before, pi) : before;
+#pragma unroll
+        for (int u = 0; u < MX_EACH; ++u) {
+            if (t + u < n) g[(size_t)(t + u) * H].w = x;
+            x = fmaxf(own[u].y + x, own[u].x);
+        }
+        __syncthreads();                        // the warps' sums are read
+    }
+    if (slot >= 0 && threadIdx.x == 0) m_state[(size_t)slot * state_ld + h] = m;
 }
 
 // ------------------------------------------------------------------------------------------------------- delta rule prep
@@ -525,6 +582,8 @@ LLMK_EXPORT int llmk_min_gru(void* out, const float* zxg, long long ld, const fl
     return LLMK_OK;
 }
 
+// Steps of up to this many token rows: a warp per (sequence, head); longer ones: a block.
+constexpr int MAXIMA_FEW_TOKENS = 64;
 // gates [n, H, 4] float32 <- (i, f, (q . k) q_scale, m before the token) per token and head; m [slots, >= H] carried in the state.
 LLMK_EXPORT int llmk_mlstm_gates(float* gates, const void* q, long long ldq, const void* k, long long ldk, const void* gi, long long ldi,
                                  const void* gf, long long ldf, const float* bi, const float* bf, float* m_state, long long state_ld,
@@ -544,6 +603,11 @@ LLMK_EXPORT int llmk_mlstm_gates(float* gates, const void* q, long long ldq, con
         LLMK_CHECK_LAUNCH_RC("mlstm_gates", llmk_launch(mlstm_gates_kernel<bf16>, grid, block, 0, st, true, gates, (const bf16*)q, ldq,
                                                         (const bf16*)k, ldk, (const bf16*)gi, ldi, (const bf16*)gf, ldf, bi, bf, cu_q,
                                                         n_seqs, n_rows, H, D, cap, q_scale));
+    if (n_rows > MAXIMA_FEW_TOKENS) {
+        LLMK_CHECK_LAUNCH_RC("mlstm_maxima", llmk_launch(mlstm_maxima_block_kernel, dim3(H, n_seqs), dim3(MX_THREADS), 0, st, true, gates, m_state,
+                                                         state_ld, cu_q, state_slots, H));
+        return LLMK_OK;
+    }
     LLMK_CHECK_LAUNCH_RC("mlstm_maxima", llmk_launch(mlstm_maxima_kernel, dim3(ceil_div(n_seqs * H, 4)), dim3(128), 0, st, true, gates,
                                                      m_state, state_ld, cu_q, state_slots, n_seqs, H));
     return LLMK_OK;
@@ -569,11 +633,20 @@ LLMK_EXPORT int llmk_delta_rule_prep(float* aux, float* dots, const void* r, lon
     return LLMK_OK;
 }
 
-// The memory's walk over each sequence's new tokens (see the top of the file).  form 0: delta, 1: mlstm.
+// Steps of more token rows than this give the mlstm form's scratch a use: the chunks of chunk_memory.cuh, where it takes the sizes.
+constexpr int CHUNKS_FROM = 64;
+// Floats of scratch that a step of `n_tokens` token rows in `n_seqs` sequences has a use for (0: none).
+LLMK_EXPORT long long llmk_memory_scan_scratch_floats(int n_tokens, int n_seqs, int H, int D, int E, int form) {
+    if (form != FORM_MLSTM || n_tokens <= CHUNKS_FROM || !chunk_memory::sizes_usable(D, E)) return 0;
+    return chunk_memory::scratch_floats(chunk_memory::CM_MAX, n_tokens, n_seqs, H, D, E);
+}
+
+// The memory's walk over each sequence's new tokens (see the top of the file).  form 0: delta, 1: mlstm.  n_tokens: rows of `out`;
+// scratch: llmk_memory_scan_scratch_floats floats, or null (the walk token by token).
 LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const void* k, long long ldk, const void* v, long long ldv,
                                  const float* aux, const float* dots, float* state, long long state_ld, const int* cu_q,
                                  const int* state_slots, int n_seqs, int H, int D, int E, int form, float r_scale, float den_eps,
-                                 int dtype, void* stream) {
+                                 int n_tokens, float* scratch, int dtype, void* stream) {
     if (n_seqs <= 0) return LLMK_OK;
     if (H <= 0 || D <= 0 || E <= 0 || D > 256) LLMK_FAIL("memory_scan: heads %d, key width %d (at most 256), value width %d", H, D, E);
     if (form != FORM_DELTA && form != FORM_MLSTM) LLMK_FAIL("memory_scan: unknown form %d", form);
@@ -582,6 +655,14 @@ LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const
     p.out = out; p.r = r; p.k = k; p.v = v; p.ldr = ldr; p.ldk = ldk; p.ldv = ldv; p.aux = aux; p.dots = dots; p.state = state;
     p.state_ld = state_ld; p.cu_q = cu_q; p.state_slots = state_slots; p.H = H; p.D = D; p.E = E; p.r_scale = r_scale; p.den_eps = den_eps;
     cudaStream_t st = (cudaStream_t)stream;
+    if (scratch && llmk_memory_scan_scratch_floats(n_tokens, n_seqs, H, D, E, form) > 0) {
+        chunk_memory::Params c = {};
+        c.q = r; c.k = k; c.v = v; c.ldq = ldr; c.ldk = ldk; c.ldv = ldv; c.out = out; c.state = state; c.state_ld = state_ld;
+        c.gates = reinterpret_cast<const float4*>(dots); c.cu_q = cu_q; c.state_slots = state_slots; c.scratch = scratch; c.H = H; c.D = D; c.E = E;
+        c.n_seqs = n_seqs; c.chunks = n_tokens / chunk_memory::C + n_seqs; c.q_scale = r_scale; c.den_eps = den_eps;
+        if (chunk_memory::usable(c, dtype == LLMK_F32 ? 4 : 2) && host_aligned16(dots))
+            return dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_MAX>(c, st) : chunk_memory::launch<bf16, chunk_memory::CM_MAX>(c, st);
+    }
     if (dtype == LLMK_F32)
         return form == FORM_DELTA ? launch_scan<float, FORM_DELTA>(p, n_seqs, st) : launch_scan<float, FORM_MLSTM>(p, n_seqs, st);
     return form == FORM_DELTA ? launch_scan<bf16, FORM_DELTA>(p, n_seqs, st) : launch_scan<bf16, FORM_MLSTM>(p, n_seqs, st);

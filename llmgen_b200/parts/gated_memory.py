@@ -105,7 +105,8 @@ class MLSTM(Mixer):
 
     def workspace_bytes(self, tokens: int) -> int:
         elem = 2 if self.dtype == torch.bfloat16 else 4
-        return tokens * (self.w_in.shape[0] * elem + self.H * 16 + self.H * self.E * (4 + elem) + self.spec.hidden_size * elem) \
+        chunks = 4 * ops.memory_scan_scratch_floats(tokens, max(1, tokens // 32), self.H, self.D, self.E, "mlstm")
+        return chunks + tokens * (self.w_in.shape[0] * elem + self.H * 16 + self.H * self.E * (4 + elem) + self.spec.hidden_size * elem) \
             + ops.SLICED_PRODUCT_BYTES
 
     def forward(self, ctx, x, cache: LayerCache):
@@ -118,8 +119,10 @@ class MLSTM(Mixer):
         ops.mlstm_gates(gates, q, k, packed[:, self.i_off:self.f_off], packed[:, self.f_off:], self.b_i, self.b_f,
                         cache.state[:, self.m_off:], ctx.cu_q, ctx.state_slots, ctx.n_seqs, H, D, float(self.spec.gate_cap), scale)
         o = ws.buffer("mlstm_o", T, H * E, torch.float32)
+        need = ops.memory_scan_scratch_floats(T, ctx.n_seqs, H, D, E, "mlstm")
+        scratch = ws.flat("mlstm_chunks", need, torch.float32) if need else None
         ops.memory_scan(o, q, k, v, None, gates, cache.state, ctx.cu_q, ctx.state_slots, ctx.n_seqs, H, D, E, "mlstm",
-                        r_scale=scale, den_eps=float(self.spec.den_eps))
+                        r_scale=scale, den_eps=float(self.spec.den_eps), scratch=scratch)
         y = ws.buffer("mlstm_y", T, H * E, self.dtype)
         ops.gated_rmsnorm(y.view(T * H, E), o.view(T * H, E), packed[:, self.g_off:self.i_off], self.out_gain, float(self.spec.eps),
                           heads=H, gains_per_head=True)

@@ -13,7 +13,7 @@ from .spec import LinearAttentionSpec, WeightDecl
 class LinearAttention(Mixer):
     """One packed projection [q | k | v | gate] -> the decayed outer-product recurrence over each sequence's new tokens,
     reading and writing the request's float32 state [heads, key_dim, value_dim] (csrc/linear_attention.cu: prompts in
-    chunks, a decoded token as a chunk of one, the tokens of a long step in segments that run side by side) -> RMSNorm over the heads side by side times sigmoid(gate), one kernel
+    chunks that run side by side, a decoded token as a chunk of one) -> RMSNorm over the heads side by side times sigmoid(gate), one kernel
     -> output projection.  q, k and v leave the product in the storage dtype; their activation, the recurrence, the
     norm and the gate are float32.
 
@@ -67,7 +67,8 @@ class LinearAttention(Mixer):
     def workspace_bytes(self, tokens: int) -> int:
         elem = 2 if self.dtype == torch.bfloat16 else 4
         wide = self.heads * self.vd
-        return tokens * (self.w_in.shape[0] * elem + wide * (4 + elem) + self.spec.hidden_size * elem) + ops.SLICED_PRODUCT_BYTES
+        chunks = 4 * ops.linear_attention_scratch_floats(tokens, max(1, tokens // 32), self.heads, self.kd, self.vd)
+        return chunks + tokens * (self.w_in.shape[0] * elem + wide * (4 + elem) + self.spec.hidden_size * elem) + ops.SLICED_PRODUCT_BYTES
 
     def forward(self, ctx, x, cache: LayerCache):
         T = ctx.n_tokens
