@@ -42,6 +42,42 @@ __global__ void embed_rows_kernel(float* __restrict__ out, const T* __restrict__
     for (int i = threadIdx.x; i < H; i += blockDim.x) dst[i] = ok ? to_float(row[i]) * scale : 0.f;
 }
 
+// The same over whole 16-byte vectors of the table (2,048 rows of 2,048 bfloat16: 12.8 -> 8.3 us).
+template <typename T>
+__global__ void embed_rows_vec_kernel(float* __restrict__ out, const T* __restrict__ table, const int* __restrict__ ids, const int* __restrict__ ids_from,
+                                      const int* __restrict__ sampled, int H, int V, int* bad, float scale, const T* __restrict__ pos_table,
+                                      const int* __restrict__ positions, int n_pos) {
+    constexpr int N = Vec16<T>::N;
+    const int t = blockIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int from = ids_from ? ids_from[t] : -1;
+    const int id = from >= 0 ? sampled[from] : ids[t];
+    const bool ok = id >= 0 && id < V;
+    if (!ok && threadIdx.x == 0 && bad) atomicAdd(bad, 1);
+    const int p = pos_table ? positions[t] : -1;
+    const bool in = p >= 0 && p < n_pos;
+    const T* row = table + (size_t)(ok ? id : 0) * H;
+    const T* prow = in ? pos_table + (size_t)p * H : nullptr;
+    float* dst = out + (size_t)t * H;
+    for (int i = threadIdx.x * N; i < H; i += blockDim.x * N) {
+        Vec16<T> x, y;
+        float v[N], q[N];
+        if (ok) {
+            x.raw = *reinterpret_cast<const decltype(x.raw)*>(row + i);
+            x.unpack(v);
+        }
+        if (in) {
+            y.raw = *reinterpret_cast<const decltype(y.raw)*>(prow + i);
+            y.unpack(q);
+        }
+#pragma unroll
+        for (int u = 0; u < N; ++u) v[u] = (ok ? v[u] * scale : 0.f) + (in ? q[u] : 0.f);
+#pragma unroll
+        for (int u = 0; u < N; u += 4) *reinterpret_cast<float4*>(dst + i + u) = make_float4(v[u], v[u + 1], v[u + 2], v[u + 3]);
+    }
+}
+
 LLMK_EXPORT int llmk_embed_rows(float* out, const void* table, const int* ids, const int* ids_from, const int* sampled,
                                 int n_tokens, int H, int V, int* bad_flag, int dtype, float scale, const void* pos_table,
                                 const int* positions, int n_pos, void* stream) {
@@ -52,6 +88,17 @@ LLMK_EXPORT int llmk_embed_rows(float* out, const void* table, const int* ids, c
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = H >= 1024 ? 256 : 128;
     cudaError_t e;
+    if ((dtype == LLMK_F32 || dtype == LLMK_BF16) && H % (dtype == LLMK_F32 ? 4 : 8) == 0 && host_aligned16(out) && host_aligned16(table) && host_aligned16(pos_table)) {
+        const int vecs = H / (dtype == LLMK_F32 ? 4 : 8), vthreads = vecs >= 256 ? 256 : ceil_div(vecs, 32) * 32;
+        if (dtype == LLMK_F32)
+            e = llmk_launch(embed_rows_vec_kernel<float>, dim3(n_tokens), dim3(vthreads), 0, s, true, out, (const float*)table, ids, ids_from, sampled, H, V, bad_flag,
+                            scale, (const float*)pos_table, positions, n_pos);
+        else
+            e = llmk_launch(embed_rows_vec_kernel<bf16>, dim3(n_tokens), dim3(vthreads), 0, s, true, out, (const bf16*)table, ids, ids_from, sampled, H, V, bad_flag,
+                            scale, (const bf16*)pos_table, positions, n_pos);
+        LLMK_CHECK_LAUNCH_RC("embed_rows", e);
+        return LLMK_OK;
+    }
     if (dtype == LLMK_F32)
         e = llmk_launch(embed_rows_kernel<float>, dim3(n_tokens), dim3(threads), 0, s, true, out, (const float*)table, ids, ids_from, sampled, H, V, bad_flag, scale,
                         (const float*)pos_table, positions, n_pos);

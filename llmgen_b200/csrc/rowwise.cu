@@ -38,6 +38,55 @@ __device__ __forceinline__ float load_sum(const void* y, size_t at, int splits, 
     return acc;
 }
 
+template <typename T, int V>
+__device__ __forceinline__ void load_sum_vec(float (&v)[V], const void* y, size_t at, int splits, long long split_stride) {
+    if constexpr (V == 1) {
+        v[0] = load_sum<T>(y, at, splits, split_stride);
+    } else if (splits == 0) {
+        if constexpr (sizeof(T) == 2) {
+            const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const T*>(y) + at);
+            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+            const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+            v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+        } else {
+            const float4 f = *reinterpret_cast<const float4*>(static_cast<const float*>(y) + at);
+            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+        }
+    } else {
+        const float* p = static_cast<const float*>(y) + at;
+        float4 acc = *reinterpret_cast<const float4*>(p);
+#pragma unroll 4
+        for (int s = 1; s < splits; ++s) {
+            const float4 f = *reinterpret_cast<const float4*>(p + (size_t)s * split_stride);
+            acc.x += f.x; acc.y += f.y; acc.z += f.z; acc.w += f.w;
+        }
+        v[0] = acc.x; v[1] = acc.y; v[2] = acc.z; v[3] = acc.w;
+    }
+}
+
+template <int V>
+__device__ __forceinline__ void load_f32_vec(float (&v)[V], const float* p) {
+    if constexpr (V == 1) {
+        v[0] = p[0];
+    } else {
+        const float4 f = *reinterpret_cast<const float4*>(p);
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+    }
+}
+
+// Four neighbouring values at once.
+template <typename T>
+__device__ __forceinline__ void store_four(T* p, float a, float b, float c, float d) {
+    if constexpr (sizeof(T) == 2) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+        *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    } else {
+        *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+    }
+}
+// Whether four values of `elem` bytes each can be read or written at once from p on.
+static bool four_ok(const void* p, int elem) { return (reinterpret_cast<uintptr_t>(p) & (size_t)(4 * elem - 1)) == 0; }
+
 template <typename T>
 __global__ void norm_add_kernel(float* __restrict__ resid, const void* __restrict__ y, const float* __restrict__ w,
                                 T* __restrict__ copy, int H, float eps, int splits, long long split_stride,
@@ -78,6 +127,54 @@ __global__ void norm_add_kernel(float* __restrict__ resid, const void* __restric
     for (int i = threadIdx.x; i < H; i += blockDim.x) copy[r * H + i] = from_float<T>(srow[i] * rinv2 * w_next[i]);
 }
 
+// The same with four neighbouring values a thread, which holds them from the products' rows to the new row: rows of up to 4,096 values, a
+// multiple of four, on 16-byte boundaries (8 for bfloat16).  2,048 rows of 2,048: 21.9 -> 14.3 us, 50 MB.
+template <typename T>
+__global__ void __launch_bounds__(1024) norm_add_vec_kernel(float* __restrict__ resid, const void* __restrict__ y, const float* __restrict__ w,
+                                                            T* __restrict__ copy, int H, float eps, int splits, long long split_stride,
+                                                            const void* __restrict__ y2, int splits2, long long split_stride2, float a, float b,
+                                                            const float* __restrict__ w_next, float eps_next) {
+    __shared__ float scratch[33];
+    const size_t r = blockIdx.x, at = r * H + 4 * threadIdx.x;
+    const int i = 4 * threadIdx.x;
+    const bool on = i < H;
+    float g[4] = {0.f, 0.f, 0.f, 0.f}, g2[4] = {0.f, 0.f, 0.f, 0.f}, v[4] = {0.f, 0.f, 0.f, 0.f}, x[4] = {0.f, 0.f, 0.f, 0.f};
+    if (on) {
+        load_f32_vec<4>(g, w + i);
+        if (w_next) load_f32_vec<4>(g2, w_next + i);
+    }
+    pdl_launch_dependents();
+    pdl_wait();
+    float ss = 0.f;
+    if (on) {
+        load_f32_vec<4>(x, resid + at);
+        load_sum_vec<T, 4>(v, y, at, splits, split_stride);
+        float u[4] = {0.f, 0.f, 0.f, 0.f};
+        if (y2) load_sum_vec<T, 4>(u, y2, at, splits2, split_stride2);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            v[c] = y2 ? a * v[c] + b * u[c] : a * v[c];
+            ss = fmaf(v[c], v[c], ss);
+        }
+    }
+    ss = block_sum(ss, scratch);
+    const float rinv = 1.0f / sqrtf(ss / (float)H + eps);
+    float ss2 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        x[c] += v[c] * rinv * g[c];
+        ss2 = fmaf(x[c], x[c], ss2);
+    }
+    if (on) *reinterpret_cast<float4*>(resid + at) = make_float4(x[0], x[1], x[2], x[3]);
+    if (!w_next) {
+        if (on && copy) store_four(copy + at, x[0], x[1], x[2], x[3]);
+        return;
+    }
+    ss2 = block_sum(ss2, scratch);
+    const float rinv2 = 1.0f / sqrtf(ss2 / (float)H + eps_next);
+    if (on) store_four(copy + at, x[0] * rinv2 * g2[0], x[1] * rinv2 * g2[1], x[2] * rinv2 * g2[2], x[3] * rinv2 * g2[3]);
+}
+
 // y2 (with its own slices) null: resid += rmsnorm(a y) w.  Else resid += rmsnorm(a y + b y2) w.  w_next non-null: `copy`
 // receives rmsnorm(new row) * w_next (eps_next inside the root) instead of the new row.
 LLMK_EXPORT int llmk_norm_add2(float* resid, const void* y, const float* w, void* copy, int n_rows, int H, float eps,
@@ -91,6 +188,19 @@ LLMK_EXPORT int llmk_norm_add2(float* resid, const void* y, const float* w, void
     const int threads = H >= 2048 ? 512 : H >= 512 ? 256 : 128;
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e;
+    const int elem = dtype == LLMK_F32 ? 4 : 2;
+    if ((dtype == LLMK_F32 || dtype == LLMK_BF16) && H % 4 == 0 && H <= 4096 && four_ok(resid, 4) && four_ok(w, 4) && four_ok(w_next, 4) &&
+        four_ok(copy, elem) && four_ok(y, splits ? 4 : elem) && four_ok(y2, splits2 ? 4 : elem) && split_stride % 4 == 0 && split_stride2 % 4 == 0) {
+        const dim3 block(ceil_div(H / 4, 32) * 32);
+        if (dtype == LLMK_F32)
+            e = llmk_launch(norm_add_vec_kernel<float>, dim3(n_rows), block, 0, s, true, resid, y, w, (float*)copy, H, eps, splits, split_stride,
+                            y2, splits2, split_stride2, a, b, w_next, eps_next);
+        else
+            e = llmk_launch(norm_add_vec_kernel<bf16>, dim3(n_rows), block, 0, s, true, resid, y, w, (bf16*)copy, H, eps, splits, split_stride,
+                            y2, splits2, split_stride2, a, b, w_next, eps_next);
+        LLMK_CHECK_LAUNCH_RC("norm_add", e);
+        return LLMK_OK;
+    }
     if (dtype == LLMK_F32) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(norm_add_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         e = llmk_launch(norm_add_kernel<float>, dim3(n_rows), dim3(threads), smem, s, true, resid, y, w, (float*)copy, H, eps, splits, split_stride,
@@ -130,42 +240,6 @@ struct ParallelAdd {
     int splits1, splits2, top, H;
     float eps;
 };
-
-template <typename T, int V>
-__device__ __forceinline__ void load_sum_vec(float (&v)[V], const void* y, size_t at, int splits, long long split_stride) {
-    if constexpr (V == 1) {
-        v[0] = load_sum<T>(y, at, splits, split_stride);
-    } else if (splits == 0) {
-        if constexpr (sizeof(T) == 2) {
-            const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const T*>(y) + at);
-            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-            const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-            v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
-        } else {
-            const float4 f = *reinterpret_cast<const float4*>(static_cast<const float*>(y) + at);
-            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-        }
-    } else {
-        const float* p = static_cast<const float*>(y) + at;
-        float4 acc = *reinterpret_cast<const float4*>(p);
-#pragma unroll 4
-        for (int s = 1; s < splits; ++s) {
-            const float4 f = *reinterpret_cast<const float4*>(p + (size_t)s * split_stride);
-            acc.x += f.x; acc.y += f.y; acc.z += f.z; acc.w += f.w;
-        }
-        v[0] = acc.x; v[1] = acc.y; v[2] = acc.z; v[3] = acc.w;
-    }
-}
-
-template <int V>
-__device__ __forceinline__ void load_f32_vec(float (&v)[V], const float* p) {
-    if constexpr (V == 1) {
-        v[0] = p[0];
-    } else {
-        const float4 f = *reinterpret_cast<const float4*>(p);
-        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-    }
-}
 
 template <typename T, int V>
 __global__ void __launch_bounds__(512) parallel_add_kernel(ParallelAdd p) {
@@ -329,8 +403,31 @@ __global__ void cast_rows_kernel(T* __restrict__ out, const float* __restrict__ 
         out[i] = from_float<T>(in[i]);
 }
 
+// Eight values at a time.
+template <typename T>
+__global__ void __launch_bounds__(256) cast_rows_vec_kernel(T* __restrict__ out, const float* __restrict__ in, long long vecs) {
+    pdl_launch_dependents();
+    pdl_wait();
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
+        float a[4], b[4];
+        load_f32_vec<4>(a, in + 8 * i);
+        load_f32_vec<4>(b, in + 8 * i + 4);
+        store_four(out + 8 * i, a[0], a[1], a[2], a[3]);
+        store_four(out + 8 * i + 4, b[0], b[1], b[2], b[3]);
+    }
+}
+
 LLMK_EXPORT int llmk_cast_rows(void* out, const float* in, long long n, int dtype, void* stream) {
     if (n <= 0) return LLMK_OK;
+    if ((dtype == LLMK_F32 || dtype == LLMK_BF16) && n % 8 == 0 && host_aligned16(out) && host_aligned16(in)) {
+        long long vblocks = (n / 8 + 255) / 256;
+        if (vblocks > device_sm_count() * 16) vblocks = device_sm_count() * 16;
+        const cudaError_t ev = dtype == LLMK_F32
+            ? llmk_launch(cast_rows_vec_kernel<float>, dim3((unsigned)vblocks), dim3(256), 0, (cudaStream_t)stream, true, (float*)out, in, n / 8)
+            : llmk_launch(cast_rows_vec_kernel<bf16>, dim3((unsigned)vblocks), dim3(256), 0, (cudaStream_t)stream, true, (bf16*)out, in, n / 8);
+        LLMK_CHECK_LAUNCH_RC("cast_rows", ev);
+        return LLMK_OK;
+    }
     long long blocks = (n + 255) / 256;
     if (blocks > device_sm_count() * 16) blocks = device_sm_count() * 16;
     cudaStream_t s = (cudaStream_t)stream;
@@ -389,9 +486,9 @@ __global__ void act_rows_kernel(T* __restrict__ out, const void* __restrict__ x,
     }
 }
 
-// The gated forms over whole 16-byte vectors: a thread takes one vector of gates, the vector of ups beside it, and writes
+// The same over whole 16-byte vectors: a thread takes one vector, or one of gates and the vector of ups beside it, and writes
 // one vector (rows that are no partial sums, column counts and strides in whole vectors).  The arithmetic is the scalar
-// kernel's.
+// kernel's.  relu2 of 2,048 rows of 6,144: 40.1 -> 11.2 us, 50 MB.
 template <typename T>
 __global__ void __launch_bounds__(256) act_rows_vec_kernel(T* __restrict__ out, const T* __restrict__ x, int n, int F, long long ld,
                                                            int mode, float alpha, float limit, int group) {
@@ -403,6 +500,20 @@ __global__ void __launch_bounds__(256) act_rows_vec_kernel(T* __restrict__ out, 
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const size_t r = (size_t)(i / vecs);
         const int f = (int)(i % vecs) * N;
+        if (mode == ACT_RELU2 || mode == ACT_TANH || mode == ACT_GELU_TANH) {
+            Vec16<T> xv, yv;
+            xv.raw = *reinterpret_cast<const decltype(xv.raw)*>(x + r * ld + f);
+            float a[N], b[N];
+            xv.unpack(a);
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const float z = fmaxf(a[k], 0.f);
+                b[k] = mode == ACT_RELU2 ? z * z : mode == ACT_TANH ? tanhf(a[k]) : gelu_tanh(a[k]);
+            }
+            yv.pack(b);
+            *reinterpret_cast<decltype(yv.raw)*>(out + (size_t)r * F + f) = yv.raw;
+            continue;
+        }
         size_t gc, uc;
         if (mode == ACT_CLAMPED_GLU) {
             gc = r * ld + f;
@@ -434,8 +545,7 @@ __global__ void __launch_bounds__(256) act_rows_vec_kernel(T* __restrict__ out, 
 template <typename T>
 static bool act_rows_vec_ok(const void* out, const void* x, int F, long long ld, int mode, int splits, int group) {
     constexpr int N = 16 / (int)sizeof(T);
-    const bool gated = mode == ACT_CLAMPED_GLU || mode == ACT_SILU_GLU || mode == ACT_GELU_TANH_GLU;
-    return gated && splits == 0 && F % N == 0 && group % N == 0 && ld % N == 0 && host_aligned16(out) && host_aligned16(x);
+    return splits == 0 && F % N == 0 && group % N == 0 && ld % N == 0 && host_aligned16(out) && host_aligned16(x);
 }
 
 LLMK_EXPORT int llmk_act_rows(void* out, const void* x, int n, int F, long long ld, int mode, float alpha, float limit,
@@ -537,6 +647,45 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_warp_kernel(T* __restrict__
     }
 }
 
+// The same with four neighbouring values a lane: TEAM threads a row (a warp for rows of up to 128 values, which are heads; else a block), each
+// holding its four from the sum of squares to the row that goes out.  Rows, gains, gates and outputs on boundaries of four values.
+// 2,048 rows of 2,048: 27.4 -> 14.0 us, 34 MB.
+template <typename T, bool WARP>
+__global__ void __launch_bounds__(WARP ? 256 : 1024) gated_rmsnorm_vec_kernel(T* __restrict__ out, const float* __restrict__ o, const T* __restrict__ g,
+                                                                              const float* __restrict__ w, int n_rows, int H, long long ldg, float eps,
+                                                                              int gate_act, int w_rows, int heads, long long ldo) {
+    __shared__ float scratch[33];
+    const size_t r = WARP ? (size_t)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;
+    const int i = 4 * (WARP ? threadIdx.x & 31 : threadIdx.x);
+    const bool on = i < H && r < (size_t)n_rows;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (WARP && r >= (size_t)n_rows) return;
+    const size_t head = r % (size_t)heads, token = r / (size_t)heads;
+    float v[4] = {0.f, 0.f, 0.f, 0.f}, gv[4] = {0.f, 0.f, 0.f, 0.f}, wv[4] = {1.f, 1.f, 1.f, 1.f};
+    if (on) {
+        load_f32_vec<4>(v, o + r * H + i);
+        load_sum_vec<T, 4>(gv, g, token * ldg + head * H + i, 0, 0);
+        if (w) load_f32_vec<4>(wv, w + (head % (size_t)w_rows) * H + i);
+    }
+    float rinv = 1.f;
+    if (w) {
+        float ss = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) ss = fmaf(v[c], v[c], ss);
+        ss = WARP ? warp_sum(ss) : block_sum(ss, scratch);
+        rinv = 1.0f / sqrtf(ss / (float)H + eps);
+    }
+    if (!on) return;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float sg = 1.0f / (1.0f + expf(-gv[c]));
+        const float gate = gate_act == GATE_SIGMOID ? sg : gate_act == GATE_SILU ? gv[c] * sg : gv[c];
+        v[c] = v[c] * rinv * wv[c] * gate;
+    }
+    store_four(out + token * ldo + head * H + i, v[0], v[1], v[2], v[3]);
+}
+
 LLMK_EXPORT int llmk_gated_rmsnorm(void* out, const float* o, const void* g, const float* w, int n_rows, int H, long long ldg,
                                    float eps, int gate_act, int w_rows, int heads, long long ldo, int dtype, void* stream) {
     if (n_rows <= 0 || H <= 0) return LLMK_OK;
@@ -545,6 +694,22 @@ LLMK_EXPORT int llmk_gated_rmsnorm(void* out, const float* o, const void* g, con
     const int threads = H >= 2048 ? 512 : H >= 512 ? 256 : 128;
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e;
+    const int elem = dtype == LLMK_F32 ? 4 : 2;
+    if ((dtype == LLMK_F32 || dtype == LLMK_BF16) && H % 4 == 0 && H <= 4096 && ldg % 4 == 0 && ldo % 4 == 0 && four_ok(o, 4) && four_ok(w, 4) &&
+        four_ok(g, elem) && four_ok(out, elem)) {
+        const bool warp = H <= 128;
+        const dim3 grid((unsigned)(warp ? ceil_div(n_rows, 8) : n_rows)), block(warp ? 256 : ceil_div(H / 4, 32) * 32);
+#define GATED_VEC(TYPE, WARP)                                                                                                                          \
+    e = llmk_launch(gated_rmsnorm_vec_kernel<TYPE, WARP>, grid, block, 0, s, true, (TYPE*)out, o, (const TYPE*)g, w, n_rows, H, ldg, eps, gate_act, w_rows, heads, ldo)
+        if (dtype == LLMK_F32) {
+            if (warp) GATED_VEC(float, true); else GATED_VEC(float, false);
+        } else {
+            if (warp) GATED_VEC(bf16, true); else GATED_VEC(bf16, false);
+        }
+#undef GATED_VEC
+        LLMK_CHECK_LAUNCH_RC("gated_rmsnorm", e);
+        return LLMK_OK;
+    }
     if (H <= 256 && n_rows >= 64 && (dtype == LLMK_F32 || dtype == LLMK_BF16)) {
         const dim3 grid((unsigned)ceil_div(n_rows, 8));
         if (dtype == LLMK_F32)
@@ -865,9 +1030,39 @@ __global__ void stream_spread_kernel(float* __restrict__ streams, float* __restr
     }
 }
 
+// The same four values at a time (2,048 rows of 2,048, four streams: 21.2 -> 12.4 us, 84 MB).
+__global__ void __launch_bounds__(256) stream_spread_vec_kernel(float4* __restrict__ streams, float4* __restrict__ row, long long n, int S, int H4, int collapse) {
+    pdl_launch_dependents();
+    pdl_wait();
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n * H4; i += (long long)gridDim.x * blockDim.x) {
+        const long long r = i / H4;
+        const int c = (int)(i % H4);
+        float4* xs = streams + (size_t)r * S * H4 + c;
+        if (collapse) {
+            float4 acc = xs[0];
+#pragma unroll 4
+            for (int s = 1; s < S; ++s) {
+                const float4 v = xs[(size_t)s * H4];
+                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+            }
+            row[i] = acc;
+        } else {
+            const float4 v = row[i];
+            for (int s = 0; s < S; ++s) xs[(size_t)s * H4] = v;
+        }
+    }
+}
+
 LLMK_EXPORT int llmk_stream_spread(float* streams, float* row, int n_rows, int S, int H, int collapse, void* stream) {
     if (n_rows <= 0) return LLMK_OK;
     if (S <= 0 || H <= 0) LLMK_FAIL("stream_spread: %d streams of %d values", S, H);
+    if (H % 4 == 0 && host_aligned16(streams) && host_aligned16(row)) {
+        long long vblocks = ((long long)n_rows * (H / 4) + 255) / 256;
+        if (vblocks > device_sm_count() * 16) vblocks = device_sm_count() * 16;
+        LLMK_CHECK_LAUNCH_RC("stream_spread", llmk_launch(stream_spread_vec_kernel, dim3((unsigned)vblocks), dim3(256), 0, (cudaStream_t)stream, true,
+                                                          reinterpret_cast<float4*>(streams), reinterpret_cast<float4*>(row), (long long)n_rows, S, H / 4, collapse));
+        return LLMK_OK;
+    }
     long long blocks = ((long long)n_rows * H + 255) / 256;
     if (blocks > device_sm_count() * 16) blocks = device_sm_count() * 16;
     LLMK_CHECK_LAUNCH_RC("stream_spread", llmk_launch(stream_spread_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, true,
