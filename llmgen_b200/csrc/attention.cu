@@ -20,6 +20,10 @@
 // sequence's own keys) and writes un-normalised partial sums
 // and (m, l); `llmk_attention_reduce` merges them as
 // sum_p e^{m_p - M} o_p / sum_p e^{m_p - M} l_p (attention.cu:186-207 in the reference).
+// float32 rows come by `cp.async`, the next tile of keys while this one is used (two tiles of 33 KB at 128 values a row, three blocks an SM).  What
+// bounds it: the reads of keys and values from shared memory for two rows a warp, and with single tokens the latency of one tile, so that a part
+// is as short as a tile.  Four layers' step of one token at 200 keys 272 -> 215 us (36 -> 15 us a layer for this kernel and the merge: parts of 32 keys instead of 128, the
+// parts' loads in the merge side by side); 480 prompt tokens 685 -> 664 us.
 //
 // Variations a model may switch on: values of another width than keys (`vd`); a bound on the scores,
 // s <- softcap * tanh(s / softcap) after the scale; a sink, one more term exp(0) in the softmax's denominator (a key of
@@ -60,20 +64,30 @@ struct AttnParams {
     int gate_heads;            // 1: the gate is one number per head, [tokens, nq]
     long long q_stride, o_stride, gate_stride;
     int max_blocks, nq, nkv, hd, vd, page_size, window, num_parts, part_size, bq, gc, chunks, sink, chunk;
+    int kld, stages;           // floats between two rows of keys in shared memory; tiles of keys on their way at a time
     float scale, softcap;
 };
+
+__device__ __forceinline__ void cp_async16(float* dst, const void* src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 __device__ __forceinline__ float gate_of(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 template <typename T, int HDL>
 __global__ void __launch_bounds__(NWARPS * 32) paged_attention_kernel(AttnParams p) {
-    extern __shared__ float smem[];
-    const int hd = p.hd, vd = p.vd;
+    extern __shared__ __align__(16) float smem[];
+    const int hd = p.hd, vd = p.vd, kld = p.kld;
     float* Qs = smem;                       // [MAX_ROWS][hd], pre-multiplied by scale
-    float* Ks = Qs + MAX_ROWS * hd;         // [KT][hd + 1]
+    float* tiles = Qs + MAX_ROWS * hd;      // [stages] of keys [KT][kld] and values [KT][vd] (or the keys' own rows)
     const bool shared_kv = p.k_scale != nullptr;
-    float* Vs = shared_kv ? Ks : Ks + KT * (hd + 1);         // [KT][vd] (or the keys' own rows)
-    const int vld = shared_kv ? hd + 1 : vd;
+    const int vld = shared_kv ? kld : vd, v_at = shared_kv ? 0 : KT * kld, tile_floats = KT * kld + (shared_kv ? 0 : KT * vd);
+    pdl_launch_dependents();
+    pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int s = p.tile_seq[blockIdx.x];
     if (s < 0) return;                      // padding of a tile list of fixed length
@@ -139,9 +153,35 @@ __global__ void __launch_bounds__(NWARPS * 32) paged_attention_kernel(AttnParams
     constexpr int VN = Vec16<T>::N;
     const int vecs = hd / VN, vvecs = shared_kv ? 0 : vd / VN;
     const bool vec_rows = hd % VN == 0 && vd % VN == 0;      // 16-byte reads of the cache's rows; else value by value
-    for (int t0 = k_beg; t0 < k_end; t0 += KT) {
+    // float32 rows of whole vectors go to shared memory as they are, the next tile's while this one is used
+    const bool async = sizeof(T) == 4 && vec_rows && p.stages == 2;
+    auto send_for = [&](int t0, float* Ks) {
+        for (int idx = threadIdx.x; idx < KT * (vecs + vvecs); idx += blockDim.x) {
+            const int key = idx / (vecs + vvecs), vec = idx % (vecs + vvecs);
+            const bool is_k = vec < vecs;
+            const int kpos = t0 + key;
+            float* dst = is_k ? Ks + key * kld + vec * VN : Ks + v_at + key * vd + (vec - vecs) * VN;
+            if (kpos < k_end) {
+                const size_t row = ((size_t)bt[kpos / p.page_size] * p.nkv + kvh) * p.page_size + kpos % p.page_size;
+                cp_async16(dst, is_k ? kc + row * hd + (size_t)vec * VN : vc + row * vd + (size_t)(vec - vecs) * VN);
+            } else {
+#pragma unroll
+                for (int i = 0; i < VN; ++i) dst[i] = 0.f;
+            }
+        }
+    };
+    if (async && k_beg < k_end) send_for(k_beg, tiles);
+    if (async) cp_async_commit();
+    int turn = 0;
+    for (int t0 = k_beg; t0 < k_end; t0 += KT, turn ^= 1) {
         __syncthreads();  // previous tile consumed (and Qs written, first time)
-        if (vec_rows) {
+        float* Ks = tiles + (async ? turn * tile_floats : 0);
+        float* Vs = Ks + v_at;
+        if (async) {
+            if (t0 + KT < k_end) send_for(t0 + KT, tiles + (turn ^ 1) * tile_floats);
+            cp_async_commit();
+            cp_async_wait<1>();
+        } else if (vec_rows) {
             for (int idx = threadIdx.x; idx < KT * (vecs + vvecs); idx += blockDim.x) {
                 const int key = idx / (vecs + vvecs), vec = idx % (vecs + vvecs);
                 const bool is_k = vec < vecs;
@@ -158,7 +198,7 @@ __global__ void __launch_bounds__(NWARPS * 32) paged_attention_kernel(AttnParams
 #pragma unroll
                     for (int i = 0; i < VN; ++i) f[i] = 0.f;
                 }
-                float* dst = is_k ? Ks + key * (hd + 1) + vec * VN : Vs + key * vd + (vec - vecs) * VN;
+                float* dst = is_k ? Ks + key * kld + vec * VN : Vs + key * vd + (vec - vecs) * VN;
 #pragma unroll
                 for (int i = 0; i < VN; ++i) dst[i] = f[i];
             }
@@ -173,7 +213,7 @@ __global__ void __launch_bounds__(NWARPS * 32) paged_attention_kernel(AttnParams
                     const size_t row = ((size_t)page * p.nkv + kvh) * p.page_size + kpos % p.page_size;
                     f = d < hd ? to_float(kc[row * hd + d]) : to_float(vc[row * vd + (d - hd)]);
                 }
-                if (d < hd) Ks[key * (hd + 1) + d] = f;
+                if (d < hd) Ks[key * kld + d] = f;
                 else Vs[key * vd + (d - hd)] = f;
             }
         }
@@ -185,7 +225,7 @@ __global__ void __launch_bounds__(NWARPS * 32) paged_attention_kernel(AttnParams
         // scores of key `lane` for both rows
         float sc[2] = {0.f, 0.f};
         {
-            const float* kr = Ks + lane * (hd + 1);
+            const float* kr = Ks + lane * kld;
             const float4* qa = reinterpret_cast<const float4*>(Qs + r_of[0] * hd);
             const float4* qb = reinterpret_cast<const float4*>(Qs + (valid[1] ? r_of[1] : r_of[0]) * hd);
             if (hd % 4 != 0) {
@@ -198,11 +238,11 @@ __global__ void __launch_bounds__(NWARPS * 32) paged_attention_kernel(AttnParams
             } else
             for (int d4 = 0; d4 < hd / 4; ++d4) {
                 const float4 a = qa[d4], b = qb[d4];
-                const float k0 = kr[4 * d4], k1 = kr[4 * d4 + 1], k2 = kr[4 * d4 + 2], k3 = kr[4 * d4 + 3];
-                sc[0] = fmaf(a.x, k0, sc[0]); sc[0] = fmaf(a.y, k1, sc[0]);
-                sc[0] = fmaf(a.z, k2, sc[0]); sc[0] = fmaf(a.w, k3, sc[0]);
-                sc[1] = fmaf(b.x, k0, sc[1]); sc[1] = fmaf(b.y, k1, sc[1]);
-                sc[1] = fmaf(b.z, k2, sc[1]); sc[1] = fmaf(b.w, k3, sc[1]);
+                const float4 k = *reinterpret_cast<const float4*>(kr + 4 * d4);      // (kld is a multiple of four here)
+                sc[0] = fmaf(a.x, k.x, sc[0]); sc[0] = fmaf(a.y, k.y, sc[0]);
+                sc[0] = fmaf(a.z, k.z, sc[0]); sc[0] = fmaf(a.w, k.w, sc[0]);
+                sc[1] = fmaf(b.x, k.x, sc[1]); sc[1] = fmaf(b.y, k.y, sc[1]);
+                sc[1] = fmaf(b.z, k.z, sc[1]); sc[1] = fmaf(b.w, k.w, sc[1]);
             }
         }
         if (shared_kv) {
@@ -235,6 +275,7 @@ __global__ void __launch_bounds__(NWARPS * 32) paged_attention_kernel(AttnParams
             for (int j = 0; j < HDL; ++j) acc[i][j] *= corr;
         }
         const int kmax = min(KT, k_end - t0);
+#pragma unroll 4
         for (int k = 0; k < kmax; ++k) {
             const float p0 = __shfl_sync(0xffffffffu, pr[0], k);
             const float p1 = __shfl_sync(0xffffffffu, pr[1], k);
@@ -324,26 +365,40 @@ __global__ void attention_reduce_kernel(T* __restrict__ out, long long o_stride,
                                         const int* __restrict__ positions) {
     const int lane = threadIdx.x & 31;
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    pdl_launch_dependents();
+    pdl_wait();
     if (row >= n_rows) return;
-    const float* ml = part_ml + (size_t)row * num_parts * 2;
+    const float* ml = part_ml + (size_t)row * num_parts * 2;         // (m, l) of every part
     float M = -INFINITY;
-    for (int pt = 0; pt < num_parts; ++pt)
+    for (int pt = lane; pt < num_parts; pt += 32)
         if (ml[2 * pt + 1] > 0.f) M = fmaxf(M, ml[2 * pt]);
+    M = warp_max(M);
     const float z = (sink && sink_values) ? sink_values[row % nq] : 0.f;
     if (sink && M > -INFINITY) M = fmaxf(M, z);
     float denom = 0.f;
-    for (int pt = 0; pt < num_parts; ++pt)
+    for (int pt = lane; pt < num_parts; pt += 32)
         if (ml[2 * pt + 1] > 0.f) denom += expf(ml[2 * pt] - M) * ml[2 * pt + 1];
+    denom = warp_sum(denom);
     if (sink && denom > 0.f) denom += expf(z - M);
     float inv = denom > 0.f ? 1.0f / denom : 0.f;
     const size_t tok = (size_t)(row / nq), head = (size_t)(row % nq);
     T* o = out + tok * o_stride + head * hd;
     const T* g = gate ? gate + tok * gate_stride + head * (gate_heads ? 1 : hd) : nullptr;
     if (g && gate_heads) inv *= gate_of(to_float(g[0]));
+    // column d of all parts (every lane calls it); a lane holds the weight of one part of each 32, the columns' loads do not wait for one another
     auto merged = [&](int d) {
         float v = 0.f;
-        for (int pt = 0; pt < num_parts; ++pt)
-            if (ml[2 * pt + 1] > 0.f) v += expf(ml[2 * pt] - M) * part_o[((size_t)row * num_parts + pt) * hd + d];
+        const float* col = part_o + (size_t)row * num_parts * hd + min(d, hd - 1);
+        for (int p0 = 0; p0 < num_parts; p0 += 32) {
+            const int held = min(32, num_parts - p0);
+            const float w = lane < held && ml[2 * (p0 + lane) + 1] > 0.f ? expf(ml[2 * (p0 + lane)] - M) : 0.f;
+#pragma unroll 8
+            for (int u = 0; u < held; ++u) {
+                const float wu = __shfl_sync(0xffffffffu, w, u);
+                const float x = col[(size_t)(p0 + u) * hd];
+                if (wu > 0.f) v += wu * x;
+            }
+        }
         return v;
     };
     if (turn_cos) {
@@ -357,7 +412,11 @@ __global__ void attention_reduce_kernel(T* __restrict__ out, long long o_stride,
         }
         return;
     }
-    for (int d = lane; d < hd; d += 32) o[d] = from_float<T>(merged(d) * inv * ((g && !gate_heads) ? gate_of(to_float(g[d])) : 1.f));
+    for (int d0 = 0; d0 < hd; d0 += 32) {
+        const int d = d0 + lane;
+        const float v = merged(d);
+        if (d < hd) o[d] = from_float<T>(v * inv * ((g && !gate_heads) ? gate_of(to_float(g[d])) : 1.f));
+    }
 }
 
 static int hdl_of(int hd) { return hd <= 32 ? 1 : hd <= 64 ? 2 : hd <= 128 ? 4 : hd <= 256 ? 8 : 16; }
@@ -369,7 +428,7 @@ static int launch_attention(const AttnParams& p, dim3 grid, size_t smem, cudaStr
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) LLMK_FAIL("paged_attention: cannot raise shared memory to %zu: %s", smem, cudaGetErrorString(e));
     }
-    paged_attention_kernel<T, HDL><<<grid, NWARPS * 32, smem, s>>>(p);
+    LLMK_CHECK_LAUNCH_RC("paged_attention", llmk_launch(paged_attention_kernel<T, HDL>, grid, dim3(NWARPS * 32), smem, s, true, p));
     return LLMK_OK;
 }
 
@@ -433,7 +492,12 @@ LLMK_EXPORT int llmk_paged_attention(void* out, long long o_stride, const void* 
     p.num_parts = num_parts; p.part_size = part_size; p.scale = scale;
     p.part_o = (float*)scratch;
     p.part_ml = num_parts > 1 ? (float*)scratch + (size_t)n_tokens * nq * num_parts * vd : nullptr;
-    const size_t smem = ((size_t)MAX_ROWS * hd + (size_t)KT * (hd + 1) + (k_scale ? 0 : (size_t)KT * vd)) * sizeof(float);
+    // rows of keys: whole vectors and four floats of padding (eight lanes that read 16 bytes of neighbouring rows touch all 32 banks), or an odd
+    // number of floats where the width is no multiple of four
+    p.kld = hd % 4 == 0 ? hd + 4 : hd + 1;
+    const size_t tile = ((size_t)KT * p.kld + (k_scale ? 0 : (size_t)KT * vd)) * sizeof(float), rows_bytes = (size_t)MAX_ROWS * hd * sizeof(float);
+    p.stages = dtype == LLMK_F32 && rows_bytes + 2 * tile <= 110 * 1024 ? 2 : 1;
+    const size_t smem = rows_bytes + (size_t)p.stages * tile;
     dim3 grid(n_tiles, nkv * p.chunks, num_parts);
     cudaStream_t s = (cudaStream_t)stream;
     int rc;
@@ -450,12 +514,13 @@ LLMK_EXPORT int llmk_paged_attention(void* out, long long o_stride, const void* 
         const int warps = 4;
         const int blocks = ceil_div(n_rows, warps);
         if (dtype == LLMK_F32)
-            attention_reduce_kernel<float><<<blocks, warps * 32, 0, s>>>((float*)out, o_stride, p.part_o, p.part_ml, n_rows, nq, vd, num_parts,
-                                                                         p.sink, sink_values, (const float*)gate, gate_stride, p.gate_heads, p.turn_cos, p.turn_sin, positions);
+            LLMK_CHECK_LAUNCH_RC("attention_reduce", llmk_launch(attention_reduce_kernel<float>, dim3(blocks), dim3(warps * 32), 0, s, true, (float*)out, o_stride, p.part_o,
+                                                                 p.part_ml, n_rows, nq, vd, num_parts, p.sink, sink_values, (const float*)gate, gate_stride, p.gate_heads,
+                                                                 p.turn_cos, p.turn_sin, positions));
         else
-            attention_reduce_kernel<bf16><<<blocks, warps * 32, 0, s>>>((bf16*)out, o_stride, p.part_o, p.part_ml, n_rows, nq, vd, num_parts,
-                                                                        p.sink, sink_values, (const bf16*)gate, gate_stride, p.gate_heads, p.turn_cos, p.turn_sin, positions);
-        LLMK_CHECK_LAUNCH("attention_reduce");
+            LLMK_CHECK_LAUNCH_RC("attention_reduce", llmk_launch(attention_reduce_kernel<bf16>, dim3(blocks), dim3(warps * 32), 0, s, true, (bf16*)out, o_stride, p.part_o,
+                                                                 p.part_ml, n_rows, nq, vd, num_parts, p.sink, sink_values, (const bf16*)gate, gate_stride, p.gate_heads,
+                                                                 p.turn_cos, p.turn_sin, positions));
     }
     return LLMK_OK;
 }

@@ -271,7 +271,7 @@ class GQAAttention(Mixer):
         if self.window or self.chunk:
             longest = min(longest, self.window or self.chunk)
         by_sms = (2 * self.sm_count + blocks - 1) // blocks
-        by_len = max(1, longest // 128)
+        by_len = max(1, longest // 32)      # a part is at least one of the kernel's tiles of 32 keys
         # under a window (as under a mask in blocks) the kernel cuts the keys a query can see, not the whole context
         return max(1, min(by_sms, by_len, 64)), 0
 
