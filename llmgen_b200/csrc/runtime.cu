@@ -685,3 +685,54 @@ LLMR_EXPORT int llmr_fill_decode(void* c, int* host, const int* offs, int n, int
     }
     return 0;
 }
+
+// The arrays of any other step, entry by entry: sequence s < n brings q_lens[s] tokens from position starts[s] on.  Sequences n .. n_seqs - 1
+// are padding: one token each that is written nowhere (single != 0), or none.  Rows beyond the sequences' own belong to none.  pos, seq_of and
+// every slots[g] hold n_tokens values, cu_q n_seqs + 1, ctx and state_slots n_seqs, every tables[g] n_seqs * max_blocks.  Returns 1 for a request
+// that was not admitted or has no table for its positions.
+LLMR_EXPORT int llmr_fill_entries(void* c, int n, int n_seqs, int n_tokens, int single, int max_blocks, const long long* reqs, const int* q_lens,
+                                  const int* starts, int* pos, int* seq_of, int* cu_q, int* ctx, int* state_slots, int** slots, int** tables) {
+    Cache* cache = static_cast<Cache*>(c);
+    const int ps = cache->page_size, n_groups = (int)cache->groups.size();
+    int t = 0;
+    cu_q[0] = 0;
+    for (int s = 0; s < n_seqs; ++s) {
+        const int len = s < n ? q_lens[s] : single ? 1 : 0, start = s < n ? starts[s] : 0;
+        if (t + len > n_tokens) {
+            snprintf(g_error, sizeof(g_error), "%d tokens do not fit a step of %d rows", t + len, n_tokens);
+            return 1;
+        }
+        for (int i = 0; i < len; ++i) {
+            pos[t + i] = start + i;
+            seq_of[t + i] = s;
+        }
+        ctx[s] = s < n ? start + len : 0;
+        state_slots[s] = s < n ? cache->slots.slot(reqs[s]) : -1;
+        if (s < n && state_slots[s] < 0) {
+            snprintf(g_error, sizeof(g_error), "request %lld was not admitted", reqs[s]);
+            return 1;
+        }
+        for (int g = 0; g < n_groups; ++g) {
+            int* row = tables[g] + (size_t)s * max_blocks;
+            int held = 0;
+            if (s < n) {
+                const std::vector<int>* table = cache->groups[g]->table(reqs[s]);
+                held = table ? std::min((int)table->size(), max_blocks) : 0;
+                if ((start + len + ps - 1) / ps > held) {
+                    snprintf(g_error, sizeof(g_error), "request %lld: no pages reserved for positions up to %d", reqs[s], start + len - 1);
+                    return 1;
+                }
+                memcpy(row, table->data(), held * sizeof(int));
+            }
+            if (held < max_blocks) memset(row + held, 0, (max_blocks - held) * sizeof(int));
+            for (int i = 0; i < len; ++i) slots[g][t + i] = s < n ? row[(start + i) / ps] * ps + (start + i) % ps : -1;
+        }
+        t += len;
+        cu_q[s + 1] = t;
+    }
+    for (; t < n_tokens; ++t) {
+        pos[t] = seq_of[t] = 0;
+        for (int g = 0; g < n_groups; ++g) slots[g][t] = -1;
+    }
+    return 0;
+}

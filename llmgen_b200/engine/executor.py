@@ -157,6 +157,7 @@ class Executor:
         self.meta_host = [torch.empty(words, dtype=torch.int32).pin_memory() for _ in range(2)]
         self.meta_events = [None, None]
         self.meta_dev = torch.zeros(words, dtype=torch.int32, device=self.device)
+        self._meta_views: Dict[Tuple[int, int, bool], torch.Tensor] = {}
         self._meta_turn = 0
         self.sample_scratch = ops.sample_scratch(max(Sm, 64), self.device)
         self.ids_host = torch.empty(max(Tm, Sm), dtype=torch.int32).pin_memory()
@@ -379,44 +380,55 @@ class Executor:
         shape: token rows beyond the step's own belong to no sequence and are written nowhere, and the sequences
         beyond its own have no tokens."""
         lim = self.limits
-        ps = lim.page_size
         S_real = len(entries)
         S = max(S_real, pad_to, shape[1] if shape else 0)
-        q_lens = [len(e.tokens) for e in entries] + [0 if shape else 1] * (S - S_real)
+        real_lens = [len(e.tokens) for e in entries]
+        q_lens = real_lens + [0 if shape else 1] * (S - S_real)
         starts = [e.start for e in entries] + [0] * (S - S_real)
         T = max(sum(q_lens), shape[0] if shape else 0)
         pure_decode = all(n == 1 for n in q_lens) and not shape
         b = StepMetaBuilder(q_lens, starts, pure_decode, lim.page_size, token_bound=shape[0] if shape else 0)
+        reqs = [self.cache.key(e.req) for e in entries]
+        n_groups, width = len(self.cache.groups), self.max_blocks
+        # everything that follows from the entries' places alone is filled natively, into slices of one array
+        sizes = [T, T, S + 1, S, S] + [T] * n_groups + [S * width] * n_groups
+        block = np.empty(sum(sizes), dtype=np.int32)
+        arrays, at, pointers = [], 0, []
+        base = block.ctypes.data
+        for size in sizes:
+            arrays.append(block[at:at + size])
+            pointers.append(base + 4 * at)
+            at += size
+        pos, seq_of, cu_q, ctx_len, state_slots = arrays[:5]
+        LL, I, P = ctypes.c_longlong * S_real, ctypes.c_int * S_real, ctypes.c_void_p * n_groups
+        rc = self._runtime.llmr_fill_entries(
+            self.cache.native_handle, ctypes.c_int(S_real), ctypes.c_int(S), ctypes.c_int(T), ctypes.c_int(0 if shape else 1), ctypes.c_int(width),
+            LL(*reqs), I(*real_lens), I(*starts[:S_real]), *(ctypes.c_void_p(x) for x in pointers[:5]),
+            P(*pointers[5:5 + n_groups]), P(*pointers[5 + n_groups:]))
+        if rc != 0:
+            raise StepError(self._runtime.llmr_last_error().decode("utf-8", "replace"))
         ids = np.zeros(T, dtype=np.int32)
-        pos = np.zeros(T, dtype=np.int32)
-        seq_of = np.zeros(T, dtype=np.int32)
-        cu_q = np.zeros(S + 1, dtype=np.int32)
-        ctx_len = np.zeros(S, dtype=np.int32)
-        state_slots = np.full(S, -1, dtype=np.int32)
-        want_rows, temps, keys = [], [], []
+        want_rows, want_pos, temps, want_reqs = [], [], [], []
         t = 0
-        for s, e in enumerate(entries):
-            n = q_lens[s]
-            ids[t:t + n] = np.asarray([0 if tok is None else tok for tok in e.tokens] if n == 1 else e.tokens, dtype=np.int32)
-            pos[t:t + n] = np.arange(e.start, e.start + n, dtype=np.int32)
-            seq_of[t:t + n] = s
-            ctx_len[s] = e.start + n
-            state_slots[s] = self.cache.state.slot(e.req)
-            want_rows += [t + w for w in e.want]
-            temps += [e.temperature] * len(e.want)
-            keys += [self.row_key(e.req, e.start + w) for w in e.want]
+        for e, n, req in zip(entries, real_lens, reqs):
+            if n == 1:
+                tok = e.tokens[0]
+                ids[t] = 0 if tok is None else tok
+            else:
+                ids[t:t + n] = e.tokens
+            want = e.want
+            want_rows += [t + w for w in want]
+            want_pos += [e.start + w for w in want]
+            temps += [e.temperature] * len(want)
+            want_reqs += [req] * len(want)
             t += n
-            cu_q[s + 1] = t
-        for s in range(S_real, S):          # padding rows: one token, no keys, written nowhere
-            if shape:
-                cu_q[s + 1] = t
-                continue
-            seq_of[t] = s
-            t += 1
-            cu_q[s + 1] = t
-            want_rows.append(t - 1)
-            temps.append(0.0)
-            keys.append(0)
+        # `row_key` of every wanted row (64-bit arithmetic that wraps)
+        keys = ((np.uint64(self.seed) + np.uint64(SEED_STRIDE) * (np.asarray(want_pos, dtype=np.uint64) + np.uint64(1)))
+                ^ (np.asarray(want_reqs, dtype=np.int64).view(np.uint64) << np.uint64(40)))
+        if not shape and S > S_real:        # padding rows are wanted too: one token each, no keys, written nowhere
+            want_rows += range(t, t + S - S_real)
+            temps += [0.0] * (S - S_real)
+            keys = np.concatenate([keys, np.zeros(S - S_real, dtype=np.uint64)])
         b.add("ids", ids)
         if pad_to > 0:
             src = np.full(T, -1, dtype=np.int32)
@@ -428,27 +440,16 @@ class Executor:
         b.add("cu_q", cu_q)
         b.add("ctx_len", ctx_len)
         b.add("state_slots", state_slots)
-        for gi, g in enumerate(self.cache.groups):
-            slots = np.full(T, -1, dtype=np.int32)
-            bt = np.zeros((S, self.max_blocks), dtype=np.int32)
-            t = 0
-            for s, e in enumerate(entries):
-                table = g.table(e.req)
-                n = q_lens[s]
-                tab = np.asarray(table, dtype=np.int32)
-                bt[s, :len(table)] = tab
-                p = np.arange(e.start, e.start + n)
-                slots[t:t + n] = tab[p // ps] * ps + p % ps
-                t += n
-            b.add(f"slots_{gi}", slots)
-            b.add(f"block_tables_{gi}", bt)
+        for gi in range(n_groups):
+            b.add(f"slots_{gi}", arrays[5 + gi])
+            b.add(f"block_tables_{gi}", arrays[5 + n_groups + gi])
         for m in self._unique_mixers:
             m.prepare_step(b)
         # what only the sampler and the gather of the wanted rows read comes last: its size is the one thing that a
         # step's shape does not fix, and nothing that a replayed graph reads lies behind it
         b.add("want_rows", np.asarray(want_rows, dtype=np.int32))
         b.add("temps", np.asarray(temps, dtype=np.float32), dtype=np.float32)
-        b.add("row_keys", np.asarray(keys, dtype=np.uint64).view(np.int32))
+        b.add("row_keys", keys.view(np.int32))
 
         turn = self._meta_turn
         self._meta_turn ^= 1
@@ -463,12 +464,7 @@ class Executor:
         ev.record()
         self.meta_events[turn] = ev
 
-        def view(name):
-            off, size, dt = layout[name]
-            v = self.meta_dev[off:off + size]
-            return v.view(torch.float32) if dt == np.float32 else v
-
-        views = {n: view(n) for n in layout}
+        views = {n: self._meta_view(*place) for n, place in layout.items()}
         longest = int(ctx_len.max()) if S else 0
         ctx = StepContext(
             n_tokens=T, n_seqs=S, dtype=self.dtype, device=self.device, workspace=self.workspace,
@@ -485,6 +481,20 @@ class Executor:
                     for gi in range(len(self.cache.groups))],
             extra=views)
         return ctx, views["want_rows"], views["temps"], views["row_keys"], len(want_rows)
+
+    def _meta_view(self, off: int, size: int, dt) -> torch.Tensor:
+        """The step arrays' device block from word `off` on.  Steps ask for the same few places again and again, and finding a view costs
+        less than making one."""
+        key = (off, size, dt == np.float32)
+        v = self._meta_views.get(key)
+        if v is None:
+            v = self.meta_dev[off:off + size]
+            if dt == np.float32:
+                v = v.view(torch.float32)
+            if len(self._meta_views) >= 4096:
+                self._meta_views.clear()
+            self._meta_views[key] = v
+        return v
 
     def row_key(self, req: Hashable, position: int) -> int:
         """The sampler's 64-bit key of the row that samples the token after `position` of `req`:

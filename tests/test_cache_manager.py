@@ -143,3 +143,16 @@ def test_storage_gives_values_their_own_width_where_a_mixer_asks_for_one():
     assert st.bytes_held() == 5 * bytes_per_page(reqs, index, 0, page, torch.float32)
     lc = st.layer_cache(1, writes=True)
     assert lc.k.shape[-1] == 64 and lc.v.shape[-1] == 16 and lc.page_size == page
+
+
+@pytest.mark.parametrize("slots", [[0], [4], [1, 2, 3], [4, 0, 2, 1], [3, 3]])
+def test_fresh_slots_are_zeroed_and_no_others(slots):
+    import torch
+    from llmgen_b200.cache.storage import CacheStorage
+    from llmgen_b200.parts.base import StateRequest
+    storage = CacheStorage({}, {0: StateRequest((2, 3), torch.float32), 1: StateRequest((4,), torch.float32)}, {}, [], 16, 5, torch.float32, "cpu")
+    for t in storage.state.values():
+        t.fill_(7.0)
+    storage.reset_state(slots)
+    for t in storage.state.values():
+        assert all(float(t[s].abs().sum()) == 0.0 if s in slots else bool((t[s] == 7.0).all()) for s in range(5))

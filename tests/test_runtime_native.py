@@ -206,3 +206,52 @@ def test_decode_step_arrays_are_filled_natively_and_rows_rewritten_only_when_a_t
     # a position without a page is refused with a message
     rc, _ = fill([11], [1], [lengths[11] + 2 * page_size], [0.0])
     assert rc == 1 and b"no page" in lib.llmr_last_error()
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_the_arrays_of_a_step_follow_the_tables(seed):
+    """`llmr_fill_entries` against the arrays written out in numpy: portions and single tokens of requests in any order, padding of either kind,
+    token rows beyond the sequences' own, two groups."""
+    rng = random.Random(100 + seed)
+    page, width = rng.choice([4, 8]), 12
+    specs = [(FULL, 0), (WINDOW, 9)] if seed % 2 else [(FULL, 0)]
+    cache = CacheManager([GroupSpec(k, w) for k, w in specs], [80] * len(specs), page, 6)
+    names, spans = ["a", 3, ("b", 1), 11, "c"], {}
+    for r in names:
+        cache.admit(r)
+        start, n = rng.randint(0, 20), rng.choice([1, 1, rng.randint(2, 17)])
+        assert cache.reserve(r, 0, start) and cache.reserve(r, start, start + n)
+        spans[r] = (start, n)
+    order = rng.sample(names, rng.randint(0, 5))
+    single = rng.choice([0, 1])
+    n_seqs = len(order) + rng.randint(0, 3)
+    own = sum(spans[r][1] for r in order)
+    T = own + (n_seqs - len(order)) * single + (0 if single else rng.randint(0, 9))
+    G = len(specs)
+    pos, seq, cu = np.full(T, 77, np.int32), np.full(T, 77, np.int32), np.full(n_seqs + 1, 77, np.int32)
+    ctx, state = np.full(n_seqs, 77, np.int32), np.full(n_seqs, 77, np.int32)
+    slots, tables = np.full((G, T), 77, np.int32), np.full((G, n_seqs, width), 77, np.int32)
+    at = lambda x: ctypes.c_void_p(x.ctypes.data)
+    arr = lambda t, v: (t * max(1, len(v)))(*v)
+    args = lambda T: (cache.native_handle, len(order), n_seqs, T, single, width, arr(ctypes.c_longlong, [cache.key(r) for r in order]),
+                      arr(ctypes.c_int, [spans[r][1] for r in order]), arr(ctypes.c_int, [spans[r][0] for r in order]), at(pos), at(seq), at(cu), at(ctx),
+                      at(state), (ctypes.c_void_p * G)(*[slots[g].ctypes.data for g in range(G)]), (ctypes.c_void_p * G)(*[tables[g].ctypes.data for g in range(G)]))
+    assert runtime().llmr_fill_entries(*args(T)) == 0
+    t = 0
+    for s in range(n_seqs):
+        start, n = spans[order[s]] if s < len(order) else (0, single)
+        assert cu[s] == t and ctx[s] == (start + n if s < len(order) else 0)
+        assert state[s] == (cache.state.slot(order[s]) if s < len(order) else -1)
+        assert pos[t:t + n].tolist() == list(range(start, start + n)) and (seq[t:t + n] == s).all()
+        for g in range(G):
+            table = cache.groups[g].table(order[s]) if s < len(order) else []
+            assert tables[g, s].tolist() == table + [0] * (width - len(table))
+            want = [table[p // page] * page + p % page for p in range(start, start + n)] if s < len(order) else [-1] * n
+            assert slots[g, t:t + n].tolist() == want
+        t += n
+    assert cu[n_seqs] == t and not pos[t:].any() and not seq[t:].any() and (slots[:, t:] == -1).all()
+    if t > 0:
+        assert runtime().llmr_fill_entries(*args(t - 1)) == 1          # more tokens than rows: refused, nothing written beyond them
+    if order:
+        cache.release(order[0])
+        assert runtime().llmr_fill_entries(*args(T)) == 1
