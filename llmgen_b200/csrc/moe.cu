@@ -29,6 +29,86 @@ constexpr int MOE_TT = 16;      // rows per tile
 constexpr int MOE_KC = 256;     // input values per pass through shared memory
 
 // ---------------------------------------------------------------------------------------------- route
+// A warp scores token t's products s [E] (with `gate_out` one more) and picks its experts; `by` [E]: what chooses (s itself where that is the
+// same), gm [groups]: room for the groups' largest.
+__device__ __forceinline__ void score_and_pick(size_t t, float* s, float* by, float* gm, bool apart, int lane, int* __restrict__ slot_expert,
+                                               float* __restrict__ slot_weight, int E, int top, int scoring, int renorm,
+                                               const float* __restrict__ choice_bias, float weight_scale, float sum_eps, int groups, int keep,
+                                               float* __restrict__ gate_out) {
+    if (gate_out && lane == 0) gate_out[t] = 1.0f / (1.0f + expf(-s[E]));
+    if (scoring == 2) {
+        // the logits choose
+    } else if (scoring == 1) {
+        float mx = -INFINITY;
+        for (int e = lane; e < E; e += 32) mx = fmaxf(mx, s[e]);
+        mx = warp_max(mx);
+        float sum = 0.f;
+        for (int e = lane; e < E; e += 32) sum += expf(s[e] - mx);
+        sum = warp_sum(sum);
+        for (int e = lane; e < E; e += 32) s[e] = expf(s[e] - mx) / sum;
+    } else {
+        for (int e = lane; e < E; e += 32) s[e] = 1.0f / (1.0f + expf(-s[e]));
+    }
+    if (apart)
+        for (int e = lane; e < E; e += 32) by[e] = s[e] + (choice_bias ? choice_bias[e] : 0.f);
+    __syncwarp();
+    if (groups > 1) {
+        const int size = E / groups;
+        for (int g = lane; g < groups; g += 32) {
+            float m = by[g * size];
+            for (int e = 1; e < size; ++e) m = fmaxf(m, by[g * size + e]);
+            gm[g] = m;
+        }
+        __syncwarp();
+        for (int g = lane; g < groups; g += 32) {
+            int before = 0;           // groups that come first: larger, or as large with a smaller index
+            for (int o = 0; o < groups; ++o) before += (gm[o] > gm[g] || (gm[o] == gm[g] && o < g)) ? 1 : 0;
+            if (before >= keep)
+                for (int e = 0; e < size; ++e) by[g * size + e] = -INFINITY;
+        }
+        __syncwarp();
+    }
+    float total = 0.f;
+    for (int c = 0; c < top; ++c) {
+        // the largest remaining score; ties and values that compare with nothing (NaN) go to the smallest index
+        float best = -INFINITY;
+        int arg = 0x7fffffff;
+        for (int e = lane; e < E; e += 32) {
+            const float v = by[e];
+            if (v > best) { best = v; arg = e; }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
+            if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
+        }
+        if (arg >= E) { arg = c < E ? c : 0; best = 0.f; }     // nothing comparable was left: a padded row's garbage
+        else if (apart) best = s[arg];                   // the correction chooses, the score weighs
+        total += best;
+        if (lane == 0) {
+            slot_expert[t * top + c] = arg;
+            slot_weight[t * top + c] = best;
+            by[arg] = -INFINITY;
+        }
+        __syncwarp();
+    }
+    if (scoring == 2) {
+        // softmax over the chosen logits; the first chosen is the largest
+        if (lane == 0) {
+            const float mx = slot_weight[t * top];
+            float sum = 0.f;
+            for (int c = 0; c < top; ++c) sum += expf(slot_weight[t * top + c] - mx);
+            for (int c = 0; c < top; ++c) slot_weight[t * top + c] = expf(slot_weight[t * top + c] - mx) / sum * weight_scale;
+        }
+        return;
+    }
+    if (lane == 0 && (renorm || weight_scale != 1.f))
+        for (int c = 0; c < top; ++c) {
+            const float w = slot_weight[t * top + c];
+            slot_weight[t * top + c] = (renorm ? w / (total + sum_eps) : w) * weight_scale;
+        }
+}
+
 // The warps share the experts (a warp per dot product, float32 sums in a fixed order), then a warp scores and picks for a
 // token.  scoring 0: sigmoid, 1: softmax over all experts, 2: the logits themselves choose, and the weights
 // are the softmax over the chosen logits.
@@ -86,82 +166,115 @@ __global__ void __launch_bounds__(TOK > 1 ? 256 : 1024) moe_route_kernel(const T
     }
     __syncthreads();
     for (int i = warp; i < n; i += nwarps) {        // a warp scores and picks for a token
-        const size_t t = t0 + i;
         float* s = sm + TOK * K + i * NE;
-        float* by = apart ? s + TOK * NE : s;
-        if (gate_out && lane == 0) gate_out[t] = 1.0f / (1.0f + expf(-s[E]));
-        if (scoring == 2) {
-            // the logits choose
-        } else if (scoring == 1) {
-            float mx = -INFINITY;
-            for (int e = lane; e < E; e += 32) mx = fmaxf(mx, s[e]);
-            mx = warp_max(mx);
-            float sum = 0.f;
-            for (int e = lane; e < E; e += 32) sum += expf(s[e] - mx);
-            sum = warp_sum(sum);
-            for (int e = lane; e < E; e += 32) s[e] = expf(s[e] - mx) / sum;
-        } else {
-            for (int e = lane; e < E; e += 32) s[e] = 1.0f / (1.0f + expf(-s[e]));
+        score_and_pick(t0 + i, s, apart ? s + TOK * NE : s, sm + TOK * K + 2 * TOK * NE + i * groups, apart, lane, slot_expert, slot_weight, E, top, scoring,
+                       renorm, choice_bias, weight_scale, sum_eps, groups, keep, gate_out);
+    }
+}
+
+// Prompts: sixteen tokens and 32 experts at a time a block, so that a value of the router is read once for sixteen tokens.  Rows and router are staged in
+// shared memory as float32, 256 values of K at a time, the next ones on their way while these are used; the eight warps share each 256 (32 apiece), and
+// a warp's lanes have 4 tokens x 4 experts each, whose vectors lie in different banks.  The warps' sums are added up in their order.  What bounds it: the
+// float32 multiply-adds.  2,048 tokens, 32 experts, width 2,048: 46 us (four tokens a block, every block reading the whole router: 134 MB through L2) ->
+// 24 us; lanes as experts that read their rows of the router from global memory: 36.
+constexpr int RT_TOK = 16, RT_EXP = 32, RT_WARPS = 8, RT_KC = 256, RT_LD = RT_KC + 4;
+template <typename T>
+__global__ void __launch_bounds__(RT_WARPS * 32) moe_route_rows_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ wr,
+                                                                       const float* __restrict__ bias, int* __restrict__ slot_expert,
+                                                                       float* __restrict__ slot_weight, int n_tokens, int K, int E, int top, int scoring,
+                                                                       int renorm, const float* __restrict__ choice_bias, float weight_scale,
+                                                                       float sum_eps, int groups, int keep, float* __restrict__ gate_out) {
+    // [2][RT_TOK + RT_EXP][RT_LD] rows and router, [RT_WARPS][RT_TOK][33] the warps' sums, [RT_TOK][NE] scores, [RT_TOK][NE] what chooses, [RT_TOK][groups]
+    extern __shared__ __align__(16) float sm[];
+    constexpr int STAGE = (RT_TOK + RT_EXP) * RT_LD, VN = Vec16<T>::N, XV = RT_TOK * RT_KC / VN / (RT_WARPS * 32);
+    const int NE = E + (gate_out ? 1 : 0);
+    const bool apart = choice_bias || groups > 1;
+    float* part = sm + 2 * STAGE;
+    float* scores = part + RT_WARPS * RT_TOK * 33;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tg = lane >> 3, eg = lane & 7;
+    const int t0 = blockIdx.x * RT_TOK, n = min(RT_TOK, n_tokens - t0);
+    const int chunks = ceil_div(K, RT_KC);
+    pdl_launch_dependents();
+    pdl_wait();
+    for (int e0 = 0; e0 < NE; e0 += RT_EXP) {
+        Vec16<T> held[XV];
+        auto ask = [&](int c) {
+            const int k0 = c * RT_KC, kc = min(RT_KC, K - k0);
+            float* ws = sm + (c & 1) * STAGE + RT_TOK * RT_LD;
+            for (int idx = tid; idx < RT_EXP * RT_KC / 4; idx += RT_WARPS * 32) {
+                const int e = idx / (RT_KC / 4), k = idx % (RT_KC / 4) * 4;
+                if (k < kc) {
+                    const uint32_t d = (uint32_t)__cvta_generic_to_shared(ws + e * RT_LD + k);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(wr + (size_t)min(e0 + e, NE - 1) * K + k0 + k) : "memory");
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < XV; ++u) {
+                const int idx = tid + u * RT_WARPS * 32, i = idx / (RT_KC / VN), k = idx % (RT_KC / VN) * VN;
+                if (i < n && k < kc) held[u].raw = *reinterpret_cast<const decltype(held[u].raw)*>(h + (size_t)(t0 + i) * ldh + k0 + k);
+            }
+        };
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        ask(0);
+        for (int c = 0; c < chunks; ++c) {
+            const int kc = min(RT_KC, K - c * RT_KC);
+            float* xs = sm + (c & 1) * STAGE;
+            const float* ws = xs + RT_TOK * RT_LD;
+#pragma unroll
+            for (int u = 0; u < XV; ++u) {
+                const int idx = tid + u * RT_WARPS * 32, i = idx / (RT_KC / VN), k = idx % (RT_KC / VN) * VN;
+                float f[VN];
+#pragma unroll
+                for (int q = 0; q < VN; ++q) f[q] = 0.f;
+                if (i < n && k < kc) held[u].unpack(f);
+#pragma unroll
+                for (int q = 0; q < VN; q += 4) *reinterpret_cast<float4*>(xs + i * RT_LD + k + q) = make_float4(f[q], f[q + 1], f[q + 2], f[q + 3]);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();                        // this chunk is there, and the one before is used by every warp
+            if (c + 1 < chunks) ask(c + 1);
+            const int k_end = min(kc, (warp + 1) * (RT_KC / RT_WARPS));
+#pragma unroll 2
+            for (int k = warp * (RT_KC / RT_WARPS); k < k_end; k += 4) {
+                float4 x[4], w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(xs + (tg + 4 * i) * RT_LD + k);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4*>(ws + (eg + 8 * j) * RT_LD + k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        acc[i][j] = fmaf(x[i].x, w[j].x, acc[i][j]);
+                        acc[i][j] = fmaf(x[i].y, w[j].y, acc[i][j]);
+                        acc[i][j] = fmaf(x[i].z, w[j].z, acc[i][j]);
+                        acc[i][j] = fmaf(x[i].w, w[j].w, acc[i][j]);
+                    }
+            }
         }
-        if (apart)
-            for (int e = lane; e < E; e += 32) by[e] = s[e] + (choice_bias ? choice_bias[e] : 0.f);
-        __syncwarp();
-        if (groups > 1) {
-            const int size = E / groups;
-            float* gm = sm + TOK * K + 2 * TOK * NE + i * groups;
-            for (int g = lane; g < groups; g += 32) {
-                float m = by[g * size];
-                for (int e = 1; e < size; ++e) m = fmaxf(m, by[g * size + e]);
-                gm[g] = m;
-            }
-            __syncwarp();
-            for (int g = lane; g < groups; g += 32) {
-                int before = 0;           // groups that come first: larger, or as large with a smaller index
-                for (int o = 0; o < groups; ++o) before += (gm[o] > gm[g] || (gm[o] == gm[g] && o < g)) ? 1 : 0;
-                if (before >= keep)
-                    for (int e = 0; e < size; ++e) by[g * size + e] = -INFINITY;
-            }
-            __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[(warp * RT_TOK + tg + 4 * i) * 33 + eg + 8 * j] = acc[i][j];
+        __syncthreads();
+        for (int idx = tid; idx < RT_TOK * RT_EXP; idx += RT_WARPS * 32) {
+            const int i = idx / RT_EXP, o = e0 + idx % RT_EXP;
+            if (o >= NE) continue;
+            float v = 0.f;
+#pragma unroll
+            for (int u = 0; u < RT_WARPS; ++u) v += part[(u * RT_TOK + i) * 33 + idx % RT_EXP];
+            scores[i * NE + o] = v + (bias && o < E ? bias[o] : 0.f);
         }
-        float total = 0.f;
-        for (int c = 0; c < top; ++c) {
-            // the largest remaining score; ties and values that compare with nothing (NaN) go to the smallest index
-            float best = -INFINITY;
-            int arg = 0x7fffffff;
-            for (int e = lane; e < E; e += 32) {
-                const float v = by[e];
-                if (v > best) { best = v; arg = e; }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
-                if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
-            }
-            if (arg >= E) { arg = c < E ? c : 0; best = 0.f; }     // nothing comparable was left: a padded row's garbage
-            else if (apart) best = s[arg];                   // the correction chooses, the score weighs
-            total += best;
-            if (lane == 0) {
-                slot_expert[t * top + c] = arg;
-                slot_weight[t * top + c] = best;
-                by[arg] = -INFINITY;
-            }
-            __syncwarp();
-        }
-        if (scoring == 2) {
-            // softmax over the chosen logits; the first chosen is the largest
-            if (lane == 0) {
-                const float mx = slot_weight[t * top];
-                float sum = 0.f;
-                for (int c = 0; c < top; ++c) sum += expf(slot_weight[t * top + c] - mx);
-                for (int c = 0; c < top; ++c) slot_weight[t * top + c] = expf(slot_weight[t * top + c] - mx) / sum * weight_scale;
-            }
-            continue;
-        }
-        if (lane == 0 && (renorm || weight_scale != 1.f))
-            for (int c = 0; c < top; ++c) {
-                const float w = slot_weight[t * top + c];
-                slot_weight[t * top + c] = (renorm ? w / (total + sum_eps) : w) * weight_scale;
-            }
+        __syncthreads();                            // (also: the staging and the sums may be written again)
+    }
+    for (int i = warp; i < n; i += RT_WARPS) {
+        float* s = scores + i * NE;
+        score_and_pick(t0 + i, s, apart ? s + RT_TOK * NE : s, scores + 2 * RT_TOK * NE + i * groups, apart, lane, slot_expert, slot_weight, E, top, scoring,
+                       renorm, choice_bias, weight_scale, sum_eps, groups, keep, gate_out);
     }
 }
 
@@ -190,6 +303,24 @@ LLMK_EXPORT int llmk_moe_route(const void* h, long long ldh, const float* wr, co
     const dim3 grid(many ? ceil_div(n_tokens, MANY) : n_tokens);
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e;
+    // prompts: sixteen tokens a block where that still gives most SMs one, rows of whole vectors
+    const size_t rows_smem = ((size_t)2 * (RT_TOK + RT_EXP) * RT_LD + RT_WARPS * RT_TOK * 33 + (size_t)RT_TOK * (2 * outputs + groups)) * sizeof(float);
+    const int vec = dtype == LLMK_F32 ? 4 : 8;
+    if ((dtype == LLMK_F32 || dtype == LLMK_BF16) && n_tokens >= RT_TOK * device_sm_count() / 2 && K % vec == 0 && ldh % vec == 0 && host_aligned16(h) &&
+        host_aligned16(wr) && rows_smem <= 200 * 1024) {
+        const dim3 rgrid(ceil_div(n_tokens, RT_TOK)), rblock(RT_WARPS * 32);
+        if (dtype == LLMK_F32) {
+            cudaFuncSetAttribute(moe_route_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            e = llmk_launch(moe_route_rows_kernel<float>, rgrid, rblock, rows_smem, s, pdl != 0, (const float*)h, ldh, wr, bias, slot_expert, slot_weight, n_tokens, K, E,
+                            top, scoring, renorm, choice_bias, weight_scale, sum_eps, groups, keep, gate_out);
+        } else {
+            cudaFuncSetAttribute(moe_route_rows_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            e = llmk_launch(moe_route_rows_kernel<bf16>, rgrid, rblock, rows_smem, s, pdl != 0, (const bf16*)h, ldh, wr, bias, slot_expert, slot_weight, n_tokens, K, E,
+                            top, scoring, renorm, choice_bias, weight_scale, sum_eps, groups, keep, gate_out);
+        }
+        LLMK_CHECK_LAUNCH_RC("moe_route", e);
+        return LLMK_OK;
+    }
 #define MOE_ROUTE_LAUNCH(TYPE, TOK)                                                                                                      \
     do {                                                                                                                                 \
         if (smem > 48 * 1024) cudaFuncSetAttribute(moe_route_kernel<TYPE, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -215,41 +346,82 @@ LLMK_EXPORT int llmk_moe_route(const void* h, long long ldh, const float* wr, co
 __global__ void moe_plan_kernel(const int* __restrict__ slot_expert, int n_slots, int E, int max_tiles, int tt, int padded,
                                 int* __restrict__ order, int* __restrict__ pos_of_slot, int* __restrict__ tile_expert,
                                 int* __restrict__ tile_start, int* __restrict__ tile_rows) {
-    extern __shared__ int sh[];     // counts [E], offsets [E], cursors [E]
+    extern __shared__ int sh[];     // counts [E], first tiles [E], cursors [E]
     int* count = sh;
-    int* offset = sh + E;
+    int* first = sh + E;
     int* cursor = sh + 2 * E;
     pdl_launch_dependents();
     pdl_wait();
     for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_slots; i += blockDim.x) {
-        const int e = slot_expert[i];
-        if (e >= 0 && e < E) atomicAdd(&count[e], 1);
+    // a thread's first slots wait in registers: they are read once (17 -> 9 us for 8,192 slots of 32 experts, most of it one thread's walk over the tiles)
+    constexpr int HELD = 8;
+    int own[HELD];
+#pragma unroll
+    for (int u = 0; u < HELD; ++u) {
+        const int i = threadIdx.x + u * (int)blockDim.x;
+        own[u] = i < n_slots ? slot_expert[i] : -1;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0, tile = 0;
-        for (int e = 0; e < E; ++e) {
-            offset[e] = at;
-            cursor[e] = at;
-            for (int r = 0; r < count[e] && tile < max_tiles; r += tt, ++tile) {
-                tile_expert[tile] = e;
-                tile_start[tile] = at + r;
-                tile_rows[tile] = min(tt, count[e] - r);
-            }
-            at += padded ? ceil_div(count[e], tt) * tt : count[e];
-        }
-        for (; tile < max_tiles; ++tile) {
-            tile_expert[tile] = -1;
-            tile_start[tile] = 0;
-            tile_rows[tile] = 0;
-        }
+#pragma unroll
+    for (int u = 0; u < HELD; ++u)
+        if (own[u] >= 0 && own[u] < E) atomicAdd(&count[own[u]], 1);
+    for (int i = threadIdx.x + HELD * blockDim.x; i < n_slots; i += blockDim.x) {
+        const int e = slot_expert[i];
+        if (e >= 0 && e < E) atomicAdd(&count[e], 1);
     }
     if (padded)
         for (int i = threadIdx.x; i < max_tiles * tt; i += blockDim.x) order[i] = -1;
     __syncthreads();
-    for (int i = threadIdx.x; i < n_slots; i += blockDim.x) {
+    if (threadIdx.x < 32) {         // where each expert's rows and tiles start: sums over the lanes, 32 experts at a time
+        const int lane = threadIdx.x;
+        int at = 0, tile = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane, c = e < E ? count[e] : 0, tiles = ceil_div(c, tt), rows = padded ? tiles * tt : c;
+            int r = rows, q = tiles;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int pr = __shfl_up_sync(0xffffffffu, r, o), pq = __shfl_up_sync(0xffffffffu, q, o);
+                if (lane >= o) {
+                    r += pr;
+                    q += pq;
+                }
+            }
+            if (e < E) {
+                cursor[e] = at + r - rows;
+                first[e] = tile + q - tiles;
+            }
+            at += __shfl_sync(0xffffffffu, r, 31);
+            tile += __shfl_sync(0xffffffffu, q, 31);
+        }
+    }
+    __syncthreads();
+    const int used = first[E - 1] + ceil_div(count[E - 1], tt);
+    for (int i = threadIdx.x; i < max_tiles; i += blockDim.x) {
+        int e = -1, start = 0, rows = 0;
+        if (i < used) {
+            int lo = 0, hi = E;     // the last expert whose first tile lies at or before this one; experts without rows share it with the next
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (first[mid] <= i) lo = mid; else hi = mid;
+            }
+            e = lo;
+            start = cursor[e] + (i - first[e]) * tt;
+            rows = min(tt, count[e] - (i - first[e]) * tt);
+        }
+        tile_expert[i] = e;
+        tile_start[i] = start;
+        tile_rows[i] = rows;
+    }
+    __syncthreads();                // the cursors move from here on
+#pragma unroll
+    for (int u = 0; u < HELD; ++u) {
+        const int i = threadIdx.x + u * (int)blockDim.x;
+        if (i >= n_slots) break;
+        const int pos = own[u] >= 0 && own[u] < E ? atomicAdd(&cursor[own[u]], 1) : -1;
+        if (pos >= 0) order[pos] = i;
+        pos_of_slot[i] = pos;
+    }
+    for (int i = threadIdx.x + HELD * blockDim.x; i < n_slots; i += blockDim.x) {
         const int e = slot_expert[i];
         if (e >= 0 && e < E) {
             const int pos = atomicAdd(&cursor[e], 1);
@@ -299,11 +471,50 @@ __global__ void moe_gather_kernel(T* __restrict__ xs, const T* __restrict__ h, l
     for (int k = threadIdx.x; k < K; k += blockDim.x) dst[k] = from_float<T>(to_float(src[k]) * w);
 }
 
+// The same with a warp a row and whole 16-byte vectors (12,288 rows of 2,048 bfloat16, 8,192 of them filled: 26.9 -> 9.8 us).
+template <typename T>
+__global__ void __launch_bounds__(256) moe_gather_vec_kernel(T* __restrict__ xs, const T* __restrict__ h, long long ldh, const int* __restrict__ order,
+                                                             const float* __restrict__ slot_weight, int n_rows, int top, int K, int scale_rows) {
+    constexpr int N = Vec16<T>::N;
+    const size_t pos = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (pos >= (size_t)n_rows) return;
+    const int slot = order[pos];
+    if (slot < 0) return;
+    const float w = scale_rows ? slot_weight[slot] : 1.f;
+    const T* src = h + (size_t)(slot / top) * ldh;
+#pragma unroll 4
+    for (int k = lane * N; k < K; k += 32 * N) {
+        Vec16<T> v;
+        v.raw = *reinterpret_cast<const decltype(v.raw)*>(src + k);
+        if (scale_rows) {
+            float f[N];
+            v.unpack(f);
+#pragma unroll
+            for (int u = 0; u < N; ++u) f[u] *= w;
+            v.pack(f);
+        }
+        *reinterpret_cast<decltype(v.raw)*>(xs + pos * K + k) = v.raw;
+    }
+}
+
 LLMK_EXPORT int llmk_moe_gather(void* xs, const void* h, long long ldh, const int* order, const float* slot_weight, int n_rows, int top,
                                 int K, int scale_rows, int dtype, void* stream) {
     if (n_rows <= 0) return LLMK_OK;
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e;
+    const int vec = dtype == LLMK_F32 ? 4 : 8;
+    if ((dtype == LLMK_F32 || dtype == LLMK_BF16) && K % vec == 0 && ldh % vec == 0 && host_aligned16(xs) && host_aligned16(h)) {
+        const dim3 grid(ceil_div(n_rows, 8));
+        if (dtype == LLMK_F32)
+            e = llmk_launch(moe_gather_vec_kernel<float>, grid, dim3(256), 0, s, true, (float*)xs, (const float*)h, ldh, order, slot_weight, n_rows, top, K, scale_rows);
+        else
+            e = llmk_launch(moe_gather_vec_kernel<bf16>, grid, dim3(256), 0, s, true, (bf16*)xs, (const bf16*)h, ldh, order, slot_weight, n_rows, top, K, scale_rows);
+        LLMK_CHECK_LAUNCH_RC("moe_gather", e);
+        return LLMK_OK;
+    }
     if (dtype == LLMK_F32)
         e = llmk_launch(moe_gather_kernel<float>, dim3(n_rows), dim3(128), 0, s, true, (float*)xs, (const float*)h, ldh, order, slot_weight, top, K, scale_rows);
     else if (dtype == LLMK_BF16)
