@@ -25,6 +25,13 @@
 //              chains: with so few warps per SM the latency of a dependent chain is what costs.
 // Statistics (m, l), the accumulator and the final division are float32.
 //
+// TERMS = 3 (`llmk_attention_tc_terms`): softmax weights that stay 32-bit.  A weight enters the second product as three bfloat16
+// terms p = p1 + p2 + p3 (24 bits of mantissa), smallest first, so every product with a bfloat16 value is what float32 arithmetic
+// would give.  P takes three arrays, so shared memory holds one buffer of them and one stage of V; pass 2 of a tile waits for the
+// P V of the tile before.  Rows of V behind a sequence's last key are cleared before they are multiplied by weights of zero, so
+// that what another request left there is nothing to this one.  The epilogue takes a sink (one more term in the denominator)
+// and an output gate.  Measured against `mma.sync` (csrc/attention_mma.cu) in the rule of its launcher.
+//
 // Tiles follow the reference's prefill kernel in spirit (src/backend/cuda/attention/attention.cu:300-466:
 // 64-query tiles, `mma.sync`, K/V through `cp.async`, group sizes 1 and 2 only); semantics follow its
 // CPU attention (src/backend/cpu/attention.zig:64-118): query j of a portion sits at position
@@ -59,19 +66,24 @@ struct Params {
     int max_blocks, nq, nkv, page_size, window, gc, bq, chunks;
     float scale_log2;
     unsigned v_lbo, v_sbo;
+    const float* sink_values;     // TERMS 3: with `sink`, the sink's score per query head [nq] (null: 0)
+    const bf16* gate;             // TERMS 3: rows of nq * HD, or (gate_heads) of nq values; null: none
+    long long gate_stride;
+    int sink, gate_heads;
 };
 
 
-template <int HD>
+template <int HD, int TERMS>
 struct Smem {
+    static constexpr int BUFFERS = TERMS == 1 ? 2 : 1;  // of V and P
     static constexpr int Q_BYTES = BM * HD * 2;
     static constexpr int KV_BYTES = BN * HD * 2;       // one K or V tile
     static constexpr int P_BYTES = BM * BN * 2;
     static constexpr int Q_OFF = 0;
     static constexpr int K_OFF = Q_OFF + Q_BYTES;       // 2 stages
-    static constexpr int V_OFF = K_OFF + 2 * KV_BYTES;  // 2 stages
-    static constexpr int P_OFF = V_OFF + 2 * KV_BYTES;  // 2 buffers
-    static constexpr int XCHG_OFF = P_OFF + 2 * P_BYTES;   // float [2][2][BM]: row maxima (and at the end sums) of the two halves
+    static constexpr int V_OFF = K_OFF + 2 * KV_BYTES;  // BUFFERS stages
+    static constexpr int P_OFF = V_OFF + BUFFERS * KV_BYTES;   // BUFFERS x TERMS
+    static constexpr int XCHG_OFF = P_OFF + BUFFERS * TERMS * P_BYTES;   // float [2][2][BM]: row maxima (and at the end sums) of the two halves
     static constexpr int BAR_OFF = XCHG_OFF + 2 * 2 * BM * 4;
     static constexpr int NUM_BARS = 14;
     // No slack for aligning the base: the kernel has no static shared memory, so the dynamic part
@@ -115,11 +127,12 @@ __device__ __forceinline__ void load_pages(uint32_t dst, const CUtensorMap* map,
     }
 }
 
-template <int HD, int PS>
-__global__ void __launch_bounds__(THREADS)
+// (one block an SM, which shared memory allows no more of anyway: said, the compiler schedules for it, 35.0 -> 34.4 us on a 2,048-token prompt)
+template <int HD, int PS, int TERMS>
+__global__ void __launch_bounds__(THREADS, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const Params p) {
-    using L = Smem<HD>;
+    using L = Smem<HD, TERMS>;
     constexpr int HB = HD / 64;                 // 64-wide blocks of the head
     constexpr uint32_t TMEM_COLS = 512;
     constexpr uint32_t S_COL0 = 0, S_COL1 = BN, O_COL0 = 2 * BN;
@@ -223,8 +236,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             int ids[BN / PS], next_ids[BN / PS];
             page_ids<PS>(next_ids, bt, kt0, last_page);
             for (int j = 0; j < n_tiles; ++j) {
-                const int st = j & 1;
-                const uint32_t round = j >> 1;
+                const int st = j & (L::BUFFERS - 1);
+                const uint32_t round = j / L::BUFFERS;
 #pragma unroll
                 for (int pg = 0; pg < BN / PS; ++pg) ids[pg] = next_ids[pg];
                 if (j + 1 < n_tiles) page_ids<PS>(next_ids, bt, kt0 + (j + 1) * BN, last_page);
@@ -242,10 +255,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const uint64_t q_desc = tc::smem_desc_sw128(tc::smem_u32(smem + L::Q_OFF));
             const uint64_t k_desc[2] = {tc::smem_desc_sw128(tc::smem_u32(smem + L::K_OFF)),
                                         tc::smem_desc_sw128(tc::smem_u32(smem + L::K_OFF + L::KV_BYTES))};
+            constexpr int LAST = L::BUFFERS - 1;
             const uint64_t p_desc[2] = {tc::smem_desc_sw128(tc::smem_u32(smem + L::P_OFF)),
-                                        tc::smem_desc_sw128(tc::smem_u32(smem + L::P_OFF + L::P_BYTES))};
+                                        tc::smem_desc_sw128(tc::smem_u32(smem + L::P_OFF + LAST * L::P_BYTES))};
             const uint64_t v_desc[2] = {tc::smem_desc_sw128_mn(tc::smem_u32(smem + L::V_OFF), p.v_lbo, p.v_sbo),
-                                        tc::smem_desc_sw128_mn(tc::smem_u32(smem + L::V_OFF + L::KV_BYTES), p.v_lbo, p.v_sbo)};
+                                        tc::smem_desc_sw128_mn(tc::smem_u32(smem + L::V_OFF + LAST * L::KV_BYTES), p.v_lbo, p.v_sbo)};
             auto issue_qk = [&](int j) -> bool {
                 const int st = j & 1;
                 if (!tc::mbar_wait(tc::smem_u32(&k_full[st]), (j >> 1) & 1, abort_flag)) return false;
@@ -266,17 +280,20 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const int st = j & 1;
                 ok = tc::mbar_wait(tc::smem_u32(p_full), j & 1, abort_flag) &&
-                     tc::mbar_wait(tc::smem_u32(&v_full[st]), (j >> 1) & 1, abort_flag);
+                     tc::mbar_wait(tc::smem_u32(&v_full[st & LAST]), (j / L::BUFFERS) & 1, abort_flag);
                 if (!ok) break;
                 tc::tc_fence_after_sync();
 #pragma unroll
-                for (int kk = 0; kk < BN / 16; ++kk) {
-                    const uint64_t da = p_desc[st] + (uint64_t)(((kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4);
-                    const uint64_t db = v_desc[st] + (uint64_t)((kk * 16 * 128) >> 4);
-                    tc::mma_bf16_ss(tmem_base + O_COL0, da, db, idesc_o, (j | kk) != 0);   // O adds up in tensor memory over the tiles
+                for (int term = TERMS - 1; term >= 0; --term) {       // smallest terms first
+#pragma unroll
+                    for (int kk = 0; kk < BN / 16; ++kk) {
+                        const uint64_t da = p_desc[st] + (uint64_t)((term * L::P_BYTES + (kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4);
+                        const uint64_t db = v_desc[st] + (uint64_t)((kk * 16 * 128) >> 4);
+                        tc::mma_bf16_ss(tmem_base + O_COL0, da, db, idesc_o, j != 0 || kk != 0 || term != TERMS - 1);   // O adds up in tensor memory over the tiles
+                    }
                 }
                 tc::mma_commit(tc::smem_u32(&o_full[st]));
-                tc::mma_commit(tc::smem_u32(&v_empty[st]));
+                tc::mma_commit(tc::smem_u32(&v_empty[st & LAST]));
                 if (j + 2 < n_tiles) ok = issue_qk(j + 2);
             }
         }
@@ -316,7 +333,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const int st = j & 1;
             const int k0 = kt0 + j * BN + half * SC;      // first key of this thread's columns
             const bool need_mask = (k0 + SC - 1 > qpos) || (k0 <= lo);
-            uint8_t* p_row = p_row0 + st * L::P_BYTES;       // P is double-buffered: P V of the tile before may still read the other
+            uint8_t* p_row = p_row0 + (st & (L::BUFFERS - 1)) * L::P_BYTES;       // P is double-buffered: P V of the tile before may still read the other
             // pass 1: the maximum of this thread's half of the row (four independent chains)
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
             if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&s_full[st]), (j >> 1) & 1, abort_flag));
@@ -351,10 +368,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const bool fix = move && m != -INFINITY && j > 0;      // O and l hold something to rescale
             const float alpha = fix ? fast_exp2((m - m_new) * sl2) : 1.f;
             if (move) m = m_new;
-            if (ok && __any_sync(0xffffffffu, fix)) {
+            bool any_fix = ok && __any_sync(0xffffffffu, fix);
+            if (any_fix || (TERMS > 1 && ok && j > 0)) {       // (one buffer of P: the P V before has to have read it in any case)
                 ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&o_full[(j - 1) & 1]), ((j - 1) >> 1) & 1, abort_flag));
                 tc::tc_fence_after_sync();
-                if (ok) {
+                if (ok && any_fix) {
 #pragma unroll
                     for (int c = 0; c < OC / 32; ++c) {
                         uint32_t o[32];
@@ -388,16 +406,37 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     for (int i = 0; i < 32; ++i) sum4[i & 3] += pv[i];
 #pragma unroll
                     for (int q8 = 0; q8 < 4; ++q8) {
-                        Vec16<bf16> pk;
-                        pk.pack(pv + q8 * 8);
                         const int chunk16 = c * 4 + q8;       // 16-byte chunk inside this half's 64 columns
-                        *reinterpret_cast<uint4*>(p_row + ((chunk16 ^ (r & 7)) << 4)) = pk.raw;
+                        uint8_t* to = p_row + ((chunk16 ^ (r & 7)) << 4);
+#pragma unroll
+                        for (int term = 0; term < TERMS; ++term) {
+                            Vec16<bf16> pk;
+                            pk.pack(pv + q8 * 8);
+                            *reinterpret_cast<uint4*>(to + term * L::P_BYTES) = pk.raw;
+                            if (term + 1 < TERMS) {            // what is left of them (exact)
+                                float head8[8];
+                                pk.unpack(head8);
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) pv[q8 * 8 + e] -= head8[e];
+                            }
+                        }
+                    }
+                }
+                if (TERMS > 1 && j == n_tiles - 1) {
+                    const int seen = first_pos + nq_tile - (kt0 + j * BN);      // keys of this tile that a row of it sees
+                    if (seen < BN) {
+                        ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&v_full[st & (L::BUFFERS - 1)]), (j / L::BUFFERS) & 1, abort_flag));
+                        uint8_t* vt = smem + L::V_OFF + (st & (L::BUFFERS - 1)) * L::KV_BYTES;
+                        for (int idx = threadIdx.x - 64; ok && idx < (BN - seen) * HB * 8; idx += 256) {
+                            const int key = seen + idx / (HB * 8), at = idx % (HB * 8);
+                            *reinterpret_cast<uint4*>(vt + (at / 8) * (BN * 128) + key * 128 + (at % 8) * 16) = make_uint4(0, 0, 0, 0);
+                        }
                     }
                 }
                 l = l * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
                 tc::fence_proxy_async();
                 tc::tc_fence_before_sync();
-                tc::mbar_arrive(tc::smem_u32(p_full));
+                if (TERMS == 1 || ok) tc::mbar_arrive(tc::smem_u32(p_full));
             }
         }
         if (ok && n_tiles > 0) {
@@ -411,7 +450,25 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         asm volatile("bar.sync %0, 64;" ::"r"(pair_barrier_end) : "memory");
         const float l_row = l + xchg[(half ^ 1) * BM + r];
         const bool writes = ok && qi < max(nq_tile, 0) && (chunk * p.gc + r % p.gc) < G;
-        const float inv = (row_valid && l_row > 0.f) ? 1.0f / l_row : 0.f;
+        float inv = (row_valid && l_row > 0.f) ? 1.0f / l_row : 0.f;
+        const bf16* gate = nullptr;
+        if constexpr (TERMS > 1) {
+            if (p.sink && inv > 0.f) {
+                const float z = p.sink_values ? p.sink_values[head] : 0.f;
+                const float mr = m * sl2 * 0.6931471805599453f;          // as a power of e
+                const float top = fmaxf(mr, z), w = expf(mr - top);
+                inv = w / (l_row * w + expf(z - top));
+            }
+            if (p.gate && writes) {
+                gate = p.gate + (size_t)(q_beg + q0 + qi) * p.gate_stride;
+                if (p.gate_heads) {
+                    inv *= 1.0f / (1.0f + expf(-__bfloat162float(gate[head])));
+                    gate = nullptr;
+                } else {
+                    gate += (size_t)head * HD + half * OC;
+                }
+            }
+        }
         bf16* o = p.out + (size_t)(q_beg + q0 + qi) * p.o_stride + (size_t)head * HD + half * OC;
 #pragma unroll
         for (int c = 0; c < OC / 32; ++c) {
@@ -428,6 +485,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     float f[8];
 #pragma unroll
                     for (int e = 0; e < 8; ++e) f[e] = inv > 0.f ? __uint_as_float(acc[i + e]) * inv : 0.f;
+                    if (TERMS > 1 && gate) {
+                        float gv[8];
+                        Vec16<bf16> gk;
+                        gk.raw = *reinterpret_cast<const uint4*>(gate + c * 32 + i);
+                        gk.unpack(gv);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) f[e] *= 1.0f / (1.0f + expf(-gv[e]));
+                    }
                     Vec16<bf16> pk;
                     pk.pack(f);
                     *reinterpret_cast<uint4*>(o + c * 32 + i) = pk.raw;
@@ -450,11 +515,11 @@ int group_chunk(int G) {
     return gc;
 }
 
-template <int HD, int PS>
+template <int HD, int PS, int TERMS = 1>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const Params& p, dim3 grid,
            cudaStream_t s) {
-    using L = Smem<HD>;
-    auto kernel = attention_tc_kernel<HD, PS>;
+    using L = Smem<HD, TERMS>;
+    auto kernel = attention_tc_kernel<HD, PS, TERMS>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
@@ -484,8 +549,7 @@ LLMK_EXPORT int llmk_attention_tc(void* out, long long o_stride, const void* q, 
                                   const int* block_tables, int max_blocks, const int* ctx_len, const int* cu_q,
                                   const int* tile_seq, const int* tile_q0, int n_tiles, int nq, int nkv, int hd,
                                   int page_size, int window, float scale, int* error_flag, unsigned v_lbo,
-                                  unsigned v_sbo, void* stream
-) {
+                                  unsigned v_sbo, void* stream) {
     if (n_tiles <= 0 || n_tokens <= 0) return LLMK_OK;
     const int bq = llmk_attention_tc_tile_queries(nq, nkv, hd, page_size);
     if (bq == 0)
@@ -495,7 +559,7 @@ LLMK_EXPORT int llmk_attention_tc(void* out, long long o_stride, const void* q, 
         !host_aligned16(vcache))
         LLMK_FAIL("attention_tc: q, out and the cache must start on 16-byte boundaries with row strides that are multiples of 8");
     if (nkv > 65535) LLMK_FAIL("attention_tc: grid too large");
-    Params p;
+    Params p = {};
     const int G = nq / nkv;
     p.gc = group_chunk(G);
     p.bq = bq;
@@ -531,5 +595,46 @@ LLMK_EXPORT int llmk_attention_tc(void* out, long long o_stride, const void* q, 
         case 32: return hd == 128 ? launch<128, 32>(mq, mk, mv, p, grid, s) : launch<64, 32>(mq, mk, mv, p, grid, s);
         case 64: return hd == 128 ? launch<128, 64>(mq, mk, mv, p, grid, s) : launch<64, 64>(mq, mk, mv, p, grid, s);
         default: return hd == 128 ? launch<128, 128>(mq, mk, mv, p, grid, s) : launch<64, 128>(mq, mk, mv, p, grid, s);
+    }
+}
+
+// The form with 32-bit softmax weights (TERMS = 3): 1 where it takes these sizes.  Head width 128 for keys and values, whole pairs of query heads
+// on a key head (64 queries x 2 heads fill a tile, and the caller's tiles are `attention_mma`'s of 64 queries).
+LLMK_EXPORT int llmk_attention_tc_terms_usable(int nq, int nkv, int hd, int vd, int page_size) {
+    if (nkv <= 0 || nq <= 0 || nq % nkv != 0 || (nq / nkv) % 2 != 0 || hd != 128 || vd != 128) return 0;
+    return page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128;
+}
+
+// As `llmk_attention_tc` without a window, tiles of 64 queries; sink, sink_values, gate as in csrc/attention_mma.cu.
+LLMK_EXPORT int llmk_attention_tc_terms(void* out, long long o_stride, const void* q, long long q_stride, int n_tokens, const void* kcache,
+                                        const void* vcache, long long num_pages, const int* block_tables, int max_blocks, const int* ctx_len,
+                                        const int* cu_q, const int* tile_seq, const int* tile_q0, int n_tiles, int nq, int nkv, int hd,
+                                        int page_size, float scale, int sink, const float* sink_values, const void* gate, long long gate_stride,
+                                        int gate_heads, int* error_flag, void* stream) {
+    if (n_tiles <= 0 || n_tokens <= 0) return LLMK_OK;
+    if (!llmk_attention_tc_terms_usable(nq, nkv, hd, hd, page_size)) LLMK_FAIL("attention_tc_terms: not taken (heads %d/%d, width %d, pages of %d)", nq, nkv, hd, page_size);
+    if (q_stride % 8 != 0 || o_stride % 8 != 0 || !host_aligned16(q) || !host_aligned16(out) || !host_aligned16(kcache) || !host_aligned16(vcache) ||
+        (gate && !gate_heads && (gate_stride % 8 != 0 || !host_aligned16(gate))))
+        LLMK_FAIL("attention_tc_terms: rows must start on 16-byte boundaries");
+    if ((long long)nkv * (nq / nkv / 2) > 0x7fffffff || n_tiles > 65535) LLMK_FAIL("attention_tc_terms: grid too large");
+    Params p = {};
+    p.gc = 2; p.bq = BM / 2; p.chunks = nq / nkv / 2;
+    p.out = (bf16*)out; p.o_stride = o_stride; p.block_tables = block_tables; p.ctx_len = ctx_len; p.cu_q = cu_q; p.tile_seq = tile_seq; p.tile_q0 = tile_q0;
+    p.error_flag = error_flag; p.max_blocks = max_blocks; p.nq = nq; p.nkv = nkv; p.page_size = page_size;
+    p.scale_log2 = scale * 1.4426950408889634f;
+    p.v_lbo = (unsigned)(BN * 128); p.v_sbo = 1024u;
+    p.sink = sink ? 1 : 0; p.sink_values = sink_values; p.gate = (const bf16*)gate; p.gate_stride = gate_stride; p.gate_heads = gate_heads ? 1 : 0;
+    CUtensorMap mq, mk, mv;
+    const uint64_t rows = (uint64_t)num_pages * nkv * page_size;
+    if (!tc_host::make_map_bf16_3d(&mq, q, hd, nq, n_tokens, hd, q_stride, p.gc, p.bq) || !tc_host::cached_map_bf16_2d(&mk, kcache, rows, hd, hd, page_size) ||
+        !tc_host::cached_map_bf16_2d(&mv, vcache, rows, hd, hd, page_size))
+        LLMK_FAIL("attention_tc_terms: cuTensorMapEncodeTiled failed");
+    const dim3 grid(nkv * p.chunks, n_tiles);
+    cudaStream_t s = (cudaStream_t)stream;
+    switch (page_size) {
+        case 16: return launch<128, 16, 3>(mq, mk, mv, p, grid, s);
+        case 32: return launch<128, 32, 3>(mq, mk, mv, p, grid, s);
+        case 64: return launch<128, 64, 3>(mq, mk, mv, p, grid, s);
+        default: return launch<128, 128, 3>(mq, mk, mv, p, grid, s);
     }
 }

@@ -625,6 +625,21 @@ def attention_mma(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vcac
     _check_sinks("attention_mma", sink, sink_values, nq)
     _check_k_scale("attention_mma", k_scale, kcache, vcache)
     tcos, tsin = _check_turn("attention_mma", turn_back, ctx_len, vd, gate, gate_per_head, nq)
+    if (q.shape[0] > 128 and window <= 0 and softcap <= 0.0 and chunk <= 0 and tcos is None and k_scale is None and vcache is not None
+            and _row_stride(q) % 8 == 0 and _row_stride(out) % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, out, kcache, vcache))
+            and (gate is None or gate_per_head or (_row_stride(gate) % 8 == 0 and gate.data_ptr() % 16 == 0)) and n_tiles <= 65535):
+        # Plain causal attention (with a sink or a gate at most) goes to the 5th-generation tensor cores where the widths fit.  16 heads on 8, pages
+        # of 16, mma.sync -> tcgen05: a prompt of 2,048 223.8 -> 65.3 us, of 512 41.9 -> 19.8, of 300 29.1 -> 15.5, 1,024 behind 3,000 keys 292.6 -> 117.  A
+        # prompt of up to 128 tokens is one tile of keys, whose set-up costs more than it saves (64: 12.1 -> 13.5): those stay.
+        tc = build.load("attention_tc")
+        if tc.llmk_attention_tc_terms_usable(c_int(nq), c_int(nkv), c_int(hd), c_int(vd), c_int(page_size)):
+            _check(tc, tc.llmk_attention_tc_terms(_ptr(out), c_longlong(_row_stride(out)), _ptr(q), c_longlong(_row_stride(q)), c_int(q.shape[0]),
+                                                  _ptr(kcache), _ptr(vcache), c_longlong(kcache.numel() // (nkv * page_size * hd)), _ptr(block_tables), c_int(max_blocks),
+                                                  _ptr(ctx_len), _ptr(cu_q), _ptr(tile_seq), _ptr(tile_q0), c_int(n_tiles), c_int(nq), c_int(nkv),
+                                                  c_int(hd), c_int(page_size), c_float(scale), c_int(1 if sink else 0), _ptr(sink_values),
+                                                  _ptr(gate), c_longlong(_row_stride(gate) if gate is not None else 0),
+                                                  c_int(1 if gate_per_head else 0), _ptr(tc_error_flag(q.device)), _stream()))
+            return
     _check(lib, lib.llmk_attention_mma(_ptr(out), c_longlong(_row_stride(out)), _ptr(q), c_longlong(_row_stride(q)), _ptr(kcache),
                                        _ptr(vcache), _ptr(block_tables), c_int(max_blocks), _ptr(ctx_len), _ptr(cu_q), _ptr(tile_seq),
                                        _ptr(tile_q0), c_int(n_tiles), c_int(nq), c_int(nkv), c_int(hd), c_int(vd), c_int(page_size),

@@ -100,7 +100,7 @@ class GQAAttention(Mixer):
     @staticmethod
     def kernel_modules(spec):
         if GQAAttention.varied(spec):
-            return ("attn_prep", "attention", "attention_mma", "rowwise") + (("recurrent",) if spec.conv is not None else ()) + GEMM_MODULES
+            return ("attn_prep", "attention", "attention_mma", "attention_tc", "rowwise") + (("recurrent",) if spec.conv is not None else ()) + GEMM_MODULES
         return ("attn_prep", "attention", "attention_decode", "attention_tc") + GEMM_MODULES
 
     @staticmethod
