@@ -617,15 +617,15 @@ def attention_mma(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vcac
                   softcap: float = 0.0, sink: bool = False, gate: Optional[torch.Tensor] = None, chunk: int = 0,
                   sink_values: Optional[torch.Tensor] = None, gate_per_head: bool = False, turn_back: Optional[tuple] = None,
                   k_scale: Optional[torch.Tensor] = None) -> None:
-    """Prompt portions in bfloat16 with 32-bit softmax weights on the tensor cores (csrc/attention_mma.cu): the same
-    result as `paged_attention` with these options, tiles of `attention_mma_tile_queries` queries."""
+    """Prompt portions in bfloat16 with 32-bit softmax weights on the tensor cores (csrc/attention_mma.cu, plain causal ones
+    csrc/attention_tc.cu): the same result as `paged_attention` with these options, tiles of `attention_mma_tile_queries` queries."""
     lib = build.load("attention_mma")
     if q.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or kcache.dtype != torch.bfloat16 or (gate is not None and gate.dtype != torch.bfloat16):
         raise KernelError("attention_mma: bfloat16 only")
     _check_sinks("attention_mma", sink, sink_values, nq)
     _check_k_scale("attention_mma", k_scale, kcache, vcache)
     tcos, tsin = _check_turn("attention_mma", turn_back, ctx_len, vd, gate, gate_per_head, nq)
-    if (q.shape[0] > 128 and window <= 0 and softcap <= 0.0 and chunk <= 0 and tcos is None and k_scale is None and vcache is not None
+    if (q.shape[0] > 128 and nq <= 65535 and window <= 0 and softcap <= 0.0 and chunk <= 0 and tcos is None and k_scale is None and vcache is not None
             and _row_stride(q) % 8 == 0 and _row_stride(out) % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, out, kcache, vcache))
             and (gate is None or gate_per_head or (_row_stride(gate) % 8 == 0 and gate.data_ptr() % 16 == 0)) and n_tiles <= 65535):
         # Plain causal attention (with a sink or a gate at most) goes to the 5th-generation tensor cores where the widths fit.  16 heads on 8, pages

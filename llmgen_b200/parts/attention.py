@@ -58,7 +58,7 @@ class GQAAttention(Mixer):
     by their root mean square after the rotation, and a mask in blocks of positions (its pages are a window group's).  The gate's matrix is packed behind q, k and v,
     the biases of q, k and v are added by the preparation kernel before the per-head norms, and bound, sink and gate
     are applied inside the attention kernels that take the steps of a layer that has any of them: in bfloat16 portions of
-    prompts run on the tensor cores with float32 softmax weights (csrc/attention_mma.cu), single decoded tokens (their
+    prompts run on the tensor cores with float32 softmax weights (csrc/attention_mma.cu; plain causal ones csrc/attention_tc.cu), single decoded tokens (their
     keys in parts), float32 and other sizes on the general kernel (csrc/attention.cu); the output projection's bias is
     added to its result (or to the first of its slices).
 
