@@ -316,6 +316,7 @@ struct ScanParams {
     const int *cu_q, *state_slots;
     int H, D, E;
     float r_scale, den_eps;
+    int* tickets;             // mlstm: [n_seqs, H], zero before and after: how many of a head's blocks are through with its n
 };
 
 // A value's bits in a 32-bit register (a 16-bit load extends into one by itself), and back.
@@ -450,9 +451,18 @@ __global__ void __launch_bounds__(LANES* CT) memory_scan_kernel(ScanParams p) {
         }
     };
     fetch(0);
+    // n is every tile's to read and one block's to write: the last one to count itself in, when its own values have arrived, knows that all
+    // others hold theirs (blocks of a head may be resident one after the other: with 200 sequences on 2 heads the first one's write
+    // reached a later one in nearly every launch).  The answer is needed at the end: counted there, 256 sequences took 419 us instead of 370.
+    int ticket = 0;
+    if (FORM == FORM_MLSTM) {
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) asm volatile("" ::"f"(nv[i]) : "memory");
+    }
     for (int c0 = 0; c0 < n; c0 += TC) {
         const int nt = min(TC, n - c0);
         __syncthreads();
+        if (FORM == FORM_MLSTM && c0 == 0 && ng && tid == 0) ticket = atomicAdd(p.tickets + (size_t)s * H + h, 1);
         put(c0);
         __syncthreads();
         if (c0 + TC < n) fetch(c0 + TC);
@@ -523,7 +533,10 @@ __global__ void __launch_bounds__(LANES* CT) memory_scan_kernel(ScanParams p) {
             if (d < D) Sg[(size_t)d * E + e] = S[i];
         }
     }
-    if (ng && tile == 0 && col == 0) {
+    // (the first warp has the ticket and the column that writes n)
+    if (FORM == FORM_MLSTM && ng && tid < 32 && __shfl_sync(0xffffffffu, ticket, 0) == (int)gridDim.x - 1) {
+        if (tid == 0) p.tickets[(size_t)s * H + h] = 0;
+        if (col != 0) return;
 #pragma unroll
         for (int i = 0; i < DPL; ++i) {
             const int d = l * DPL + i;
@@ -643,17 +656,19 @@ LLMK_EXPORT long long llmk_memory_scan_scratch_floats(int n_tokens, int n_seqs, 
 
 // The memory's walk over each sequence's new tokens (see the top of the file).  form 0: delta, 1: mlstm.  n_tokens: rows of `out`;
 // scratch: llmk_memory_scan_scratch_floats floats, or null (the walk token by token).
+// tickets (mlstm): n_seqs * H ints that are zero, and zero again afterwards.
 LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const void* k, long long ldk, const void* v, long long ldv,
                                  const float* aux, const float* dots, float* state, long long state_ld, const int* cu_q,
                                  const int* state_slots, int n_seqs, int H, int D, int E, int form, float r_scale, float den_eps,
-                                 int n_tokens, float* scratch, int dtype, void* stream) {
+                                 int n_tokens, float* scratch, int* tickets, int dtype, void* stream) {
     if (n_seqs <= 0) return LLMK_OK;
     if (H <= 0 || D <= 0 || E <= 0 || D > 256) LLMK_FAIL("memory_scan: heads %d, key width %d (at most 256), value width %d", H, D, E);
     if (form != FORM_DELTA && form != FORM_MLSTM) LLMK_FAIL("memory_scan: unknown form %d", form);
     if (form == FORM_DELTA && !aux) LLMK_FAIL("memory_scan: the delta form needs its vectors");
+    if (form == FORM_MLSTM && !tickets) LLMK_FAIL("memory_scan: the mlstm form needs its tickets");
     ScanParams p;
     p.out = out; p.r = r; p.k = k; p.v = v; p.ldr = ldr; p.ldk = ldk; p.ldv = ldv; p.aux = aux; p.dots = dots; p.state = state;
-    p.state_ld = state_ld; p.cu_q = cu_q; p.state_slots = state_slots; p.H = H; p.D = D; p.E = E; p.r_scale = r_scale; p.den_eps = den_eps;
+    p.state_ld = state_ld; p.cu_q = cu_q; p.state_slots = state_slots; p.H = H; p.D = D; p.E = E; p.r_scale = r_scale; p.den_eps = den_eps; p.tickets = tickets;
     cudaStream_t st = (cudaStream_t)stream;
     if (scratch && llmk_memory_scan_scratch_floats(n_tokens, n_seqs, H, D, E, form) > 0) {
         chunk_memory::Params c = {};

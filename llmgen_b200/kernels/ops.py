@@ -1178,25 +1178,29 @@ def memory_scan_scratch_floats(n_tokens: int, n_seqs: int, heads: int, dim: int,
 
 def memory_scan(out: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, aux: Optional[torch.Tensor], dots: torch.Tensor,
                 state: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor, n_seqs: int, heads: int, dim: int, vdim: int,
-                form: str, r_scale: float = 1.0, den_eps: float = 0.0, scratch: Optional[torch.Tensor] = None) -> None:
+                form: str, r_scale: float = 1.0, den_eps: float = 0.0, scratch: Optional[torch.Tensor] = None, tickets: Optional[torch.Tensor] = None) -> None:
     """A matrix memory S [dim, vdim] per head walked over each sequence's new tokens (csrc/memory_scan.cu); out float32
     [n, heads vdim].  "delta": S_t = diag(w) S - b (u^T S) + k v^T, o = S_t^T r, with `aux` and `dots` from `delta_rule_prep`.
     "mlstm": S_t = keep S + take k v^T, n_t = keep n + take k, o = S_t^T q / (max(|n_t . q|, exp(-m_t)) + den_eps), q = r r_scale,
     with `dots` from `mlstm_gates`.  state float32 [slots, >= heads dim vdim (+ heads dim for n)].  With `scratch` (float32,
-    `memory_scan_scratch_floats` values) long steps are taken in chunks of tokens that run side by side."""
+    `memory_scan_scratch_floats` values) long steps are taken in chunks of tokens that run side by side.  `tickets` (mlstm: int32, n_seqs * heads values): an array
+    that is zero, and zero again afterwards, for a caller that keeps one; steps that may run at the same time have one each."""
     lib = build.load("memory_scan")
     chunks = memory_scan_scratch_floats(out.shape[0], n_seqs, heads, dim, vdim, form) if scratch is not None else 0
     if chunks and (scratch.dtype != torch.float32 or scratch.numel() < chunks):
         raise KernelError(f"memory_scan: a step of {out.shape[0]} tokens takes {chunks} float32 of scratch")
     need = heads * dim * vdim + (heads * dim if form == "mlstm" else 0)
     if out.dtype != torch.float32 or not out.is_contiguous() or state.dtype != torch.float32 or state.shape[1] < need \
-            or dots.dtype != torch.float32 or r.dtype != k.dtype or r.dtype != v.dtype:
+            or dots.dtype != torch.float32 or r.dtype != k.dtype or r.dtype != v.dtype \
+            or (tickets is not None and (tickets.dtype != torch.int32 or tickets.numel() < n_seqs * heads or not tickets.is_contiguous())):
         raise KernelError("memory_scan: out, dots and state are float32; r, k, v share the storage dtype")
+    if tickets is None and form == "mlstm":
+        tickets = torch.zeros(n_seqs * heads, dtype=torch.int32, device=out.device)
     _check(lib, lib.llmk_memory_scan(_ptr(out), _ptr(r), c_longlong(_row_stride(r)), _ptr(k), c_longlong(_row_stride(k)), _ptr(v),
                                      c_longlong(_row_stride(v)), _ptr(aux), _ptr(dots), _ptr(state), c_longlong(_row_stride(state)),
                                      _ptr(cu_q), _ptr(state_slots), c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim),
                                      c_int(MEMORY_FORMS[form]), c_float(r_scale), c_float(den_eps), c_int(out.shape[0]),
-                                     _ptr(scratch if chunks else None), c_int(dtype_code(r.dtype)), _stream()), 3 if chunks else 1)
+                                     _ptr(scratch if chunks else None), _ptr(tickets), c_int(dtype_code(r.dtype)), _stream()), 3 if chunks else 1)
 
 
 # ------------------------------------------------------------------------------ recurrent mixers

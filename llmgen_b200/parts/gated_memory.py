@@ -121,8 +121,9 @@ class MLSTM(Mixer):
         o = ws.buffer("mlstm_o", T, H * E, torch.float32)
         need = ops.memory_scan_scratch_floats(T, ctx.n_seqs, H, D, E, "mlstm")
         scratch = ws.flat("mlstm_chunks", need, torch.float32) if need else None
+        tickets = ws.flat("mlstm_tickets", max(ctx.n_seqs, ctx.max_seqs_bound) * H, torch.int32, zero=True)
         ops.memory_scan(o, q, k, v, None, gates, cache.state, ctx.cu_q, ctx.state_slots, ctx.n_seqs, H, D, E, "mlstm",
-                        r_scale=scale, den_eps=float(self.spec.den_eps), scratch=scratch)
+                        r_scale=scale, den_eps=float(self.spec.den_eps), scratch=scratch, tickets=tickets)
         y = ws.buffer("mlstm_y", T, H * E, self.dtype)
         ops.gated_rmsnorm(y.view(T * H, E), o.view(T * H, E), packed[:, self.g_off:self.i_off], self.out_gain, float(self.spec.eps),
                           heads=H, gains_per_head=True)
