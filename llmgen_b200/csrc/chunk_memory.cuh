@@ -19,12 +19,17 @@
 // six products, 4 M of them), the rest the conversion of what is staged, and the latency of one block an SM.
 //
 // Measured (us, one sequence, 16 heads of 128 x 128, bfloat16 rows, before -> now), and the error against float64 of the rows:
-//   linear attention   2,048 tokens 352 -> 108 (segments of 256 tokens walked 32 at a time on the CUDA cores), 1.9e-7 -> 0.9e-7;  512: 203 -> 43;  96: 50 -> 38
-//   running maximum    2,048 tokens 798 -> 82 (a walk token by token), 7.4e-7 -> 6.5e-7;  512: 202 -> 34;  96: 41 -> 31
-// Steps of up to 64 tokens keep the walks: one launch, and no state but the request's own to write.
+//   linear attention   2,048 tokens 353 -> 113 (segments of 256 tokens walked 32 at a time on the CUDA cores), 1.9e-7 -> 0.9e-7;  512: 203 -> 44
+//   running maximum    2,048 tokens 1,139 -> 105 with its gates (a walk token by token), 7.4e-7 -> 6.5e-7;  512: 324 -> 42
+// What a sequence brings decides, not what the step brings: sequences of up to few_of(form) tokens keep the walks (one launch, and no state but the
+// request's own to write), in steps of any size, so that a token's sums do not depend on which other requests share its step.  The walk is
+// launched behind the chunks and skips the sequences that they took.  Walk -> chunks
+// (us, constant decay / running maximum): one sequence of 96 tokens 50 -> 37 / 68 -> 39, 8 of 60 tokens - / 124 -> 73, 32 of 64 - / 478 -> 248; a step that counted
+// its rows instead took 417 -> 1,090 / 185 -> 1,051 for a token each of 128 sequences and 729 -> 2,069 / 697 -> 2,015 for 10 tokens each of 200.
 // A value that is no number reaches the outputs of its sequence from the sixteen tokens it lies in on, not only from its own token on.
 #pragma once
 #include "common.cuh"
+#include <algorithm>
 
 namespace chunk_memory {
 
@@ -33,6 +38,7 @@ constexpr int EB = 64;          // value columns at a time
 constexpr int THREADS = 256;
 constexpr int LDE = EB + 8, LDP = C + 8;      // rows of 144 bytes: eight rows' 16 bytes lie in different banks
 enum { CM_CONST = 0, CM_MAX = 1 };
+__host__ __device__ constexpr int few_of(int form) { return form == CM_CONST ? 64 : 48; }       // sequences of more tokens are taken in chunks
 
 struct Params {
     const void *q, *k, *v;      // storage type, rows ldq / ldk / ldv apart, heads side by side
@@ -43,14 +49,27 @@ struct Params {
     const float* decay;         // CM_CONST: [H]
     const float4* gates;        // CM_MAX: [tokens, H] = (i, f, -, m before the token)
     const int *cu_q, *state_slots;
-    float* scratch;             // [chunks][H][D E (+ D)], then the chunks' decays [chunks][H]
-    int H, D, E, n_seqs, chunks, silu;      // chunks: the most that the step can have
+    float* scratch;             // [chunks][H][entries], the chunks' decays [chunks][H]
+    int H, D, E, n_seqs, silu;
+    int chunks, longs;          // the most chunks, and sequences taken in chunks, that the step can have
+    int entries;                // of a head's state: D E, CM_MAX D E + D
     float q_scale, den_eps;
+    __host__ __device__ float* decays() const { return scratch + (size_t)chunks * H * entries; }
 };
 
 inline bool sizes_usable(int D, int E) { return (D == 64 || D == 128) && E % EB == 0; }
+inline int most_longs(int form, int n_tokens, int n_seqs) { return std::min(n_seqs, n_tokens / (few_of(form) + 1)); }
+// What the step's shape says: a sequence's chunks are at most its tokens / C and one more.
+inline void shape(Params& p, int form, int n_tokens) {
+    p.longs = most_longs(form, n_tokens, p.n_seqs);
+    p.chunks = n_tokens / C + p.longs;
+    p.entries = p.D * p.E + (form == CM_MAX ? p.D : 0);
+}
+// (0: no sequence can be long enough)
 inline long long scratch_floats(int form, int n_tokens, int n_seqs, int H, int D, int E) {
-    return (long long)(n_tokens / C + n_seqs) * H * ((long long)D * E + (form == CM_MAX ? D : 0) + 1);
+    if (n_tokens <= few_of(form) || n_seqs <= 0 || !sizes_usable(D, E)) return 0;
+    const long long chunks = n_tokens / C + most_longs(form, n_tokens, n_seqs);
+    return chunks * H * ((long long)D * E + (form == CM_MAX ? D : 0) + 1);
 }
 
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const bf16* p) {
@@ -119,29 +138,49 @@ __device__ __forceinline__ void mma_terms(Sums<N8>& s, int n, const uint32_t (&a
 
 __device__ __forceinline__ float act(float x, int silu) { return silu ? __fdividef(x, 1.0f + __expf(-x)) : x; }
 
-// Which sequence and which of its chunks chunk number `c` of the step is (s = -1: the step has fewer).  All threads of a warp.
+// Which sequence and which of its chunks chunk number `c` of the step is (s = -1: the step has fewer); or, with BY_SEQUENCE, which sequence the
+// c-th of those taken in chunks is.  All threads of a warp.
 struct Place {
     int s, chunk, base;         // base: number of the sequence's first chunk
 };
+template <int FORM, bool BY_SEQUENCE>
 __device__ __forceinline__ Place place_of(const int* __restrict__ cu_q, int n_seqs, int c) {
     const int lane = threadIdx.x & 31;
-    int before = 0;
-    for (int s0 = 0; s0 < n_seqs; s0 += 32) {
-        const int s = s0 + lane;
-        const int n = s < n_seqs ? ceil_div(max(0, cu_q[s + 1] - cu_q[s]), C) : 0;
-        int upto = n;
+    int before = 0, seen = 0;                   // chunks, and sequences with chunks, of the sequences passed
+    for (int s0 = 0; s0 < n_seqs; s0 += 128) {  // four in a row a lane
+        const int s = s0 + 4 * lane;
+        int at[5], n[4], chunks = 0, longs = 0;
+#pragma unroll
+        for (int u = 0; u < 5; ++u) at[u] = cu_q[min(s + u, n_seqs)];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            n[u] = at[u + 1] - at[u] > few_of(FORM) ? ceil_div(at[u + 1] - at[u], C) : 0;
+            chunks += n[u];
+            longs += n[u] > 0 ? 1 : 0;
+        }
+        int upto = chunks, longs_upto = longs;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int x = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += x;
+            const int x = __shfl_up_sync(0xffffffffu, upto, o), y = BY_SEQUENCE ? __shfl_up_sync(0xffffffffu, longs_upto, o) : 0;
+            if (lane >= o) {
+                upto += x;
+                longs_upto += y;
+            }
         }
-        const unsigned holds = __ballot_sync(0xffffffffu, before + upto > c);
+        const unsigned holds = __ballot_sync(0xffffffffu, BY_SEQUENCE ? seen + longs_upto > c : before + upto > c);
         if (holds) {
-            const int at = __ffs(holds) - 1;
-            const int base = before + __shfl_sync(0xffffffffu, upto - n, at);
-            return {s0 + at, c - base, base};
+            const int owner = __ffs(holds) - 1;
+            int base = before + upto - chunks, skip = BY_SEQUENCE ? c - (seen + longs_upto - longs) : 0, u = 0;      // (the owner's are used)
+            for (; u < 3; ++u) {
+                if (BY_SEQUENCE ? n[u] > 0 && skip == 0 : c < base + n[u]) break;
+                if (BY_SEQUENCE && n[u] > 0) --skip;
+                base += n[u];
+            }
+            base = __shfl_sync(0xffffffffu, base, owner);
+            return {s0 + 4 * owner + __shfl_sync(0xffffffffu, u, owner), c - base, base};
         }
         before += __shfl_sync(0xffffffffu, upto, 31);
+        if (BY_SEQUENCE) seen += __shfl_sync(0xffffffffu, longs_upto, 31);
     }
     return {-1, 0, 0};
 }
@@ -258,8 +297,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_local_kernel(Params p
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_launch_dependents();
     pdl_wait();
-    const Place at = place_of(p.cu_q, p.n_seqs, blockIdx.x);
-    if (at.s < 0 || (FORM == CM_CONST && p.state_slots[at.s] < 0)) return;
+    const Place at = place_of<FORM, false>(p.cu_q, p.n_seqs, blockIdx.x);
+    if (at.s < 0) return;
+    if (FORM == CM_CONST && p.state_slots[at.s] < 0) return;
     const int q_beg = p.cu_q[at.s], t0 = q_beg + at.chunk * C, n = min(C, p.cu_q[at.s + 1] - t0);
     Rows<T, NT, D> keys;
     Rows<T, 3, EB> values;
@@ -270,11 +310,8 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_local_kernel(Params p
     keys.put(Ks, n, p.silu, nullptr);
     __syncthreads();
     if (tid < C) wj[tid] = tid < n ? weight<FORM>(w, n - 1, tid) : 0.f;
-    float* dst = p.scratch + ((size_t)blockIdx.x * p.H + h) * ((size_t)D * p.E + (FORM == CM_MAX ? D : 0));
-    if (tid == 0) {
-        float* gains = p.scratch + (size_t)p.chunks * p.H * ((size_t)D * p.E + (FORM == CM_MAX ? D : 0));
-        gains[(size_t)blockIdx.x * p.H + h] = from_start<FORM>(w, n - 1);
-    }
+    float* dst = p.scratch + ((size_t)blockIdx.x * p.H + h) * p.entries;
+    if (tid == 0) p.decays()[(size_t)blockIdx.x * p.H + h] = from_start<FORM>(w, n - 1);
     __syncthreads();
     const int d0 = 16 * (warp % ROW_WARPS), e_warp = (warp / ROW_WARPS) * (N8 * 8);
     for (int e0 = 0; e0 < p.E; e0 += EB) {
@@ -319,42 +356,50 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_local_kernel(Params p
 
 // ----------------------------------------------------------------------------------------------------------------- scan
 // A thread per entry of the state (CM_MAX: of n too): a chunk's sum is replaced by the state before it, eight chunks' values asked for at once.
+// Blocks take (sequence, head, 256 entries) one after the other, those of sequences in chunks only: the most that a shape can have would be
+// 262,144 blocks for 256 sequences of 16 heads of 128 x 128.
 template <int FORM>
 __global__ void __launch_bounds__(THREADS) chunk_memory_scan_kernel(Params p) {
-    const int s = blockIdx.x, h = blockIdx.y, entry = blockIdx.z * THREADS + threadIdx.x;
-    const int entries = p.D * p.E + (FORM == CM_MAX ? p.D : 0);
+    const int per_head = ceil_div(p.entries, THREADS);
     pdl_launch_dependents();
     pdl_wait();
-    const int slot = p.state_slots[s], n_tok = p.cu_q[s + 1] - p.cu_q[s];
-    if (n_tok <= 0 || (slot < 0 && FORM == CM_CONST)) return;
-    int base = 0;
-    for (int i = 0; i < s; ++i) base += ceil_div(max(0, p.cu_q[i + 1] - p.cu_q[i]), C);
-    if (entry >= entries) return;
-    const int count = ceil_div(n_tok, C);
-    float* Sg = nullptr;
-    if (slot >= 0) {
-        const int DE = p.D * p.E;
-        Sg = p.state + (size_t)slot * p.state_ld + (entry < DE ? (size_t)h * DE + entry : (size_t)p.H * DE + (size_t)h * p.D + (entry - DE));
-    }
-    const size_t stride = (size_t)p.H * entries;
-    float* at = p.scratch + ((size_t)base * p.H + h) * entries + entry;
-    const float* gain = p.scratch + (size_t)p.chunks * p.H * entries + (size_t)base * p.H + h;
-    float S = Sg ? *Sg : 0.f;
-    for (int c0 = 0; c0 < count; c0 += 8) {
+    for (int item = blockIdx.x; item < p.longs * p.H * per_head; item += gridDim.x) {
+        const Place seq = place_of<FORM, true>(p.cu_q, p.n_seqs, item / (per_head * p.H));
+        if (seq.s < 0) return;
+        const int s = seq.s, h = item / per_head % p.H, part = item % per_head, entry = part * THREADS + (int)threadIdx.x;
+        const int slot = p.state_slots[s];
+        if (FORM == CM_CONST && slot < 0) continue;
+        const int count = ceil_div(p.cu_q[s + 1] - p.cu_q[s], C);
+        const bool on = entry < p.entries;
+        float* Sg = nullptr;
+        if (slot >= 0 && on) {
+            const int DE = p.D * p.E;
+            Sg = p.state + (size_t)slot * p.state_ld + (entry < DE ? (size_t)h * DE + entry : (size_t)p.H * DE + (size_t)h * p.D + (entry - DE));
+        }
+        const size_t stride = (size_t)p.H * p.entries;
+        float* at = p.scratch + ((size_t)seq.base * p.H + h) * p.entries + entry;
+        const float* gain = p.decays() + (size_t)seq.base * p.H + h;
+        float S = Sg ? *Sg : 0.f;
         float add[8], g[8];
+        auto ask = [&](int c0) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            add[u] = c0 + u < count ? at[(size_t)(c0 + u) * stride] : 0.f;
-            g[u] = c0 + u < count ? gain[(size_t)(c0 + u) * p.H] : 0.f;
-        }
+            for (int u = 0; u < 8; ++u) {
+                add[u] = on && c0 + u < count ? at[(size_t)(c0 + u) * stride] : 0.f;
+                g[u] = c0 + u < count ? gain[(size_t)(c0 + u) * p.H] : 0.f;
+            }
+        };
+        ask(0);
+        for (int c0 = 0; c0 < count; c0 += 8) {
+            if (c0 > 0) ask(c0);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            if (c0 + u >= count) break;
-            at[(size_t)(c0 + u) * stride] = S;
-            S = fmaf(g[u], S, add[u]);
+            for (int u = 0; u < 8; ++u) {
+                if (c0 + u >= count) break;
+                if (on) at[(size_t)(c0 + u) * stride] = S;
+                S = fmaf(g[u], S, add[u]);
+            }
         }
+        if (Sg) *Sg = S;
     }
-    if (Sg) *Sg = S;
 }
 
 // ------------------------------------------------------------------------------------------------------------------ out
@@ -379,10 +424,10 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_launch_dependents();
     pdl_wait();
-    const Place at = place_of(p.cu_q, p.n_seqs, blockIdx.x);
+    const Place at = place_of<FORM, false>(p.cu_q, p.n_seqs, blockIdx.x);
     if (at.s < 0 || (FORM == CM_CONST && p.state_slots[at.s] < 0)) return;
     const int q_beg = p.cu_q[at.s], t0 = q_beg + at.chunk * C, n = min(C, p.cu_q[at.s + 1] - t0);
-    const float* before = p.scratch + ((size_t)blockIdx.x * p.H + h) * ((size_t)D * p.E + (FORM == CM_MAX ? D : 0));
+    const float* before = p.scratch + ((size_t)blockIdx.x * p.H + h) * p.entries;
     // the state's entries of 64 columns, float4 a thread and turn: asked for early, put down where the keys were
     constexpr int SV = D * EB / 4 / THREADS;
     float4 held[SV];
@@ -555,9 +600,10 @@ int launch_width(const Params& p, cudaStream_t s) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
     if (e != cudaSuccess) LLMK_FAIL("chunk_memory: cannot raise shared memory: %s", cudaGetErrorString(e));
     const dim3 grid(p.chunks, p.H);
-    const int entries = p.D * p.E + (FORM == CM_MAX ? p.D : 0);
+    const long long items = (long long)p.longs * p.H * ceil_div(p.entries, THREADS);
+    const dim3 scan((unsigned)std::min<long long>(items, 8 * device_sm_count()));
     LLMK_CHECK_LAUNCH_RC("chunk_memory_local", llmk_launch(k1, grid, dim3(THREADS), local, s, true, p));
-    LLMK_CHECK_LAUNCH_RC("chunk_memory_scan", llmk_launch(chunk_memory_scan_kernel<FORM>, dim3(p.n_seqs, p.H, ceil_div(entries, THREADS)), dim3(THREADS), 0, s, true, p));
+    LLMK_CHECK_LAUNCH_RC("chunk_memory_scan", llmk_launch(chunk_memory_scan_kernel<FORM>, scan, dim3(THREADS), 0, s, true, p));
     LLMK_CHECK_LAUNCH_RC("chunk_memory_out", llmk_launch(k3, grid, dim3(THREADS), out, s, true, p));
     return LLMK_OK;
 }

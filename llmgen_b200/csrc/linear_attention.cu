@@ -22,8 +22,9 @@
 // state), and a third launch adds that state's share, lambda^(i+1) S_before^T q_i, to the segment's outputs.  A
 // prompt's chunks then no longer form one chain of dependent steps on a handful of SMs.
 //
-// Steps of more than 64 tokens with key widths of 64 or 128, value widths in runs of 64 and rows of 16-byte vectors take the
-// chunks of 64 tokens of chunk_memory.cuh instead, whose products run on the tensor cores at 32-bit precision.
+// Sequences of more than 64 tokens with key widths of 64 or 128, value widths in runs of 64 and rows of 16-byte vectors take the
+// chunks of 64 tokens of chunk_memory.cuh instead, whose products run on the tensor cores at 32-bit precision; the walk
+// above, launched behind them without segments, then takes the step's other sequences.
 //
 // A sequence whose state slot is negative or that brings no tokens (the padding of a step laid out for replay) is
 // skipped.
@@ -53,10 +54,10 @@ struct LinAttnParams {
     // empty state; `seg_state` [segments of all sequences][heads][dim][vdim] receives each segment's end state
     int segments, n_seqs;
     float* seg_state;
+    int in_chunks;              // != 0: sequences of more tokens than chunk_memory leaves were taken in chunks
 };
 
 constexpr int LA_SEG = 256;     // tokens per segment (a multiple of the chunk)
-constexpr int LA_CHUNKS_FROM = 64;      // steps of more tokens take the chunks of chunk_memory.cuh where it takes the sizes
 
 // Index of sequence s's first segment among all segments of the step, and how many it has.
 __device__ __forceinline__ int la_segment_base(const int* cu_q, int s, int& count) {
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(LA_WARPS * 32) linear_attention_kernel(LinAttn
     pdl_wait();
     const int slot = p.state_slots[s];
     int t_beg = p.cu_q[s], n_tok = p.cu_q[s + 1] - t_beg;
-    if (slot < 0 || n_tok <= 0) return;
+    if (slot < 0 || n_tok <= 0 || (p.in_chunks && n_tok > chunk_memory::few_of(chunk_memory::CM_CONST))) return;
     float* Sg = p.state + (((size_t)slot * p.heads + h) * D) * E;
     const bool local = p.segments > 1;      // this block runs one segment from an empty state
     if (local) {
@@ -412,47 +413,51 @@ static int dispatch_linear_attention(const LinAttnParams& p, dim3 grid, size_t s
     return launch_linear_attention<T, 32>(p, grid, smem, s);
 }
 
-// q, k, v: pointers to the first row's q, k and v inside the packed projection (rows `ld` elements apart, heads
-// side by side); out float32 [tokens, heads * vdim]; state float32 [slots, heads, dim, vdim]; decay float32 [heads].
-// Floats of scratch that a step of `n_tokens` tokens in `n_seqs` sequences needs for its segments' states (0: the step
-// runs without segments).
+// Floats of scratch that a step of `n_tokens` tokens in `n_seqs` sequences needs for its chunks' or segments' states (0: none).
 LLMK_EXPORT long long llmk_linear_attention_scratch_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim) {
-    long long need = 0;
-    if (n_tokens > LA_SEG) need = (long long)(n_tokens / LA_SEG + n_seqs) * heads * dim * vdim;
-    if (n_tokens > LA_CHUNKS_FROM && chunk_memory::sizes_usable(dim, vdim))
-        need = std::max(need, chunk_memory::scratch_floats(chunk_memory::CM_CONST, n_tokens, n_seqs, heads, dim, vdim));
-    return need;
+    const long long segments = n_tokens > LA_SEG ? (long long)(n_tokens / LA_SEG + n_seqs) * heads * dim * vdim : 0;
+    return std::max(segments, chunk_memory::scratch_floats(chunk_memory::CM_CONST, n_tokens, n_seqs, heads, dim, vdim));
 }
 
-// n_tokens: rows of `out` (all tokens of the step).  With more than LA_SEG of them a sequence's tokens are cut into
-// segments that run side by side (three launches: segments from an empty state, the scan over their end states, the
-// carried state's share of the outputs) and `seg_state` must hold llmk_linear_attention_scratch_floats(...) floats.
+// q, k, v: pointers to the first row's q, k and v inside the packed projection (rows `ld` elements apart, heads
+// side by side); out float32 [tokens, heads * vdim]; state float32 [slots, heads, dim, vdim]; decay float32 [heads].
+// n_tokens: rows of `out` (all tokens of the step).  longest: the most tokens that one of its sequences brings (0: not known).
+// scratch: llmk_linear_attention_scratch_floats floats, or null.  What takes no chunks is walked; with more
+// than LA_SEG tokens in segments that run side by side (three launches: segments from an empty state, the scan over their end states, the
+// carried state's share of the outputs), whose states the scratch must hold.
 LLMK_EXPORT int llmk_linear_attention(float* out, const void* q, const void* k, const void* v, long long ld, float* state,
                                       const float* decay, const int* cu_q, const int* state_slots, int n_seqs, int heads,
-                                      int dim, int vdim, int silu, int n_tokens, float* seg_state, int dtype, void* stream) {
+                                      int dim, int vdim, int silu, int n_tokens, int longest, float* scratch, int dtype, void* stream) {
     if (n_seqs <= 0) return LLMK_OK;
     if (heads <= 0 || dim <= 0 || vdim <= 0) LLMK_FAIL("linear_attention: bad sizes (heads %d, dim %d, vdim %d)", heads, dim, vdim);
     if (dim > 32 * LA_WARPS) LLMK_FAIL("linear_attention: dim %d is more than %d", dim, 32 * LA_WARPS);
     if (heads > 65535) LLMK_FAIL("linear_attention: too many heads");
+    if (dtype != LLMK_F32 && dtype != LLMK_BF16) LLMK_FAIL("linear_attention: unknown dtype %d", dtype);
+    const int most = longest > 0 ? std::min(longest, n_tokens) : n_tokens;
     LinAttnParams p;
     p.q = q; p.k = k; p.v = v; p.ld = ld; p.out = out; p.state = state; p.decay = decay; p.cu_q = cu_q;
     p.state_slots = state_slots; p.heads = heads; p.dim = dim; p.vdim = vdim; p.silu = silu;
     p.n_seqs = n_seqs;
-    p.segments = n_tokens > LA_SEG ? ceil_div(n_tokens, LA_SEG) : 1;
-    p.seg_state = seg_state;
-    if (p.segments > 1 && !seg_state) LLMK_FAIL("linear_attention: %d tokens need scratch for the segments' states", n_tokens);
-    if (dtype != LLMK_F32 && dtype != LLMK_BF16) LLMK_FAIL("linear_attention: unknown dtype %d", dtype);
+    p.segments = most > LA_SEG ? ceil_div(most, LA_SEG) : 1;
+    p.seg_state = scratch;
+    p.in_chunks = 0;
     const int vsplits = ceil_div(vdim, LA_EV);
-    if ((long long)vsplits * p.segments > 65535) LLMK_FAIL("linear_attention: too many segments");
-    if (n_tokens > LA_CHUNKS_FROM && seg_state) {
+    if (most > chunk_memory::few_of(chunk_memory::CM_CONST) && scratch) {
         chunk_memory::Params c = {};
         c.q = q; c.k = k; c.v = v; c.ldq = c.ldk = c.ldv = ld; c.out = out; c.state = state; c.state_ld = (long long)heads * dim * vdim;
-        c.decay = decay; c.cu_q = cu_q; c.state_slots = state_slots; c.scratch = seg_state; c.H = heads; c.D = dim; c.E = vdim;
-        c.n_seqs = n_seqs; c.chunks = n_tokens / chunk_memory::C + n_seqs; c.silu = silu; c.q_scale = 1.f;
-        if (chunk_memory::usable(c, dtype == LLMK_F32 ? 4 : 2))
-            return dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_CONST>(c, (cudaStream_t)stream)
-                                     : chunk_memory::launch<bf16, chunk_memory::CM_CONST>(c, (cudaStream_t)stream);
+        c.decay = decay; c.cu_q = cu_q; c.state_slots = state_slots; c.scratch = scratch; c.H = heads; c.D = dim; c.E = vdim;
+        c.n_seqs = n_seqs; c.silu = silu; c.q_scale = 1.f;
+        chunk_memory::shape(c, chunk_memory::CM_CONST, n_tokens);
+        if (chunk_memory::usable(c, dtype == LLMK_F32 ? 4 : 2)) {
+            const int rc = dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_CONST>(c, (cudaStream_t)stream)
+                                             : chunk_memory::launch<bf16, chunk_memory::CM_CONST>(c, (cudaStream_t)stream);
+            if (rc != LLMK_OK) return rc;
+            p.in_chunks = 1;
+            p.segments = 1;
+        }
     }
+    if (p.segments > 1 && !scratch) LLMK_FAIL("linear_attention: %d tokens need scratch for the segments' states", n_tokens);
+    if ((long long)vsplits * p.segments > 65535) LLMK_FAIL("linear_attention: too many segments");
     const size_t smem = ((size_t)LA_C * (((dim + 3) & ~3) + dim + 1) + (size_t)dim * LA_C + LA_C * LA_EV + LA_C * (LA_C + 1) +
                          (size_t)dim * LA_EV + LA_C + 1) * sizeof(float);
     dim3 grid(n_seqs, heads, vsplits * p.segments);

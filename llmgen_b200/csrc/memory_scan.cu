@@ -20,10 +20,11 @@
 // A step's sequences are given as everywhere else: sequence s owns token rows [cu_q[s], cu_q[s+1]), its state lies in
 // slot state_slots[s] (-1: none; the sequence then starts from zeros and leaves nothing).  Rows beyond cu_q[n_seqs]
 // belong to no sequence and are skipped, sequences without tokens too, so every launch here follows from a step's shape.
-// Prompts through the mlstm form with key widths of 64 or 128 and value widths in runs of 64 take the chunks of chunk_memory.cuh.
+// Sequences of more than 48 tokens through the mlstm form, with key widths of 64 or 128 and value widths in runs of 64, take the chunks of
+// chunk_memory.cuh; the walk then takes the step's other sequences.
 // States, gates, decays, their logarithms and exponentials, unit norms and the recurrences are float32 arithmetic in both
 // storage dtypes.  The arithmetic of a token of a walk does not depend on where a step was cut;
-// in chunks its sums are grouped by the chunks of its step.
+// in chunks its sums are grouped by the chunks of its own sequence's portion, whatever else the step holds.
 #define LLMK_MODULE_NAME "memory_scan"
 #include "common.cuh"
 #include "chunk_memory.cuh"
@@ -153,21 +154,13 @@ __global__ void mlstm_gates_kernel(float* __restrict__ gates, const T* __restric
     }
 }
 
-// A warp per (sequence, head) takes the tokens 32 at a time: gates[t, h].w <- m_(t-1), the maximum before the token.  A token's
+// Sequence s and head h by a warp, the tokens 32 at a time: gates[t, h].w <- m_(t-1), the maximum before the token.  A token's
 // step m -> max(f + m, i) composes with the next, (f1, i1) then (f2, i2) = (f1 + f2, max(i1 + f2, i2)), so five rounds over the
 // lanes give every token's maximum.  What the memory's step needs follows from (i, f, m_(t-1)) alone, m_t = max(f + m_(t-1), i),
 // keep = exp(f + m_(t-1) - m_t), take = exp(i - m_t), exp(-m_t), and is made where it is used.
-__global__ void mlstm_maxima_kernel(float* __restrict__ gates, float* __restrict__ m_state, long long state_ld,
-                                    const int* __restrict__ cu_q, const int* __restrict__ state_slots, int n_seqs, int H) {
+__device__ __forceinline__ void maxima_by_warp(float* __restrict__ gates, float* __restrict__ m_state, long long state_ld, int q_beg, int n, int slot,
+                                               int h, int H) {
     const int lane = threadIdx.x & 31;
-    const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    pdl_launch_dependents();
-    pdl_wait();
-    if (idx >= n_seqs * H) return;
-    const int s = idx / H, h = idx % H;
-    const int q_beg = cu_q[s], n = cu_q[s + 1] - q_beg;
-    if (n <= 0) return;
-    const int slot = state_slots[s];
     float m = slot >= 0 ? m_state[(size_t)slot * state_ld + h] : 0.f;
     float4* g = reinterpret_cast<float4*>(gates);
     for (int t0 = 0; t0 < n; t0 += 32) {
@@ -195,9 +188,20 @@ __global__ void mlstm_maxima_kernel(float* __restrict__ gates, float* __restrict
     }
     if (slot >= 0 && lane == 0) m_state[(size_t)slot * state_ld + h] = m;
 }
+__global__ void mlstm_maxima_kernel(float* __restrict__ gates, float* __restrict__ m_state, long long state_ld,
+                                    const int* __restrict__ cu_q, const int* __restrict__ state_slots, int n_seqs, int H) {
+    const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    pdl_launch_dependents();
+    pdl_wait();
+    if (idx >= n_seqs * H) return;
+    const int s = idx / H, q_beg = cu_q[s], n = cu_q[s + 1] - q_beg;
+    if (n > 0) maxima_by_warp(gates, m_state, state_ld, q_beg, n, state_slots[s], idx % H, H);
+}
 
-// The same for steps of many tokens: a block per (sequence, head) takes 2,048 tokens at a time, eight in a row a thread, whose steps compose
+// The same for steps that may hold long sequences: a block per (sequence, head) takes 2,048 tokens at a time, eight in a row a thread, whose steps compose
 // in the thread, over the warp's lanes and over the warps (48 us a warp, 2,048 tokens on 16 heads; nearly all of it the wait for gates).
+// Sequences of up to MAXIMA_FEW_TOKENS are a warp's here too: how a token's sums are grouped follows from its own sequence.
+constexpr int MAXIMA_FEW_TOKENS = 64;
 constexpr int MX_THREADS = 256, MX_EACH = 8;
 __global__ void __launch_bounds__(MX_THREADS) mlstm_maxima_block_kernel(float* __restrict__ gates, float* __restrict__ m_state, long long state_ld,
                                                                         const int* __restrict__ cu_q, const int* __restrict__ state_slots, int H) {
@@ -209,6 +213,10 @@ __global__ void __launch_bounds__(MX_THREADS) mlstm_maxima_block_kernel(float* _
     const int q_beg = cu_q[s], n = cu_q[s + 1] - q_beg;
     if (n <= 0) return;
     const int slot = state_slots[s];
+    if (n <= MAXIMA_FEW_TOKENS) {
+        if (warp == 0) maxima_by_warp(gates, m_state, state_ld, q_beg, n, slot, h, H);
+        return;
+    }
     float m = slot >= 0 ? m_state[(size_t)slot * state_ld + h] : 0.f;
     float4* g = reinterpret_cast<float4*>(gates) + (size_t)q_beg * H + h;
     for (int t0 = 0; t0 < n; t0 += MX_THREADS * MX_EACH) {
@@ -317,6 +325,7 @@ struct ScanParams {
     int H, D, E;
     float r_scale, den_eps;
     int* tickets;             // mlstm: [n_seqs, H], zero before and after: how many of a head's blocks are through with its n
+    int in_chunks;            // != 0: sequences of more tokens than chunk_memory leaves were taken in chunks
 };
 
 // A value's bits in a 32-bit register (a 16-bit load extends into one by itself), and back.
@@ -371,7 +380,7 @@ __global__ void __launch_bounds__(LANES* CT) memory_scan_kernel(ScanParams p) {
     pdl_launch_dependents();
     pdl_wait();
     const int q_beg = p.cu_q[s], n = p.cu_q[s + 1] - q_beg;
-    if (n <= 0) return;
+    if (n <= 0 || (FORM == FORM_MLSTM && p.in_chunks && n > chunk_memory::few_of(chunk_memory::CM_MAX))) return;
     const int slot = p.state_slots[s];
     float* Sg = slot >= 0 ? p.state + (size_t)slot * p.state_ld + (size_t)h * D * E : nullptr;
     float* ng = (slot >= 0 && FORM == FORM_MLSTM) ? p.state + (size_t)slot * p.state_ld + (size_t)H * D * E + (size_t)h * D : nullptr;
@@ -595,13 +604,12 @@ LLMK_EXPORT int llmk_min_gru(void* out, const float* zxg, long long ld, const fl
     return LLMK_OK;
 }
 
-// Steps of up to this many token rows: a warp per (sequence, head); longer ones: a block.
-constexpr int MAXIMA_FEW_TOKENS = 64;
 // gates [n, H, 4] float32 <- (i, f, (q . k) q_scale, m before the token) per token and head; m [slots, >= H] carried in the state.
+// longest: the most tokens that one of the step's sequences brings (0: not known).
 LLMK_EXPORT int llmk_mlstm_gates(float* gates, const void* q, long long ldq, const void* k, long long ldk, const void* gi, long long ldi,
                                  const void* gf, long long ldf, const float* bi, const float* bf, float* m_state, long long state_ld,
                                  const int* cu_q, const int* state_slots, int n_seqs, int n_rows, int H, int D, float cap, float q_scale,
-                                 int dtype, void* stream) {
+                                 int longest, int dtype, void* stream) {
     if (n_seqs <= 0 || n_rows <= 0) return LLMK_OK;
     if (!(cap > 0.f)) LLMK_FAIL("mlstm_gates: the gates' bound must be positive");
     if (!host_aligned16(gates)) LLMK_FAIL("mlstm_gates: the gates' array must lie on a 16-byte boundary");
@@ -616,7 +624,7 @@ LLMK_EXPORT int llmk_mlstm_gates(float* gates, const void* q, long long ldq, con
         LLMK_CHECK_LAUNCH_RC("mlstm_gates", llmk_launch(mlstm_gates_kernel<bf16>, grid, block, 0, st, true, gates, (const bf16*)q, ldq,
                                                         (const bf16*)k, ldk, (const bf16*)gi, ldi, (const bf16*)gf, ldf, bi, bf, cu_q,
                                                         n_seqs, n_rows, H, D, cap, q_scale));
-    if (n_rows > MAXIMA_FEW_TOKENS) {
+    if (n_rows > MAXIMA_FEW_TOKENS && (longest <= 0 || longest > MAXIMA_FEW_TOKENS)) {
         LLMK_CHECK_LAUNCH_RC("mlstm_maxima", llmk_launch(mlstm_maxima_block_kernel, dim3(H, n_seqs), dim3(MX_THREADS), 0, st, true, gates, m_state,
                                                          state_ld, cu_q, state_slots, H));
         return LLMK_OK;
@@ -646,21 +654,19 @@ LLMK_EXPORT int llmk_delta_rule_prep(float* aux, float* dots, const void* r, lon
     return LLMK_OK;
 }
 
-// Steps of more token rows than this give the mlstm form's scratch a use: the chunks of chunk_memory.cuh, where it takes the sizes.
-constexpr int CHUNKS_FROM = 64;
 // Floats of scratch that a step of `n_tokens` token rows in `n_seqs` sequences has a use for (0: none).
 LLMK_EXPORT long long llmk_memory_scan_scratch_floats(int n_tokens, int n_seqs, int H, int D, int E, int form) {
-    if (form != FORM_MLSTM || n_tokens <= CHUNKS_FROM || !chunk_memory::sizes_usable(D, E)) return 0;
-    return chunk_memory::scratch_floats(chunk_memory::CM_MAX, n_tokens, n_seqs, H, D, E);
+    return form == FORM_MLSTM ? chunk_memory::scratch_floats(chunk_memory::CM_MAX, n_tokens, n_seqs, H, D, E) : 0;
 }
 
 // The memory's walk over each sequence's new tokens (see the top of the file).  form 0: delta, 1: mlstm.  n_tokens: rows of `out`;
-// scratch: llmk_memory_scan_scratch_floats floats, or null (the walk token by token).
+// longest: the most tokens that one of the step's sequences brings (0: not known); scratch: llmk_memory_scan_scratch_floats floats, or null (every
+// sequence is walked token by token).
 // tickets (mlstm): n_seqs * H ints that are zero, and zero again afterwards.
 LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const void* k, long long ldk, const void* v, long long ldv,
                                  const float* aux, const float* dots, float* state, long long state_ld, const int* cu_q,
                                  const int* state_slots, int n_seqs, int H, int D, int E, int form, float r_scale, float den_eps,
-                                 int n_tokens, float* scratch, int* tickets, int dtype, void* stream) {
+                                 int n_tokens, int longest, float* scratch, int* tickets, int dtype, void* stream) {
     if (n_seqs <= 0) return LLMK_OK;
     if (H <= 0 || D <= 0 || E <= 0 || D > 256) LLMK_FAIL("memory_scan: heads %d, key width %d (at most 256), value width %d", H, D, E);
     if (form != FORM_DELTA && form != FORM_MLSTM) LLMK_FAIL("memory_scan: unknown form %d", form);
@@ -670,13 +676,18 @@ LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const
     p.out = out; p.r = r; p.k = k; p.v = v; p.ldr = ldr; p.ldk = ldk; p.ldv = ldv; p.aux = aux; p.dots = dots; p.state = state;
     p.state_ld = state_ld; p.cu_q = cu_q; p.state_slots = state_slots; p.H = H; p.D = D; p.E = E; p.r_scale = r_scale; p.den_eps = den_eps; p.tickets = tickets;
     cudaStream_t st = (cudaStream_t)stream;
-    if (scratch && llmk_memory_scan_scratch_floats(n_tokens, n_seqs, H, D, E, form) > 0) {
+    p.in_chunks = 0;
+    if (scratch && (longest <= 0 || longest > chunk_memory::few_of(chunk_memory::CM_MAX)) && llmk_memory_scan_scratch_floats(n_tokens, n_seqs, H, D, E, form) > 0) {
         chunk_memory::Params c = {};
         c.q = r; c.k = k; c.v = v; c.ldq = ldr; c.ldk = ldk; c.ldv = ldv; c.out = out; c.state = state; c.state_ld = state_ld;
         c.gates = reinterpret_cast<const float4*>(dots); c.cu_q = cu_q; c.state_slots = state_slots; c.scratch = scratch; c.H = H; c.D = D; c.E = E;
-        c.n_seqs = n_seqs; c.chunks = n_tokens / chunk_memory::C + n_seqs; c.q_scale = r_scale; c.den_eps = den_eps;
-        if (chunk_memory::usable(c, dtype == LLMK_F32 ? 4 : 2) && host_aligned16(dots))
-            return dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_MAX>(c, st) : chunk_memory::launch<bf16, chunk_memory::CM_MAX>(c, st);
+        c.n_seqs = n_seqs; c.q_scale = r_scale; c.den_eps = den_eps;
+        chunk_memory::shape(c, chunk_memory::CM_MAX, n_tokens);
+        if (chunk_memory::usable(c, dtype == LLMK_F32 ? 4 : 2) && host_aligned16(dots)) {
+            const int rc = dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_MAX>(c, st) : chunk_memory::launch<bf16, chunk_memory::CM_MAX>(c, st);
+            if (rc != LLMK_OK) return rc;
+            p.in_chunks = 1;
+        }
     }
     if (dtype == LLMK_F32)
         return form == FORM_DELTA ? launch_scan<float, FORM_DELTA>(p, n_seqs, st) : launch_scan<float, FORM_MLSTM>(p, n_seqs, st);

@@ -1132,12 +1132,13 @@ def min_gru(out: torch.Tensor, zxg: torch.Tensor, bias_z: Optional[torch.Tensor]
 
 def mlstm_gates(gates: torch.Tensor, q: torch.Tensor, k: torch.Tensor, gi: torch.Tensor, gf: torch.Tensor, bias_i: Optional[torch.Tensor],
                 bias_f: Optional[torch.Tensor], m_state: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor, n_seqs: int,
-                heads: int, dim: int, cap: float, q_scale: float) -> None:
+                heads: int, dim: int, cap: float, q_scale: float, longest: int = 0) -> None:
     """gates float32 [n, heads, 4] <- (i, f, (q . k) q_scale, m_(t-1)) of a matrix memory with a running maximum:
     i = cap tanh((gi + bias_i) / cap), f = logsigmoid(cap tanh((gf + bias_f) / cap)), m_t = max(f + m_(t-1), i) (from which
     `memory_scan` makes keep = exp(f + m_(t-1) - m_t), take = exp(i - m_t) and exp(-m_t)); m is carried in `m_state` (float32
     [slots, >= heads]).  q, k [n, heads dim] and gi, gf
-    [n, heads] of the storage dtype with any row stride.  Two launches (csrc/memory_scan.cu)."""
+    [n, heads] of the storage dtype with any row stride.  `longest`: the most tokens that one of the step's sequences brings, where
+    the caller knows it (0: not known).  Two launches (csrc/memory_scan.cu)."""
     lib = build.load("memory_scan")
     n = q.shape[0]
     if gates.dtype != torch.float32 or not gates.is_contiguous() or gates.numel() < n * heads * 4 or m_state.dtype != torch.float32:
@@ -1145,8 +1146,8 @@ def mlstm_gates(gates: torch.Tensor, q: torch.Tensor, k: torch.Tensor, gi: torch
     _check(lib, lib.llmk_mlstm_gates(_ptr(gates), _ptr(q), c_longlong(_row_stride(q)), _ptr(k), c_longlong(_row_stride(k)), _ptr(gi),
                                      c_longlong(_row_stride(gi)), _ptr(gf), c_longlong(_row_stride(gf)), _ptr(bias_i), _ptr(bias_f),
                                      _ptr(m_state), c_longlong(_row_stride(m_state)), _ptr(cu_q), _ptr(state_slots), c_int(n_seqs),
-                                     c_int(n), c_int(heads), c_int(dim), c_float(cap), c_float(q_scale), c_int(dtype_code(q.dtype)),
-                                     _stream()), 2)
+                                     c_int(n), c_int(heads), c_int(dim), c_float(cap), c_float(q_scale), c_int(longest),
+                                     c_int(dtype_code(q.dtype)), _stream()), 2)
 
 
 def delta_rule_prep(aux: torch.Tensor, dots: torch.Tensor, r: torch.Tensor, k: torch.Tensor, a: torch.Tensor, decay: torch.Tensor,
@@ -1178,12 +1179,14 @@ def memory_scan_scratch_floats(n_tokens: int, n_seqs: int, heads: int, dim: int,
 
 def memory_scan(out: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, aux: Optional[torch.Tensor], dots: torch.Tensor,
                 state: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor, n_seqs: int, heads: int, dim: int, vdim: int,
-                form: str, r_scale: float = 1.0, den_eps: float = 0.0, scratch: Optional[torch.Tensor] = None, tickets: Optional[torch.Tensor] = None) -> None:
+                form: str, r_scale: float = 1.0, den_eps: float = 0.0, scratch: Optional[torch.Tensor] = None, longest: int = 0,
+                tickets: Optional[torch.Tensor] = None) -> None:
     """A matrix memory S [dim, vdim] per head walked over each sequence's new tokens (csrc/memory_scan.cu); out float32
     [n, heads vdim].  "delta": S_t = diag(w) S - b (u^T S) + k v^T, o = S_t^T r, with `aux` and `dots` from `delta_rule_prep`.
     "mlstm": S_t = keep S + take k v^T, n_t = keep n + take k, o = S_t^T q / (max(|n_t . q|, exp(-m_t)) + den_eps), q = r r_scale,
     with `dots` from `mlstm_gates`.  state float32 [slots, >= heads dim vdim (+ heads dim for n)].  With `scratch` (float32,
-    `memory_scan_scratch_floats` values) long steps are taken in chunks of tokens that run side by side.  `tickets` (mlstm: int32, n_seqs * heads values): an array
+    `memory_scan_scratch_floats` values) sequences of more than 48 tokens are taken in chunks that run side by side.  `longest`:
+    the most tokens that one of the step's sequences brings, where the caller knows it (0: not known).  `tickets` (mlstm: int32, n_seqs * heads values): an array
     that is zero, and zero again afterwards, for a caller that keeps one; steps that may run at the same time have one each."""
     lib = build.load("memory_scan")
     chunks = memory_scan_scratch_floats(out.shape[0], n_seqs, heads, dim, vdim, form) if scratch is not None else 0
@@ -1199,8 +1202,8 @@ def memory_scan(out: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: torch.Te
     _check(lib, lib.llmk_memory_scan(_ptr(out), _ptr(r), c_longlong(_row_stride(r)), _ptr(k), c_longlong(_row_stride(k)), _ptr(v),
                                      c_longlong(_row_stride(v)), _ptr(aux), _ptr(dots), _ptr(state), c_longlong(_row_stride(state)),
                                      _ptr(cu_q), _ptr(state_slots), c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim),
-                                     c_int(MEMORY_FORMS[form]), c_float(r_scale), c_float(den_eps), c_int(out.shape[0]),
-                                     _ptr(scratch if chunks else None), _ptr(tickets), c_int(dtype_code(r.dtype)), _stream()), 3 if chunks else 1)
+                                     c_int(MEMORY_FORMS[form]), c_float(r_scale), c_float(den_eps), c_int(out.shape[0]), c_int(longest),
+                                     _ptr(scratch if chunks else None), _ptr(tickets), c_int(dtype_code(r.dtype)), _stream()), 4 if chunks else 1)
 
 
 # ------------------------------------------------------------------------------ recurrent mixers
@@ -1448,10 +1451,11 @@ def linear_attention_scratch_floats(n_tokens: int, n_seqs: int, heads: int, dim:
 
 def linear_attention(out: torch.Tensor, packed: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor,
                      decay: torch.Tensor, cu_q: torch.Tensor, state_slots: torch.Tensor, n_seqs: int, heads: int, dim: int,
-                     vdim: int, silu: bool = True, scratch: Optional[torch.Tensor] = None) -> None:
+                     vdim: int, silu: bool = True, scratch: Optional[torch.Tensor] = None, longest: int = 0) -> None:
     """The decayed outer-product recurrence over each sequence's new tokens (csrc/linear_attention.cu).  `packed`
     [tokens, >= ...] holds q, k (heads x dim) and v (heads x vdim) at the column offsets given; `state` float32
-    [slots, heads, dim, vdim] is read and written at each sequence's slot; out float32 [tokens, heads * vdim]."""
+    [slots, heads, dim, vdim] is read and written at each sequence's slot; out float32 [tokens, heads * vdim].
+    `longest`: the most tokens that one of the step's sequences brings, where the caller knows it (0: not known)."""
     lib = build.load("linear_attention")
     if out.dtype != torch.float32 or state.dtype != torch.float32 or decay.dtype != torch.float32 or not out.is_contiguous():
         raise KernelError("linear_attention: out, state and decay are float32")
@@ -1460,14 +1464,14 @@ def linear_attention(out: torch.Tensor, packed: torch.Tensor, q_off: int, k_off:
     es = packed.element_size()
     base = packed.data_ptr()
     n_tokens = out.shape[0]
-    need = linear_attention_scratch_floats(n_tokens, n_seqs, heads, dim, vdim)
+    need = linear_attention_scratch_floats(n_tokens, n_seqs, heads, dim, vdim) if longest <= 0 or longest > 64 else 0
     if need and (scratch is None or scratch.dtype != torch.float32 or scratch.numel() < need):
         raise KernelError(f"linear_attention: a step of {n_tokens} tokens needs {need} float32 of scratch")
     _check(lib, lib.llmk_linear_attention(_ptr(out), c_void_p(base + q_off * es), c_void_p(base + k_off * es), c_void_p(base + v_off * es),
                                           c_longlong(_row_stride(packed)), _ptr(state), _ptr(decay), _ptr(cu_q), _ptr(state_slots),
-                                          c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim), c_int(1 if silu else 0),
-                                          c_int(n_tokens), _ptr(scratch if need else None), c_int(dtype_code(packed.dtype)), _stream()),
-           3 if need else 1)
+                                          c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim), c_int(1 if silu else 0), c_int(n_tokens),
+                                          c_int(longest), _ptr(scratch if need else None), c_int(dtype_code(packed.dtype)), _stream()),
+           4 if need else 1)
 
 
 # ------------------------------------------------------------------------------ latent attention

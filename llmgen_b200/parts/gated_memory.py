@@ -112,18 +112,19 @@ class MLSTM(Mixer):
     def forward(self, ctx, x, cache: LayerCache):
         T, ws = ctx.n_tokens, ctx.workspace
         H, D, E = self.H, self.D, self.E
+        longest = 1 if ctx.pure_decode else 0
         packed = linear(x, self.w_in, ws.buffer("mlstm_in", T, self.w_in.shape[0], self.dtype))
         q, k, v = packed[:, :self.k_off], packed[:, self.k_off:self.v_off], packed[:, self.v_off:self.g_off]
         gates = ws.buffer("mlstm_gates", T, 4 * H, torch.float32)
         scale = float(D) ** -0.5
         ops.mlstm_gates(gates, q, k, packed[:, self.i_off:self.f_off], packed[:, self.f_off:], self.b_i, self.b_f,
-                        cache.state[:, self.m_off:], ctx.cu_q, ctx.state_slots, ctx.n_seqs, H, D, float(self.spec.gate_cap), scale)
+                        cache.state[:, self.m_off:], ctx.cu_q, ctx.state_slots, ctx.n_seqs, H, D, float(self.spec.gate_cap), scale, longest=longest)
         o = ws.buffer("mlstm_o", T, H * E, torch.float32)
-        need = ops.memory_scan_scratch_floats(T, ctx.n_seqs, H, D, E, "mlstm")
+        need = 0 if ctx.pure_decode else ops.memory_scan_scratch_floats(T, ctx.n_seqs, H, D, E, "mlstm")
         scratch = ws.flat("mlstm_chunks", need, torch.float32) if need else None
         tickets = ws.flat("mlstm_tickets", max(ctx.n_seqs, ctx.max_seqs_bound) * H, torch.int32, zero=True)
         ops.memory_scan(o, q, k, v, None, gates, cache.state, ctx.cu_q, ctx.state_slots, ctx.n_seqs, H, D, E, "mlstm",
-                        r_scale=scale, den_eps=float(self.spec.den_eps), scratch=scratch, tickets=tickets)
+                        r_scale=scale, den_eps=float(self.spec.den_eps), scratch=scratch, tickets=tickets, longest=longest)
         y = ws.buffer("mlstm_y", T, H * E, self.dtype)
         ops.gated_rmsnorm(y.view(T * H, E), o.view(T * H, E), packed[:, self.g_off:self.i_off], self.out_gain, float(self.spec.eps),
                           heads=H, gains_per_head=True)

@@ -76,10 +76,11 @@ class LinearAttention(Mixer):
         wide = self.heads * self.vd
         packed = linear(x, self.w_in, ws.buffer("linattn_in", T, self.w_in.shape[0], self.dtype))
         o = ws.buffer("linattn_o", T, wide, torch.float32)
-        need = ops.linear_attention_scratch_floats(T, ctx.n_seqs, self.heads, self.kd, self.vd)
+        need = 0 if ctx.pure_decode else ops.linear_attention_scratch_floats(T, ctx.n_seqs, self.heads, self.kd, self.vd)
         scratch = ws.flat("linattn_segments", need, torch.float32) if need else None
         ops.linear_attention(o, packed, 0, self.k_off, self.v_off, cache.state, self.decay, ctx.cu_q, ctx.state_slots,
-                             ctx.n_seqs, self.heads, self.kd, self.vd, silu=self.spec.activation == "silu", scratch=scratch)
+                             ctx.n_seqs, self.heads, self.kd, self.vd, silu=self.spec.activation == "silu", scratch=scratch,
+                             longest=1 if ctx.pure_decode else 0)
         y = ws.buffer("linattn_y", T, wide, self.dtype)
         if self.spec.gate_proj:
             ops.gated_rmsnorm(y, o, packed[:, self.g_off:], self.norm_gain, self.norm_eps)

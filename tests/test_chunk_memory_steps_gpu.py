@@ -1,0 +1,97 @@
+"""Matrix memories in steps of many sequences (csrc/chunk_memory.cuh beside the walks of csrc/linear_attention.cu and csrc/memory_scan.cu): what a
+sequence's tokens give follows from its own portion and state, whatever else the step holds."""
+import pytest
+import torch
+
+from llmgen_b200.kernels import ops
+
+pytestmark = pytest.mark.gpu
+DT = {"float32": torch.float32, "bfloat16": torch.bfloat16}
+DEV = "cuda:0"
+H, D, E, CAP = 2, 64, 64, 12.0
+SIZE = H * D * E + H * D + H
+
+
+def rnd(shape, seed, scale=1.0, dtype=torch.float32):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).to(dtype)
+
+
+def ints(values):
+    return torch.tensor(values, dtype=torch.int32, device=DEV)
+
+
+def offsets(lens):
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    return ints(cu)
+
+
+def linear(x, state, lens, longest=0, scratch=True):
+    """One step over rows x [n, H (2 D + E)] of sequences of `lens` tokens, sequence s in state[s]; the outputs."""
+    n = len(x)
+    out = torch.full((n, H * E), 3.0, device=DEV)
+    need = ops.linear_attention_scratch_floats(n, len(lens), H, D, E) if scratch else 0
+    ops.linear_attention(out, x, 0, H * D, 2 * H * D, state, torch.tensor([0.97, 0.5], device=DEV), offsets(lens), ints(list(range(len(lens)))), len(lens), H, D, E,
+                         scratch=torch.full((need,), float("nan"), device=DEV) if need else None, **({"longest": longest} if longest else {}))
+    return out
+
+
+def mlstm(x, state, lens, longest=0, scratch=True):
+    """The same for the memory under a running maximum; the gates' columns follow q, k and v."""
+    n, slots = len(x), ints(list(range(len(lens))))
+    q, k, v = x[:, :H * D], x[:, H * D:2 * H * D], x[:, 2 * H * D:2 * H * D + H * E]
+    gates, at, hint = torch.zeros(n, 4 * H, device=DEV), H * (2 * D + E), {"longest": longest} if longest else {}
+    ops.mlstm_gates(gates, q, k, x[:, at:at + H], x[:, at + H:at + 2 * H], None, torch.tensor([3.0, 0.0], device=DEV), state[:, H * D * E + H * D:], offsets(lens),
+                    slots, len(lens), H, D, CAP, D ** -0.5, **hint)
+    out = torch.full((n, H * E), 3.0, device=DEV)
+    need = ops.memory_scan_scratch_floats(n, len(lens), H, D, E, "mlstm") if scratch else 0
+    ops.memory_scan(out, q, k, v, None, gates, state, offsets(lens), slots, len(lens), H, D, E, "mlstm", r_scale=D ** -0.5, den_eps=1e-6,
+                    scratch=torch.full((need,), float("nan"), device=DEV) if need else None, **hint)
+    return out
+
+
+def fresh(form, n):
+    return rnd((n, H, D, E), 1, 0.3).to(DEV) if form is linear else rnd((n, SIZE), 1, 0.3).to(DEV)
+
+
+def rows(n, dtype, seed=2):
+    return rnd((n, H * (2 * D + E) + 8), seed, 0.7, DT[dtype]).to(DEV)
+
+
+LENS = [1] * 150
+for at, n in ((0, 130), (30, 32), (37, 64), (40, 65), (70, 48), (71, 49), (100, 0), (131, 300), (149, 200)):
+    LENS[at] = n
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("form", [linear, mlstm])
+def test_a_sequence_gives_what_it_gives_alone(form, dtype):
+    x, state = rows(sum(LENS), dtype), fresh(form, len(LENS))
+    before = state.clone()
+    out = form(x, state, LENS)
+    at = 0
+    for s, n in enumerate(LENS):
+        if s in (0, 1, 30, 37, 40, 70, 71, 72, 131, 148, 149):
+            own = before[s:s + 1].clone()
+            assert torch.equal(form(x[at:at + n], own, [n]), out[at:at + n]), (s, n)
+            assert torch.equal(own, state[s:s + 1]), (s, n)
+        at += n
+    assert torch.equal(state[100], before[100])
+
+
+@pytest.mark.parametrize("form", [linear, mlstm])
+def test_scratch_follows_what_long_sequences_can_be_there(form):
+    entries = D * E + (D if form is mlstm else 0)
+    need = ops.memory_scan_scratch_floats if form is mlstm else ops.linear_attention_scratch_floats
+    last = ("mlstm",) if form is mlstm else ()
+    few = need(256, 8, H, D, E, *last)
+    # 256 tokens are at most four whole chunks and the shorter chunks of five sequences of more than 48 tokens
+    assert 0 < few <= need(256, 256, H, D, E, *last) <= 9 * H * (entries + 2) + 256 * H
+
+
+@pytest.mark.parametrize("form", [linear, mlstm])
+def test_single_tokens_are_walked_without_scratch(form):
+    x, lens = rows(200, "bfloat16"), [1] * 200
+    a, b = fresh(form, 200), fresh(form, 200)
+    assert torch.equal(form(x, a, lens, longest=1, scratch=False), form(x, b, lens)) and torch.equal(a, b)
