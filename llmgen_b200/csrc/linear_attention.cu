@@ -413,21 +413,28 @@ static int dispatch_linear_attention(const LinAttnParams& p, dim3 grid, size_t s
     return launch_linear_attention<T, 32>(p, grid, smem, s);
 }
 
-// Floats of scratch that a step of `n_tokens` tokens in `n_seqs` sequences needs for its chunks' or segments' states (0: none).
-LLMK_EXPORT long long llmk_linear_attention_scratch_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim) {
-    const long long segments = n_tokens > LA_SEG ? (long long)(n_tokens / LA_SEG + n_seqs) * heads * dim * vdim : 0;
-    return std::max(segments, chunk_memory::scratch_floats(chunk_memory::CM_CONST, n_tokens, n_seqs, heads, dim, vdim));
+// Floats of scratch with which a step of `n_tokens` tokens in `n_seqs` sequences runs as fast as it can (0: it needs none): the chunks' where the
+// sizes allow them (`vectors`: the rows are 16-byte vectors), and else the segments'.  Without `vectors` as much as either may need.
+static long long segment_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim) {
+    return n_tokens > LA_SEG ? (long long)(n_tokens / LA_SEG + n_seqs) * heads * dim * vdim : 0;
+}
+LLMK_EXPORT long long llmk_linear_attention_scratch_floats(int n_tokens, int n_seqs, int heads, int dim, int vdim, int vectors) {
+    const long long chunks = chunk_memory::scratch_floats(chunk_memory::CM_CONST, n_tokens, n_seqs, heads, dim, vdim);
+    if (vectors && chunk_memory::sizes_usable(dim, vdim)) return chunks;
+    return std::max(chunks, segment_floats(n_tokens, n_seqs, heads, dim, vdim));
 }
 
 // q, k, v: pointers to the first row's q, k and v inside the packed projection (rows `ld` elements apart, heads
 // side by side); out float32 [tokens, heads * vdim]; state float32 [slots, heads, dim, vdim]; decay float32 [heads].
 // n_tokens: rows of `out` (all tokens of the step).  longest: the most tokens that one of its sequences brings (0: not known).
-// scratch: llmk_linear_attention_scratch_floats floats, or null.  What takes no chunks is walked; with more
+// scratch: `scratch_floats` floats, or null.  Where they do not hold the chunks' (llmk_linear_attention_scratch_floats) the step is walked; with more
 // than LA_SEG tokens in segments that run side by side (three launches: segments from an empty state, the scan over their end states, the
-// carried state's share of the outputs), whose states the scratch must hold.
+// carried state's share of the outputs), whose states the scratch must hold.  launches receives how many kernels were launched.
 LLMK_EXPORT int llmk_linear_attention(float* out, const void* q, const void* k, const void* v, long long ld, float* state,
                                       const float* decay, const int* cu_q, const int* state_slots, int n_seqs, int heads,
-                                      int dim, int vdim, int silu, int n_tokens, int longest, float* scratch, int dtype, void* stream) {
+                                      int dim, int vdim, int silu, int n_tokens, int longest, float* scratch, long long scratch_floats,
+                                      int* launches, int dtype, void* stream) {
+    *launches = 0;
     if (n_seqs <= 0) return LLMK_OK;
     if (heads <= 0 || dim <= 0 || vdim <= 0) LLMK_FAIL("linear_attention: bad sizes (heads %d, dim %d, vdim %d)", heads, dim, vdim);
     if (dim > 32 * LA_WARPS) LLMK_FAIL("linear_attention: dim %d is more than %d", dim, 32 * LA_WARPS);
@@ -442,7 +449,7 @@ LLMK_EXPORT int llmk_linear_attention(float* out, const void* q, const void* k, 
     p.seg_state = scratch;
     p.in_chunks = 0;
     const int vsplits = ceil_div(vdim, LA_EV);
-    if (most > chunk_memory::few_of(chunk_memory::CM_CONST) && scratch) {
+    if (most > chunk_memory::few_of(chunk_memory::CM_CONST) && scratch && scratch_floats >= chunk_memory::scratch_floats(chunk_memory::CM_CONST, n_tokens, n_seqs, heads, dim, vdim)) {
         chunk_memory::Params c = {};
         c.q = q; c.k = k; c.v = v; c.ldq = c.ldk = c.ldv = ld; c.out = out; c.state = state; c.state_ld = (long long)heads * dim * vdim;
         c.decay = decay; c.cu_q = cu_q; c.state_slots = state_slots; c.scratch = scratch; c.H = heads; c.D = dim; c.E = vdim;
@@ -452,12 +459,15 @@ LLMK_EXPORT int llmk_linear_attention(float* out, const void* q, const void* k, 
             const int rc = dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_CONST>(c, (cudaStream_t)stream)
                                              : chunk_memory::launch<bf16, chunk_memory::CM_CONST>(c, (cudaStream_t)stream);
             if (rc != LLMK_OK) return rc;
+            *launches = 3;
             p.in_chunks = 1;
             p.segments = 1;
         }
     }
-    if (p.segments > 1 && !scratch) LLMK_FAIL("linear_attention: %d tokens need scratch for the segments' states", n_tokens);
+    if (p.segments > 1 && (!scratch || scratch_floats < segment_floats(n_tokens, n_seqs, heads, dim, vdim)))
+        LLMK_FAIL("linear_attention: a step of %d tokens needs %lld float32 of scratch", n_tokens, segment_floats(n_tokens, n_seqs, heads, dim, vdim));
     if ((long long)vsplits * p.segments > 65535) LLMK_FAIL("linear_attention: too many segments");
+    *launches += p.segments > 1 ? 3 : 1;
     const size_t smem = ((size_t)LA_C * (((dim + 3) & ~3) + dim + 1) + (size_t)dim * LA_C + LA_C * LA_EV + LA_C * (LA_C + 1) +
                          (size_t)dim * LA_EV + LA_C + 1) * sizeof(float);
     dim3 grid(n_seqs, heads, vsplits * p.segments);

@@ -661,12 +661,13 @@ LLMK_EXPORT long long llmk_memory_scan_scratch_floats(int n_tokens, int n_seqs, 
 
 // The memory's walk over each sequence's new tokens (see the top of the file).  form 0: delta, 1: mlstm.  n_tokens: rows of `out`;
 // longest: the most tokens that one of the step's sequences brings (0: not known); scratch: llmk_memory_scan_scratch_floats floats, or null (every
-// sequence is walked token by token).
+// sequence is walked token by token); launches receives how many kernels were launched.
 // tickets (mlstm): n_seqs * H ints that are zero, and zero again afterwards.
 LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const void* k, long long ldk, const void* v, long long ldv,
                                  const float* aux, const float* dots, float* state, long long state_ld, const int* cu_q,
                                  const int* state_slots, int n_seqs, int H, int D, int E, int form, float r_scale, float den_eps,
-                                 int n_tokens, int longest, float* scratch, int* tickets, int dtype, void* stream) {
+                                 int n_tokens, int longest, float* scratch, int* tickets, int* launches, int dtype, void* stream) {
+    *launches = 0;
     if (n_seqs <= 0) return LLMK_OK;
     if (H <= 0 || D <= 0 || E <= 0 || D > 256) LLMK_FAIL("memory_scan: heads %d, key width %d (at most 256), value width %d", H, D, E);
     if (form != FORM_DELTA && form != FORM_MLSTM) LLMK_FAIL("memory_scan: unknown form %d", form);
@@ -686,9 +687,11 @@ LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const
         if (chunk_memory::usable(c, dtype == LLMK_F32 ? 4 : 2) && host_aligned16(dots)) {
             const int rc = dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_MAX>(c, st) : chunk_memory::launch<bf16, chunk_memory::CM_MAX>(c, st);
             if (rc != LLMK_OK) return rc;
+            *launches = 3;
             p.in_chunks = 1;
         }
     }
+    *launches += 1;
     if (dtype == LLMK_F32)
         return form == FORM_DELTA ? launch_scan<float, FORM_DELTA>(p, n_seqs, st) : launch_scan<float, FORM_MLSTM>(p, n_seqs, st);
     return form == FORM_DELTA ? launch_scan<bf16, FORM_DELTA>(p, n_seqs, st) : launch_scan<bf16, FORM_MLSTM>(p, n_seqs, st);

@@ -1199,11 +1199,13 @@ def memory_scan(out: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: torch.Te
         raise KernelError("memory_scan: out, dots and state are float32; r, k, v share the storage dtype")
     if tickets is None and form == "mlstm":
         tickets = torch.zeros(n_seqs * heads, dtype=torch.int32, device=out.device)
+    launched = c_int(0)
     _check(lib, lib.llmk_memory_scan(_ptr(out), _ptr(r), c_longlong(_row_stride(r)), _ptr(k), c_longlong(_row_stride(k)), _ptr(v),
                                      c_longlong(_row_stride(v)), _ptr(aux), _ptr(dots), _ptr(state), c_longlong(_row_stride(state)),
                                      _ptr(cu_q), _ptr(state_slots), c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim),
                                      c_int(MEMORY_FORMS[form]), c_float(r_scale), c_float(den_eps), c_int(out.shape[0]), c_int(longest),
-                                     _ptr(scratch if chunks else None), _ptr(tickets), c_int(dtype_code(r.dtype)), _stream()), 4 if chunks else 1)
+                                     _ptr(scratch if chunks else None), _ptr(tickets), ctypes.byref(launched), c_int(dtype_code(r.dtype)), _stream()), 0)
+    _Counter.launches += launched.value
 
 
 # ------------------------------------------------------------------------------ recurrent mixers
@@ -1442,11 +1444,12 @@ def decay_scan(out: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Ten
 
 
 # ------------------------------------------------------------------------------ linear attention
-def linear_attention_scratch_floats(n_tokens: int, n_seqs: int, heads: int, dim: int, vdim: int) -> int:
-    """float32 values of scratch `linear_attention` needs for a step of this shape (0: none)."""
+def linear_attention_scratch_floats(n_tokens: int, n_seqs: int, heads: int, dim: int, vdim: int, vectors: bool = False) -> int:
+    """float32 values of scratch with which `linear_attention` takes a step of this shape as fast as it can (0: none).  `vectors`: its q, k
+    and v are known to be rows of whole 16-byte vectors; otherwise what other rows need is counted too."""
     lib = build.load("linear_attention")
     lib.llmk_linear_attention_scratch_floats.restype = c_longlong
-    return int(lib.llmk_linear_attention_scratch_floats(c_int(n_tokens), c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim)))
+    return int(lib.llmk_linear_attention_scratch_floats(c_int(n_tokens), c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim), c_int(1 if vectors else 0)))
 
 
 def linear_attention(out: torch.Tensor, packed: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor,
@@ -1454,8 +1457,10 @@ def linear_attention(out: torch.Tensor, packed: torch.Tensor, q_off: int, k_off:
                      vdim: int, silu: bool = True, scratch: Optional[torch.Tensor] = None, longest: int = 0) -> None:
     """The decayed outer-product recurrence over each sequence's new tokens (csrc/linear_attention.cu).  `packed`
     [tokens, >= ...] holds q, k (heads x dim) and v (heads x vdim) at the column offsets given; `state` float32
-    [slots, heads, dim, vdim] is read and written at each sequence's slot; out float32 [tokens, heads * vdim].
-    `longest`: the most tokens that one of the step's sequences brings, where the caller knows it (0: not known)."""
+    [slots, heads, dim, vdim] is read and written at each sequence's slot; out float32 [tokens, heads * vdim].  With `scratch`
+    (float32, `linear_attention_scratch_floats` values; more than 256 tokens need it unless no sequence has as many) sequences
+    of more than 64 tokens are taken in chunks that run side by side.  `longest`: the most tokens that one of the step's
+    sequences brings, where the caller knows it (0: not known)."""
     lib = build.load("linear_attention")
     if out.dtype != torch.float32 or state.dtype != torch.float32 or decay.dtype != torch.float32 or not out.is_contiguous():
         raise KernelError("linear_attention: out, state and decay are float32")
@@ -1463,15 +1468,15 @@ def linear_attention(out: torch.Tensor, packed: torch.Tensor, q_off: int, k_off:
         raise KernelError(f"linear_attention: state must be [slots, {heads}, {dim}, {vdim}], got {list(state.shape)}")
     es = packed.element_size()
     base = packed.data_ptr()
-    n_tokens = out.shape[0]
-    need = linear_attention_scratch_floats(n_tokens, n_seqs, heads, dim, vdim) if longest <= 0 or longest > 64 else 0
-    if need and (scratch is None or scratch.dtype != torch.float32 or scratch.numel() < need):
-        raise KernelError(f"linear_attention: a step of {n_tokens} tokens needs {need} float32 of scratch")
+    if scratch is not None and (scratch.dtype != torch.float32 or not scratch.is_contiguous()):
+        scratch = None
+    launched = c_int(0)
     _check(lib, lib.llmk_linear_attention(_ptr(out), c_void_p(base + q_off * es), c_void_p(base + k_off * es), c_void_p(base + v_off * es),
                                           c_longlong(_row_stride(packed)), _ptr(state), _ptr(decay), _ptr(cu_q), _ptr(state_slots),
-                                          c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim), c_int(1 if silu else 0), c_int(n_tokens),
-                                          c_int(longest), _ptr(scratch if need else None), c_int(dtype_code(packed.dtype)), _stream()),
-           4 if need else 1)
+                                          c_int(n_seqs), c_int(heads), c_int(dim), c_int(vdim), c_int(1 if silu else 0), c_int(out.shape[0]),
+                                          c_int(longest), _ptr(scratch), c_longlong(scratch.numel() if scratch is not None else 0),
+                                          ctypes.byref(launched), c_int(dtype_code(packed.dtype)), _stream()), 0)
+    _Counter.launches += launched.value
 
 
 # ------------------------------------------------------------------------------ latent attention

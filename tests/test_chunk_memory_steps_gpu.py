@@ -95,3 +95,33 @@ def test_single_tokens_are_walked_without_scratch(form):
     x, lens = rows(200, "bfloat16"), [1] * 200
     a, b = fresh(form, 200), fresh(form, 200)
     assert torch.equal(form(x, a, lens, longest=1, scratch=False), form(x, b, lens)) and torch.equal(a, b)
+
+
+def launched(f):
+    before = ops.launches()
+    f()
+    return ops.launches() - before
+
+
+@pytest.mark.parametrize("n", [65, 100, 256])
+def test_linear_attention_of_up_to_256_tokens_needs_no_scratch(n):
+    x, want_state, state = rows(n, "bfloat16"), fresh(linear, 1), fresh(linear, 1)
+    want, out = linear(x, want_state, [n]), linear(x, state, [n], scratch=False)
+    # (float32 sums of at most 256 terms of the same size in another order)
+    assert float((out - want).norm() / want.norm()) < 2e-6 and float((state - want_state).norm() / want_state.norm()) < 2e-6
+
+
+def test_a_step_that_needs_scratch_for_its_segments_says_so():
+    x, state = rows(257, "bfloat16"), fresh(linear, 1)
+    with pytest.raises(ops.KernelError, match="scratch"):
+        linear(x, state, [257], scratch=False)
+
+
+def test_launches_are_counted_as_they_happen():
+    x, wide = rows(200, "bfloat16"), rows(200, "bfloat16")[:, 1:]        # (the second's rows start off 16-byte boundaries)
+    assert launched(lambda: linear(x, fresh(linear, 1), [200])) == 4
+    assert launched(lambda: linear(wide, fresh(linear, 1), [200])) == 1
+    assert launched(lambda: linear(x, fresh(linear, 1), [200], scratch=False)) == 1
+    assert launched(lambda: linear(x, fresh(linear, 200), [1] * 200, longest=1)) == 1
+    assert launched(lambda: mlstm(x, fresh(mlstm, 1), [200])) == 2 + 4
+    assert launched(lambda: mlstm(wide, fresh(mlstm, 1), [200])) == 2 + 1
