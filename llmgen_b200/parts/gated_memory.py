@@ -105,9 +105,11 @@ class MLSTM(Mixer):
 
     def workspace_bytes(self, tokens: int) -> int:
         elem = 2 if self.dtype == torch.bfloat16 else 4
-        chunks = 4 * ops.memory_scan_scratch_floats(tokens, max(1, tokens // 32), self.H, self.D, self.E, "mlstm")
-        return chunks + tokens * (self.w_in.shape[0] * elem + self.H * 16 + self.H * self.E * (4 + elem) + self.spec.hidden_size * elem) \
+        return 4 * self._chunk_floats(tokens, max(1, tokens // 32)) + tokens * (self.w_in.shape[0] * elem + self.H * 16 + self.H * self.E * (4 + elem) + self.spec.hidden_size * elem) \
             + ops.SLICED_PRODUCT_BYTES
+
+    def _chunk_floats(self, tokens: int, seqs: int) -> int:
+        return ops.memory_scan_scratch_floats(tokens, seqs, self.H, self.D, self.E, "mlstm")
 
     def forward(self, ctx, x, cache: LayerCache):
         T, ws = ctx.n_tokens, ctx.workspace
@@ -120,8 +122,11 @@ class MLSTM(Mixer):
         ops.mlstm_gates(gates, q, k, packed[:, self.i_off:self.f_off], packed[:, self.f_off:], self.b_i, self.b_f,
                         cache.state[:, self.m_off:], ctx.cu_q, ctx.state_slots, ctx.n_seqs, H, D, float(self.spec.gate_cap), scale, longest=longest)
         o = ws.buffer("mlstm_o", T, H * E, torch.float32)
-        need = 0 if ctx.pure_decode else ops.memory_scan_scratch_floats(T, ctx.n_seqs, H, D, E, "mlstm")
-        scratch = ws.flat("mlstm_chunks", need, torch.float32) if need else None
+        scratch = None
+        if not ctx.pure_decode and self._chunk_floats(T, ctx.n_seqs):
+            # one buffer for every shape of step, so that none is outgrown (a graph that was captured keeps the buffers it uses)
+            rows, seqs = max(T, ws.default_rows), max(ctx.n_seqs, ctx.max_seqs_bound)
+            scratch = ws.flat("mlstm_chunks", self._chunk_floats(rows, seqs), torch.float32)
         tickets = ws.flat("mlstm_tickets", max(ctx.n_seqs, ctx.max_seqs_bound) * H, torch.int32, zero=True)
         ops.memory_scan(o, q, k, v, None, gates, cache.state, ctx.cu_q, ctx.state_slots, ctx.n_seqs, H, D, E, "mlstm",
                         r_scale=scale, den_eps=float(self.spec.den_eps), scratch=scratch, tickets=tickets, longest=longest)

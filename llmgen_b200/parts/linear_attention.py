@@ -67,8 +67,15 @@ class LinearAttention(Mixer):
     def workspace_bytes(self, tokens: int) -> int:
         elem = 2 if self.dtype == torch.bfloat16 else 4
         wide = self.heads * self.vd
-        chunks = 4 * ops.linear_attention_scratch_floats(tokens, max(1, tokens // 32), self.heads, self.kd, self.vd)
-        return chunks + tokens * (self.w_in.shape[0] * elem + wide * (4 + elem) + self.spec.hidden_size * elem) + ops.SLICED_PRODUCT_BYTES
+        return 4 * self._chunk_floats(tokens, max(1, tokens // 32)) + tokens * (self.w_in.shape[0] * elem + wide * (4 + elem) + self.spec.hidden_size * elem) + ops.SLICED_PRODUCT_BYTES
+
+    def _chunk_floats(self, tokens: int, seqs: int) -> int:
+        return ops.linear_attention_scratch_floats(tokens, seqs, self.heads, self.kd, self.vd, vectors=self._rows_are_vectors())
+
+    def _rows_are_vectors(self) -> bool:
+        """Whether q, k and v of the packed projection lie on 16-byte boundaries in every row."""
+        per = 8 if self.dtype == torch.bfloat16 else 4
+        return all(n % per == 0 for n in (self.w_in.shape[0], self.k_off, self.v_off))
 
     def forward(self, ctx, x, cache: LayerCache):
         T = ctx.n_tokens
@@ -76,8 +83,11 @@ class LinearAttention(Mixer):
         wide = self.heads * self.vd
         packed = linear(x, self.w_in, ws.buffer("linattn_in", T, self.w_in.shape[0], self.dtype))
         o = ws.buffer("linattn_o", T, wide, torch.float32)
-        need = 0 if ctx.pure_decode else ops.linear_attention_scratch_floats(T, ctx.n_seqs, self.heads, self.kd, self.vd)
-        scratch = ws.flat("linattn_segments", need, torch.float32) if need else None
+        scratch = None
+        if not ctx.pure_decode and self._chunk_floats(T, ctx.n_seqs):
+            # one buffer for every shape of step, so that none is outgrown (a graph that was captured keeps the buffers it uses)
+            rows, seqs = max(T, ws.default_rows), max(ctx.n_seqs, ctx.max_seqs_bound)
+            scratch = ws.flat("linattn_chunks", self._chunk_floats(rows, seqs), torch.float32)
         ops.linear_attention(o, packed, 0, self.k_off, self.v_off, cache.state, self.decay, ctx.cu_q, ctx.state_slots,
                              ctx.n_seqs, self.heads, self.kd, self.vd, silu=self.spec.activation == "silu", scratch=scratch,
                              longest=1 if ctx.pure_decode else 0)

@@ -125,3 +125,38 @@ def test_launches_are_counted_as_they_happen():
     assert launched(lambda: linear(x, fresh(linear, 200), [1] * 200, longest=1)) == 1
     assert launched(lambda: mlstm(x, fresh(mlstm, 1), [200])) == 2 + 4
     assert launched(lambda: mlstm(wide, fresh(mlstm, 1), [200])) == 2 + 1
+
+
+def a_mixer(form):
+    """(the part, the state's shape) of one layer around the memory."""
+    from llmgen_b200.parts.registry import build_mixer, mixer_class
+    from llmgen_b200.parts.spec import LinearAttentionSpec, MLSTMSpec
+    from llmgen_b200.weights import weights_from_dict
+    W, w = 64, lambda i, rows, cols: rnd((rows, cols), i, 0.1, torch.bfloat16)
+    if form is linear:
+        spec = LinearAttentionSpec(hidden_size=W, num_heads=H, key_dim=D, value_dim=E, decay=(0.9, 0.5), q_proj="q", k_proj="k", v_proj="v", o_proj="o")
+        tensors, shape = {}, (H, D, E)
+    else:
+        spec = MLSTMSpec(hidden_size=W, num_heads=H, key_dim=D, value_dim=E, gate_cap=CAP, eps=1e-5, q_proj="q", k_proj="k", v_proj="v", i_proj="i", f_proj="f",
+                         gate_proj="g", o_proj="o", out_gain="n", den_eps=1e-6)
+        tensors, shape = {"i": w(5, H, W), "f": w(6, H, W), "g": w(7, H * E, W), "n": torch.ones(H * E)}, (SIZE,)
+    tensors.update({"q": w(1, H * D, W), "k": w(2, H * D, W), "v": w(3, H * E, W), "o": w(4, W, H * E)})
+    return build_mixer(spec, weights_from_dict(tensors, mixer_class(spec).weight_decls(spec)), torch.bfloat16, DEV), shape
+
+
+@pytest.mark.parametrize("form", [linear, mlstm])
+def test_a_workspace_keeps_one_array_for_the_chunks(form):
+    """Steps of rising sizes, as when graphs are captured: no array is outgrown, and what is held is what was said to be."""
+    from llmgen_b200.parts.base import LayerCache
+    from tests.util import manual_context
+    part, shape = a_mixer(form)
+    workspace = None
+    for lens in ([1] * 80, [1] * 256, [100], [60] * 3, [500], [300, 1, 1], [70] * 14, [1024]):
+        ctx = manual_context(lens, [0] * len(lens), [[0] * 64] * len(lens), 16, torch.bfloat16, max_step_tokens=1024)
+        ctx.max_seqs_bound = 256
+        workspace = ctx.workspace = workspace or ctx.workspace
+        part.forward(ctx, rnd((sum(lens), 64), 9, 1.0, torch.bfloat16).to(DEV), LayerCache(state=torch.zeros(len(lens), *shape, device=DEV)))
+    torch.cuda.synchronize()
+    held = [b for name, b in workspace._buffers.items() if "chunks" in name]
+    assert len(held) == 1 and all(b.numel() < 4096 for b in workspace._retired)
+    assert held[0].numel() * 4 <= part.workspace_bytes(1024) and workspace.bytes_held() <= part.workspace_bytes(1024) + ops.SLICED_PRODUCT_BYTES + (1 << 20)
