@@ -26,7 +26,9 @@
 // launched behind the chunks and skips the sequences that they took.  Walk -> chunks
 // (us, constant decay / running maximum): one sequence of 96 tokens 50 -> 37 / 68 -> 39, 8 of 60 tokens - / 124 -> 73, 32 of 64 - / 478 -> 248; a step that counted
 // its rows instead took 417 -> 1,090 / 185 -> 1,051 for a token each of 128 sequences and 729 -> 2,069 / 697 -> 2,015 for 10 tokens each of 200.
-// A value that is no number reaches the outputs of its sequence from the sixteen tokens it lies in on, not only from its own token on.
+// Terms of bfloat16 are made of ordinary numbers only: an infinity would fall apart into inf - inf, and products of sixteen keys at a time would
+// carry what is no number to tokens before it.  A head of a sequence whose tokens or state hold a value beyond 1e38, an infinity or a NaN, or whose
+// gates add up to more than two floats can tell apart, is left to the walk too (the check reads the queries once more, and the state once).
 #pragma once
 #include "common.cuh"
 #include <algorithm>
@@ -49,12 +51,14 @@ struct Params {
     const float* decay;         // CM_CONST: [H]
     const float4* gates;        // CM_MAX: [tokens, H] = (i, f, -, m before the token)
     const int *cu_q, *state_slots;
-    float* scratch;             // [chunks][H][entries], the chunks' decays [chunks][H]
+    float* scratch;             // [chunks][H][entries], the chunks' decays [chunks][H], and as ints [chunks][H] and [n_seqs][H]: left to the walk
     int H, D, E, n_seqs, silu;
     int chunks, longs;          // the most chunks, and sequences taken in chunks, that the step can have
     int entries;                // of a head's state: D E, CM_MAX D E + D
     float q_scale, den_eps;
     __host__ __device__ float* decays() const { return scratch + (size_t)chunks * H * entries; }
+    __host__ __device__ int* chunk_odd() const { return reinterpret_cast<int*>(decays() + (size_t)chunks * H); }
+    __host__ __device__ int* odd() const { return chunk_odd() + (size_t)chunks * H; }
 };
 
 inline bool sizes_usable(int D, int E) { return (D == 64 || D == 128) && E % EB == 0; }
@@ -69,7 +73,12 @@ inline void shape(Params& p, int form, int n_tokens) {
 inline long long scratch_floats(int form, int n_tokens, int n_seqs, int H, int D, int E) {
     if (n_tokens <= few_of(form) || n_seqs <= 0 || !sizes_usable(D, E)) return 0;
     const long long chunks = n_tokens / C + most_longs(form, n_tokens, n_seqs);
-    return chunks * H * ((long long)D * E + (form == CM_MAX ? D : 0) + 1);
+    return chunks * H * ((long long)D * E + (form == CM_MAX ? D : 0) + 2) + (long long)n_seqs * H;
+}
+// What the walk behind the chunks skips: head h of sequence s.  odd: Params::odd(), null where no chunks were launched.
+template <int FORM>
+__device__ __forceinline__ bool taken(const int* __restrict__ odd, int n_tokens, int s, int h, int H) {
+    return odd && n_tokens > few_of(FORM) && !odd[(size_t)s * H + h];
 }
 
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const bf16* p) {
@@ -85,6 +94,8 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint3
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// No ordinary number, or one beyond what a bfloat16 can hold (3.3e38) with room to spare.
+__device__ __forceinline__ bool odd_value(float x) { return !(fabsf(x) < 1e38f); }
 // (x, y) as NT pairs of bfloat16, the most significant first.
 template <int NT>
 __device__ __forceinline__ void terms(uint32_t (&t)[NT], float x, float y) {
@@ -224,6 +235,15 @@ __device__ __forceinline__ void make_weights(Weights& w, const Params& p, int h,
         w.lo[2 * tid + u] = (float)(F - (double)(float)F);
     }
 }
+// Whether a thread's token has gates that are no numbers, or sums of them of which `hi` and `lo` keep too little: up to 2^20 they hold 2^-28, and
+// differences of two sums are exponents.
+template <int FORM>
+__device__ __forceinline__ bool weights_odd(const Weights& w, int n) {
+    const int i = threadIdx.x;
+    if (i >= n) return false;
+    if (FORM == CM_CONST) return odd_value(w.pw[C]);
+    return !(fabsf(w.hi[i]) <= 1048576.f) || odd_value(w.gate[i]) || odd_value(w.top[i]) || odd_value(w.m_before);
+}
 // The weight of token j in what token i (or the state after it) holds, i >= j.
 template <int FORM>
 __device__ __forceinline__ float weight(const Weights& w, int i, int j) {
@@ -239,6 +259,7 @@ __device__ __forceinline__ float from_start(const Weights& w, int i) {
 
 // COLS columns of a chunk's rows on their way into shared memory: `ask` sends for a thread's 16-byte vectors, all at once, and `put` writes them
 // as NT terms, times `scale` per row (null: 1), zeros beyond the chunk's n tokens.
+// `odd`: whether one of the thread's values is none that terms can be made of.
 template <typename T, int NT, int COLS>
 struct Rows {
     static constexpr int VN = Vec16<T>::N, LD = COLS + 8, EACH = C * COLS / VN / THREADS;
@@ -249,6 +270,18 @@ struct Rows {
             const int idx = threadIdx.x + i * THREADS, r = idx / (COLS / VN), c = idx % (COLS / VN) * VN;
             if (r < n) held[i].raw = *reinterpret_cast<const decltype(held[i].raw)*>(src + (size_t)r * ld + c);
         }
+    }
+    __device__ __forceinline__ bool odd(int n) const {
+        bool any = false;
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            float f[VN];
+            held[i].unpack(f);
+            const bool row = (threadIdx.x + i * THREADS) / (COLS / VN) < n;
+#pragma unroll
+            for (int u = 0; u < VN; ++u) any |= row && odd_value(f[u]);
+        }
+        return any;
     }
     __device__ __forceinline__ void put(bf16* dst, int n, int silu, const float* scale) {
 #pragma unroll
@@ -284,7 +317,8 @@ struct Rows {
 template <typename T, int FORM> constexpr int input_terms() { return sizeof(T) == 2 && FORM == CM_MAX ? 1 : 3; }
 
 // ---------------------------------------------------------------------------------------------------------------- local
-// Block (chunk, head): dS [D, E], 64 columns at a time; warp w has rows 16 (w % (D / 16)) of D and, with D = 64, half of the columns.
+// Block (chunk, head): dS [D, E], 64 columns at a time; warp w has rows 16 (w % (D / 16)) of D and, with D = 64, half of the columns.  It also looks
+// for values that the terms cannot hold, in the chunk's rows, its gates and its share of the state that the sequence comes with.
 template <typename T, int FORM, int D>
 __global__ void __launch_bounds__(THREADS, 2) chunk_memory_local_kernel(Params p) {
     constexpr int NT = input_terms<T, FORM>(), LDD = D + 8;
@@ -299,16 +333,38 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_local_kernel(Params p
     pdl_wait();
     const Place at = place_of<FORM, false>(p.cu_q, p.n_seqs, blockIdx.x);
     if (at.s < 0) return;
-    if (FORM == CM_CONST && p.state_slots[at.s] < 0) return;
-    const int q_beg = p.cu_q[at.s], t0 = q_beg + at.chunk * C, n = min(C, p.cu_q[at.s + 1] - t0);
+    const int slot = p.state_slots[at.s];
+    if (FORM == CM_CONST && slot < 0) return;
+    const int q_beg = p.cu_q[at.s], q_end = p.cu_q[at.s + 1], t0 = q_beg + at.chunk * C, n = min(C, q_end - t0);
     Rows<T, NT, D> keys;
     Rows<T, 3, EB> values;
     const T* vp = static_cast<const T*>(p.v) + (size_t)t0 * p.ldv + (size_t)h * p.E;
     keys.ask(static_cast<const T*>(p.k) + (size_t)t0 * p.ldk + (size_t)h * D, p.ldk, n);
     values.ask(vp, p.ldv, n);
     make_weights<FORM>(w, p, h, t0, n);
+    bool odd = keys.odd(n);
     keys.put(Ks, n, p.silu, nullptr);
+    {
+        Rows<T, NT, D> queries;
+        queries.ask(static_cast<const T*>(p.q) + (size_t)t0 * p.ldq + (size_t)h * D, p.ldq, n);
+        if (slot >= 0) {
+            const float* Sg = p.state + (size_t)slot * p.state_ld;
+            const int DE = D * p.E, step = ceil_div(q_end - q_beg, C) * THREADS;
+            for (int i0 = at.chunk * THREADS + tid; i0 < p.entries; i0 += 16 * step) {       // sixteen asked for at once
+                float x[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    const int i = i0 + u * step;
+                    x[u] = i < p.entries ? Sg[i < DE ? (size_t)h * DE + i : (size_t)p.H * DE + (size_t)h * D + (i - DE)] : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 16; ++u) odd |= odd_value(x[u]);
+            }
+        }
+        odd |= queries.odd(n);
+    }
     __syncthreads();
+    odd |= weights_odd<FORM>(w, n);
     if (tid < C) wj[tid] = tid < n ? weight<FORM>(w, n - 1, tid) : 0.f;
     float* dst = p.scratch + ((size_t)blockIdx.x * p.H + h) * p.entries;
     if (tid == 0) p.decays()[(size_t)blockIdx.x * p.H + h] = from_start<FORM>(w, n - 1);
@@ -316,6 +372,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_local_kernel(Params p
     const int d0 = 16 * (warp % ROW_WARPS), e_warp = (warp / ROW_WARPS) * (N8 * 8);
     for (int e0 = 0; e0 < p.E; e0 += EB) {
         if (e0 > 0) __syncthreads();            // the columns before are used
+        odd |= values.odd(n);
         values.put(Vs, n, p.silu, wj);
         __syncthreads();
         if (e0 + EB < p.E) values.ask(vp + e0 + EB, p.ldv, n);
@@ -352,6 +409,8 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_memory_local_kernel(Params p
         }
         dst[(size_t)D * p.E + tid] = s;
     }
+    const int any = __syncthreads_or(odd);
+    if (tid == 0) p.chunk_odd()[(size_t)blockIdx.x * p.H + h] = any;
 }
 
 // ----------------------------------------------------------------------------------------------------------------- scan
@@ -389,6 +448,11 @@ __global__ void __launch_bounds__(THREADS) chunk_memory_scan_kernel(Params p) {
             }
         };
         ask(0);
+        bool any = false;
+        for (int c = threadIdx.x & 31; c < count; c += 32) any |= p.chunk_odd()[(size_t)(seq.base + c) * p.H + h] != 0;
+        any = __any_sync(0xffffffffu, any);
+        if (part == 0 && threadIdx.x == 0) p.odd()[(size_t)s * p.H + h] = any;
+        if (any) continue;
         for (int c0 = 0; c0 < count; c0 += 8) {
             if (c0 > 0) ask(c0);
 #pragma unroll
@@ -426,6 +490,7 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
     pdl_wait();
     const Place at = place_of<FORM, false>(p.cu_q, p.n_seqs, blockIdx.x);
     if (at.s < 0 || (FORM == CM_CONST && p.state_slots[at.s] < 0)) return;
+    const int left = p.odd()[(size_t)at.s * p.H + h];
     const int q_beg = p.cu_q[at.s], t0 = q_beg + at.chunk * C, n = min(C, p.cu_q[at.s + 1] - t0);
     const float* before = p.scratch + ((size_t)blockIdx.x * p.H + h) * p.entries;
     // the state's entries of 64 columns, float4 a thread and turn: asked for early, put down where the keys were
@@ -446,6 +511,7 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
         keys.ask(static_cast<const T*>(p.k) + (size_t)t0 * p.ldk + (size_t)h * D, p.ldk, n);
         values.ask(vp, p.ldv, n);
         ask(0);
+        if (left) return;                       // (all threads of the block)
         make_weights<FORM>(w, p, h, t0, n);
         queries.put(Qs, n, p.silu, nullptr);
         keys.put(Ks, n, p.silu, nullptr);

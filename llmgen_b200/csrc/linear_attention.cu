@@ -54,7 +54,7 @@ struct LinAttnParams {
     // empty state; `seg_state` [segments of all sequences][heads][dim][vdim] receives each segment's end state
     int segments, n_seqs;
     float* seg_state;
-    int in_chunks;              // != 0: sequences of more tokens than chunk_memory leaves were taken in chunks
+    const int* odd;             // sequences taken in chunks are skipped (chunk_memory::taken); null: none were
 };
 
 constexpr int LA_SEG = 256;     // tokens per segment (a multiple of the chunk)
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(LA_WARPS * 32) linear_attention_kernel(LinAttn
     pdl_wait();
     const int slot = p.state_slots[s];
     int t_beg = p.cu_q[s], n_tok = p.cu_q[s + 1] - t_beg;
-    if (slot < 0 || n_tok <= 0 || (p.in_chunks && n_tok > chunk_memory::few_of(chunk_memory::CM_CONST))) return;
+    if (slot < 0 || n_tok <= 0 || chunk_memory::taken<chunk_memory::CM_CONST>(p.odd, n_tok, s, h, p.heads)) return;
     float* Sg = p.state + (((size_t)slot * p.heads + h) * D) * E;
     const bool local = p.segments > 1;      // this block runs one segment from an empty state
     if (local) {
@@ -447,7 +447,7 @@ LLMK_EXPORT int llmk_linear_attention(float* out, const void* q, const void* k, 
     p.n_seqs = n_seqs;
     p.segments = most > LA_SEG ? ceil_div(most, LA_SEG) : 1;
     p.seg_state = scratch;
-    p.in_chunks = 0;
+    p.odd = nullptr;
     const int vsplits = ceil_div(vdim, LA_EV);
     if (most > chunk_memory::few_of(chunk_memory::CM_CONST) && scratch && scratch_floats >= chunk_memory::scratch_floats(chunk_memory::CM_CONST, n_tokens, n_seqs, heads, dim, vdim)) {
         chunk_memory::Params c = {};
@@ -460,7 +460,7 @@ LLMK_EXPORT int llmk_linear_attention(float* out, const void* q, const void* k, 
                                              : chunk_memory::launch<bf16, chunk_memory::CM_CONST>(c, (cudaStream_t)stream);
             if (rc != LLMK_OK) return rc;
             *launches = 3;
-            p.in_chunks = 1;
+            p.odd = c.odd();
             p.segments = 1;
         }
     }

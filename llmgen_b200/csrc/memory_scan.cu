@@ -325,7 +325,7 @@ struct ScanParams {
     int H, D, E;
     float r_scale, den_eps;
     int* tickets;             // mlstm: [n_seqs, H], zero before and after: how many of a head's blocks are through with its n
-    int in_chunks;            // != 0: sequences of more tokens than chunk_memory leaves were taken in chunks
+    const int* odd;           // sequences taken in chunks are skipped (chunk_memory::taken); null: none were
 };
 
 // A value's bits in a 32-bit register (a 16-bit load extends into one by itself), and back.
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(LANES* CT) memory_scan_kernel(ScanParams p) {
     pdl_launch_dependents();
     pdl_wait();
     const int q_beg = p.cu_q[s], n = p.cu_q[s + 1] - q_beg;
-    if (n <= 0 || (FORM == FORM_MLSTM && p.in_chunks && n > chunk_memory::few_of(chunk_memory::CM_MAX))) return;
+    if (n <= 0 || (FORM == FORM_MLSTM && chunk_memory::taken<chunk_memory::CM_MAX>(p.odd, n, s, h, H))) return;
     const int slot = p.state_slots[s];
     float* Sg = slot >= 0 ? p.state + (size_t)slot * p.state_ld + (size_t)h * D * E : nullptr;
     float* ng = (slot >= 0 && FORM == FORM_MLSTM) ? p.state + (size_t)slot * p.state_ld + (size_t)H * D * E + (size_t)h * D : nullptr;
@@ -677,7 +677,7 @@ LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const
     p.out = out; p.r = r; p.k = k; p.v = v; p.ldr = ldr; p.ldk = ldk; p.ldv = ldv; p.aux = aux; p.dots = dots; p.state = state;
     p.state_ld = state_ld; p.cu_q = cu_q; p.state_slots = state_slots; p.H = H; p.D = D; p.E = E; p.r_scale = r_scale; p.den_eps = den_eps; p.tickets = tickets;
     cudaStream_t st = (cudaStream_t)stream;
-    p.in_chunks = 0;
+    p.odd = nullptr;
     if (scratch && (longest <= 0 || longest > chunk_memory::few_of(chunk_memory::CM_MAX)) && llmk_memory_scan_scratch_floats(n_tokens, n_seqs, H, D, E, form) > 0) {
         chunk_memory::Params c = {};
         c.q = r; c.k = k; c.v = v; c.ldq = ldr; c.ldk = ldk; c.ldv = ldv; c.out = out; c.state = state; c.state_ld = state_ld;
@@ -688,7 +688,7 @@ LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const
             const int rc = dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_MAX>(c, st) : chunk_memory::launch<bf16, chunk_memory::CM_MAX>(c, st);
             if (rc != LLMK_OK) return rc;
             *launches = 3;
-            p.in_chunks = 1;
+            p.odd = c.odd();
         }
     }
     *launches += 1;

@@ -160,3 +160,55 @@ def test_a_workspace_keeps_one_array_for_the_chunks(form):
     held = [b for name, b in workspace._buffers.items() if "chunks" in name]
     assert len(held) == 1 and all(b.numel() < 4096 for b in workspace._retired)
     assert held[0].numel() * 4 <= part.workspace_bytes(1024) and workspace.bytes_held() <= part.workspace_bytes(1024) + ops.SLICED_PRODUCT_BYTES + (1 << 20)
+
+
+def same(a, b):
+    return torch.allclose(a, b, rtol=0, atol=0, equal_nan=True)
+
+
+# what a value of `where` (head 1, sequence 1) is made, at which of its 200 tokens
+ODD = [("v", float("inf"), 70), ("v", float("nan"), 127), ("k", float("-inf"), 10), ("k", float("nan"), 199), ("q", float("inf"), 64), ("q", float("nan"), 130),
+       ("v", 2.9e38, 100), ("state", float("inf"), -1), ("state", float("nan"), -1), ("n", float("inf"), -1), ("f", float("-inf"), 90), ("f", -3e6, 30), ("i", float("-inf"), 77), ("f", float("nan"), 150)]
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("form", [linear, mlstm])
+@pytest.mark.parametrize("where,value,token", ODD)
+def test_what_is_no_ordinary_number_goes_the_way_of_the_walk(where, value, token, form, dtype, monkeypatch):
+    """Infinities, NaN, values beyond what bfloat16 terms hold, gates that close at once: the sequence's head gives what the walk token by token
+    gives, from its own token on and not before, and nothing else changes."""
+    if form is linear and where in ("n", "f", "i"):
+        pytest.skip("gates and n belong to the running maximum")
+    lens = [100, 200, 30, 130]
+    x, state = rows(sum(lens), dtype), fresh(form, len(lens))
+    clean_state = state.clone()
+    clean = form(x, clean_state, lens)
+    x = x.clone()
+    if where in ("q", "k", "v"):
+        x[100 + token, {"q": 0, "k": H * D, "v": 2 * H * D}[where] + D + 5] = value
+    elif where == "state":
+        state.view(len(lens), -1)[1, D * E + 3 * E + 7] = value
+    elif where == "n":
+        state[1, H * D * E + D + 4] = value
+    elif where in ("f", "i"):
+        def gates_with(gates, *args, _inner=ops.mlstm_gates, **kwargs):
+            _inner(gates, *args, **kwargs)
+            row = (100 if len(gates) == sum(lens) else 0) + token
+            gates.view(len(gates), H, 4)[row, 1, 1 if where == "f" else 0] = value
+        monkeypatch.setattr(ops, "mlstm_gates", gates_with)
+    alone = state[1:2].clone()
+    out, walk = form(x, state, lens), form(x[100:300], alone, [200], scratch=False)
+    at = slice(E, 2 * E)
+    assert same(out[100:300, at], walk[:, at])
+    entries = torch.zeros(SIZE if form is mlstm else H * D * E, dtype=torch.bool, device=DEV)
+    entries[D * E:2 * D * E] = True
+    if form is mlstm:
+        entries[H * D * E + D:H * D * E + 2 * D] = True
+        entries[H * D * E + H * D:] = state.view(len(lens), -1)[1, H * D * E + H * D:] == alone[0, H * D * E + H * D:]      # (m is the gates' kernel's)
+    assert same(state.view(len(lens), -1)[1][entries], alone.view(-1)[entries])
+    assert bool(torch.isfinite(out[100:100 + max(token, 0), at]).all()) and (where not in ("q", "k", "v") or abs(value) < 1e39 or not bool(torch.isfinite(out[100 + token, at]).all()))
+    out[100:300, at] = clean[100:300, at]
+    assert same(out, clean)
+    others = ~entries if form is linear else ~entries & (torch.arange(SIZE, device=DEV) < H * D * E + H * D)
+    assert same(state.view(len(lens), -1)[1][others], clean_state.view(len(lens), -1)[1][others])
+    assert same(state[[0, 2, 3]], clean_state[[0, 2, 3]])
