@@ -109,7 +109,7 @@ __device__ __forceinline__ void score_and_pick(size_t t, float* s, float* by, fl
         }
 }
 
-// The warps share the experts (a warp per dot product, float32 sums in a fixed order), then a warp scores and picks for a
+// The warps share the experts (a warp per dot product, float32 sums in a fixed order, which is the same for any number of tokens), then a warp scores and picks for a
 // token.  scoring 0: sigmoid, 1: softmax over all experts, 2: the logits themselves choose, and the weights
 // are the softmax over the chosen logits.
 // TOK tokens per block: a prompt's rows share what a block reads of the router; steps of a few tokens take a token a block
@@ -173,103 +173,110 @@ __global__ void __launch_bounds__(TOK > 1 ? 256 : 1024) moe_route_kernel(const T
 }
 
 // Prompts: sixteen tokens and 32 experts at a time a block, so that a value of the router is read once for sixteen tokens.  Rows and router are staged in
-// shared memory as float32, 256 values of K at a time, the next ones on their way while these are used; the eight warps share each 256 (32 apiece), and
-// a warp's lanes have 4 tokens x 4 experts each, whose vectors lie in different banks.  The warps' sums are added up in their order.  What bounds it: the
-// float32 multiply-adds.  2,048 tokens, 32 experts, width 2,048: 46 us (four tokens a block, every block reading the whole router: 134 MB through L2) ->
-// 24 us; lanes as experts that read their rows of the router from global memory: 36.
-constexpr int RT_TOK = 16, RT_EXP = 32, RT_WARPS = 8, RT_KC = 256, RT_LD = RT_KC + 4;
+// shared memory, 256 values of K at a time in a ring of three.  A warp has 8 tokens x 8 experts, its lanes
+// share K as a warp of the kernel above does: lane l multiplies values 4 l .. 4 l + 3 of each 128 in their order, and the lanes' sums are added up in pairs 16,
+// 8, 4, 2 and 1 lanes apart.  A token's scores, and the experts that a close call chooses, therefore do not depend on how many
+// tokens share its step.  What bounds it: the
+// float32 multiply-adds and their reads of shared memory, by about the same.  2,048 tokens, 32 experts, width 2,048: 36.0 us (four tokens a block, every block
+// reading the whole router: 134 MB through L2) -> 17.6.
+constexpr int RT_TOK = 16, RT_EXP = 32, RT_WARPS = 8, RT_KC = 256, RT_SUB = 8, RT_STAGES = 3;
+constexpr size_t rt_stage_bytes(int elem) { return (size_t)RT_TOK * RT_KC * elem + (size_t)RT_EXP * RT_KC * sizeof(float); }
+// One round: a lane's 2 M sums are added to those of the lane `apart` away, and each lane of the pair keeps half of them.
+template <int M>
+__device__ __forceinline__ void pair_sums(float (&v)[RT_SUB * RT_SUB], int lane, int apart) {
+    const bool upper = lane & apart;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+        const float give = upper ? v[i] : v[M + i], keep = upper ? v[M + i] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, apart);
+    }
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ float4 four_values(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 four_values(const bf16* p) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
+}
 template <typename T>
 __global__ void __launch_bounds__(RT_WARPS * 32) moe_route_rows_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ wr,
                                                                        const float* __restrict__ bias, int* __restrict__ slot_expert,
                                                                        float* __restrict__ slot_weight, int n_tokens, int K, int E, int top, int scoring,
                                                                        int renorm, const float* __restrict__ choice_bias, float weight_scale,
                                                                        float sum_eps, int groups, int keep, float* __restrict__ gate_out) {
-    // [2][RT_TOK + RT_EXP][RT_LD] rows and router, [RT_WARPS][RT_TOK][33] the warps' sums, [RT_TOK][NE] scores, [RT_TOK][NE] what chooses, [RT_TOK][groups]
+    // [RT_STAGES] of router [RT_EXP][RT_KC] and rows [RT_TOK][RT_KC], [RT_TOK][NE] scores, [RT_TOK][NE] what chooses, [RT_TOK][groups]
     extern __shared__ __align__(16) float sm[];
-    constexpr int STAGE = (RT_TOK + RT_EXP) * RT_LD, VN = Vec16<T>::N, XV = RT_TOK * RT_KC / VN / (RT_WARPS * 32);
+    constexpr int STAGE = (int)(rt_stage_bytes(sizeof(T)) / sizeof(float)), VN = Vec16<T>::N;
+    static_assert(RT_WARPS * RT_SUB * RT_SUB == RT_TOK * RT_EXP && RT_KC % 128 == 0, "a warp's share of a block's outputs");
     const int NE = E + (gate_out ? 1 : 0);
     const bool apart = choice_bias || groups > 1;
-    float* part = sm + 2 * STAGE;
-    float* scores = part + RT_WARPS * RT_TOK * 33;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tg = lane >> 3, eg = lane & 7;
+    float* scores = sm + RT_STAGES * STAGE;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i0 = RT_SUB * (warp % (RT_TOK / RT_SUB)), j0 = RT_SUB * (warp / (RT_TOK / RT_SUB));      // the warp's tokens and experts of the block's
     const int t0 = blockIdx.x * RT_TOK, n = min(RT_TOK, n_tokens - t0);
     const int chunks = ceil_div(K, RT_KC);
     pdl_launch_dependents();
     pdl_wait();
     for (int e0 = 0; e0 < NE; e0 += RT_EXP) {
-        Vec16<T> held[XV];
         auto ask = [&](int c) {
-            const int k0 = c * RT_KC, kc = min(RT_KC, K - k0);
-            float* ws = sm + (c & 1) * STAGE + RT_TOK * RT_LD;
-            for (int idx = tid; idx < RT_EXP * RT_KC / 4; idx += RT_WARPS * 32) {
-                const int e = idx / (RT_KC / 4), k = idx % (RT_KC / 4) * 4;
-                if (k < kc) {
-                    const uint32_t d = (uint32_t)__cvta_generic_to_shared(ws + e * RT_LD + k);
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(wr + (size_t)min(e0 + e, NE - 1) * K + k0 + k) : "memory");
+            if (c < chunks) {
+                const int k0 = c * RT_KC, kc = min(RT_KC, K - k0);
+                float* ws = sm + (c % RT_STAGES) * STAGE;
+                T* xs = reinterpret_cast<T*>(ws + RT_EXP * RT_KC);
+                for (int idx = tid; idx < RT_EXP * RT_KC / 4; idx += RT_WARPS * 32) {
+                    const int e = idx / (RT_KC / 4), k = idx % (RT_KC / 4) * 4;
+                    if (k < kc) cp_async16(ws + e * RT_KC + k, wr + (size_t)min(e0 + e, NE - 1) * K + k0 + k);
+                }
+                for (int idx = tid; idx < RT_TOK * RT_KC / VN; idx += RT_WARPS * 32) {      // (rows beyond the step's are not written and not used)
+                    const int i = idx / (RT_KC / VN), k = idx % (RT_KC / VN) * VN;
+                    if (i < n && k < kc) cp_async16(xs + i * RT_KC + k, h + (size_t)(t0 + i) * ldh + k0 + k);
                 }
             }
-#pragma unroll
-            for (int u = 0; u < XV; ++u) {
-                const int idx = tid + u * RT_WARPS * 32, i = idx / (RT_KC / VN), k = idx % (RT_KC / VN) * VN;
-                if (i < n && k < kc) held[u].raw = *reinterpret_cast<const decltype(held[u].raw)*>(h + (size_t)(t0 + i) * ldh + k0 + k);
-            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        float acc[4][4];
+        float acc[RT_SUB * RT_SUB];         // [token][expert]
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-        ask(0);
+        for (int u = 0; u < RT_SUB * RT_SUB; ++u) acc[u] = 0.f;
+        for (int c = 0; c < RT_STAGES - 1; ++c) ask(c);
         for (int c = 0; c < chunks; ++c) {
             const int kc = min(RT_KC, K - c * RT_KC);
-            float* xs = sm + (c & 1) * STAGE;
-            const float* ws = xs + RT_TOK * RT_LD;
-#pragma unroll
-            for (int u = 0; u < XV; ++u) {
-                const int idx = tid + u * RT_WARPS * 32, i = idx / (RT_KC / VN), k = idx % (RT_KC / VN) * VN;
-                float f[VN];
-#pragma unroll
-                for (int q = 0; q < VN; ++q) f[q] = 0.f;
-                if (i < n && k < kc) held[u].unpack(f);
-#pragma unroll
-                for (int q = 0; q < VN; q += 4) *reinterpret_cast<float4*>(xs + i * RT_LD + k + q) = make_float4(f[q], f[q + 1], f[q + 2], f[q + 3]);
-            }
-            asm volatile("cp.async.wait_all;" ::: "memory");
+            const float* ws = sm + (c % RT_STAGES) * STAGE;
+            const T* xs = reinterpret_cast<const T*>(ws + RT_EXP * RT_KC);
+            asm volatile("cp.async.wait_group %0;" ::"n"(RT_STAGES - 2) : "memory");
             __syncthreads();                        // this chunk is there, and the one before is used by every warp
-            if (c + 1 < chunks) ask(c + 1);
-            const int k_end = min(kc, (warp + 1) * (RT_KC / RT_WARPS));
-#pragma unroll 2
-            for (int k = warp * (RT_KC / RT_WARPS); k < k_end; k += 4) {
-                float4 x[4], w[4];
+            ask(c + RT_STAGES - 1);
+            for (int k = 4 * lane; k < kc; k += 128) {
+                float4 w[RT_SUB];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(xs + (tg + 4 * i) * RT_LD + k);
+                for (int j = 0; j < RT_SUB; ++j) w[j] = *reinterpret_cast<const float4*>(ws + (j0 + j) * RT_KC + k);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4*>(ws + (eg + 8 * j) * RT_LD + k);
+                for (int i = 0; i < RT_SUB; ++i) {
+                    const float4 x = four_values(xs + (i0 + i) * RT_KC + k);
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        acc[i][j] = fmaf(x[i].x, w[j].x, acc[i][j]);
-                        acc[i][j] = fmaf(x[i].y, w[j].y, acc[i][j]);
-                        acc[i][j] = fmaf(x[i].z, w[j].z, acc[i][j]);
-                        acc[i][j] = fmaf(x[i].w, w[j].w, acc[i][j]);
+                    for (int j = 0; j < RT_SUB; ++j) {
+                        float& a = acc[i * RT_SUB + j];
+                        a = fmaf(x.x, w[j].x, a);
+                        a = fmaf(x.y, w[j].y, a);
+                        a = fmaf(x.z, w[j].z, a);
+                        a = fmaf(x.w, w[j].w, a);
                     }
+                }
             }
         }
+        // each round leaves half of the outputs to each lane of a pair; lane l ends with outputs 2 l and 2 l + 1
+        __syncwarp();
+        pair_sums<32>(acc, lane, 16);
+        pair_sums<16>(acc, lane, 8);
+        pair_sums<8>(acc, lane, 4);
+        pair_sums<4>(acc, lane, 2);
+        pair_sums<2>(acc, lane, 1);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) part[(warp * RT_TOK + tg + 4 * i) * 33 + eg + 8 * j] = acc[i][j];
-        __syncthreads();
-        for (int idx = tid; idx < RT_TOK * RT_EXP; idx += RT_WARPS * 32) {
-            const int i = idx / RT_EXP, o = e0 + idx % RT_EXP;
-            if (o >= NE) continue;
-            float v = 0.f;
-#pragma unroll
-            for (int u = 0; u < RT_WARPS; ++u) v += part[(u * RT_TOK + i) * 33 + idx % RT_EXP];
-            scores[i * NE + o] = v + (bias && o < E ? bias[o] : 0.f);
+        for (int u = 0; u < 2; ++u) {
+            const int at = 2 * lane + u, i = i0 + at / RT_SUB, o = e0 + j0 + at % RT_SUB;
+            if (o < NE) scores[i * NE + o] = acc[u] + (bias && o < E ? bias[o] : 0.f);
         }
-        __syncthreads();                            // (also: the staging and the sums may be written again)
+        __syncthreads();                            // (also: the staging may be written again)
     }
     for (int i = warp; i < n; i += RT_WARPS) {
         float* s = scores + i * NE;
@@ -304,19 +311,24 @@ LLMK_EXPORT int llmk_moe_route(const void* h, long long ldh, const float* wr, co
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e;
     // prompts: sixteen tokens a block where that gives three eighths of the SMs one, rows of whole vectors.  32 experts, us, four tokens a
-    // block -> sixteen: width 512, 600 tokens 12.3 -> 13.9, 900 15.6 -> 14.5, 2,048 18.4 -> 15.5; width 2,048, 600 tokens 29.6 -> 25.5, 900 38.2 ->
-    // 26.6, 2,048 43.1 -> 27.4; width 4,096, 900 55.9 -> 41.2, 2,048 97.2 -> 42.6
-    const size_t rows_smem = ((size_t)2 * (RT_TOK + RT_EXP) * RT_LD + RT_WARPS * RT_TOK * 33 + (size_t)RT_TOK * (2 * outputs + groups)) * sizeof(float);
+    // block -> sixteen: width 512, 900 tokens 13.0 -> 8.8, 2,048 14.3 -> 8.9; width 2,048, 900 32.4 -> 17.3, 2,048 36.0 -> 17.6; width 4,096,
+    // 900 52.3 -> 28.8, 2,048 93.7 -> 28.9.  A block by itself takes as long for a few tokens as for sixteen times as many blocks (17 us at width 2,048).
+    const size_t rows_smem = RT_STAGES * rt_stage_bytes(dtype == LLMK_F32 ? 4 : 2) + (size_t)RT_TOK * (2 * outputs + groups) * sizeof(float);
     const int vec = dtype == LLMK_F32 ? 4 : 8;
     if ((dtype == LLMK_F32 || dtype == LLMK_BF16) && n_tokens >= RT_TOK * device_sm_count() * 3 / 8 && K % vec == 0 && ldh % vec == 0 && host_aligned16(h) &&
         host_aligned16(wr) && rows_smem <= 200 * 1024) {
         const dim3 rgrid(ceil_div(n_tokens, RT_TOK)), rblock(RT_WARPS * 32);
+        static bool configured = false;
+        if (!configured) {
+            e = cudaFuncSetAttribute(moe_route_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(moe_route_rows_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            if (e != cudaSuccess) LLMK_FAIL("moe_route: cannot raise shared memory: %s", cudaGetErrorString(e));
+            configured = true;
+        }
         if (dtype == LLMK_F32) {
-            cudaFuncSetAttribute(moe_route_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
             e = llmk_launch(moe_route_rows_kernel<float>, rgrid, rblock, rows_smem, s, pdl != 0, (const float*)h, ldh, wr, bias, slot_expert, slot_weight, n_tokens, K, E,
                             top, scoring, renorm, choice_bias, weight_scale, sum_eps, groups, keep, gate_out);
         } else {
-            cudaFuncSetAttribute(moe_route_rows_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
             e = llmk_launch(moe_route_rows_kernel<bf16>, rgrid, rblock, rows_smem, s, pdl != 0, (const bf16*)h, ldh, wr, bias, slot_expert, slot_weight, n_tokens, K, E,
                             top, scoring, renorm, choice_bias, weight_scale, sum_eps, groups, keep, gate_out);
         }

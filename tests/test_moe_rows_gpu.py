@@ -86,3 +86,23 @@ def test_rows_are_gathered_and_added_up(K, dtype):
         terms = torch.where(pos[:, None] >= 0, rows[pos.clamp(min=0).long()].double() * weight[:n * t].double()[:, None], torch.zeros(1, dtype=torch.float64))
         bound = terms.abs().view(n, t, K).sum(1) * (t + 1) * 2.0 ** -24
         assert bool(((got.cpu().double() - terms.view(n, t, K).sum(1)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("E,K,top,gate,scoring", [(32, 2048, 4, False, "sigmoid"), (33, 1032, 3, True, "softmax"), (8, 72, 2, False, "sigmoid"), (70, 520, 8, True, "sigmoid")])
+def test_a_tokens_experts_do_not_depend_on_how_many_tokens_share_the_step(E, K, top, gate, scoring, dtype):
+    """The same bits whichever kernel takes the step: one token a block, four, sixteen."""
+    n = 1190
+    h, router, bias = rnd((n, K), 1, 1.0, DT[dtype]).to(DEV), rnd((E + int(gate), K), 2, K ** -0.5).to(DEV), rnd((E,), 3).to(DEV)
+
+    def route(rows):
+        m = len(rows)
+        expert, weight, out = torch.full((m, top), -7, dtype=torch.int32, device=DEV), torch.zeros(m, top, device=DEV), torch.zeros(m, device=DEV)
+        ops.moe_route(rows, router, expert.view(-1), weight.view(-1), top, scoring, False, bias=bias, gate_out=out if gate else None)
+        return expert, weight, out
+    whole = route(h)
+    for size in (1, 37, 601):
+        parts = [route(h[i:i + size]) for i in range(0, n if size > 1 else 20, size)]
+        for got, want in zip(zip(*parts), whole):
+            got = torch.cat(got)
+            assert torch.equal(got, want[:len(got)])
