@@ -625,10 +625,10 @@ def attention_mma(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vcac
     _check_sinks("attention_mma", sink, sink_values, nq)
     _check_k_scale("attention_mma", k_scale, kcache, vcache)
     tcos, tsin = _check_turn("attention_mma", turn_back, ctx_len, vd, gate, gate_per_head, nq)
-    if (q.shape[0] > 128 and nq <= 65535 and window <= 0 and softcap <= 0.0 and chunk <= 0 and tcos is None and k_scale is None and vcache is not None
+    if (q.shape[0] > 128 and scale > 0.0 and nq <= 65535 and window <= 0 and softcap <= 0.0 and chunk <= 0 and tcos is None and k_scale is None and vcache is not None
             and _row_stride(q) % 8 == 0 and _row_stride(out) % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in (q, out, kcache, vcache))
             and (gate is None or gate_per_head or (_row_stride(gate) % 8 == 0 and gate.data_ptr() % 16 == 0)) and n_tiles <= 65535):
-        # Plain causal attention (with a sink or a gate at most) goes to the 5th-generation tensor cores where the widths fit.  16 heads on 8, pages
+        # Plain causal attention (with a sink or a gate at most, a positive scale) goes to the 5th-generation tensor cores where the widths fit.  16 heads on 8, pages
         # of 16, mma.sync -> tcgen05: a prompt of 2,048 223.8 -> 65.3 us, of 512 41.9 -> 19.8, of 300 29.1 -> 15.5, 1,024 behind 3,000 keys 292.6 -> 117.  A
         # prompt of up to 128 tokens is one tile of keys, whose set-up costs more than it saves (64: 12.1 -> 13.5): those stay.
         tc = build.load("attention_tc")

@@ -1,0 +1,60 @@
+"""Causal attention with 32-bit softmax weights on the 5th-generation tensor cores beside the same on `mma.sync` (csrc/attention_mma.cu, which a window wider
+than everything sends a step to): what is no number, scales that are not positive, many keys, and weights of which the last bits decide."""
+import pytest
+import torch
+
+from llmgen_b200.kernels import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+HD, PAGE, WIDE = 128, 16, 1 << 24
+
+
+def rnd(shape, seed, scale=1.0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).to(torch.bfloat16)
+
+
+def ints(values):
+    return torch.tensor(values, dtype=torch.int32, device=DEV)
+
+
+def attend(q, ks, vs, news, window=0, scale=HD ** -0.5):
+    """q [tokens, heads, HD] of sequences with keys ks[s], values vs[s] [ctx, kv heads, HD] and news[s] new tokens."""
+    T, nq, nkv = q.shape[0], q.shape[1], ks[0].shape[1]
+    blocks = [-(-len(k) // PAGE) for k in ks]
+    most = max(blocks)
+    kc, vc = (torch.zeros(sum(blocks), nkv, PAGE, HD, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    bt, at, tiles, cu = torch.zeros(len(ks), most, dtype=torch.int32), 0, [], [0]
+    for s, (k, v, n, m) in enumerate(zip(ks, vs, news, blocks)):
+        bt[s, :m] = torch.arange(at, at + m, dtype=torch.int32)
+        for cache, x in ((kc, k), (vc, v)):
+            padded = torch.zeros(m * PAGE, nkv, HD, dtype=torch.bfloat16)
+            padded[:len(x)] = x
+            cache[at:at + m] = padded.view(m, PAGE, nkv, HD).transpose(1, 2).to(DEV)
+        at += m
+        tiles += [(s, q0) for q0 in range(0, n, 64)]
+        cu.append(cu[-1] + n)
+    out = torch.full((T, nq * HD), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.attention_mma(out, q.reshape(T, nq * HD).to(DEV), kc, vc, bt.to(DEV), most, ints([len(k) for k in ks]), ints(cu), ints([t[0] for t in tiles]),
+                      ints([t[1] for t in tiles]), len(tiles), nq, nkv, HD, HD, PAGE, window, scale)
+    torch.cuda.synchronize()
+    ops.check_tc_errors(out.device)
+    return out.view(T, nq, HD)
+
+
+def plain(q, k, v, scale=HD ** -0.5):
+    """One sequence in float64, its last len(q) tokens."""
+    n, ctx, group = len(q), len(k), q.shape[1] // k.shape[1]
+    k, v = (x.double().repeat_interleave(group, 1) for x in (k, v))
+    z = torch.einsum("thd,jhd->htj", q.double(), k) * scale
+    z = z.masked_fill((torch.arange(ctx)[None, :] > torch.arange(ctx - n, ctx)[:, None])[None], float("-inf"))
+    return torch.einsum("htj,jhd->thd", torch.softmax(z, 2), v)
+
+
+@pytest.mark.parametrize("scale", [-0.09, 0.0])
+def test_a_scale_that_is_not_positive(scale):
+    """Scores of up to a hundred either way: against the largest product instead of the largest score the powers would overflow."""
+    q, k, v = rnd((200, 4, HD), 1, 24.0), rnd((300, 2, HD), 2), rnd((300, 2, HD), 3)
+    got, want = attend(q, [k], [v], [200], scale=scale).cpu().double(), plain(q, k, v, scale)
+    # one rounding to bfloat16 (2^-8 of the value at most), and before it float32 sums: 300 terms, scores of 128 products each, as good as 128 2^-24 of the sum of their magnitudes
+    assert bool(((got - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -24 * (300 + 128 * 0.09 * 4.5 * float(q.double().abs().sum(2).max())) * 4.5).all())
