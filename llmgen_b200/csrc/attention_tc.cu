@@ -454,6 +454,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const float l_row = l + xchg[(half ^ 1) * BM + r];
         const bool writes = ok && qi < max(nq_tile, 0) && (chunk * p.gc + r % p.gc) < G;
         float inv = (row_valid && l_row > 0.f) ? 1.0f / l_row : 0.f;
+        if (TERMS > 1 && row_valid && l_row != l_row) inv = l_row;      // a score that is no number: its row is none
         const bf16* gate = nullptr;
         if constexpr (TERMS > 1) {
             if (p.sink && inv > 0.f) {
@@ -487,7 +488,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 for (int i = 0; i < 32; i += 8) {
                     float f[8];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) f[e] = inv > 0.f ? __uint_as_float(acc[i + e]) * inv : 0.f;
+                    for (int e = 0; e < 8; ++e) f[e] = (inv > 0.f || (TERMS > 1 && inv != inv)) ? __uint_as_float(acc[i + e]) * inv : 0.f;
                     if (TERMS > 1 && gate) {
                         float gv[8];
                         Vec16<bf16> gk;

@@ -58,3 +58,23 @@ def test_a_scale_that_is_not_positive(scale):
     got, want = attend(q, [k], [v], [200], scale=scale).cpu().double(), plain(q, k, v, scale)
     # one rounding to bfloat16 (2^-8 of the value at most), and before it float32 sums: 300 terms, scores of 128 products each, as good as 128 2^-24 of the sum of their magnitudes
     assert bool(((got - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -24 * (300 + 128 * 0.09 * 4.5 * float(q.double().abs().sum(2).max())) * 4.5).all())
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_what_is_no_number_stays_visible(value):
+    q, k, v = rnd((300, 4, HD), 1), rnd((300, 2, HD), 2), rnd((300, 2, HD), 3)
+    clean = attend(q, [k], [v], [300])
+    bad = q.clone()
+    bad[150, 1, 7] = value
+    for window in (0, WIDE):
+        out = attend(bad, [k], [v], [300], window=window)
+        assert bool(torch.isnan(out[150, 1]).all())                      # its own row and head
+    out = attend(bad, [k], [v], [300])
+    out[150, 1] = clean[150, 1]
+    assert torch.equal(out, clean)                                       # and no other
+    bad = k.clone()
+    bad[100, 0, 7] = float("nan")
+    out = attend(q, [bad], [v], [300])
+    assert bool(torch.isnan(out[100:, :2]).all())                        # every row that sees the key, in the heads that read it
+    out[100:, :2] = clean[100:, :2]
+    assert torch.equal(out, clean)
