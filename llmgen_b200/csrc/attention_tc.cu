@@ -26,8 +26,11 @@
 // Statistics (m, l), the accumulator and the final division are float32.
 //
 // TERMS = 3 (`llmk_attention_tc_terms`): softmax weights that stay 32-bit.  A weight enters the second product as three bfloat16
-// terms p = p1 + p2 + p3 (24 bits of mantissa), smallest first, so every product with a bfloat16 value is what float32 arithmetic
-// would give.  P takes three arrays, so shared memory holds one buffer of them and one stage of V; pass 2 of a tile waits for the
+// terms p = p1 + p2 + p3 (24 bits of mantissa), so every product with a bfloat16 value is what float32 arithmetic
+// would give.  The tensor cores cut off what an accumulator cannot hold, always towards zero, with every MMA: p1 V has one accumulator, p2 V and p3 V,
+// 2^-8 of it and below, another, so that a tile cuts the large sum 8 times and not 24.  Outputs that round to another bfloat16 than the float64 result
+// does, 256 rows, scores of sigma 4, mma.sync / one accumulator / two: 2,048 keys 0.185 / 0.199 / 0.157 %, 16,384 1.28 / 1.36 / 1.17, 32,768 2.23 / 2.41 / 2.06 (sigma 1:
+// 3.06 / 3.06 / 2.40); the second accumulator costs no time (2,048 tokens 61.5 us).  P takes three arrays, so shared memory holds one buffer of them and one stage of V; pass 2 of a tile waits for the
 // P V of the tile before.  Rows of V behind a sequence's last key are cleared before they are multiplied by weights of zero, so
 // that what another request left there is nothing to this one.  The epilogue takes a sink (one more term in the denominator)
 // and an output gate.  What bounds it is what bounds the other form, and P V of a tile (24 MMAs) before the next tile's pass 2.  16 heads on 8,
@@ -138,7 +141,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     using L = Smem<HD, TERMS>;
     constexpr int HB = HD / 64;                 // 64-wide blocks of the head
     constexpr uint32_t TMEM_COLS = 512;
-    constexpr uint32_t S_COL0 = 0, S_COL1 = BN, O_COL0 = 2 * BN;
+    constexpr uint32_t S_COL0 = 0, S_COL1 = BN, O_COL0 = 2 * BN, REST_COL0 = O_COL0 + HD;      // REST: TERMS 3, O of the smaller terms
+    static_assert(TERMS == 1 || REST_COL0 + HD <= TMEM_COLS, "two accumulators");
     extern __shared__ __align__(1024) uint8_t smem[];
     // A tile whose sequence is -1 is padding of a list of fixed length (a launch shape kept for replay): the
     // block leaves before it sets anything up.  The list is read ahead of `griddepcontrol.wait`: it belongs
@@ -287,12 +291,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 if (!ok) break;
                 tc::tc_fence_after_sync();
 #pragma unroll
-                for (int term = TERMS - 1; term >= 0; --term) {       // smallest terms first
+                for (int term = TERMS - 1; term >= 0; --term) {       // (the smaller terms, smallest first, have an accumulator of their own)
 #pragma unroll
                     for (int kk = 0; kk < BN / 16; ++kk) {
                         const uint64_t da = p_desc[st] + (uint64_t)((term * L::P_BYTES + (kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4);
                         const uint64_t db = v_desc[st] + (uint64_t)((kk * 16 * 128) >> 4);
-                        tc::mma_bf16_ss(tmem_base + O_COL0, da, db, idesc_o, j != 0 || kk != 0 || term != TERMS - 1);   // O adds up in tensor memory over the tiles
+                        // O adds up in tensor memory over the tiles
+                        tc::mma_bf16_ss(tmem_base + (term == 0 ? O_COL0 : REST_COL0), da, db, idesc_o, j != 0 || kk != 0 || (term != 0 && term != TERMS - 1));
                     }
                 }
                 tc::mma_commit(tc::smem_u32(&o_full[st]));
@@ -336,7 +341,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const int st = j & 1;
             const int k0 = kt0 + j * BN + half * SC;      // first key of this thread's columns
             const bool need_mask = (k0 + SC - 1 > qpos) || (k0 <= lo);
-            uint8_t* p_row = p_row0 + (st & (L::BUFFERS - 1)) * L::P_BYTES;       // P is double-buffered: P V of the tile before may still read the other
+            uint8_t* p_row = p_row0 + (st & (L::BUFFERS - 1)) * L::P_BYTES;       // two buffers: P V of the tile before may still read the other; one (TERMS 3): it is waited for below
             // pass 1: the maximum of this thread's half of the row (four independent chains)
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
             if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&s_full[st]), (j >> 1) & 1, abort_flag));
@@ -377,12 +382,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc::tc_fence_after_sync();
                 if (ok && any_fix) {
 #pragma unroll
-                    for (int c = 0; c < OC / 32; ++c) {
+                    for (int c = 0; c < (TERMS > 1 ? 2 : 1) * (OC / 32); ++c) {
+                        const uint32_t at = c < OC / 32 ? o_addr + c * 32 : o_addr + (REST_COL0 - O_COL0) + (c - OC / 32) * 32;
                         uint32_t o[32];
-                        tc::tmem_ld_32x32_wait(o_addr + c * 32, o);
+                        tc::tmem_ld_32x32_wait(at, o);
 #pragma unroll
                         for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                        tc::tmem_st_32x32(o_addr + c * 32, o);
+                        tc::tmem_st_32x32(at, o);
                     }
                     tc::tmem_st_wait();
                 }
@@ -479,6 +485,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             uint32_t acc[32];
             if (ok && n_tiles > 0) {                     // uniform over the warp: the load is a warp's instruction
                 tc::tmem_ld_32x32_wait(o_addr + c * 32, acc);
+                if constexpr (TERMS > 1) {
+                    uint32_t rest[32];
+                    tc::tmem_ld_32x32_wait(o_addr + (REST_COL0 - O_COL0) + c * 32, rest);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) + __uint_as_float(rest[i]));
+                }
             } else {
 #pragma unroll
                 for (int i = 0; i < 32; ++i) acc[i] = 0u;

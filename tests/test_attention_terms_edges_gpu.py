@@ -78,3 +78,13 @@ def test_what_is_no_number_stays_visible(value):
     assert bool(torch.isnan(out[100:, :2]).all())                        # every row that sees the key, in the heads that read it
     out[100:, :2] = clean[100:, :2]
     assert torch.equal(out, clean)
+
+
+@pytest.mark.parametrize("ctx,sharp", [(512, 1.0), (4096, 1.0), (4096, 4.0), (16384, 4.0)])
+def test_many_keys_lose_no_more_than_on_the_other_tensor_path(ctx, sharp):
+    """Values that round to another bfloat16 than the float64 result does: no more of them than `mma.sync` gives, whose sums are float32 too."""
+    n, nq = 200, 4
+    q, k, v = rnd((n, nq, HD), 1, sharp), rnd((ctx, 2, HD), 2), rnd((ctx, 2, HD), 3) + 1
+    want = plain(q, k, v).to(torch.bfloat16)
+    wrong = [int((attend(q, [k], [v], [n], window=window).cpu() != want).sum()) for window in (0, WIDE)]
+    assert wrong[0] <= wrong[1], wrong
