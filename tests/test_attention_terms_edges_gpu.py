@@ -88,3 +88,33 @@ def test_many_keys_lose_no_more_than_on_the_other_tensor_path(ctx, sharp):
     want = plain(q, k, v).to(torch.bfloat16)
     wrong = [int((attend(q, [k], [v], [n], window=window).cpu() != want).sum()) for window in (0, WIDE)]
     assert wrong[0] <= wrong[1], wrong
+
+
+def test_the_last_bits_of_a_weight_count():
+    """Eight keys, seven of them the row's best (weight 1) and one of weight p = exp(-d): values -t1, -t2, 0, .., 1 with t1 + t2 the two leading bfloat16 terms of p
+    leave p - t1 - t2, which weights kept in one or two terms do not have."""
+    seqs, nq, nkv = 40, 4, 2
+    low = 4 - (torch.arange(seqs * nkv).double().view(seqs, nkv) + 7) * 2.0 ** -6              # the weak key's score: a bfloat16 value (4 - d, d up to 1.4)
+    p = torch.exp(low - 4)
+    t1 = p.float().to(torch.bfloat16).double()
+    t2 = (p - t1).float().to(torch.bfloat16).double()
+    ks, vs = [], []
+    for s in range(seqs):
+        k, v = torch.zeros(8, nkv, HD), rnd((8, nkv, HD), s).float()
+        k[:7, :, 0], k[7, :, 0] = 4.0, low[s].float()
+        v[:, :, 5] = 0.0
+        v[0, :, 5], v[1, :, 5], v[7, :, 5] = -t1[s].float(), -t2[s].float(), 1.0
+        assert torch.equal(k.to(torch.bfloat16).float(), k) and torch.equal(v[:2, :, 5].to(torch.bfloat16).float(), v[:2, :, 5])
+        ks.append(k.to(torch.bfloat16)), vs.append(v.to(torch.bfloat16))
+    q = torch.zeros(seqs * 8, nq, HD)
+    q[:, :, 0] = 8.0
+    group = nq // nkv
+    p, left = (x.repeat_interleave(group, 1) for x in (p, p - t1 - t2))
+    # float32: the exponent is a difference of numbers of up to 6 (2^-23 of them each), the power good to 2 units (2^-22), p's own rounding 2^-24; the sums cancel
+    # exactly but for it.  Then one rounding to bfloat16 of the result.
+    bound = left.abs() * 2.0 ** -8 + p * (2 * 6 * 2.0 ** -24 + 2.0 ** -22 + 2.0 ** -24)
+    one, two = (t1 - t1 - t2).repeat_interleave(group, 1), torch.zeros_like(left)
+    assert bool(((one - left).abs() > bound).all()) and float(((two - left).abs() > bound).double().mean()) > 0.25      # what fewer terms give is found
+    for window in (0, WIDE):
+        got = attend(q.to(torch.bfloat16), ks, vs, [8] * seqs, window=window, scale=0.125).cpu().double().view(seqs, 8, nq, HD)[:, 7, :, 5]
+        assert bool(((got * (7 + p) - left).abs() <= bound).all()), float(((got * (7 + p) - left).abs() - bound).max())
