@@ -260,8 +260,8 @@ class GQAAttention(Mixer):
         else:
             self._tiles(builder, self.bq)
 
-    def _split(self, ctx):
-        """(num_parts, part_size) for flash-decoding; only pure-decode steps are split."""
+    def _split(self, ctx, least: int = 32):
+        """(num_parts, part_size) for flash-decoding; only pure-decode steps are split.  `least`: keys that a part has at least."""
         if not ctx.pure_decode:
             return 1, 0
         G = self.nq // self.nkv
@@ -271,9 +271,13 @@ class GQAAttention(Mixer):
         if self.window or self.chunk:
             longest = min(longest, self.window or self.chunk)
         by_sms = (2 * self.sm_count + blocks - 1) // blocks
-        by_len = max(1, longest // 32)      # a part is at least one of the kernel's tiles of 32 keys
-        # under a window (as under a mask in blocks) the kernel cuts the keys a query can see, not the whole context
-        return max(1, min(by_sms, by_len, 64)), 0
+        # under a window (as under a mask in blocks) the kernel cuts the keys a query can see, not the whole context.  Parts of 128 keys, or of
+        # `least` where those are twice as many at least, and then a power of two of them (general kernel, us: 8 sequences on 8 key heads of 500 keys
+        # 4 parts 41.9, 5 43.3, 8 34.5; 4 sequences 4 parts 35.1, 8 24.2, 10 27.2; one sequence 4 parts 32.1, 16 16.6; at 1,500 keys 8
+        # sequences 4 parts 97, 5 85)
+        coarse = max(1, min(by_sms, longest // 128, 64))
+        fine = 1 << (max(1, min(by_sms, longest // least, 64)).bit_length() - 1)
+        return (fine if fine >= 2 * coarse else coarse), 0
 
     def workspace_bytes(self, tokens: int) -> int:
         """Bytes of activations this part keeps in the step's workspace for `tokens` rows: the packed projection
@@ -393,8 +397,10 @@ class GQAAttention(Mixer):
         # single decoded tokens: the keys in parts that are merged afterwards (the sink enters once, in the merge)
         parts, part_size = self._split(ctx)
         if ctx.pure_decode and gate is None and self.mma_tile_queries():
+            parts = self._split(ctx, least=128)[0]
             # in bfloat16 without a gate: the parts of a token's keys are the blocks of a cluster, one an SM (8 sequences of 514 keys
-            # on 4 key heads: 13.8 us with 4 parts, 31.9 with 8, whose blocks do not fit the SMs together)
+            # on 4 key heads: 13.8 us with 4 parts, 31.9 with 8, whose blocks do not fit the SMs together; 4 sequences 11.6 and 17.0, 2 on 8
+            # key heads 11.2 and 16.6, although theirs would)
             blocks = max(1, ctx.n_seqs * self.nkv * ((self.nq // self.nkv + 15) // 16))
             parts = max(1, min(parts, self.sm_count // blocks))
             ops.attention_mma_parts(o, q, cache.k, cache.v, group.block_tables, group.max_blocks, ctx.ctx_len, ctx.cu_q, ctx.n_seqs, self.nq,
@@ -495,8 +501,9 @@ class GQAAttention(Mixer):
                               float(spec.scale), softcap=self.softcap, sink=self.sink, sink_values=self.sink_scores, chunk=self.chunk,
                               k_scale=cache.k_scale)
         elif ctx.pure_decode and self.mma_tile_queries():
-            # single tokens in bfloat16: the parts of a token's keys are the blocks of a cluster
-            parts = min(self._split(ctx)[0], ops.ATTENTION_MMA_MAX_PARTS)
+            # single tokens in bfloat16: the parts of a token's keys are the blocks of a cluster, tiles of 64 keys at least; three fit an SM here (8
+            # sequences on 4 key heads, 4 and 8 parts: 500 keys 11.8 and 10.2 us, 200 keys 9.3 and 10.0; one sequence 10.3 and 8.4)
+            parts = min(self._split(ctx, least=64)[0], ops.ATTENTION_MMA_MAX_PARTS)
             ops.attention_mma_parts(o, q, cache.k, None, group.block_tables, group.max_blocks, ctx.ctx_len, ctx.cu_q, ctx.n_seqs, nq, nk, hd, hd,
                                     cache.page_size, self.window, float(spec.scale), parts, softcap=self.softcap, sink=self.sink,
                                     chunk=self.chunk, sink_values=self.sink_scores, k_scale=cache.k_scale)
