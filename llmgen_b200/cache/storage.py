@@ -68,19 +68,23 @@ class CacheStorage:
                           writes=writes, state=self.state.get(cache_id), k_scale=self.scales.get(cache_id))
 
     def reset_state(self, slots: Sequence[int]) -> None:
-        """Zero the state of slots that were just handed to new requests: a fill per run of neighbouring slots.  (An index array would be
-        copied to the device first, which waits for everything in the stream: 220 us of a prompt's step of 600.)"""
+        """Zero the state of slots that were just handed to new requests: one fill a layer, of neighbouring slots as a slice, of scattered ones by an
+        index array out of pinned memory.  (Out of pageable memory its copy would wait for everything in the stream: 220 us of a prompt's
+        step of 600.)"""
         if not slots or not self.state:
             return
-        runs, order = [], sorted(set(slots))
-        for slot in order:
-            if runs and runs[-1][1] == slot:
-                runs[-1][1] = slot + 1
-            else:
-                runs.append([slot, slot + 1])
-        for t in self.state.values():
-            for first, end in runs:
+        order = sorted(set(slots))
+        first, end = order[0], order[-1] + 1
+        if end - first == len(order):
+            for t in self.state.values():
                 t[first:end].zero_()
+            return
+        idx = torch.tensor(order, dtype=torch.long)
+        device = next(iter(self.state.values())).device
+        if device.type == "cuda":
+            idx = idx.pin_memory().to(device, non_blocking=True)
+        for t in self.state.values():
+            t.index_fill_(0, idx, 0)
 
     def bytes_held(self) -> int:
         n = sum(t.numel() * t.element_size() for kv in self.kv.values() for t in kv if t is not None)

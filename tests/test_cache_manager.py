@@ -156,3 +156,23 @@ def test_fresh_slots_are_zeroed_and_no_others(slots):
     storage.reset_state(slots)
     for t in storage.state.values():
         assert all(float(t[s].abs().sum()) == 0.0 if s in slots else bool((t[s] == 7.0).all()) for s in range(5))
+
+
+def test_scattered_fresh_slots_take_one_fill_a_layer():
+    import torch
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from llmgen_b200.cache.storage import CacheStorage
+    from llmgen_b200.parts.base import StateRequest
+
+    class Fills(TorchDispatchMode):
+        seen = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen += func._schema.name in ("aten::zero_", "aten::fill_", "aten::index_fill_")
+            return func(*args, **(kwargs or {}))
+    layers = 12
+    storage = CacheStorage({}, {i: StateRequest((3,), torch.float32) for i in range(layers)}, {}, [], 16, 40, torch.float32, "cpu")
+    for slots in (list(range(0, 40, 2)), list(range(7, 19))):
+        with Fills() as fills:
+            storage.reset_state(slots)
+        assert fills.seen == layers
