@@ -238,7 +238,8 @@ def attn_prep(qkv, kcache: Optional[torch.Tensor], vcache: Optional[torch.Tensor
 
 # ------------------------------------------------------------------------- matrix products
 def gemm_simt(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, accumulate: bool = False) -> None:
-    """out[M, N] = a[M, K] @ w[N, K]^T on the CUDA cores (float32 multiply-add, fixed k order)."""
+    """out[M, N] = a[M, K] @ w[N, K]^T on the CUDA cores (float32 multiply-add, fixed k order).  Like the other products it may read `w`,
+    a weight, while the kernel launched before it is still running: that kernel must not be what writes `w`."""
     lib = build.load("gemm_simt")
     M, K = a.shape
     N = w.shape[0]
