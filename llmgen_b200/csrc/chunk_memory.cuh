@@ -657,14 +657,18 @@ inline bool usable(const Params& p, int elem) {
 }
 
 template <typename T, int FORM, int D>
-int launch_width(const Params& p, cudaStream_t s) {
+static int launch_width(const Params& p, cudaStream_t s) {
     constexpr int NT = input_terms<T, FORM>();
     const size_t local = (size_t)(NT * C * (D + 8) + 3 * C * LDE) * sizeof(bf16), out = OutLayout<T, FORM, D>::bytes();
     auto k1 = chunk_memory_local_kernel<T, FORM, D>;
     auto k3 = chunk_memory_out_kernel<T, FORM, D>;
-    cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)local);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
-    if (e != cudaSuccess) LLMK_FAIL("chunk_memory: cannot raise shared memory: %s", cudaGetErrorString(e));
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)local);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
+        if (e != cudaSuccess) LLMK_FAIL("chunk_memory: cannot raise shared memory: %s", cudaGetErrorString(e));
+        configured = true;
+    }
     const dim3 grid(p.chunks, p.H);
     const long long items = (long long)p.longs * p.H * ceil_div(p.entries, THREADS);
     const dim3 scan((unsigned)std::min<long long>(items, 8 * device_sm_count()));
@@ -674,7 +678,7 @@ int launch_width(const Params& p, cudaStream_t s) {
     return LLMK_OK;
 }
 template <typename T, int FORM>
-int launch(const Params& p, cudaStream_t s) {
+static int launch(const Params& p, cudaStream_t s) {
     return p.D == 64 ? launch_width<T, FORM, 64>(p, s) : launch_width<T, FORM, 128>(p, s);
 }
 

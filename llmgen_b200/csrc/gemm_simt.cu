@@ -339,12 +339,16 @@ __global__ void __launch_bounds__(TTHREADS, 3) gemm_f32_tile_kernel(GemmF32Param
 }
 
 constexpr size_t F32_SMEM_MAX = 200 * 1024;
-template <typename Kernel>
-static int launch_f32(Kernel kernel, const GemmF32Params& p, int tiles_n, int blocks, int tiles_m, size_t smem, cudaStream_t s) {
-    // one bound for every size of this kernel: launches recorded into graphs keep theirs
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F32_SMEM_MAX);
-    if (e != cudaSuccess) LLMK_FAIL("gemm_simt: cannot raise shared memory to %zu: %s", F32_SMEM_MAX, cudaGetErrorString(e));
-    LLMK_CHECK_LAUNCH_RC("gemm_simt", llmk_launch_cluster(kernel, dim3(tiles_n, blocks, tiles_m), dim3(RWARPS * 32), smem, s, true, (unsigned)blocks, p));
+template <void (*KERNEL)(GemmF32Params)>
+static int launch_f32(const GemmF32Params& p, int tiles_n, int blocks, int tiles_m, size_t smem, cudaStream_t s) {
+    // one bound for every size of this kernel, set once: launches recorded into graphs keep theirs
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F32_SMEM_MAX);
+        if (e != cudaSuccess) LLMK_FAIL("gemm_simt: cannot raise shared memory to %zu: %s", F32_SMEM_MAX, cudaGetErrorString(e));
+        configured = true;
+    }
+    LLMK_CHECK_LAUNCH_RC("gemm_simt", llmk_launch_cluster(KERNEL, dim3(tiles_n, blocks, tiles_m), dim3(RWARPS * 32), smem, s, true, (unsigned)blocks, p));
     return LLMK_OK;
 }
 
@@ -375,7 +379,7 @@ static int launch_rows(GemmF32Params p, cudaStream_t s) {
     }
     if (best == 0) return -1;
     p.per_block = ceil_div(p.groups, best);
-    return launch_f32(gemm_f32_rows_kernel<TM>, p, tiles, best, 1, rows_smem(TM, p.per_block), s);
+    return launch_f32<gemm_f32_rows_kernel<TM>>(p, tiles, best, 1, rows_smem(TM, p.per_block), s);
 }
 
 // More rows: the groups that an SM has to walk, with the cost of filling a ring (and of the exchange) for each of its blocks; one block
@@ -402,7 +406,7 @@ static int launch_tile(GemmF32Params p, cudaStream_t s) {
         }
     }
     p.per_block = ceil_div(p.groups, best);
-    return launch_f32(gemm_f32_tile_kernel<TM, TN>, p, ceil_div(p.N, L::BN_), best, ceil_div(p.M, L::BM), L::RING + (best > 1 ? p.per_block : 1) * part, s);
+    return launch_f32<gemm_f32_tile_kernel<TM, TN>>(p, ceil_div(p.N, L::BN_), best, ceil_div(p.M, L::BM), L::RING + (best > 1 ? p.per_block : 1) * part, s);
 }
 
 static int gemm_f32(void* C, const void* A, const void* W, int M, int N, int K, long long lda, long long ldw, long long ldc,
