@@ -19,8 +19,8 @@
 // six products, 4 M of them), the rest the conversion of what is staged, and the latency of one block an SM.
 //
 // Measured (us, one sequence, 16 heads of 128 x 128, bfloat16 rows, before -> now), and the error against float64 of the rows:
-//   linear attention   2,048 tokens 353 -> 113 (segments of 256 tokens walked 32 at a time on the CUDA cores), 1.9e-7 -> 0.9e-7;  512: 203 -> 44
-//   running maximum    2,048 tokens 1,139 -> 105 with its gates (a walk token by token), 7.4e-7 -> 6.5e-7;  512: 324 -> 42
+//   linear attention   2,048 tokens 353 -> 115 (segments of 256 tokens walked 32 at a time on the CUDA cores), 1.9e-7 -> 0.9e-7;  512: 203 -> 45
+//   running maximum    2,048 tokens 1,139 -> 106 with its gates (a walk token by token), 7.4e-7 -> 6.5e-7;  512: 324 -> 43
 // What a sequence brings decides, not what the step brings: sequences of up to few_of(form) tokens keep the walks (one launch, and no state but the
 // request's own to write), in steps of any size, so that a token's sums do not depend on which other requests share its step.  The walk is
 // launched behind the chunks and skips the sequences that they took.  Walk -> chunks
@@ -154,46 +154,44 @@ __device__ __forceinline__ float act(float x, int silu) { return silu ? __fdivid
 struct Place {
     int s, chunk, base;         // base: number of the sequence's first chunk
 };
+template <int FORM>
+__device__ __forceinline__ int chunks_of(const int* __restrict__ cu_q, int s) {
+    const int tokens = cu_q[s + 1] - cu_q[s];
+    return tokens > few_of(FORM) ? ceil_div(tokens, C) : 0;
+}
 template <int FORM, bool BY_SEQUENCE>
 __device__ __forceinline__ Place place_of(const int* __restrict__ cu_q, int n_seqs, int c) {
-    const int lane = threadIdx.x & 31;
-    int before = 0, seen = 0;                   // chunks, and sequences with chunks, of the sequences passed
-    for (int s0 = 0; s0 < n_seqs; s0 += 128) {  // four in a row a lane
-        const int s = s0 + 4 * lane;
-        int at[5], n[4], chunks = 0, longs = 0;
-#pragma unroll
-        for (int u = 0; u < 5; ++u) at[u] = cu_q[min(s + u, n_seqs)];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            n[u] = at[u + 1] - at[u] > few_of(FORM) ? ceil_div(at[u + 1] - at[u], C) : 0;
-            chunks += n[u];
-            longs += n[u] > 0 ? 1 : 0;
-        }
-        int upto = chunks, longs_upto = longs;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int x = __shfl_up_sync(0xffffffffu, upto, o), y = BY_SEQUENCE ? __shfl_up_sync(0xffffffffu, longs_upto, o) : 0;
-            if (lane >= o) {
-                upto += x;
-                longs_upto += y;
-            }
-        }
-        const unsigned holds = __ballot_sync(0xffffffffu, BY_SEQUENCE ? seen + longs_upto > c : before + upto > c);
-        if (holds) {
-            const int owner = __ffs(holds) - 1;
-            int base = before + upto - chunks, skip = BY_SEQUENCE ? c - (seen + longs_upto - longs) : 0, u = 0;      // (the owner's are used)
-            for (; u < 3; ++u) {
-                if (BY_SEQUENCE ? n[u] > 0 && skip == 0 : c < base + n[u]) break;
-                if (BY_SEQUENCE && n[u] > 0) --skip;
-                base += n[u];
-            }
-            base = __shfl_sync(0xffffffffu, base, owner);
-            return {s0 + 4 * owner + __shfl_sync(0xffffffffu, u, owner), c - base, base};
-        }
-        before += __shfl_sync(0xffffffffu, upto, 31);
-        if (BY_SEQUENCE) seen += __shfl_sync(0xffffffffu, longs_upto, 31);
+    const int lane = threadIdx.x & 31, each = ceil_div(n_seqs, 32), s0 = lane * each, s1 = min(n_seqs, s0 + each);      // a run of sequences a lane
+    int count = 0, found = 0;                   // their chunks, and what is counted: chunks, or sequences that have any
+#pragma unroll 4
+    for (int s = s0; s < s1; ++s) {
+        const int n = chunks_of<FORM>(cu_q, s);
+        count += n;
+        found += BY_SEQUENCE ? n > 0 : n;
     }
-    return {-1, 0, 0};
+    int base = count, upto = found;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, base, o), y = BY_SEQUENCE ? __shfl_up_sync(0xffffffffu, upto, o) : x;
+        if (lane >= o) {
+            base += x;
+            upto += y;
+        }
+    }
+    const unsigned holds = __ballot_sync(0xffffffffu, upto > c);
+    if (!holds) return {-1, 0, 0};
+    const int owner = __ffs(holds) - 1;
+    base -= count;
+    int s = s0, left = c - (upto - found);      // (the owner's are used)
+    if (lane == owner)
+        for (;; ++s) {
+            const int n = chunks_of<FORM>(cu_q, s), step = BY_SEQUENCE ? n > 0 : n;
+            if (left < step) break;
+            left -= step;
+            base += n;
+        }
+    base = __shfl_sync(0xffffffffu, base, owner);
+    return {__shfl_sync(0xffffffffu, s, owner), c - base, base};
 }
 
 // What the weights of a chunk follow from, per token i: CM_MAX the sums F_i = f_1 + .. + f_i as two floats, i and m; CM_CONST powers of the decay.
