@@ -10,6 +10,8 @@
 //   OUT_DIRECT         C[m, n]                      (splits == 1), bfloat16 or float32
 //   OUT_GATED          C[m, j] = silu(gate) * up    (splits == 1), W interleaving gate and up rows in groups of 16
 //   OUT_PARTIAL        P[split, m, n] float32       the consumer adds the `splits` slices in a fixed order
+//   OUT_CLUSTER        C[m, n]                      the slices of K of a tile are a thread-block cluster and are added up through
+//                                                   its shared memory: what OUT_DIRECT becomes where W has few rows (`direct_splits`)
 //   OUT_CLUSTER_GATED  C[m, j] = silu(gate) * up    the slices of K of a tile are a thread-block cluster (2 or 4
 //                                                   blocks) and are added up through its shared memory
 // Consumers of partial sums are the residual add + RMSNorm and the q/k-norm + rotary + cache-write
@@ -26,6 +28,8 @@
 // The reference uses a one-warp-per-output-row GEMV for M <= 2 and cuBLAS above
 // (src/backend/cuda/linear/linear.cu:22-96); this kernel covers both ranges up to 256 rows.
 #include <string.h>
+
+#include <algorithm>
 #define LLMK_MODULE_NAME "gemm_skinny"
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -38,7 +42,8 @@ constexpr int BW = 128;          // rows of W per block
 constexpr int BK = 64;           // one 128-byte swizzle row of bfloat16
 constexpr int UMMA_K = 16;
 constexpr int THREADS = 192;
-enum { OUT_DIRECT = 0, OUT_PARTIAL = 1, OUT_GATED = 2, OUT_CLUSTER_GATED = 5 };
+enum { OUT_DIRECT = 0, OUT_PARTIAL = 1, OUT_GATED = 2, OUT_CLUSTER = 4, OUT_CLUSTER_GATED = 5 };
+constexpr bool in_cluster(int mode) { return mode == OUT_CLUSTER || mode == OUT_CLUSTER_GATED; }
 
 // A ring stage holds a tile of W and one of X.
 template <int MPAD, int STAGES>
@@ -69,7 +74,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same for all lanes, and known to be)
     const int n0 = blockIdx.x * BW;
     const int split = blockIdx.y;
     const int num_kb = (K + BK - 1) / BK;
@@ -96,31 +101,36 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
+    // The whole warp walks the loops of both issuing roles and one lane issues: what the instructions are given is then known to be the same for all
+    // lanes and kept where they read it.
     if (warp == 0) {
-        if (lane == 0) {
-            pdl_launch_dependents();   // at once: releasing the next kernel later (after the loads, after the products) was slower
+        {
+            const bool issues = tc::elect_one();
+            if (issues) pdl_launch_dependents();   // at once: releasing the next kernel later (after the loads, after the products) was slower
             // W is written by no kernel of the step: its first loads go out before the wait.
             const int first = min(nkb, STAGES);
             for (int i = 0; i < first; ++i) {
+                if (!issues) break;
                 const uint32_t bar = tc::smem_u32(&full[i]);
                 tc::mbar_expect_tx(bar, L::STAGE_BYTES);
                 tc::tma_load_2d(tc::smem_u32(smem + i * L::STAGE_BYTES), &map_w, bar, (kb0 + i) * BK, n0);
             }
             pdl_wait();   // X was written by the kernel before this one
             for (int i = 0; i < first; ++i)
-                tc::tma_load_2d(tc::smem_u32(smem + i * L::STAGE_BYTES + L::W_BYTES), &map_x, tc::smem_u32(&full[i]),
+                if (issues) tc::tma_load_2d(tc::smem_u32(smem + i * L::STAGE_BYTES + L::W_BYTES), &map_x, tc::smem_u32(&full[i]),
                                 (kb0 + i) * BK, 0);
             int issued = first;
             for (int kb = first; kb < nkb; ++kb) {
                 const int s = kb % STAGES;
                 const uint32_t round = kb / STAGES;
-                if (!tc::mbar_wait(tc::smem_u32(&empty[s]), (round & 1) ^ 1, abort_flag)) break;
+                if (!tc::mbar_wait_warp(tc::smem_u32(&empty[s]), (round & 1) ^ 1, abort_flag)) break;
+                issued = kb + 1;
+                if (!issues) continue;
                 const uint32_t bar = tc::smem_u32(&full[s]);
                 tc::mbar_expect_tx(bar, L::STAGE_BYTES);
                 const uint32_t dst = tc::smem_u32(smem + s * L::STAGE_BYTES);
                 tc::tma_load_2d(dst, &map_w, bar, (kb0 + kb) * BK, n0);
                 tc::tma_load_2d(dst + L::W_BYTES, &map_x, bar, (kb0 + kb) * BK, 0);
-                issued = kb + 1;
             }
             if (*abort_flag) {
                 // Let the copies that are in flight land before the block's memory is given up.
@@ -133,15 +143,17 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            const bool issues = tc::elect_one();
             constexpr uint32_t idesc = tc::idesc_bf16_f32(BW, MPAD);
             bool ok = true;
             for (int kb = 0; kb < nkb && ok; ++kb) {
                 const int s = kb % STAGES;
                 const uint32_t round = kb / STAGES;
-                ok = tc::mbar_wait(tc::smem_u32(&full[s]), round & 1, abort_flag);
+                ok = tc::mbar_wait_warp(tc::smem_u32(&full[s]), round & 1, abort_flag);
                 if (!ok) break;
                 tc::tc_fence_after_sync();
+                if (!issues) continue;
                 const uint32_t w_addr = tc::smem_u32(smem + s * L::STAGE_BYTES);
                 const uint32_t x_addr = w_addr + L::W_BYTES;
 #pragma unroll
@@ -152,7 +164,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 }
                 tc::mma_commit(tc::smem_u32(&empty[s]));
             }
-            if (ok) tc::mma_commit(tc::smem_u32(acc_full));
+            if (ok && issues) tc::mma_commit(tc::smem_u32(acc_full));
         }
     } else {
         // Epilogue: warp w may touch tensor-memory lanes 32 * (w % 4) .. + 31; a lane is a row of W
@@ -172,7 +184,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 for (int i = 0; i < 16; ++i) {
                     const int m = c0 + i;
                     const float v = __uint_as_float(r[i]);
-                    if constexpr (MODE == OUT_CLUSTER_GATED) {
+                    if constexpr (in_cluster(MODE)) {
                         // this block's slice of the sum, for the cluster to add up: [row of X][row of W]
                         if (m < M) reinterpret_cast<float*>(smem)[m * BW + quarter * 32 + lane] = v;
                     } else if constexpr (MODE == OUT_GATED) {
@@ -196,6 +208,29 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         tc::tmem_dealloc(tmem_base, TMEM_COLS);
     }
     if (threadIdx.x == 0 && *abort_flag && error_flag) atomicExch(error_flag, 1);
+    if constexpr (MODE == OUT_CLUSTER) {
+        // The blocks of a cluster hold the slices of K of one tile, each its float32 slice in its own shared memory (over the TMA
+        // ring, which is idle by now): block r adds up every S-th row of X over the blocks, in slice order.  Nobody leaves before
+        // all have read.
+        cluster_sync_all();
+        const int S = (int)gridDim.y, rank = (int)cluster_ctarank();
+        const uint32_t red = tc::smem_u32(smem);
+        for (int idx = threadIdx.x; idx < ceil_div(M - rank, S) * BW; idx += THREADS) {
+            const int m = rank + idx / BW * S, col = idx % BW;
+            const uint32_t local = red + (uint32_t)(m * BW + col) * 4u;
+            float v = 0.f;
+            for (int q0 = 0; q0 < S; q0 += 4) {                 // four reads on their way at a time
+                float x[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) x[q] = cluster_ld_f32(cluster_map_shared(local, (uint32_t)min(q0 + q, S - 1)));
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (q0 + q < S) v += x[q];
+            }
+            if (n0 + col < N) C[(size_t)m * ldc + n0 + col] = from_float<TC>(v);
+        }
+        cluster_sync_all();
+    }
     if constexpr (MODE == OUT_CLUSTER_GATED) {
         // The blocks of a cluster hold the slices of K of one tile.  Each left its float32 slice in its own
         // shared memory (over the TMA ring, which is idle by now).  W interleaves gate and up rows in groups of
@@ -234,7 +269,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int M, int N, 
         if (e != cudaSuccess) LLMK_FAIL("gemm_skinny: cannot raise shared memory to %d: %s", L::TOTAL, cudaGetErrorString(e));
         configured = true;
     }
-    if constexpr (MODE == OUT_CLUSTER_GATED) {
+    if constexpr (in_cluster(MODE)) {
         LLMK_CHECK_LAUNCH_RC("gemm_skinny", llmk_launch_cluster(kernel, dim3(ceil_div(N, BW), splits), dim3(THREADS), L::TOTAL, s,
                                                                 true, (unsigned)splits, mw, mx, (TC*)C, M, N, K, ldc,
                                                                 kb_per_split, error_flag));
@@ -258,12 +293,22 @@ int dispatch_rows(const CUtensorMap& mw, const void* X, void* C, int M, int N, i
         case 64: return launch<TC, 64, 4, MODE>(mw, mx, C, M, N, K, ldc, splits, kb_per_split, error_flag, s);
         default: break;
     }
-    if constexpr (MODE == OUT_CLUSTER_GATED) {
+    if constexpr (in_cluster(MODE)) {
         LLMK_FAIL("gemm_skinny: the sum over a cluster takes at most 64 rows, not %d", M);
     } else {
         if (mpad == 128) return launch<TC, 128, 6, MODE>(mw, mx, C, M, N, K, ldc, splits, kb_per_split, error_flag, s);
         return launch<TC, 256, 4, MODE>(mw, mx, C, M, N, K, ldc, splits, kb_per_split, error_flag, s);
     }
+}
+
+// Into how many slices of K, a cluster's blocks, a product written directly is cut: W of fewer rows than keep half of the SMs busy is
+// pulled by few of them at some 40 GB/s each.  At most 8 slices, of four steps of 64 at least; from N and K alone, so that
+// a row's sum does not depend on M.
+int direct_splits(int N, int K) {
+    const int tiles = ceil_div(N, BW), num_kb = ceil_div(K, BK);
+    int splits = std::min(std::min(device_sm_count() / tiles, num_kb / 4), 8);
+    if (splits < 2) return 1;
+    return ceil_div(num_kb, ceil_div(num_kb, splits));          // none is left empty
 }
 
 }  // namespace
@@ -333,6 +378,12 @@ LLMK_EXPORT int llmk_gemm_skinny(void* C, const void* X, const void* W, int M, i
     }
     if (mode == OUT_CLUSTER_GATED) return dispatch_rows<bf16, OUT_CLUSTER_GATED>(mw, X, C, M, N, K, ldx, ldc, splits, per, error_flag, s);
     if (mode != OUT_DIRECT) LLMK_FAIL("gemm_skinny: unknown mode %d", mode);
+    const int cut = M <= 64 ? direct_splits(N, K) : 1;
+    if (cut > 1) {
+        const int kb = ceil_div(num_kb, cut);
+        if (out_dtype == LLMK_BF16) return dispatch_rows<bf16, OUT_CLUSTER>(mw, X, C, M, N, K, ldx, ldc, cut, kb, error_flag, s);
+        if (out_dtype == LLMK_F32) return dispatch_rows<float, OUT_CLUSTER>(mw, X, C, M, N, K, ldx, ldc, cut, kb, error_flag, s);
+    }
     if (out_dtype == LLMK_BF16) return dispatch_rows<bf16, OUT_DIRECT>(mw, X, C, M, N, K, ldx, ldc, 1, per, error_flag, s);
     if (out_dtype == LLMK_F32) return dispatch_rows<float, OUT_DIRECT>(mw, X, C, M, N, K, ldx, ldc, 1, per, error_flag, s);
     LLMK_FAIL("gemm_skinny: unknown output dtype %d", out_dtype);
