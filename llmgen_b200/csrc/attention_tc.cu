@@ -120,17 +120,21 @@ __device__ __forceinline__ void page_ids(int (&ids)[BN / PS], const int* bt, int
 // is (page * nkv + kvh) * PS (a page already given back by a window, id -1, is replaced by the last page: its keys
 // are masked).
 template <int HB, int PS>
-__device__ __forceinline__ void load_pages(uint32_t dst, const CUtensorMap* map, uint32_t bar, const int (&ids)[BN / PS],
+__device__ __forceinline__ void load_pages(bool issues, uint32_t dst, const CUtensorMap* map, uint32_t bar, const int (&ids)[BN / PS],
                                            const int* bt, int last_page, int nkv, int kvh) {
-    tc::mbar_expect_tx(bar, BN * HB * 128);
+    int row[BN / PS];
 #pragma unroll
     for (int pg = 0; pg < BN / PS; ++pg) {
         int page = ids[pg];
         if (page < 0) page = __ldg(bt + last_page);
-        const int row = (page * nkv + kvh) * PS;
-#pragma unroll
-        for (int h = 0; h < HB; ++h) tc::tma_load_2d(dst + h * BN * 128 + pg * PS * 128, map, bar, h * 64, row);
+        row[pg] = (page * nkv + kvh) * PS;
     }
+    if (!issues) return;
+    tc::mbar_expect_tx(bar, BN * HB * 128);
+#pragma unroll
+    for (int pg = 0; pg < BN / PS; ++pg)
+#pragma unroll
+        for (int h = 0; h < HB; ++h) tc::tma_load_2d(dst + h * BN * 128 + pg * PS * 128, map, bar, h * 64, row[pg]);
 }
 
 // (one block an SM, which shared memory allows no more of anyway: said, the compiler schedules for it, 35.0 -> 34.4 us on a 2,048-token prompt)
@@ -170,7 +174,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NUM_BARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same for all lanes, and known to be)
     const int G = p.nq / p.nkv;
     // heads vary fastest over the grid: the caller lists the tiles heaviest first, and the blocks of a
     // grid start in the order of their linear index, so the long tiles of every head start first
@@ -213,13 +217,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
     const int head0 = kvh * G + chunk * p.gc;
 
+    // The whole warp walks the loops of an issuing role and one lane issues: what the instructions are given is then known to be the same for all
+    // lanes and kept where they read it.
+    const bool issues = tc::elect_one();
     if (warp == 0) {
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0) {
             const uint32_t qbar = tc::smem_u32(q_full);
-            tc::mbar_expect_tx(qbar, L::Q_BYTES);
+            if (issues) tc::mbar_expect_tx(qbar, L::Q_BYTES);
 #pragma unroll
             for (int h = 0; h < HB; ++h)
-                tc::tma_load_3d(tc::smem_u32(smem + L::Q_OFF + h * BM * 128), &map_q, qbar, h * 64, head0, q_beg + q0);
+                if (issues) tc::tma_load_3d(tc::smem_u32(smem + L::Q_OFF + h * BM * 128), &map_q, qbar, h * 64, head0, q_beg + q0);
             const int* bt = p.block_tables + (size_t)s * p.max_blocks;
             const int last_page = (ctx - 1) / PS;
             int ids[BN / PS], next_ids[BN / PS];
@@ -230,14 +237,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
                 for (int pg = 0; pg < BN / PS; ++pg) ids[pg] = next_ids[pg];
                 if (j + 1 < n_tiles) page_ids<PS>(next_ids, bt, kt0 + (j + 1) * BN, last_page);
-                if (!tc::mbar_wait(tc::smem_u32(&k_empty[st]), (round & 1) ^ 1, abort_flag)) break;
-                load_pages<HB, PS>(tc::smem_u32(smem + L::K_OFF + st * L::KV_BYTES), &map_k, tc::smem_u32(&k_full[st]), ids, bt,
+                if (!tc::mbar_wait_warp(tc::smem_u32(&k_empty[st]), (round & 1) ^ 1, abort_flag)) break;
+                load_pages<HB, PS>(issues, tc::smem_u32(smem + L::K_OFF + st * L::KV_BYTES), &map_k, tc::smem_u32(&k_full[st]), ids, bt,
                                    last_page, p.nkv, kvh);
             }
         }
     } else if (warp == 10) {
         // V producer: a ring of its own, so that K of the next tiles never waits for a V slot.
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0) {
             const int* bt = p.block_tables + (size_t)s * p.max_blocks;
             const int last_page = (ctx - 1) / PS;
             int ids[BN / PS], next_ids[BN / PS];
@@ -248,13 +255,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
                 for (int pg = 0; pg < BN / PS; ++pg) ids[pg] = next_ids[pg];
                 if (j + 1 < n_tiles) page_ids<PS>(next_ids, bt, kt0 + (j + 1) * BN, last_page);
-                if (!tc::mbar_wait(tc::smem_u32(&v_empty[st]), (round & 1) ^ 1, abort_flag)) break;
-                load_pages<HB, PS>(tc::smem_u32(smem + L::V_OFF + st * L::KV_BYTES), &map_v, tc::smem_u32(&v_full[st]), ids, bt,
+                if (!tc::mbar_wait_warp(tc::smem_u32(&v_empty[st]), (round & 1) ^ 1, abort_flag)) break;
+                load_pages<HB, PS>(issues, tc::smem_u32(smem + L::V_OFF + st * L::KV_BYTES), &map_v, tc::smem_u32(&v_full[st]), ids, bt,
                                    last_page, p.nkv, kvh);
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && n_tiles > 0) {
+        if (n_tiles > 0) {
             constexpr uint32_t idesc_s = tc::idesc_bf16_f32(BM, BN);
             constexpr uint32_t idesc_o = tc::idesc_bf16_f32_b_mn(BM, HD);
             // descriptors of the four operands, built once: a step along K (or along the keys) adds to the start
@@ -269,8 +276,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                                         tc::smem_desc_sw128_mn(tc::smem_u32(smem + L::V_OFF + LAST * L::KV_BYTES), p.v_lbo, p.v_sbo)};
             auto issue_qk = [&](int j) -> bool {
                 const int st = j & 1;
-                if (!tc::mbar_wait(tc::smem_u32(&k_full[st]), (j >> 1) & 1, abort_flag)) return false;
+                if (!tc::mbar_wait_warp(tc::smem_u32(&k_full[st]), (j >> 1) & 1, abort_flag)) return false;
                 tc::tc_fence_after_sync();
+                if (!issues) return true;
 #pragma unroll
                 for (int k = 0; k < HD / 16; ++k) {
                     const uint64_t off = (uint64_t)(((k / 4) * (BM * 128) + (k % 4) * 32) >> 4);
@@ -280,18 +288,19 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc::mma_commit(tc::smem_u32(&k_empty[st]));
                 return true;
             };
-            bool ok = tc::mbar_wait(tc::smem_u32(q_full), 0, abort_flag);
+            bool ok = tc::mbar_wait_warp(tc::smem_u32(q_full), 0, abort_flag);
             if (ok) tc::tc_fence_after_sync();
             ok = ok && issue_qk(0);
             if (ok && n_tiles > 1) ok = issue_qk(1);
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const int st = j & 1;
-                ok = tc::mbar_wait(tc::smem_u32(p_full), j & 1, abort_flag) &&
-                     tc::mbar_wait(tc::smem_u32(&v_full[st & LAST]), (j / L::BUFFERS) & 1, abort_flag);
+                ok = tc::mbar_wait_warp(tc::smem_u32(p_full), j & 1, abort_flag) &&
+                     tc::mbar_wait_warp(tc::smem_u32(&v_full[st & LAST]), (j / L::BUFFERS) & 1, abort_flag);
                 if (!ok) break;
                 tc::tc_fence_after_sync();
 #pragma unroll
                 for (int term = TERMS - 1; term >= 0; --term) {       // (the smaller terms, smallest first, have an accumulator of their own)
+                    if (!issues) break;
 #pragma unroll
                     for (int kk = 0; kk < BN / 16; ++kk) {
                         const uint64_t da = p_desc[st] + (uint64_t)((term * L::P_BYTES + (kk / 4) * (BM * 128) + (kk % 4) * 32) >> 4);
@@ -300,8 +309,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         tc::mma_bf16_ss(tmem_base + (term == 0 ? O_COL0 : REST_COL0), da, db, idesc_o, j != 0 || kk != 0 || (term != 0 && term != TERMS - 1));
                     }
                 }
-                tc::mma_commit(tc::smem_u32(&o_full[st]));
-                tc::mma_commit(tc::smem_u32(&v_empty[st & LAST]));
+                if (issues) {
+                    tc::mma_commit(tc::smem_u32(&o_full[st]));
+                    tc::mma_commit(tc::smem_u32(&v_empty[st & LAST]));
+                }
                 if (j + 2 < n_tiles) ok = issue_qk(j + 2);
             }
         }
