@@ -328,24 +328,59 @@ attn_prep_vec_kernel(const T* __restrict__ qkv, long long row_stride, T* __restr
     }
 }
 
+// Eight bytes from each half of a row: two float32 or four bfloat16 values twice.
+template <typename T>
+struct Halves {
+    uint2 lo, hi;
+    __device__ __forceinline__ void unpack(float* f) const {
+        Vec16<T> v;
+        if constexpr (sizeof(T) == 4) v.raw = make_float4(__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(hi.x), __uint_as_float(hi.y));
+        else v.raw = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        v.unpack(f);
+    }
+    __device__ __forceinline__ void pack(const float* f) {
+        Vec16<T> v;
+        v.pack(f);
+        if constexpr (sizeof(T) == 4) {
+            lo = make_uint2(__float_as_uint(v.raw.x), __float_as_uint(v.raw.y));
+            hi = make_uint2(__float_as_uint(v.raw.z), __float_as_uint(v.raw.w));
+        } else {
+            lo = make_uint2(v.raw.x, v.raw.y);
+            hi = make_uint2(v.raw.z, v.raw.w);
+        }
+    }
+};
+template <int N>
+__device__ __forceinline__ void load_floats(float* f, const float* src) {
+    if constexpr (N == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(src);
+        f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+    } else {
+        const float2 v = *reinterpret_cast<const float2*>(src);
+        f[0] = v.x; f[1] = v.y;
+    }
+}
+
 // The same, a warp taking `U` rounds of rows of ONE token at a time: position, slot, the lane's cos and
 // sin values and its gains are read once for U * 32 / LPR rows (16 heads of 128 in bfloat16) instead of
-// once a row, and the U loads of the rows are in flight together.
+// once a row, and the U loads of the rows are in flight together.  A lane holds EPL / 2 neighbouring values of a row's low half and the
+// same of its high half, so the pairs that the rotation mixes lie in one lane: 8-byte accesses, but no exchange of
+// every value and half the cos and sin values a lane, and registers for more warps (bound by the loads in flight: 34 MB for 2,048 tokens of 32 heads
+// of 128; with a lane's values in one piece and eight rounds 700 / 2,048 / 8,000 tokens took 5.8 / 10.7 / 43.2 us).
 template <typename T, int LPR, int U>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 attn_prep_token_kernel(const T* __restrict__ qkv, long long row_stride, T* __restrict__ q_out, long long q_stride,
                        T* __restrict__ kcache, T* __restrict__ vcache, const int* __restrict__ positions,
                        const int* __restrict__ slots, const float* __restrict__ cos_tab,
                        const float* __restrict__ sin_tab, const float* __restrict__ q_gain,
                        const float* __restrict__ k_gain, int n_tokens, int nq, int nk, int nkv_cache, int hd,
                        int page_size, float eps, float q_off, float k_off) {
-    constexpr int EPL = Vec16<T>::N;            // elements per lane
+    constexpr int EPL = Vec16<T>::N, HALF = EPL / 2;       // elements per lane
     constexpr int RPW = 32 / LPR;               // rows per round
     constexpr int RC = U * RPW;                 // rows per item
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
-    const int sub = lane % LPR;                 // which vector of the row
-    const int half_lanes = LPR / 2;
+    const int low = lane % LPR * HALF, high = hd / 2 + low;      // where this lane's values lie in a row
     const int heads = nq + 2 * nk;
     const int chunks = (heads + RC - 1) / RC;
     const unsigned n_items = (unsigned)n_tokens * (unsigned)chunks;
@@ -355,46 +390,40 @@ attn_prep_token_kernel(const T* __restrict__ qkv, long long row_stride, T* __res
     // the gains are weights: read before the wait
     float gq[EPL], gk[EPL];
 #pragma unroll
-    for (int i = 0; i < EPL; i += 4) {
-        const float4 a = q_gain ? *reinterpret_cast<const float4*>(q_gain + sub * EPL + i) : make_float4(1.f, 1.f, 1.f, 1.f);
-        const float4 b = k_gain ? *reinterpret_cast<const float4*>(k_gain + sub * EPL + i) : make_float4(1.f, 1.f, 1.f, 1.f);
-        gq[i] = a.x + q_off; gq[i + 1] = a.y + q_off; gq[i + 2] = a.z + q_off; gq[i + 3] = a.w + q_off;
-        gk[i] = b.x + k_off; gk[i + 1] = b.y + k_off; gk[i + 2] = b.z + k_off; gk[i + 3] = b.w + k_off;
+    for (int i = 0; i < HALF; ++i) {
+        gq[i] = (q_gain ? q_gain[low + i] : 1.f) + q_off;
+        gq[HALF + i] = (q_gain ? q_gain[high + i] : 1.f) + q_off;
+        gk[i] = (k_gain ? k_gain[low + i] : 1.f) + k_off;
+        gk[HALF + i] = (k_gain ? k_gain[high + i] : 1.f) + k_off;
     }
-    const float sign = sub < half_lanes ? -1.f : 1.f;      // low half: x cos - y sin; high half: x cos + y sin
     pdl_wait();
     for (unsigned item = warp_id; item < n_items; item += n_warps) {
         const int t = (int)(item / (unsigned)chunks);
         const int h0 = (int)(item - (unsigned)t * (unsigned)chunks) * RC + lane / LPR;
-        const T* src = qkv + (size_t)t * row_stride + sub * EPL;
-        Vec16<T> x[U];
+        const T* src = qkv + (size_t)t * row_stride;
+        Halves<T> x[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int h = h0 + u * RPW;
-            if (h < heads) x[u].raw = *reinterpret_cast<const decltype(x[u].raw)*>(src + (size_t)h * hd);
-            else x[u].raw = decltype(x[u].raw){};
+            if (h < heads) {
+                x[u].lo = *reinterpret_cast<const uint2*>(src + (size_t)h * hd + low);
+                x[u].hi = *reinterpret_cast<const uint2*>(src + (size_t)h * hd + high);
+            } else {
+                x[u].lo = x[u].hi = make_uint2(0u, 0u);
+            }
         }
         const int slot = slots ? slots[t] : -1;
-        float cv[EPL], sv[EPL];
+        float cv[HALF], sv[HALF];
         if (cos_tab) {
-            const int pos = positions[t];
-            const int p0 = (sub % half_lanes) * EPL;          // index of the pair inside the half
-            const float* c = cos_tab + (size_t)pos * (hd / 2) + p0;
-            const float* sn = sin_tab + (size_t)pos * (hd / 2) + p0;
-#pragma unroll
-            for (int i = 0; i < EPL; i += 4) {
-                const float4 a = *reinterpret_cast<const float4*>(c + i);
-                const float4 b = *reinterpret_cast<const float4*>(sn + i);
-                cv[i] = a.x; cv[i + 1] = a.y; cv[i + 2] = a.z; cv[i + 3] = a.w;
-                sv[i] = sign * b.x; sv[i + 1] = sign * b.y; sv[i + 2] = sign * b.z; sv[i + 3] = sign * b.w;
-            }
+            const size_t at = (size_t)positions[t] * (hd / 2) + low;
+            load_floats<HALF>(cv, cos_tab + at);
+            load_floats<HALF>(sv, sin_tab + at);
         }
         const int page = slot >= 0 ? slot / page_size : 0;
         const int in_page = slot - page * page_size;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int h = h0 + u * RPW;
-            const bool live = h < heads;
             const bool is_q = h < nq;
             const bool is_v = h >= nq + nk;
             float f[EPL];
@@ -412,14 +441,7 @@ attn_prep_token_kernel(const T* __restrict__ qkv, long long row_stride, T* __res
 #pragma unroll
                 for (int i = 0; i < EPL; ++i) f[i] = f[i] * rinv * (is_q ? gq[i] : gk[i]);
             }
-            float partner[EPL];
-#pragma unroll
-            for (int i = 0; i < EPL; ++i) partner[i] = __shfl_xor_sync(0xffffffffu, f[i], half_lanes);
-            if (!is_v && cos_tab) {
-#pragma unroll
-                for (int i = 0; i < EPL; ++i) f[i] = f[i] * cv[i] + partner[i] * sv[i];
-            }
-            if (!live) continue;
+            if (h >= heads) continue;
             T* dst = nullptr;
             if (is_q) {
                 dst = q_out + (size_t)t * q_stride + (size_t)h * hd;
@@ -429,9 +451,19 @@ attn_prep_token_kernel(const T* __restrict__ qkv, long long row_stride, T* __res
                 if (cache) dst = cache + (((size_t)page * nkv_cache + kvh) * page_size + in_page) * hd;
             }
             if (dst) {
-                Vec16<T> y;
-                y.pack(f);
-                *reinterpret_cast<decltype(y.raw)*>(dst + sub * EPL) = is_v ? x[u].raw : y.raw;
+                if (!is_v) {
+                    if (cos_tab) {
+#pragma unroll
+                        for (int i = 0; i < HALF; ++i) {
+                            const float a = f[i], b = f[HALF + i];
+                            f[i] = a * cv[i] + b * -sv[i];
+                            f[HALF + i] = b * cv[i] + a * sv[i];
+                        }
+                    }
+                    x[u].pack(f);
+                }
+                *reinterpret_cast<uint2*>(dst + low) = x[u].lo;
+                *reinterpret_cast<uint2*>(dst + high) = x[u].hi;
             }
         }
     }
@@ -469,11 +501,11 @@ static bool launch_vec(const void* qkv, long long row_stride, void* q_out, long 
                            row_stride, (T*)q_out, q_stride, (T*)kcache, (T*)vcache, positions, slots, cos_tab, sin_tab,     \
                            q_gain, k_gain, n_tokens, nq, nk, nkv_cache, hd, page_size, eps, q_off, k_off);                  \
     } while (0)
-        // eight rounds of rows in flight per warp: 13.3 us on 2,048 tokens of 32 heads of 128 in bfloat16,
-        // 15.2 us with four, 14.5 us a row at a time
-        if (lpr == 8) LAUNCH_TOKEN(8, 8);
-        else if (lpr == 16) LAUNCH_TOKEN(16, 8);
-        else LAUNCH_TOKEN(32, 8);
+        // four rounds of rows in flight a warp, three blocks an SM: 700 / 2,048 / 8,000 tokens of 32 heads of 128 in bfloat16 4.1 / 9.9 / 34.3 us;
+        // eight rounds at two blocks 5.5 / 10.5 / 42.7, four at four blocks (registers to memory) 5.8 / 9.8 / 34.8, two at five 5.8 / 12.7 / 43.3
+        if (lpr == 8) LAUNCH_TOKEN(8, 4);
+        else if (lpr == 16) LAUNCH_TOKEN(16, 4);
+        else LAUNCH_TOKEN(32, 4);
 #undef LAUNCH_TOKEN
         return true;
     }
