@@ -795,6 +795,10 @@ LLMK_EXPORT int llmk_concat_stream(void* out, const float* resid, const void* de
 // streams [n, S, H] float32.  With y (an array of T or float32 slices, times a, or a y + b y2): every stream is rewritten from all the old
 // ones, x_t <- sum_s mix[s * S + t] x_s + out_coef[t] y.  With next_in: normed[r, :] = rmsnorm(sum_t next_in[t] x_t) * next_gain
 // (the new streams), the input of the sublayer that follows.  Either half may be absent.  A block per token row.
+//
+// What bounds it is the streams' traffic (2,048 rows of 2,048, four streams: 134 MB a step, 21 us), so the first and the last step of a
+// pass take less of it: `one` [n, H] stands for streams that are all still equal to this row (none is read), and `sum` [n, H]
+// receives the new streams' sum, in the order of the streams, where nothing else is needed of them (none is written).
 constexpr int MAX_STREAMS = 16;
 
 // MS: the most streams this instance takes (4, 8 or 16); the loops over streams are unrolled to it, except the outer one of 16.
@@ -803,7 +807,7 @@ __global__ void __launch_bounds__(512) stream_step_kernel(float* __restrict__ st
                                    const void* __restrict__ y2, int splits2, long long split_stride2, float a, float b,
                                    const float* __restrict__ mix, const float* __restrict__ out_coef,
                                    const float* __restrict__ next_in, const float* __restrict__ next_gain, float eps,
-                                   T* __restrict__ normed, int S, int H) {
+                                   T* __restrict__ normed, int S, int H, const float* one, float* sum) {
     extern __shared__ float srow[];  // H floats + 33 scratch + S * S + 2 * S coefficients
     float* scratch = srow + H;
     float* coef = scratch + 33;      // mix [S, S], out [S], in [S]
@@ -824,8 +828,8 @@ __global__ void __launch_bounds__(512) stream_step_kernel(float* __restrict__ st
         float x[MS];
 #pragma unroll
         for (int s = 0; s < MS; ++s)
-            if (s < S) x[s] = xs[(size_t)s * H + i];
-        float u = 0.f;
+            if (s < S) x[s] = one ? one[r * H + i] : xs[(size_t)s * H + i];
+        float u = 0.f, total = 0.f;
         if (y) {
             float v = load_sum<T>(y, r * H + i, splits, split_stride);
             v = y2 ? a * v + b * load_sum<T>(y2, r * H + i, splits2, split_stride2) : a * v;
@@ -837,7 +841,8 @@ __global__ void __launch_bounds__(512) stream_step_kernel(float* __restrict__ st
 #pragma unroll
                     for (int s = 0; s < MS; ++s)
                         if (s < S) acc = fmaf(coef[s * S + t], x[s], acc);
-                    xs[(size_t)t * H + i] = acc;
+                    if (sum) total = t == 0 ? acc : total + acc;
+                    else xs[(size_t)t * H + i] = acc;
                     u = fmaf(coef[S * S + S + t], acc, u);
                 }
             }
@@ -846,6 +851,7 @@ __global__ void __launch_bounds__(512) stream_step_kernel(float* __restrict__ st
             for (int t = 0; t < MS; ++t)
                 if (t < S) u = fmaf(coef[S * S + S + t], x[t], u);
         }
+        if (sum) sum[r * H + i] = total;
         if (next_in) {
             srow[i] = u;
             ss = fmaf(u, u, ss);
@@ -884,7 +890,7 @@ __global__ void __launch_bounds__(1024) stream_step_vec_kernel(float* __restrict
                                    const void* __restrict__ y2, int splits2, long long split_stride2, float a, float b,
                                    const float* __restrict__ mix, const float* __restrict__ out_coef,
                                    const float* __restrict__ next_in, const float* __restrict__ next_gain, float eps,
-                                   T* __restrict__ normed, int S, int H) {
+                                   T* __restrict__ normed, int S, int H, const float* one, float* sum) {
     __shared__ float scratch[33];
     __shared__ float coef[MS * MS + 2 * MS];      // mix [S, S], out [S], in [S]
     const size_t r = blockIdx.x;
@@ -905,11 +911,11 @@ __global__ void __launch_bounds__(1024) stream_step_vec_kernel(float* __restrict
     float u[4] = {0.f, 0.f, 0.f, 0.f};
     if (on) {
         float* xs = streams + r * S * H + i;
-        float x[MS][4];
+        float x[MS][4], total[4];
 #pragma unroll
         for (int s = 0; s < MS; ++s) {
             if (s < S) {
-                const float4 v = *reinterpret_cast<const float4*>(xs + (size_t)s * H);
+                const float4 v = *reinterpret_cast<const float4*>(one ? one + r * H + i : xs + (size_t)s * H);
                 x[s][0] = v.x; x[s][1] = v.y; x[s][2] = v.z; x[s][3] = v.w;
             }
         }
@@ -933,11 +939,17 @@ __global__ void __launch_bounds__(1024) stream_step_vec_kernel(float* __restrict
                             for (int c = 0; c < 4; ++c) acc[c] = fmaf(m, x[s][c], acc[c]);
                         }
                     }
-                    *reinterpret_cast<float4*>(xs + (size_t)t * H) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                    if (sum) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) total[c] = t == 0 ? acc[c] : total[c] + acc[c];
+                    } else {
+                        *reinterpret_cast<float4*>(xs + (size_t)t * H) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                    }
 #pragma unroll
                     for (int c = 0; c < 4; ++c) u[c] = fmaf(in, acc[c], u[c]);
                 }
             }
+            if (sum) *reinterpret_cast<float4*>(sum + r * H + i) = make_float4(total[0], total[1], total[2], total[3]);
         } else {
 #pragma unroll
             for (int t = 0; t < MS; ++t)
@@ -967,10 +979,11 @@ __global__ void __launch_bounds__(1024) stream_step_vec_kernel(float* __restrict
 LLMK_EXPORT int llmk_stream_step(float* streams, const void* y, int splits, long long split_stride, const void* y2, int splits2,
                                  long long split_stride2, float a, float b, const float* mix, const float* out_coef,
                                  const float* next_in, const float* next_gain, float eps, void* normed, int n_rows, int S, int H,
-                                 int dtype, void* stream) {
+                                 const float* one, float* sum, int dtype, void* stream) {
     if (n_rows <= 0) return LLMK_OK;
     if (S <= 0 || S > MAX_STREAMS || H <= 0 || !streams) LLMK_FAIL("stream_step: %d streams (at most %d) of %d values", S, MAX_STREAMS, H);
     if (y && (!mix || !out_coef)) LLMK_FAIL("stream_step: a sublayer's output needs the streams' coefficients");
+    if (sum && !y) LLMK_FAIL("stream_step: the streams' sum is taken as they are rewritten");
     if (next_in && (!next_gain || !normed)) LLMK_FAIL("stream_step: the next sublayer's input needs gains and a place");
     const size_t smem = ((size_t)H + 33 + S * S + 2 * S) * sizeof(float);
     if (smem > 200 * 1024) LLMK_FAIL("stream_step: a row of %d values does not fit shared memory", H);
@@ -979,12 +992,13 @@ LLMK_EXPORT int llmk_stream_step(float* streams, const void* y, int splits, long
     cudaError_t e;
     const size_t vec = dtype == LLMK_F32 ? 16 : 8;
     if (S <= 8 && H % 4 == 0 && H <= 4096 && (dtype == LLMK_F32 || dtype == LLMK_BF16) && host_aligned16(streams) && host_aligned16(next_gain) &&
+        host_aligned16(one) && host_aligned16(sum) &&
         (reinterpret_cast<uintptr_t>(y) & (splits ? 15 : vec - 1)) == 0 && (reinterpret_cast<uintptr_t>(y2) & (splits2 ? 15 : vec - 1)) == 0 &&
         split_stride % 4 == 0 && split_stride2 % 4 == 0 && (reinterpret_cast<uintptr_t>(normed) & (vec - 1)) == 0) {
         const dim3 block(ceil_div(H / 4, 32) * 32);
 #define STREAM_STEP_VEC(TYPE, MS)                                                                                                     \
     e = llmk_launch(stream_step_vec_kernel<TYPE, MS>, dim3(n_rows), block, 0, st, true, streams, y, splits, split_stride, y2, splits2, \
-                    split_stride2, a, b, mix, out_coef, next_in, next_gain, eps, (TYPE*)normed, S, H)
+                    split_stride2, a, b, mix, out_coef, next_in, next_gain, eps, (TYPE*)normed, S, H, one, sum)
         if (dtype == LLMK_F32) {
             if (S <= 4) STREAM_STEP_VEC(float, 4); else STREAM_STEP_VEC(float, 8);
         } else {
@@ -998,7 +1012,7 @@ LLMK_EXPORT int llmk_stream_step(float* streams, const void* y, int splits, long
     do {                                                                                                                               \
         if (smem > 48 * 1024) cudaFuncSetAttribute(stream_step_kernel<TYPE, MS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         e = llmk_launch(stream_step_kernel<TYPE, MS>, dim3(n_rows), dim3(threads), smem, st, true, streams, y, splits, split_stride, y2, \
-                        splits2, split_stride2, a, b, mix, out_coef, next_in, next_gain, eps, (TYPE*)normed, S, H);                    \
+                        splits2, split_stride2, a, b, mix, out_coef, next_in, next_gain, eps, (TYPE*)normed, S, H, one, sum);          \
     } while (0)
     if (dtype == LLMK_F32) {
         if (S <= 4) STREAM_STEP_LAUNCH(float, 4); else if (S <= 8) STREAM_STEP_LAUNCH(float, 8); else STREAM_STEP_LAUNCH(float, 16);

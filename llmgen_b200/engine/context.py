@@ -173,6 +173,8 @@ class StepContext:
     max_seqs_bound: int = 0      # most sequences any step of this engine has
     serial: bool = False         # True: one kernel after the other (times of single kernels are being taken)
     side_stream: object = None   # a second stream for work that may run beside the step's own (None: there is none)
+    streams_equal: object = None     # a row per token that all residual streams still equal (they are not in memory yet)
+    streams_total: object = None     # where the last block leaves the sum of its streams (None: it leaves the streams)
     stream_copy_of: object = None   # the residual buffer whose rows the workspace's "stream_copy" holds in the storage dtype
 
     def array(self, name: str) -> torch.Tensor:

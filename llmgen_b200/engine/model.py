@@ -17,6 +17,7 @@ import torch
 from ..kernels import build as kernel_build
 from ..kernels import ops
 from ..parts.base import LayerCache
+from ..parts.block import MultiStreamBlock
 from ..parts.linear import linear
 from ..parts.reentry import Reentry
 from ..parts.registry import build_block, build_norm, model_kernel_modules
@@ -109,16 +110,23 @@ class DecoderModel:
         ctx.normed_for = None
         ctx.side_stream = None if ctx.serial else self.side_stream
         stream = resid
+        ctx.streams_equal = ctx.streams_total = None
         n_streams = int(getattr(self.spec, "residual_streams", 0) or 0)
         if n_streams > 0:
-            # layers that keep several residual streams: every stream starts as the embedding's output
+            # layers that keep several residual streams: every stream starts as the embedding's output, and is that row until a block
+            # rewrites them; the last block leaves their sum
             resid = ctx.workspace.buffer("residual_streams", T, n_streams * H, torch.float32)
-            ops.stream_spread(resid.view(T, n_streams, H), stream)
+            ctx.streams_equal = stream
         order = self.spec.run_order
         for n, (item, cache, before) in enumerate(zip(order, caches, self.before)):
+            keeps_streams = isinstance(self.layers[item.layer], MultiStreamBlock)
+            if ctx.streams_equal is not None and (before is not None or not keeps_streams):
+                ops.stream_spread(resid.view(T, n_streams, H), stream)
+                ctx.streams_equal = None
             if before is not None:
                 before.forward(ctx, resid, delta, x0)
                 delta = None
+            ctx.streams_total = stream if n_streams > 0 and keeps_streams and n + 1 == len(order) else None
             # blocks that prepare the next block's input are told which block that is (none behind a re-entry step)
             ctx.next_block = (self.layers[order[n + 1].layer] if n + 1 < len(order) and self.before[n + 1] is None else None)
             delta = self.layers[item.layer].forward(ctx, resid, delta, cache)
@@ -126,7 +134,11 @@ class DecoderModel:
         if n_streams > 0:
             if delta is not None:
                 raise ValueError("a model with residual streams is made of blocks that finish their own sums")
-            ops.stream_spread(resid.view(T, n_streams, H), stream, collapse=True)     # the stream is the sum of the streams
+            if ctx.streams_equal is not None:
+                ops.stream_spread(resid.view(T, n_streams, H), stream)
+            if ctx.streams_total is None:
+                ops.stream_spread(resid.view(T, n_streams, H), stream, collapse=True)     # the stream is the sum of the streams
+            ctx.streams_equal = ctx.streams_total = None
             resid = stream
         return resid, delta
 

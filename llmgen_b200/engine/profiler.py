@@ -455,7 +455,9 @@ def _cost_stream_step(a, info: PassInfo) -> Tuple[int, int]:
     n, S, H = a["streams"].shape
     wrote = a.get("y") is not None
     flops = n * H * ((2 * S * S + 2 * S if wrote else 0) + (2 * S + 5 if a.get("next_in") is not None else 0))
-    return flops, _nbytes(a["streams"]) * (2 if wrote else 1) + _nbytes(a.get("y")) + _nbytes(a.get("normed"))
+    read = _nbytes(a["streams"]) // (S if a.get("all_equal") is not None else 1)
+    written = _nbytes(a["streams"]) // (S if a.get("total") is not None else 1) if wrote else 0
+    return flops, read + written + _nbytes(a.get("y")) + _nbytes(a.get("normed"))
 
 
 def _cost_attn_prep_rows(a, info: PassInfo) -> Tuple[int, int]:

@@ -1003,11 +1003,14 @@ MAX_STREAMS = 16
 
 
 def stream_step(streams: torch.Tensor, y, mix: Optional[torch.Tensor], out_coef: Optional[torch.Tensor], next_in: Optional[torch.Tensor],
-                next_gain: Optional[torch.Tensor], eps: float, normed: Optional[torch.Tensor], dtype: torch.dtype) -> None:
+                next_gain: Optional[torch.Tensor], eps: float, normed: Optional[torch.Tensor], dtype: torch.dtype,
+                all_equal: Optional[torch.Tensor] = None, total: Optional[torch.Tensor] = None) -> None:
     """One step of a layer that keeps S residual streams per token, `streams` float32 [n, S, H] (csrc/rowwise.cu).  With `y` (a
     sublayer's output: an array of the storage dtype, a `Partials`, or a `WeightedPair` of two such): every stream is rewritten
     from all the old ones, x_t <- sum_s mix[s, t] x_s + out_coef[t] y.  With `next_in`: normed [n, H] (storage dtype) =
-    rmsnorm(sum_t next_in[t] x_t) * next_gain over the new streams.  Either half may be left out."""
+    rmsnorm(sum_t next_in[t] x_t) * next_gain over the new streams.  Either half may be left out.  `all_equal` (float32 [n, H]): every
+    stream still equals this row, which is read in their place; `total` (float32 [n, H], may be the same array): receives the sum of the new
+    streams, which are not written."""
     lib = build.load("rowwise")
     if streams.dtype != torch.float32 or streams.dim() != 3 or not streams.is_contiguous():
         raise KernelError("stream_step: the streams are a contiguous float32 [n, S, H] array")
@@ -1032,9 +1035,12 @@ def stream_step(streams: torch.Tensor, y, mix: Optional[torch.Tensor], out_coef:
     if next_in is not None and (next_in.numel() != S or next_gain is None or next_gain.numel() != H or normed is None
                                 or normed.dtype != dtype or tuple(normed.shape) != (n, H) or not normed.is_contiguous()):
         raise KernelError("stream_step: the next sublayer's input needs in [S], gains [H] and a place [n, H]")
+    for row in (all_equal, total):
+        if row is not None and (row.dtype != torch.float32 or tuple(row.shape) != (n, H) or not row.is_contiguous()):
+            raise KernelError("stream_step: rows that stand for all streams are float32 [n, H], contiguous")
     _check(lib, lib.llmk_stream_step(_ptr(streams), _ptr(src), c_int(splits), c_longlong(stride), _ptr(src2), c_int(splits2),
                                      c_longlong(stride2), c_float(a), c_float(b), _ptr(mix), _ptr(out_coef), _ptr(next_in),
-                                     _ptr(next_gain), c_float(eps), _ptr(normed), c_int(n), c_int(S), c_int(H),
+                                     _ptr(next_gain), c_float(eps), _ptr(normed), c_int(n), c_int(S), c_int(H), _ptr(all_equal), _ptr(total),
                                      c_int(dtype_code(dtype)), _stream()))
 
 

@@ -206,7 +206,8 @@ class MultiStreamBlock(Part):
     mult write[t] y, and in the same pass reads the streams for the sublayer that follows, norm(sum_t read[t] x_t) (the next block's
     mixer included, when the run list's next item is a block of this kind: the model names it in `ctx.next_block`).  The
     coefficients stay float32; `mult write` is folded at load.  A block whose input nobody prepared reads the streams itself.
-    It finishes its sums and hands on nothing to add."""
+    It finishes its sums and hands on nothing to add.  While `ctx.streams_equal` holds a row, the streams are all equal to it and not in
+    memory yet; with `ctx.streams_total` the block is the last one and leaves the sum of its streams there, not the streams."""
 
     @staticmethod
     def weight_decls(spec: MultiStreamBlockSpec):
@@ -277,22 +278,25 @@ class MultiStreamBlock(Part):
             raise ValueError("multi-stream block: it runs on the model's array of streams and takes no pending sum")
         streams = resid.view(T, self.S, H)
         normed = ctx.workspace.buffer("block_normed", T, H, self.dtype)
+        equal, total = getattr(ctx, "streams_equal", None), getattr(ctx, "streams_total", None)
         if getattr(ctx, "normed_for", None) is not self:
-            ops.stream_step(streams, None, None, None, self.read1, self.gain1, self.mixer_norm.eps, normed, self.dtype)
+            ops.stream_step(streams, None, None, None, self.read1, self.gain1, self.mixer_norm.eps, normed, self.dtype, all_equal=equal)
         ctx.normed_for = None
         follower = getattr(ctx, "next_block", None)
         follow = follower if isinstance(follower, MultiStreamBlock) and follower.S == self.S else None
         mixed = self.mixer.forward(ctx, normed, cache)
         if self.ffn is not None:
-            ops.stream_step(streams, mixed, self.mix1, self.write1, self.read2, self.gain2, self.ffn_norm.eps, normed, self.dtype)
+            ops.stream_step(streams, mixed, self.mix1, self.write1, self.read2, self.gain2, self.ffn_norm.eps, normed, self.dtype, all_equal=equal)
+            equal = None
             mixed = self.ffn.forward(ctx, normed)
             mix, write = self.mix2, self.write2
         else:
             mix, write = self.mix1, self.write1
         if follow is not None:
-            ops.stream_step(streams, mixed, mix, write, follow.read1, follow.gain1, follow.mixer_norm.eps, normed, self.dtype)
+            ops.stream_step(streams, mixed, mix, write, follow.read1, follow.gain1, follow.mixer_norm.eps, normed, self.dtype, all_equal=equal)
         else:
-            ops.stream_step(streams, mixed, mix, write, None, None, 0.0, None, self.dtype)
+            ops.stream_step(streams, mixed, mix, write, None, None, 0.0, None, self.dtype, all_equal=equal, total=total)
+        ctx.streams_equal = None
         ctx.normed_for = follow
         return None
 
