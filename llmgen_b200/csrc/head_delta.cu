@@ -9,7 +9,8 @@
 //                       the outputs  o_i = e^(L_i) S^T q_i + sum_(j <= i) e^(L_i - L_j) (q_i . k_j) u_j,  and the state after the chunk
 //                       e^(L_n) S + sum_j e^(L_n - L_j) k_j u_j^T.  What does not need the state (the two triangular systems' solutions
 //                       W = (I + M)^-1 diag(beta e^L) K and (I + M)^-1 diag(beta) V, the matrix of the read-out) is made for all chunks
-//                       side by side; the walk over the chunks then touches the state once a chunk instead of once a token
+//                       side by side; the walk over the chunks then touches the state once a chunk instead of once a token, and leaves it for
+//                       the outputs, again of all chunks side by side
 //   head_delta_step     steps of a few tokens (single decoded tokens above all) in one launch: all of the preparation, the
 //                       recurrence, each head's RMSNorm and the gate silu(z)
 //
@@ -450,7 +451,8 @@ struct ChunkParams {
     float* qs;               // [places][G][CHUNK][DP]
     float* ks;               // [places][G][CHUNK * DP], in the order the walk's threads read it: see `key_place`
     float* w;                // [places][H][CHUNK][DP]
-    float* uv;               // [places][H][CHUNK][EP]
+    float* uv;               // [places][H][CHUNK][EP]: (I + M)^-1 diag(beta) V, rewritten by the walk as U
+    float* states;           // [places][H][DP][EP]: the state before each chunk
     float* p;                // [places][H][CHUNK][CHUNK]
     float* dec;              // [places][H][2][CHUNK]: e^(L_i), e^(L_n - L_i)
     int n_seqs, n_tokens, H, G, D, E, EP, vec_ok;
@@ -693,30 +695,30 @@ __device__ __forceinline__ void reduce_scatter(float (&v)[N], int lane) {
     }
 }
 
-// The walk: block (sequence, head, COLS value columns), the state's columns in shared memory.  A chunk takes three steps:
-//   1  rows of W and of Q times S: a thread has 4 rows, all columns, and one of 8 slices of the key channels; warps 0 .. 3 hold W's rows
-//      and leave U, warps 4 .. 7 hold Q's
+// The walk: block (sequence, head, COLS value columns), the state's columns in shared memory.  It leaves the state before every chunk
+// and the chunk's U to `chunk_out_kernel`, which makes the outputs of all chunks side by side; what is left of a chunk takes two steps:
+//   1  U = (..) - W S: a thread has 4 rows of W, all columns, and one of 16 slices of the key channels
 //   2  S <- e^(L_n) S + K^T (U scaled): a thread has 4 key channels, all columns, and one slice of the chunk's tokens
-//   3  (warps 4 .. 7) the outputs: e^(L_i) times the rows of step 1 + P U
-// Operands of W, Q, K and P are used by one thread each and go from global memory straight into registers, asked for a step ahead.
+// Operands are used by one thread each and go from global memory straight into registers, asked for a step ahead.  What bounds it is the
+// chain of a chunk's steps (two barriers, two sums over lanes) on eight warps an SM; with the outputs in the walk, a third of the operations
+// more and a third step, 2,048 tokens of 16 heads of 128 x 128 took 209 us.
 template <int DP, int COLS>
 __global__ void __launch_bounds__(CTHREADS) chunk_scan_kernel(ChunkParams p) {
-    constexpr int KR = DP / 32;                    // runs of four key channels a thread has in step 1
+    constexpr int SL = 16, KR = DP > 4 * SL ? DP / (4 * SL) : 1;      // slices of key channels in step 1, runs of four channels of a slice
     constexpr int TS = CTHREADS / (DP / 4);        // slices of tokens in step 2
     constexpr int TR = CHUNK / TS;                 // tokens of one
     constexpr int SQ = 4 * COLS + 4;               // four rows of S side by side, padded: slices read different banks
     constexpr int UL = COLS + 4;                   // a row of U
     constexpr int NV = 4 * COLS;                   // outputs of a thread before the slices are summed up
+    constexpr int KEEP = NV / SL;                  // what a lane keeps of them: 2 or 4 values of one row
     __shared__ __align__(16) float S[DP / 4 * SQ];
-    __shared__ __align__(16) float U[2][CHUNK / 4 * SQ];   // as the outputs read it (four rows side by side), two chunks in turn
-    __shared__ __align__(16) float Ud[CHUNK * UL];         // times e^(L_n - L_j)
+    __shared__ __align__(16) float Ud[CHUNK * UL];         // U times e^(L_n - L_j)
     const int s = blockIdx.x, h = blockIdx.y, e0 = blockIdx.z * COLS, tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int kvh = h / (p.H / p.G);
-    const int ks = lane & 7, rt = warp * 4 + (lane >> 3);  // slice of key channels, row tile (0 .. 15: W, 16 .. 31: Q)
-    const bool reads_out = rt >= 16;
-    const int row0 = (reads_out ? rt - 16 : rt) * 4;
+    const int ks = lane & (SL - 1), row0 = (warp * 2 + lane / SL) * 4;
     const int ts = tid & (TS - 1), d0 = tid / TS * 4;
+    const int row = row0 + ks * KEEP / COLS, col = ks * KEEP % COLS;
     pdl_launch_dependents();
     pdl_wait();
     const int q_beg = p.cu_q[s], n = p.cu_q[s + 1] - q_beg;
@@ -728,14 +730,27 @@ __global__ void __launch_bounds__(CTHREADS) chunk_scan_kernel(ChunkParams p) {
         S[(d >> 2) * SQ + (d & 3) * COLS + c] = (st && d < D && e0 + c < E) ? st[(size_t)d * E + e0 + c] : 0.f;
     }
     const int place0 = q_beg / CHUNK + s, chunks = ceil_div(n, CHUNK);
-    float4 a4[4][KR], k4[TR], p4[4][2];
+    float4 a4[4][KR], k4[TR];
+    float uv[KEEP], scale, keep;
     auto load_rows = [&](int c) {
-        const size_t place = place0 + c;
-        const float* src = reads_out ? p.qs + ((place * p.G + kvh) * CHUNK + row0) * DP : p.w + ((place * p.H + h) * CHUNK + row0) * DP;
+        const size_t ph = (size_t)(place0 + c) * p.H + h;
+        const float* src = p.w + (ph * CHUNK + row0) * DP;
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int i = 0; i < KR; ++i) a4[r][i] = *reinterpret_cast<const float4*>(src + r * DP + i * 32 + ks * 4);
+            for (int i = 0; i < KR; ++i)
+                if ((i * SL + ks) * 4 < DP) a4[r][i] = *reinterpret_cast<const float4*>(src + r * DP + (i * SL + ks) * 4);
+        const float* u = p.uv + (ph * CHUNK + row) * p.EP + e0 + col;
+        if constexpr (KEEP == 4) {
+            const float4 x = *reinterpret_cast<const float4*>(u);
+            uv[0] = x.x; uv[1] = x.y; uv[2] = x.z; uv[3] = x.w;
+        } else {
+            const float2 x = *reinterpret_cast<const float2*>(u);
+            uv[0] = x.x; uv[1] = x.y;
+        }
+        const float* dec = p.dec + ph * 2 * CHUNK;
+        scale = dec[CHUNK + row];
+        keep = dec[CHUNK - 1];
     };
     auto load_keys = [&](int c) {
         const float* src = p.ks + ((size_t)(place0 + c) * p.G + kvh) * CHUNK * DP + tid * 4;
@@ -747,13 +762,18 @@ __global__ void __launch_bounds__(CTHREADS) chunk_scan_kernel(ChunkParams p) {
     __syncthreads();
     for (int c = 0; c < chunks; ++c) {
         const size_t ph = (size_t)(place0 + c) * p.H + h;
-        const float* dec = p.dec + ph * 2 * CHUNK;
+        // the state before the chunk
+        for (int idx = tid; idx < DP * COLS / 4; idx += CTHREADS) {
+            const int d = idx / (COLS / 4), c4 = idx % (COLS / 4) * 4;
+            *reinterpret_cast<float4*>(p.states + (ph * DP + d) * p.EP + e0 + c4) = *reinterpret_cast<const float4*>(S + (d >> 2) * SQ + (d & 3) * COLS + c4);
+        }
         float v[NV];
 #pragma unroll
         for (int i = 0; i < NV; ++i) v[i] = 0.f;
 #pragma unroll
         for (int i = 0; i < KR; ++i) {
-            const float* sr = S + (i * 8 + ks) * SQ;
+            if ((i * SL + ks) * 4 >= DP) break;
+            const float* sr = S + (i * SL + ks) * SQ;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 float4 sv[COLS / 4];
@@ -772,37 +792,24 @@ __global__ void __launch_bounds__(CTHREADS) chunk_scan_kernel(ChunkParams p) {
                 }
             }
         }
-        // what the slices add up to: this lane keeps NV / 8 values of one row
-        constexpr int KEEP = NV / 8;
-        const int at = ks * KEEP, row = row0 + at / COLS, col = at % COLS;
-        float4 uv[KEEP / 4];
-        if (!reads_out) {
+        reduce_scatter<NV, SL>(v, ks);
+        {
+            float x[KEEP];
 #pragma unroll
-            for (int u = 0; u < KEEP / 4; ++u) uv[u] = *reinterpret_cast<const float4*>(p.uv + (ph * CHUNK + row) * p.EP + e0 + col + 4 * u);
-        }
-        const float scale = reads_out ? dec[row] : dec[CHUNK + row], keep = dec[CHUNK - 1];
-        reduce_scatter<NV, 8>(v, ks);
-        float* ur = U[c & 1];
-        if (!reads_out) {
-#pragma unroll
-            for (int u = 0; u < KEEP / 4; ++u) {
-                const float4 x = make_float4(uv[u].x - v[4 * u], uv[u].y - v[4 * u + 1], uv[u].z - v[4 * u + 2], uv[u].w - v[4 * u + 3]);
-                *reinterpret_cast<float4*>(ur + (row >> 2) * SQ + (row & 3) * COLS + col + 4 * u) = x;
-                *reinterpret_cast<float4*>(Ud + row * UL + col + 4 * u) = make_float4(scale * x.x, scale * x.y, scale * x.z, scale * x.w);
+            for (int u = 0; u < KEEP; ++u) x[u] = uv[u] - v[u];
+            float* to = p.uv + (ph * CHUNK + row) * p.EP + e0 + col;
+            float* ud = Ud + row * UL + col;
+            if constexpr (KEEP == 4) {
+                *reinterpret_cast<float4*>(to) = make_float4(x[0], x[1], x[2], x[3]);
+                *reinterpret_cast<float4*>(ud) = make_float4(scale * x[0], scale * x[1], scale * x[2], scale * x[3]);
+            } else {
+                *reinterpret_cast<float2*>(to) = make_float2(x[0], x[1]);
+                *reinterpret_cast<float2*>(ud) = make_float2(scale * x[0], scale * x[1]);
             }
         }
-        float o[KEEP];
-#pragma unroll
-        for (int i = 0; i < KEEP; ++i) o[i] = scale * v[i];
+        const float decay = keep;
         __syncthreads();                     // U is there, and S has been read
         if (c + 1 < chunks) load_rows(c + 1);
-        if (reads_out) {
-            const float* src = p.p + (ph * CHUNK + row0) * CHUNK;
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) p4[r][i] = *reinterpret_cast<const float4*>(src + r * CHUNK + i * 32 + ks * 4);
-        }
 #pragma unroll
         for (int i = 0; i < NV; ++i) v[i] = 0.f;
 #pragma unroll
@@ -831,55 +838,119 @@ __global__ void __launch_bounds__(CTHREADS) chunk_scan_kernel(ChunkParams p) {
 #pragma unroll
                 for (int u = 0; u < KEEP2 / 4; ++u) {
                     float4 x = *reinterpret_cast<float4*>(sr + 4 * u);
-                    x.x = fmaf(keep, x.x, v[4 * u]);
-                    x.y = fmaf(keep, x.y, v[4 * u + 1]);
-                    x.z = fmaf(keep, x.z, v[4 * u + 2]);
-                    x.w = fmaf(keep, x.w, v[4 * u + 3]);
+                    x.x = fmaf(decay, x.x, v[4 * u]);
+                    x.y = fmaf(decay, x.y, v[4 * u + 1]);
+                    x.z = fmaf(decay, x.z, v[4 * u + 2]);
+                    x.w = fmaf(decay, x.w, v[4 * u + 3]);
                     *reinterpret_cast<float4*>(sr + 4 * u) = x;
                 }
             } else {
 #pragma unroll
-                for (int i = 0; i < KEEP2; ++i) sr[i] = fmaf(keep, sr[i], v[i]);
+                for (int i = 0; i < KEEP2; ++i) sr[i] = fmaf(decay, sr[i], v[i]);
             }
         }
         __syncthreads();                     // S is the state after the chunk
-        if (reads_out) {
-#pragma unroll
-            for (int i = 0; i < NV; ++i) v[i] = 0.f;
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float* uj = ur + (i * 8 + ks) * SQ + q * COLS;
-                    float4 u4[COLS / 4];
-#pragma unroll
-                    for (int u = 0; u < COLS / 4; ++u) u4[u] = *reinterpret_cast<const float4*>(uj + 4 * u);
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        const float w = q == 0 ? p4[r][i].x : q == 1 ? p4[r][i].y : q == 2 ? p4[r][i].z : p4[r][i].w;
-#pragma unroll
-                        for (int u = 0; u < COLS / 4; ++u) {
-                            v[r * COLS + 4 * u] = fmaf(w, u4[u].x, v[r * COLS + 4 * u]);
-                            v[r * COLS + 4 * u + 1] = fmaf(w, u4[u].y, v[r * COLS + 4 * u + 1]);
-                            v[r * COLS + 4 * u + 2] = fmaf(w, u4[u].z, v[r * COLS + 4 * u + 2]);
-                            v[r * COLS + 4 * u + 3] = fmaf(w, u4[u].w, v[r * COLS + 4 * u + 3]);
-                        }
-                    }
-                }
-            }
-            reduce_scatter<NV, 8>(v, ks);
-            if (c * CHUNK + row < n) {
-                float* dst = p.out + (size_t)(q_beg + c * CHUNK + row) * ((size_t)p.H * E) + (size_t)h * E + e0 + col;
-#pragma unroll
-                for (int i = 0; i < KEEP; ++i)
-                    if (e0 + col + i < E) dst[i] = o[i] + v[i];
-            }
-        }
     }
     if (st) {
         for (int idx = tid; idx < DP * COLS; idx += CTHREADS) {
             const int d = idx / COLS, c = idx % COLS;
             if (d < D && e0 + c < E) st[(size_t)d * E + e0 + c] = S[(d >> 2) * SQ + (d & 3) * COLS + c];
+        }
+    }
+}
+
+// The outputs of all chunks side by side: block (place, head, 128 value columns), o_i = e^(L_i) S^T q_i + sum_j P_ij u_j as one product
+// of 64 rows over key channels, then tokens, in slices of 16 by cp.async in a ring of three.  A thread has rows ty + 8 i and columns
+// 4 tx .. and 64 + 4 tx ..: 64 sums from 16 values read a step, which keeps the multiply-adds and the reads of shared memory even.
+constexpr int OTHREADS = 128, OK = 16, OROWS = CHUNK, OCOLS = 128, OLD = OK + 4, OSTAGES = 3;
+template <int DP>
+__global__ void __launch_bounds__(OTHREADS) chunk_out_kernel(ChunkParams p) {
+    __shared__ __align__(16) float As[OSTAGES][OROWS * OLD];
+    __shared__ __align__(16) float Bs[OSTAGES][OK * OCOLS];
+    const int place = blockIdx.x, h = blockIdx.y, e0 = blockIdx.z * OCOLS, tid = threadIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
+    int lo = 0, hi = p.n_seqs;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (p.cu_q[mid] / CHUNK + mid <= place) lo = mid; else hi = mid;
+    }
+    const int q_beg = p.cu_q[lo], first = (place - q_beg / CHUNK - lo) * CHUNK;
+    const int n = min(CHUNK, p.cu_q[lo + 1] - q_beg - first);
+    if (n <= 0) return;
+    const size_t ph = (size_t)place * p.H + h;
+    const int cols = min(OCOLS, p.EP - e0);            // a multiple of 16
+    const float* q = p.qs + ((size_t)place * p.G + h / (p.H / p.G)) * CHUNK * DP;
+    const float* P = p.p + ph * CHUNK * CHUNK;
+    const float* S = p.states + ph * DP * p.EP + e0;
+    const float* U = p.uv + ph * CHUNK * p.EP + e0;
+    constexpr int FIRST = DP / OK, SLICES = FIRST + CHUNK / OK;
+    auto load = [&](int i) {
+        if (i < SLICES) {
+            const bool inner = i >= FIRST;
+            const int k0 = (inner ? i - FIRST : i) * OK, ld = inner ? CHUNK : DP;
+            const float* a = (inner ? P : q) + k0;
+            const float* b = (inner ? U : S) + (size_t)k0 * p.EP;
+            for (int idx = tid; idx < OROWS * OK / 4; idx += OTHREADS)
+                cp_async16(As[i % OSTAGES] + idx / (OK / 4) * OLD + idx % (OK / 4) * 4, a + (size_t)(idx / (OK / 4)) * ld + idx % (OK / 4) * 4);
+            for (int idx = tid; idx < OK * OCOLS / 4; idx += OTHREADS) {
+                const int k = idx / (OCOLS / 4), c = idx % (OCOLS / 4) * 4;
+                if (c < cols) cp_async16(Bs[i % OSTAGES] + k * OCOLS + c, b + (size_t)k * p.EP + c);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int tx = tid % 16, ty = tid / 16;
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int i = 0; i < OSTAGES - 1; ++i) load(i);
+    for (int s = 0; s < SLICES; ++s) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(OSTAGES - 2) : "memory");
+        __syncthreads();                     // the slice is there, and the one before has been read
+        load(s + OSTAGES - 1);
+        if (s == FIRST) {
+            const float* dec = p.dec + ph * 2 * CHUNK;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float scale = dec[ty + 8 * i];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][j] *= scale;
+            }
+        }
+        const float* a = As[s % OSTAGES] + ty * OLD;
+        const float* b = Bs[s % OSTAGES] + tx * 4;
+#pragma unroll
+        for (int k = 0; k < OK; k += 4) {
+            float4 av[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) av[i] = *reinterpret_cast<const float4*>(a + 8 * i * OLD + k);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float4 b0 = *reinterpret_cast<const float4*>(b + (k + u) * OCOLS), b1 = *reinterpret_cast<const float4*>(b + (k + u) * OCOLS + 64);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float x = u == 0 ? av[i].x : u == 1 ? av[i].y : u == 2 ? av[i].z : av[i].w;
+                    acc[i][0] = fmaf(x, b0.x, acc[i][0]); acc[i][1] = fmaf(x, b0.y, acc[i][1]);
+                    acc[i][2] = fmaf(x, b0.z, acc[i][2]); acc[i][3] = fmaf(x, b0.w, acc[i][3]);
+                    acc[i][4] = fmaf(x, b1.x, acc[i][4]); acc[i][5] = fmaf(x, b1.y, acc[i][5]);
+                    acc[i][6] = fmaf(x, b1.z, acc[i][6]); acc[i][7] = fmaf(x, b1.w, acc[i][7]);
+                }
+            }
+        }
+    }
+    const int E = p.E;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int row = ty + 8 * i;
+        if (row >= n) continue;
+        float* dst = p.out + (size_t)(q_beg + first + row) * ((size_t)p.H * E) + (size_t)h * E;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int e = e0 + (j & 4) * 16 + tx * 4 + (j & 3);
+            if (e < E) dst[e] = acc[i][j];
         }
     }
 }
@@ -891,7 +962,7 @@ static int chunk_places(int n_tokens, int n_seqs) { return n_tokens / CHUNK + st
 LLMK_EXPORT long long llmk_head_delta_chunk_floats(int n_tokens, int n_seqs, int H, int G, int D, int E) {
     if (n_tokens <= 0 || n_seqs <= 0 || D <= 0 || D > 128 || E <= 0 || H <= 0 || G <= 0) return 0;
     const long long dp = chunk_width(D), ep = ceil_div(E, 16) * 16;
-    return (long long)chunk_places(n_tokens, n_seqs) * CHUNK * (2 * G * dp + H * (dp + ep + CHUNK + 2));
+    return (long long)chunk_places(n_tokens, n_seqs) * (CHUNK * (2 * G * dp + H * (dp + ep + CHUNK + 2)) + H * dp * ep);
 }
 
 template <int DP>
@@ -907,9 +978,11 @@ static cudaError_t launch_chunks(const ChunkParams& p, int places, cudaStream_t 
     cudaError_t e = llmk_launch(chunk_prep_kernel<DP>, dim3(places, p.H), dim3(CTHREADS), smem, s, true, p);
     if (e != cudaSuccess) return e;
     // sixteen columns a block where eight would not fit the SMs side by side
-    if (p.H * ceil_div(p.E, 8) <= device_sm_count())
-        return llmk_launch(chunk_scan_kernel<DP, 8>, dim3(p.n_seqs, p.H, ceil_div(p.E, 8)), dim3(CTHREADS), 0, s, true, p);
-    return llmk_launch(chunk_scan_kernel<DP, 16>, dim3(p.n_seqs, p.H, ceil_div(p.E, 16)), dim3(CTHREADS), 0, s, true, p);
+    e = p.H * ceil_div(p.E, 8) <= device_sm_count()
+            ? llmk_launch(chunk_scan_kernel<DP, 8>, dim3(p.n_seqs, p.H, p.EP / 8), dim3(CTHREADS), 0, s, true, p)
+            : llmk_launch(chunk_scan_kernel<DP, 16>, dim3(p.n_seqs, p.H, p.EP / 16), dim3(CTHREADS), 0, s, true, p);
+    if (e != cudaSuccess) return e;
+    return llmk_launch(chunk_out_kernel<DP>, dim3(places, p.H, ceil_div(p.EP, OCOLS)), dim3(OTHREADS), 0, s, true, p);
 }
 
 // scratch: llmk_head_delta_chunk_floats(...) floats on a 16-byte boundary.  qkv and gates as `head_delta_prep` leaves them.
@@ -931,6 +1004,7 @@ LLMK_EXPORT int llmk_head_delta_chunks(float* out, const float* qkv, const float
     p.uv = p.w + rows * H * dp;
     p.p = p.uv + rows * H * ep;
     p.dec = p.p + rows * H * CHUNK;
+    p.states = p.dec + rows * H * 2;
     p.n_seqs = n_seqs; p.n_tokens = n_tokens; p.H = H; p.G = G; p.D = D; p.E = E; p.EP = (int)ep;
     p.vec_ok = (D % 4 == 0 && E % 4 == 0 && (2 * G * D + H * E) % 4 == 0 && host_aligned16(qkv)) ? 1 : 0;
     cudaStream_t s = (cudaStream_t)stream;
