@@ -4,7 +4,7 @@
 // epilogue warps read it back with `tcgen05.ld`, round once and store.
 //
 // A block computes 128 x BN output tiles (BN = 64, 128 or 256) one after the other, 192 threads
-// (or two blocks of a cluster compute tiles of 256 rows together, see `gemm_pair_kernel`):
+// (from 4,096 rows on, two blocks of a cluster compute 256 x 256 tiles together, see PAIR below):
 //   warp 0     TMA producer: for every 64-wide slice of K, one A box [128, 64] and one W box
 //              [BN, 64] into a ring of STAGES buffers; `full[s]` counts the bytes.
 //   warp 1     owns the tensor memory (two accumulators of BN columns) and issues the MMAs: 4
@@ -31,7 +31,6 @@
 #include "common.cuh"
 #include "tcgen05.cuh"
 
-#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
@@ -44,11 +43,11 @@ constexpr int BK = 64;           // one 128-byte swizzle row of bfloat16
 constexpr int UMMA_K = 16;
 constexpr int THREADS = 192;
 
-template <int W_ROWS, int STAGES, int KS = 1>
+template <int BN, int STAGES, int MB, bool PAIR = false, int KS = 1>
 struct Smem {
     static constexpr int A_BYTES = BM * BK * 2;        // one block of 128 rows of A
-    static constexpr int B_BYTES = W_ROWS * BK * 2;
-    static constexpr int SUB_BYTES = A_BYTES + B_BYTES;             // one step of 64 along K: A, then W
+    static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;   // a pair's blocks hold half of the W rows each
+    static constexpr int SUB_BYTES = MB * A_BYTES + B_BYTES;        // one step of 64 along K: A blocks, then W
     static constexpr int STAGE_BYTES = KS * SUB_BYTES;              // a stage of the ring holds KS such steps
     // the epilogue's staging: per epilogue warp two slabs of 32 rows x 64 bfloat16 columns (128-byte swizzle)
     static constexpr int SLAB_BYTES = 32 * 128;
@@ -82,169 +81,34 @@ __device__ __forceinline__ float gate_act(float g) {
 }
 
 
-// What the epilogue warps do with one tile: `acc` is the warp's 32 lanes of an accumulator of `width` columns (a multiple of 32), its
-// rows are row0 .. row0 + 31 and its columns begin at n0.
-template <typename TC, int ACT>
-__device__ __forceinline__ void store_tile(const CUtensorMap& map_c, int store_by_tma, uint32_t slabs, uint32_t& box_iter, uint32_t acc,
-                                           int row0, int n0, int width, int split, TC* __restrict__ C, int M, int N, long long ldc) {
-    constexpr bool GATED = is_glu(ACT);
-    constexpr int SLAB_BYTES = 32 * 128;
-    const int lane = threadIdx.x & 31;
-    if (row0 >= M) return;                                  // uniform over the warp
-    int c0 = 0;
-    if constexpr (sizeof(TC) == 2) {
-        if (store_by_tma) {
-            // Row-per-thread stores to global memory are slow and hold up the TMA loads of the next
-            // tile (measured: 4.3 us a tile against 1 us without them).  Each warp rounds its 32
-            // rows into a slab of shared memory, 64 output columns at a time, in the layout of a
-            // 128-byte-swizzled box (a lane's 16-byte pieces then fall into different banks), and
-            // one lane hands the slab to TMA, which writes whole rows and clips at M and N.
-            constexpr int ACC_COLS = GATED ? 128 : 64;          // accumulator columns per 64 output columns
-#pragma unroll 1
-            for (; c0 + ACC_COLS <= width; c0 += ACC_COLS) {
-                if (n0 + c0 >= N) return;
-                const uint32_t slab = slabs + (uint32_t)(box_iter & 1) * SLAB_BYTES;
-                if (lane == 0) tc::bulk_wait_read<1>();         // the store that read this slab two boxes ago
-                __syncwarp();
-#pragma unroll
-                for (int h = 0; h < ACC_COLS / 32; ++h) {
-                    uint32_t r[32];
-                    tc::tmem_ld_32x32_wait(acc + (uint32_t)(c0 + 32 * h), r);
-                    if constexpr (GATED) {
-                        float o[16];
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = gate_act<ACT>(__uint_as_float(r[i])) * __uint_as_float(r[16 + i]);
-#pragma unroll
-                        for (int q = 0; q < 2; ++q) {
-                            Vec16<bf16> v;
-                            v.pack(o + 8 * q);
-                            const int chunk = 2 * h + q;
-                            tc::st_shared_v4(slab + (uint32_t)lane * 128 + (uint32_t)((chunk ^ (lane & 7)) << 4), v.raw);
-                        }
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            float f[8];
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) f[j] = plain_act<ACT>(__uint_as_float(r[8 * q + j]));
-                            Vec16<bf16> v;
-                            v.pack(f);
-                            const int chunk = 4 * h + q;
-                            tc::st_shared_v4(slab + (uint32_t)lane * 128 + (uint32_t)((chunk ^ (lane & 7)) << 4), v.raw);
-                        }
-                    }
-                }
-                tc::fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) {
-                    tc::tma_store_2d(&map_c, slab, GATED ? (n0 + c0) / 2 : n0 + c0, row0);
-                    tc::bulk_commit();
-                }
-                ++box_iter;
-            }
-        }
-    }
-    if constexpr (sizeof(TC) == 4 && !GATED) {
-        if (store_by_tma) {
-            // float32 slices: slabs of 32 rows x 32 columns (128 bytes a row), handed to TMA the same way
-#pragma unroll 1
-            for (; c0 < width; c0 += 32) {
-                if (n0 + c0 >= N) return;
-                const uint32_t slab = slabs + (uint32_t)(box_iter & 1) * SLAB_BYTES;
-                if (lane == 0) tc::bulk_wait_read<1>();
-                __syncwarp();
-                uint32_t r[32];
-                tc::tmem_ld_32x32_wait(acc + (uint32_t)c0, r);
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    tc::st_shared_v4(slab + (uint32_t)lane * 128 + (uint32_t)((q ^ (lane & 7)) << 4),
-                                     make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]));
-                tc::fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) {
-                    tc::tma_store_3d(&map_c, slab, n0 + c0, row0, split);
-                    tc::bulk_commit();
-                }
-                ++box_iter;
-            }
-        }
-    }
-    // results TMA cannot address, and a last half of a box
-    const int row = row0 + lane;
-    const int n_out = GATED ? N / 2 : N;
-    const bool vec_ok = (ldc % (16 / (int)sizeof(TC)) == 0) && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
-#pragma unroll 1
-    for (; c0 < width; c0 += 32) {
-        if (n0 + c0 >= N) return;                           // uniform over the warp
-        uint32_t r[32];
-        __syncwarp();
-        tc::tmem_ld_32x32_wait(acc + (uint32_t)c0, r);
-        if (row >= M) {
-            // nothing to store for this lane; it still takes part in the loads above
-        } else if constexpr (GATED) {
-            // columns [c0, c0 + 16) are gates, [c0 + 16, c0 + 32) the matching ups
-            const int j0 = (n0 + c0) / 2;
-            float o[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = gate_act<ACT>(__uint_as_float(r[i])) * __uint_as_float(r[16 + i]);
-            TC* dst = C + (size_t)row * ldc + j0;
-            if (vec_ok && j0 + 16 <= n_out) {
-                if constexpr (sizeof(TC) == 2) {
-                    Vec16<bf16> v0, v1;
-                    v0.pack(o);
-                    v1.pack(o + 8);
-                    reinterpret_cast<uint4*>(dst)[0] = v0.raw;
-                    reinterpret_cast<uint4*>(dst)[1] = v1.raw;
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        reinterpret_cast<float4*>(dst)[i] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-                }
-            } else {
-                for (int i = 0; i < 16; ++i)
-                    if (j0 + i < n_out) dst[i] = from_float<TC>(o[i]);
-            }
-        } else {
-            TC* dst = C + ((size_t)split * M + row) * ldc + n0 + c0;
-            if (vec_ok && n0 + c0 + 32 <= N) {
-                if constexpr (sizeof(TC) == 2) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        float f[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) f[j] = plain_act<ACT>(__uint_as_float(r[8 * i + j]));
-                        Vec16<bf16> v;
-                        v.pack(f);
-                        reinterpret_cast<uint4*>(dst)[i] = v.raw;
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        reinterpret_cast<float4*>(dst)[i] =
-                            make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
-                                        __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
-                }
-            } else {
-                for (int i = 0; i < 32; ++i)
-                    if (n0 + c0 + i < N) dst[i] = from_float<TC>(plain_act<ACT>(__uint_as_float(r[i])));
-            }
-        }
-    }
-}
-
 // Persistent: block b computes tiles b, b + gridDim.x, ... (tile t = (t % m_tiles) rows, (t / m_tiles)
-// columns, so blocks that run together share W tiles).  Two accumulators of BN columns are used in turn: while
+// columns, so blocks that run together share W tiles).  A tile is MB blocks of 128 rows by BN
+// columns: with MB = 2 the two MMAs of a k-step share the W tile, which halves what the block pulls
+// from L2 per flop (the wide products are bound by that, not by the tensor core).  When two
+// accumulator sets fit into tensor memory (2 * MB * BN <= 512 columns) they are used in turn: while
 // the epilogue warps read tile i out of one, the MMA warp fills the other with tile i + 1; the TMA
 // ring runs on across tiles either way.
-template <typename TC, int BN, int STAGES, int ACT, int KS = 1>
+//
+// PAIR: the kernel runs as clusters of two blocks (an SM pair) and a tile is 256 rows by BN columns,
+// computed by `tcgen05.mma.cta_group::2`.  Each block loads its 128 rows of A and its half of the W
+// rows (no multicast: every block loads what it holds), so a block pulls A + W/2 per k-step where a
+// lone block pulls A + W: the wide products are bound by what the SMs pull from L2.  The bytes of
+// both blocks are counted on the `full` barriers of the block of rank 0, which issues the MMAs; its
+// commits arrive on the `empty` and `acc_full` barriers of both blocks; the epilogue warps of both
+// release an accumulator set on rank 0's `acc_empty`.  Each block reads its own 128 rows of the
+// accumulator out of its own tensor memory.
+template <typename TC, int BN, int STAGES, int ACT, int MB, bool PAIR = false, int KS = 1>
 __global__ void __launch_bounds__(THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ CUtensorMap map_c, int store_by_tma, int splits,
                TC* __restrict__ C, int M, int N, int K, long long ldc, int* error_flag,
                const int* __restrict__ tile_group) {
-    using L = Smem<BN, STAGES, KS>;
-    constexpr int W_OFF = KS * L::A_BYTES;          // a stage: A's KS steps, then W's
-    constexpr uint32_t TMEM_COLS = 2 * BN;                         // 128, 256 or 512: a power of two
+    static_assert(!PAIR || MB == 1, "a pair of blocks takes one block of rows each");
+    constexpr bool GATED = is_glu(ACT);
+    using L = Smem<BN, STAGES, MB, PAIR, KS>;
+    constexpr int ROWS = (PAIR ? 2 : MB) * BM;                     // rows of a tile
+    constexpr int ACC_SETS = 2 * MB * BN <= 512 ? 2 : 1;
+    constexpr uint32_t TMEM_COLS = ACC_SETS * MB * BN;             // 128, 256 or 512: a power of two
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
@@ -255,9 +119,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NUM_BARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same for all lanes, and known to be)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_kb = (K + BK - 1) / BK;
-    const int m_tiles = (M + BM - 1) / BM;
+    const int m_tiles = (M + ROWS - 1) / ROWS;
     const int n_tiles = (N + BN - 1) / BN;
     const int total_tiles = m_tiles * n_tiles;
     // K may be cut into `splits` slices (float32 results only): work item i is slice i / total_tiles of tile
@@ -266,7 +130,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // a stage of the ring holds KS steps of 64 along K under one barrier (the hand-over of a stage costs about as
     // much as the copy of a narrow tile's step, so narrow tiles take two steps a stage); a slice begins on a stage
     const int kb_per_split = ((num_kb + splits - 1) / splits + KS - 1) / KS * KS;
-    const int unit = (int)blockIdx.x, units = (int)gridDim.x;
+    const uint32_t rank = PAIR ? cluster_ctarank() : 0u;           // which block of the pair
+    const int unit = PAIR ? (int)blockIdx.x / 2 : (int)blockIdx.x; // this block's (or pair's) place in the grid
+    const int units = PAIR ? (int)gridDim.x / 2 : (int)gridDim.x;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
@@ -276,45 +142,50 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(tc::smem_u32(&acc_full[i]), 1);
-            tc::mbar_init(tc::smem_u32(&acc_empty[i]), 4);
+            tc::mbar_init(tc::smem_u32(&acc_empty[i]), PAIR ? 8 : 4);
         }
         tc::fence_barrier_init();
         tc::prefetch_tensormap(&map_a);
         tc::prefetch_tensormap(&map_w);
     }
     if (warp == 1) {
-        tc::tmem_alloc(tc::smem_u32(tmem_slot), TMEM_COLS);
-        tc::tmem_relinquish();
+        if constexpr (PAIR) {
+            tc::tmem_alloc_pair(tc::smem_u32(tmem_slot), TMEM_COLS);
+            tc::tmem_relinquish_pair();
+        } else {
+            tc::tmem_alloc(tc::smem_u32(tmem_slot), TMEM_COLS);
+            tc::tmem_relinquish();
+        }
     }
     tc::tc_fence_before_sync();
-    __syncthreads();
+    if constexpr (PAIR) {
+        __syncwarp();
+        cluster_sync_all();     // both blocks' barriers and tensor memory are ready before either uses the other's
+    } else {
+        __syncthreads();
+    }
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        {
-            // The whole warp walks the loops of both issuing roles and one lane issues: what the instructions are given is then known to be the
-            // same for all lanes and kept where they read it.
-            const bool issues = tc::elect_one();
-            if (issues) pdl_launch_dependents();
-            // KS steps of 64 along K of an operand (what lies beyond K is filled with zeros and counts its bytes all the same)
-            auto load = [&](const CUtensorMap* map, uint32_t dst, uint32_t step_bytes, uint32_t bar, int kb, int row) {
-#pragma unroll
-                for (int h = 0; h < KS; ++h) tc::tma_load_2d(dst + h * step_bytes, map, bar, (kb + h) * BK, row);
-            };
+        if (lane == 0) {
+            pdl_launch_dependents();
             // W is a weight: no kernel of the stream writes it, so the first slices of it are asked for before the
             // wait for the kernel that makes A, and arrive while that kernel ends.
             uint32_t w_ahead = 0;
-            if (unit < total_items && !tile_group) {      // (which rows of W a grouped tile reads is known only after the wait)
-                const int tile = unit % total_tiles, kb0 = (unit / total_tiles) * kb_per_split;
-                const int sts = (min(num_kb, kb0 + kb_per_split) - kb0 + KS - 1) / KS;     // stages of the first item
-                w_ahead = (uint32_t)(sts < STAGES ? sts : STAGES);
-                const int n0 = (tile / m_tiles) * BN;
-                for (uint32_t i = 0; i < w_ahead; ++i) {
-                    const uint32_t bar = tc::smem_u32(&full[i]);
-                    if (issues) {
+            if constexpr (!PAIR) {
+                if (unit < total_items && !tile_group) {      // (which rows of W a grouped tile reads is known only after the wait)
+                    const int tile = unit % total_tiles, kb0 = (unit / total_tiles) * kb_per_split;
+                    const int sts = (min(num_kb, kb0 + kb_per_split) - kb0 + KS - 1) / KS;     // stages of the first item
+                    w_ahead = (uint32_t)(sts < STAGES ? sts : STAGES);
+                    const int n0 = (tile / m_tiles) * BN;
+                    for (uint32_t i = 0; i < w_ahead; ++i) {
+                        const uint32_t bar = tc::smem_u32(&full[i]);
                         tc::mbar_expect_tx(bar, L::STAGE_BYTES);
-                        load(&map_w, tc::smem_u32(smem + i * L::STAGE_BYTES) + W_OFF, L::B_BYTES, bar, kb0 + (int)i * KS, n0);
+#pragma unroll
+                        for (int h = 0; h < KS; ++h)      // a step beyond K is filled with zeros and counts its bytes all the same
+                            tc::tma_load_2d(tc::smem_u32(smem + i * L::STAGE_BYTES + h * L::SUB_BYTES) + MB * L::A_BYTES, &map_w, bar,
+                                            (kb0 + (int)i * KS + h) * BK, n0);
                     }
                 }
             }
@@ -323,8 +194,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             bool ok = true;
             for (int item = unit; item < total_items && ok; item += units) {
                 const int tile = item % total_tiles, split = item / total_tiles;
-                const int m0 = (tile % m_tiles) * BM;
-                int n0 = (tile / m_tiles) * BN;
+                const int m0 = (tile % m_tiles) * ROWS + (int)rank * BM;
+                int n0 = (tile / m_tiles) * BN + (PAIR ? (int)rank * (BN / 2) : 0);
                 if (tile_group) {
                     // grouped: the 128 rows of this tile belong to one group, whose matrix is rows [g N, (g + 1) N) of W
                     const int g = tile_group[tile % m_tiles];
@@ -335,19 +206,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 for (int kb = split * kb_per_split; kb < kb_end; kb += KS, ++it) {
                     const int s = it % STAGES;
                     const uint32_t round = it / STAGES;
-                    if (!tc::mbar_wait_warp(tc::smem_u32(&empty[s]), (round & 1) ^ 1, abort_flag)) { ok = false; break; }
+                    if (!tc::mbar_wait(tc::smem_u32(&empty[s]), (round & 1) ^ 1, abort_flag)) { ok = false; break; }
                     const uint32_t bar = tc::smem_u32(&full[s]);
-                    const bool w_here = it < w_ahead;       // its bytes are expected and W is on its way
-                    const uint32_t dst = tc::smem_u32(smem + s * L::STAGE_BYTES);
-                    if (issues) {
+                    if constexpr (PAIR) {
+                        // both blocks' bytes are counted on rank 0's barrier
+                        if (rank == 0) tc::mbar_expect_tx(bar, 2 * L::STAGE_BYTES);
+                        const uint32_t bar0 = cluster_map_shared(bar, 0);
+#pragma unroll
+                        for (int h = 0; h < KS; ++h) {
+                            const uint32_t a_dst = tc::smem_u32(smem + s * L::STAGE_BYTES + h * L::SUB_BYTES);
+                            tc::tma_load_2d_pair(a_dst, &map_a, bar0, (kb + h) * BK, m0);
+                            tc::tma_load_2d_pair(a_dst + L::A_BYTES, &map_w, bar0, (kb + h) * BK, n0);
+                        }
+                    } else {
+                        const bool w_here = it < w_ahead;       // its bytes are expected and W is on its way
                         if (!w_here) tc::mbar_expect_tx(bar, L::STAGE_BYTES);
-                        load(&map_a, dst, L::A_BYTES, bar, kb, m0);
-                        if (!w_here) load(&map_w, dst + W_OFF, L::B_BYTES, bar, kb, n0);
+#pragma unroll
+                        for (int h = 0; h < KS; ++h) {
+                            const uint32_t a_dst = tc::smem_u32(smem + s * L::STAGE_BYTES + h * L::SUB_BYTES);
+#pragma unroll
+                            for (int i = 0; i < MB; ++i) tc::tma_load_2d(a_dst + i * L::A_BYTES, &map_a, bar, (kb + h) * BK, m0 + i * BM);
+                            if (!w_here) tc::tma_load_2d(a_dst + MB * L::A_BYTES, &map_w, bar, (kb + h) * BK, n0);
+                        }
                     }
                 }
             }
-            if (*abort_flag) {
-                // Let the copies that are in flight land before the block's memory is given up.
+            if (*abort_flag && rank == 0) {
+                // Let the copies that are in flight land before the block's memory is given up (rank 0's
+                // barriers count the other block's copies too, and that block leaves only after rank 0).
                 for (uint32_t k = it > (uint32_t)STAGES ? it - STAGES : 0; k < it; ++k) {
                     const long long t0 = clock64();
                     while (!tc::mbar_try_wait(tc::smem_u32(&full[k % STAGES]), (k / STAGES) & 1) &&
@@ -357,9 +243,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        {
-            const bool issues = tc::elect_one();
-            constexpr uint32_t idesc = tc::idesc_bf16_f32(BM, BN);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = tc::idesc_bf16_f32(PAIR ? 2 * BM : BM, BN);
             // The descriptor of the ring's first byte, built once: every operand tile's descriptor is this one plus
             // its byte offset in units of 16 (the start address is the descriptor's lowest field); built per
             // instruction they cost the one issuing thread a few per cent (11.1 -> 10.9 us, 15.2 -> 14.9 us on the
@@ -376,40 +261,52 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 const int split = item / total_tiles;
                 const int kb_begin = split * kb_per_split, kb_end = min(num_kb, (split + 1) * kb_per_split);
-                const int buf = tile_iter & 1;
-                // the epilogue must have read this accumulator before it is filled again
-                ok = tc::mbar_wait_warp(tc::smem_u32(&acc_empty[buf]), ((tile_iter / 2) & 1) ^ 1, abort_flag);
+                const int buf = tile_iter % ACC_SETS;
+                // the epilogue must have read this accumulator set before it is filled again
+                ok = tc::mbar_wait(tc::smem_u32(&acc_empty[buf]), ((tile_iter / ACC_SETS) & 1) ^ 1, abort_flag);
                 if (!ok) break;
                 tc::tc_fence_after_sync();
-                const uint32_t acc = tmem_base + (uint32_t)(buf * BN);
+                const uint32_t acc = tmem_base + (uint32_t)(buf * MB * BN);
                 for (int kb = kb_begin; kb < kb_end; kb += KS, ++it) {
                     const int s = it % STAGES;
                     const uint32_t round = it / STAGES;
-                    ok = tc::mbar_wait_warp(tc::smem_u32(&full[s]), round & 1, abort_flag);
+                    ok = tc::mbar_wait(tc::smem_u32(&full[s]), round & 1, abort_flag);
                     if (!ok) break;
                     tc::tc_fence_after_sync();
-                    if (!issues) continue;
 #pragma unroll
                     for (int h = 0; h < KS; ++h) {
                         if (kb + h >= kb_end) break;            // a step beyond K holds zeros: nothing to add
-                        const uint64_t a_desc = ring_desc + (uint64_t)((s * L::STAGE_BYTES + h * L::A_BYTES) >> 4);
-                        const uint64_t b_desc = ring_desc + (uint64_t)((s * L::STAGE_BYTES + W_OFF + h * L::B_BYTES) >> 4);
+                        const uint64_t a_desc = ring_desc + (uint64_t)((s * L::STAGE_BYTES + h * L::SUB_BYTES) >> 4);
+                        const uint64_t b_desc = a_desc + (uint64_t)((MB * L::A_BYTES) >> 4);
                         const bool first = kb + h == kb_begin;
 #pragma unroll
                         for (int k = 0; k < BK / UMMA_K; ++k) {
-                            const uint64_t at = (uint64_t)((k * UMMA_K * 2) >> 4);
-                            tc::mma_bf16_ss(acc, a_desc + at, b_desc + at, idesc, !first || k != 0);
+                            const uint64_t db = b_desc + (uint64_t)((k * UMMA_K * 2) >> 4);
+                            const bool add = !first || k != 0;
+                            if constexpr (PAIR) {
+                                tc::mma_bf16_ss_pair(acc, a_desc + (uint64_t)((k * UMMA_K * 2) >> 4), db, idesc, add);
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < MB; ++i)
+                                    tc::mma_bf16_ss(acc + (uint32_t)(i * BN), a_desc + (uint64_t)((i * L::A_BYTES + k * UMMA_K * 2) >> 4),
+                                                    db, idesc, add);
+                            }
                         }
                     }
-                    tc::mma_commit(tc::smem_u32(&empty[s]));
+                    if constexpr (PAIR) tc::mma_commit_pair(tc::smem_u32(&empty[s]), (uint16_t)3);
+                    else tc::mma_commit(tc::smem_u32(&empty[s]));
                 }
-                if (ok && issues) tc::mma_commit(tc::smem_u32(&acc_full[buf]));
+                if (ok) {
+                    if constexpr (PAIR) tc::mma_commit_pair(tc::smem_u32(&acc_full[buf]), (uint16_t)3);
+                    else tc::mma_commit(tc::smem_u32(&acc_full[buf]));
+                }
             }
         }
     } else {
         // Epilogue: warp w may touch tensor-memory lanes 32 * (w % 4) .. + 31.
         const int quarter = warp & 3;
-        const uint32_t slabs = tc::smem_u32(smem + L::STAGING_OFFSET) + (uint32_t)quarter * 2 * L::SLAB_BYTES;
+        const int n_out = GATED ? N / 2 : N;
+        const bool vec_ok = (ldc % (16 / (int)sizeof(TC)) == 0) && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
         bool ok = true;
         int tile_iter = 0;
         uint32_t box_iter = 0;          // boxes this warp has handed to TMA
@@ -420,242 +317,189 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 --tile_iter;
                 continue;
             }
-            const int buf = tile_iter & 1;
-            ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&acc_full[buf]), (tile_iter / 2) & 1, abort_flag));
+            const int buf = tile_iter % ACC_SETS;
+            const int m0 = (tile % m_tiles) * ROWS + (int)rank * BM, n0 = (tile / m_tiles) * BN;
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&acc_full[buf]), (tile_iter / ACC_SETS) & 1, abort_flag));
             if (!ok) break;
             tc::tc_fence_after_sync();
-            store_tile<TC, ACT>(map_c, store_by_tma, slabs, box_iter, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN),
-                                (tile % m_tiles) * BM + quarter * 32, (tile / m_tiles) * BN, BN, split, C, M, N, ldc);
-            // this warp has read its lanes of the accumulator: let the MMA warp fill it again
+            if constexpr (sizeof(TC) == 2 && MB == 1) {
+                if (store_by_tma) {
+                    // Row-per-thread stores to global memory are slow and hold up the TMA loads of the next
+                    // tile (measured: 4.3 us a tile against 1 us without them).  Each warp rounds its 32
+                    // rows into a slab of shared memory, 64 output columns at a time, in the layout of a
+                    // 128-byte-swizzled box (a lane's 16-byte pieces then fall into different banks), and
+                    // one lane hands the slab to TMA, which writes whole rows and clips at M and N.
+                    constexpr int ACC_COLS = GATED ? 128 : 64;          // accumulator columns per 64 output columns
+                    const uint32_t slabs = tc::smem_u32(smem + L::STAGING_OFFSET) + (uint32_t)quarter * 2 * L::SLAB_BYTES;
+                    const uint32_t acc0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
+                    const bool rows_live = m0 + quarter * 32 < M;      // uniform over the warp
+#pragma unroll 1
+                    for (int c0 = 0; c0 < BN; c0 += ACC_COLS) {
+                        if (n0 + c0 >= N || !rows_live) break;
+                        const uint32_t slab = slabs + (uint32_t)(box_iter & 1) * L::SLAB_BYTES;
+                        if (lane == 0) tc::bulk_wait_read<1>();         // the store that read this slab two boxes ago
+                        __syncwarp();
+#pragma unroll
+                        for (int h = 0; h < ACC_COLS / 32; ++h) {
+                            uint32_t r[32];
+                            tc::tmem_ld_32x32_wait(acc0 + (uint32_t)(c0 + 32 * h), r);
+                            if constexpr (GATED) {
+                                float o[16];
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) o[i] = gate_act<ACT>(__uint_as_float(r[i])) * __uint_as_float(r[16 + i]);
+#pragma unroll
+                                for (int q = 0; q < 2; ++q) {
+                                    Vec16<bf16> v;
+                                    v.pack(o + 8 * q);
+                                    const int chunk = 2 * h + q;
+                                    tc::st_shared_v4(slab + (uint32_t)lane * 128 + (uint32_t)((chunk ^ (lane & 7)) << 4), v.raw);
+                                }
+                            } else {
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) {
+                                    float f[8];
+#pragma unroll
+                                    for (int j = 0; j < 8; ++j) f[j] = plain_act<ACT>(__uint_as_float(r[8 * q + j]));
+                                    Vec16<bf16> v;
+                                    v.pack(f);
+                                    const int chunk = 4 * h + q;
+                                    tc::st_shared_v4(slab + (uint32_t)lane * 128 + (uint32_t)((chunk ^ (lane & 7)) << 4), v.raw);
+                                }
+                            }
+                        }
+                        tc::fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tc::tma_store_2d(&map_c, slab, GATED ? (n0 + c0) / 2 : n0 + c0, m0 + quarter * 32);
+                            tc::bulk_commit();
+                        }
+                        ++box_iter;
+                    }
+                    tc::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if constexpr (PAIR) tc::mbar_arrive_cluster(cluster_map_shared(tc::smem_u32(&acc_empty[buf]), 0));
+                        else tc::mbar_arrive(tc::smem_u32(&acc_empty[buf]));
+                    }
+                    continue;
+                }
+            }
+            if constexpr (sizeof(TC) == 4 && MB == 1 && !GATED) {
+                if (store_by_tma) {
+                    // float32 slices: slabs of 32 rows x 32 columns (128 bytes a row), handed to TMA the same way
+                    const uint32_t slabs = tc::smem_u32(smem + L::STAGING_OFFSET) + (uint32_t)quarter * 2 * L::SLAB_BYTES;
+                    const uint32_t acc0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BN);
+                    const bool rows_live = m0 + quarter * 32 < M;      // uniform over the warp
+#pragma unroll 1
+                    for (int c0 = 0; c0 < BN; c0 += 32) {
+                        if (n0 + c0 >= N || !rows_live) break;
+                        const uint32_t slab = slabs + (uint32_t)(box_iter & 1) * L::SLAB_BYTES;
+                        if (lane == 0) tc::bulk_wait_read<1>();
+                        __syncwarp();
+                        uint32_t r[32];
+                        tc::tmem_ld_32x32_wait(acc0 + (uint32_t)c0, r);
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            tc::st_shared_v4(slab + (uint32_t)lane * 128 + (uint32_t)((q ^ (lane & 7)) << 4),
+                                             make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]));
+                        tc::fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tc::tma_store_3d(&map_c, slab, n0 + c0, m0 + quarter * 32, split);
+                            tc::bulk_commit();
+                        }
+                        ++box_iter;
+                    }
+                    tc::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if constexpr (PAIR) tc::mbar_arrive_cluster(cluster_map_shared(tc::smem_u32(&acc_empty[buf]), 0));
+                        else tc::mbar_arrive(tc::smem_u32(&acc_empty[buf]));
+                    }
+                    continue;
+                }
+            }
+#pragma unroll 1
+            for (int cc = 0; cc < MB * BN; cc += 32) {
+                const int mb = cc / BN, c0 = cc % BN;          // which block of rows, which columns of it
+                const int row = m0 + mb * BM + quarter * 32 + lane;
+                const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * MB * BN + mb * BN);
+                if (n0 + c0 >= N || m0 + mb * BM >= M) continue;   // uniform over the warp
+                uint32_t r[32];
+                __syncwarp();
+                tc::tmem_ld_32x32_wait(acc + (uint32_t)c0, r);
+                if (row >= M) {
+                    // nothing to store for this lane; it still takes part in the loads above
+                } else if constexpr (GATED) {
+                    // columns [c0, c0 + 16) are gates, [c0 + 16, c0 + 32) the matching ups
+                    const int j0 = (n0 + c0) / 2;
+                    float o[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) o[i] = gate_act<ACT>(__uint_as_float(r[i])) * __uint_as_float(r[16 + i]);
+                    TC* dst = C + (size_t)row * ldc + j0;
+                    if (vec_ok && j0 + 16 <= n_out) {
+                        if constexpr (sizeof(TC) == 2) {
+                            Vec16<bf16> v0, v1;
+                            v0.pack(o);
+                            v1.pack(o + 8);
+                            reinterpret_cast<uint4*>(dst)[0] = v0.raw;
+                            reinterpret_cast<uint4*>(dst)[1] = v1.raw;
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                reinterpret_cast<float4*>(dst)[i] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+                        }
+                    } else {
+                        for (int i = 0; i < 16; ++i)
+                            if (j0 + i < n_out) dst[i] = from_float<TC>(o[i]);
+                    }
+                } else {
+                    TC* dst = C + ((size_t)split * M + row) * ldc + n0 + c0;
+                    if (vec_ok && n0 + c0 + 32 <= N) {
+                        if constexpr (sizeof(TC) == 2) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                float f[8];
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) f[j] = plain_act<ACT>(__uint_as_float(r[8 * i + j]));
+                                Vec16<bf16> v;
+                                v.pack(f);
+                                reinterpret_cast<uint4*>(dst)[i] = v.raw;
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                reinterpret_cast<float4*>(dst)[i] =
+                                    make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
+                                                __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
+                        }
+                    } else {
+                        for (int i = 0; i < 32; ++i)
+                            if (n0 + c0 + i < N) dst[i] = from_float<TC>(plain_act<ACT>(__uint_as_float(r[i])));
+                    }
+                }
+            }
+            // this warp has read its lanes of the half: let the MMA warp fill it again
             tc::tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(tc::smem_u32(&acc_empty[buf]));
+            if (lane == 0) {
+                if constexpr (PAIR) tc::mbar_arrive_cluster(cluster_map_shared(tc::smem_u32(&acc_empty[buf]), 0));
+                else tc::mbar_arrive(tc::smem_u32(&acc_empty[buf]));
+            }
         }
         if (lane == 0) tc::bulk_wait_read<0>();     // the slabs are read before the block's memory is given up
     }
     tc::tc_fence_before_sync();
-    __syncthreads();
-    if (warp == 1) {
-        tc::tc_fence_after_sync();
-        tc::tmem_dealloc(tmem_base, TMEM_COLS);
-    }
-    if (threadIdx.x == 0 && *abort_flag && error_flag) atomicExch(error_flag, 1);
-}
-
-// ------------------------------------------------------------------------------------------- pairs of blocks
-// The same product by clusters of two blocks (an SM pair): a tile is 256 rows by up to 256 columns, computed by
-// `tcgen05.mma.cta_group::2`.  Each block loads its 128 rows of A and its half of the tile's W rows (no multicast: every block
-// loads what it holds), so a block pulls 32 KB per step of 64 along K for 128 x 256 outputs where a lone block pulls 48 KB: the
-// products are bound by what the SMs pull from L2.  The bytes of both blocks are counted on the `full` barriers of the block of
-// rank 0, which issues the MMAs; its commits arrive on the `empty` and `acc_full` barriers of both blocks; the epilogue warps of
-// both release an accumulator on rank 0's `acc_empty`.  Each block reads its own 128 rows of the accumulator out of its own
-// tensor memory.
-//
-// PairPlan: the tiles of a launch have two widths, so that the last round over the SM pairs is as full as the others: `wide` tiles of
-// PAIR_BN columns from a panel's (256 rows') first column on, in whole rounds, and what is left of every panel in tiles of
-// `narrow` columns.  A stage holds two steps of 64 along K (with one, tiles of 128 columns took 287 ns a step instead of 215).
-constexpr int PAIR_BN = 256, PAIR_STAGES = 3, PAIR_KS = 2;
-struct PairPlan {
-    int panels;         // of 256 rows
-    int panels_hi;      // the first of them have `wide_hi` wide tiles each, the others one less
-    int wide_hi;
-    int wide_items;     // wide tiles in all
-    int narrow;         // width of the narrow tiles, a multiple of 32; 0: none
-    int narrow_hi;      // narrow tiles of each of the first panels
-    int total;          // tiles in all
-};
-struct PairTile { int m0, n0, width; };
-__device__ __forceinline__ PairTile pair_tile(const PairPlan& p, int item) {
-    PairTile t;
-    if (item < p.wide_items) {
-        t.m0 = item % p.panels * 2 * BM;
-        t.n0 = item / p.panels * PAIR_BN;
-        t.width = PAIR_BN;
-        return t;
-    }
-    int j = item - p.wide_items, panel, c;
-    if (j < p.panels * p.narrow_hi) {
-        panel = j % p.panels;
-        c = j / p.panels;
-    } else {                                     // panels with one wide tile less have more narrow ones
-        j -= p.panels * p.narrow_hi;
-        const int lo = p.panels - p.panels_hi;
-        panel = p.panels_hi + j % lo;
-        c = p.narrow_hi + j / lo;
-    }
-    t.m0 = panel * 2 * BM;
-    t.n0 = (p.wide_hi - (panel < p.panels_hi ? 0 : 1)) * PAIR_BN + c * p.narrow;
-    t.width = p.narrow;
-    return t;
-}
-
-template <typename TC, int ACT>
-__global__ void __launch_bounds__(THREADS)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
-                 const __grid_constant__ CUtensorMap map_w_narrow, const __grid_constant__ CUtensorMap map_c, int store_by_tma,
-                 const PairPlan plan, TC* __restrict__ C, int M, int N, int K, long long ldc, int* error_flag) {
-    constexpr int STAGES = PAIR_STAGES, KS = PAIR_KS;
-    using L = Smem<PAIR_BN / 2, STAGES, KS>;
-    constexpr int W_OFF = KS * L::A_BYTES;          // a stage: A's KS steps, then W's
-    constexpr uint32_t TMEM_COLS = 2 * PAIR_BN;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFFSET);
-    uint64_t* full = bars;
-    uint64_t* empty = bars + STAGES;
-    uint64_t* acc_full = bars + 2 * STAGES;         // 2
-    uint64_t* acc_empty = bars + 2 * STAGES + 2;    // 2, eight arrivals each (one per epilogue warp of either block)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NUM_BARS);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same for all lanes, and known to be)
-    const int num_kb = (K + BK - 1) / BK;
-    const uint32_t rank = cluster_ctarank();                        // which block of the pair
-    const int unit = (int)blockIdx.x / 2, units = (int)gridDim.x / 2;
-
-    if (threadIdx.x == 0) {
-        *abort_flag = 0;
-        for (int s = 0; s < STAGES; ++s) {
-            tc::mbar_init(tc::smem_u32(&full[s]), 1);
-            tc::mbar_init(tc::smem_u32(&empty[s]), 1);
-        }
-        for (int i = 0; i < 2; ++i) {
-            tc::mbar_init(tc::smem_u32(&acc_full[i]), 1);
-            tc::mbar_init(tc::smem_u32(&acc_empty[i]), 8);
-        }
-        tc::fence_barrier_init();
-        tc::prefetch_tensormap(&map_a);
-        tc::prefetch_tensormap(&map_w);
-        if (plan.narrow) tc::prefetch_tensormap(&map_w_narrow);
-    }
-    if (warp == 1) {
-        tc::tmem_alloc_pair(tc::smem_u32(tmem_slot), TMEM_COLS);
-        tc::tmem_relinquish_pair();
-    }
-    tc::tc_fence_before_sync();
-    __syncwarp();
-    cluster_sync_all();         // both blocks' barriers and tensor memory are ready before either uses the other's
-    tc::tc_fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;
-
-    if (warp == 0) {
-        {
-            const bool issues = tc::elect_one();
-            if (issues) pdl_launch_dependents();
-            // a stage is KS steps of 64 along K (what lies beyond K is filled with zeros and counts its bytes all the same)
-            const int stages = (num_kb + KS - 1) / KS;
-            auto stage_bytes = [](const PairTile& t) { return 2 * KS * (L::A_BYTES + t.width / 2 * BK * 2); };      // of both blocks
-            auto load = [&](const CUtensorMap* map, uint32_t dst, uint32_t step_bytes, uint32_t bar, int st, int row) {
-#pragma unroll
-                for (int h = 0; h < KS; ++h) tc::tma_load_2d_pair(dst + h * step_bytes, map, bar, (st * KS + h) * BK, row);
-            };
-            auto load_w = [&](const PairTile& t, int s, int st) {
-                load(t.width == PAIR_BN ? &map_w : &map_w_narrow, tc::smem_u32(smem + s * L::STAGE_BYTES) + W_OFF, (uint32_t)(t.width / 2 * BK * 2),
-                     cluster_map_shared(tc::smem_u32(&full[s]), 0), st, t.n0 + (int)rank * (t.width / 2));
-            };
-            // the first stages of W before the wait for the kernel that makes A, as in `gemm_tc_kernel`
-            const uint32_t w_ahead = (uint32_t)min(stages, STAGES);
-            {
-                const PairTile t = pair_tile(plan, unit);
-                for (uint32_t i = 0; i < w_ahead; ++i) {
-                    if (!issues) continue;
-                    if (rank == 0) tc::mbar_expect_tx(tc::smem_u32(&full[i]), stage_bytes(t));
-                    load_w(t, (int)i, (int)i);
-                }
-            }
-            pdl_wait();   // A was written by the kernel before this one
-            uint32_t it = 0;        // stages loaded so far, over all tiles of this block
-            bool ok = true;
-            for (int item = unit; item < plan.total && ok; item += units) {
-                const PairTile t = pair_tile(plan, item);
-                for (int st = 0; st < stages; ++st, ++it) {
-                    const int s = it % STAGES;
-                    if (!tc::mbar_wait_warp(tc::smem_u32(&empty[s]), ((it / STAGES) & 1) ^ 1, abort_flag)) { ok = false; break; }
-                    if (!issues) continue;
-                    const bool w_here = it < w_ahead;       // its bytes are expected and W is on its way
-                    // both blocks' bytes are counted on rank 0's barrier
-                    if (!w_here && rank == 0) tc::mbar_expect_tx(tc::smem_u32(&full[s]), stage_bytes(t));
-                    load(&map_a, tc::smem_u32(smem + s * L::STAGE_BYTES), L::A_BYTES, cluster_map_shared(tc::smem_u32(&full[s]), 0), st,
-                         t.m0 + (int)rank * BM);
-                    if (!w_here) load_w(t, s, st);
-                }
-            }
-            if (*abort_flag && rank == 0) {
-                // Let the copies that are in flight land before the block's memory is given up (rank 0's
-                // barriers count the other block's copies too, and that block leaves only after rank 0).
-                for (uint32_t k = it > (uint32_t)STAGES ? it - STAGES : 0; k < it; ++k) {
-                    const long long t0 = clock64();
-                    while (!tc::mbar_try_wait(tc::smem_u32(&full[k % STAGES]), (k / STAGES) & 1) &&
-                           clock64() - t0 < tc::WAIT_LIMIT_CYCLES) {
-                    }
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (rank == 0) {
-            const bool issues = tc::elect_one();
-            const uint64_t ring_desc = tc::smem_desc_sw128(tc::smem_u32(smem));
-            uint32_t it = 0;
-            bool ok = true;
-            int tile_iter = 0;
-            for (int item = unit; item < plan.total && ok; item += units, ++tile_iter) {
-                const int width = pair_tile(plan, item).width;
-                const uint32_t idesc = tc::idesc_bf16_f32(2 * BM, width);
-                const uint64_t w_step = (uint64_t)((width / 2 * BK * 2) >> 4);
-                const int buf = tile_iter & 1;
-                // the epilogue must have read this accumulator before it is filled again
-                ok = tc::mbar_wait_warp(tc::smem_u32(&acc_empty[buf]), ((tile_iter / 2) & 1) ^ 1, abort_flag);
-                if (!ok) break;
-                tc::tc_fence_after_sync();
-                const uint32_t acc = tmem_base + (uint32_t)(buf * PAIR_BN);
-                for (int kb = 0; kb < num_kb; kb += KS, ++it) {
-                    const int s = it % STAGES;
-                    ok = tc::mbar_wait_warp(tc::smem_u32(&full[s]), (it / STAGES) & 1, abort_flag);
-                    if (!ok) break;
-                    tc::tc_fence_after_sync();
-                    if (!issues) continue;
-#pragma unroll
-                    for (int h = 0; h < KS; ++h) {
-                        if (kb + h >= num_kb) break;            // a step beyond K holds zeros: nothing to add
-                        const uint64_t a_desc = ring_desc + (uint64_t)((s * L::STAGE_BYTES + h * L::A_BYTES) >> 4);
-                        const uint64_t b_desc = ring_desc + (uint64_t)((s * L::STAGE_BYTES + W_OFF) >> 4) + (uint64_t)h * w_step;
-#pragma unroll
-                        for (int k = 0; k < BK / UMMA_K; ++k) {
-                            const uint64_t at = (uint64_t)((k * UMMA_K * 2) >> 4);
-                            tc::mma_bf16_ss_pair(acc, a_desc + at, b_desc + at, idesc, kb + h != 0 || k != 0);
-                        }
-                    }
-                    tc::mma_commit_pair(tc::smem_u32(&empty[s]), (uint16_t)3);
-                }
-                if (ok && issues) tc::mma_commit_pair(tc::smem_u32(&acc_full[buf]), (uint16_t)3);
-            }
-        }
+    if constexpr (PAIR) {
+        __syncwarp();
+        cluster_sync_all();     // neither block leaves, or frees tensor memory, while the other may still use it
     } else {
-        const int quarter = warp & 3;
-        const uint32_t slabs = tc::smem_u32(smem + L::STAGING_OFFSET) + (uint32_t)quarter * 2 * L::SLAB_BYTES;
-        bool ok = true;
-        int tile_iter = 0;
-        uint32_t box_iter = 0;
-        for (int item = unit; item < plan.total && ok; item += units, ++tile_iter) {
-            const PairTile t = pair_tile(plan, item);
-            const int buf = tile_iter & 1;
-            ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&acc_full[buf]), (tile_iter / 2) & 1, abort_flag));
-            if (!ok) break;
-            tc::tc_fence_after_sync();
-            store_tile<TC, ACT>(map_c, store_by_tma, slabs, box_iter, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * PAIR_BN),
-                                t.m0 + (int)rank * BM + quarter * 32, t.n0, t.width, 0, C, M, N, ldc);
-            tc::tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive_cluster(cluster_map_shared(tc::smem_u32(&acc_empty[buf]), 0));
-        }
-        if (lane == 0) tc::bulk_wait_read<0>();
+        __syncthreads();
     }
-    tc::tc_fence_before_sync();
-    __syncwarp();
-    cluster_sync_all();         // neither block leaves, or frees tensor memory, while the other may still use it
     if (warp == 1) {
         tc::tc_fence_after_sync();
-        tc::tmem_dealloc_pair(tmem_base, TMEM_COLS);
+        if constexpr (PAIR) tc::tmem_dealloc_pair(tmem_base, TMEM_COLS);
+        else tc::tmem_dealloc(tmem_base, TMEM_COLS);
     }
     if (threadIdx.x == 0 && *abort_flag && error_flag) atomicExch(error_flag, 1);
 }
@@ -713,114 +557,49 @@ bool get_slice_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t c
     return true;
 }
 
-// bfloat16 results leave through shared memory and TMA stores of [32 rows x 64 columns] boxes
-// where TMA can address C (16-byte aligned base and rows), float32 slices in boxes of 32 columns; otherwise the threads store their rows.
-// (A TMA store clips at the tensor's last column in units of 16 bytes, measured: with a width that is no
-// multiple of 16 bytes it writes up to 7 bfloat16 columns beyond it, so such results are stored by the threads.)
-template <typename TC, int ACT>
-int store_map(CUtensorMap* mc, void* C, int M, int N, long long ldc, int splits) {
-    constexpr bool GATED = is_glu(ACT);
-    const int n_out = GATED ? N / 2 : N;
-    if (!g_store_by_tma || !host_aligned16(C)) return 0;
-    if (sizeof(TC) == 2 && ldc % 8 == 0 && n_out % 8 == 0) return get_map(mc, C, M, n_out, ldc, 32) ? 1 : 0;
-    if (sizeof(TC) == 4 && !GATED && ldc % 4 == 0 && N % 4 == 0) return get_slice_map(mc, C, M, N, ldc, splits) ? 1 : 0;
-    return 0;
-}
-
-// w_rows: rows of the array W (N, or those of all groups)
-template <typename TC, int BN, int STAGES, int ACT, int KS = 1>
-int launch(const void* A, const void* W, void* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
-           int* error_flag, int pdl, cudaStream_t s, uint64_t w_rows, int splits = 1, const int* tile_group = nullptr) {
+template <typename TC, int BN, int STAGES, int ACT, int MB, bool PAIR = false, int KS = 1>
+int launch(const CUtensorMap& ma, const CUtensorMap& mw, void* C, int M, int N, int K, long long ldc,
+           int* error_flag, int pdl, cudaStream_t s, int splits = 1, const int* tile_group = nullptr) {
     static_assert(ACT != ACT_RELU2 || sizeof(TC) == 2, "the squared relu is built for bfloat16 results");
-    using L = Smem<BN, STAGES, KS>;
-    auto kernel = gemm_tc_kernel<TC, BN, STAGES, ACT, KS>;
+    constexpr bool GATED = is_glu(ACT);
+    using L = Smem<BN, STAGES, MB, PAIR, KS>;
+    auto kernel = gemm_tc_kernel<TC, BN, STAGES, ACT, MB, PAIR, KS>;
     static bool configured = false;   // per instantiation
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
         if (e != cudaSuccess) LLMK_FAIL("gemm_tc: cannot raise shared memory to %d: %s", L::TOTAL, cudaGetErrorString(e));
         configured = true;
     }
-    CUtensorMap ma, mw, mc{};
-    if (!get_map(&ma, A, M, K, lda, BM) || !get_map(&mw, W, w_rows, K, ldw, BN))
-        LLMK_FAIL("gemm_tc: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%lld ldw=%lld)", M, N, K, lda, ldw);
-    const int store_by_tma = store_map<TC, ACT>(&mc, C, M, N, ldc, splits);
+    // bfloat16 results leave through shared memory and TMA stores of [32 rows x 64 columns] boxes
+    // where TMA can address C (16-byte aligned base and rows); otherwise the threads store their rows
+    CUtensorMap mc{};
+    int store_by_tma = 0;
+    // (a TMA store clips at the tensor's last column in units of 16 bytes, measured: with a width that is no
+    // multiple of 16 bytes it writes up to 7 bfloat16 columns beyond it, so such results are stored by the threads)
+    if (sizeof(TC) == 2 && MB == 1 && g_store_by_tma && host_aligned16(C) && ldc % 8 == 0 && (GATED ? N / 2 : N) % 8 == 0)
+        store_by_tma = get_map(&mc, C, M, GATED ? N / 2 : N, ldc, 32) ? 1 : 0;
+    if (sizeof(TC) == 4 && MB == 1 && !GATED && g_store_by_tma && host_aligned16(C) && ldc % 4 == 0 && N % 4 == 0)
+        store_by_tma = get_slice_map(&mc, C, M, N, ldc, splits) ? 1 : 0;
     const int NUM_SMS = device_sm_count();
-    const int tiles = ceil_div(N, BN) * ceil_div(M, BM) * splits;
-    LLMK_CHECK_LAUNCH_RC("gemm_tc", llmk_launch(kernel, dim3(tiles < NUM_SMS ? tiles : NUM_SMS), dim3(THREADS), L::TOTAL, s,
-                                                pdl != 0, ma, mw, mc, store_by_tma, splits, (TC*)C, M, N, K, ldc,
-                                                error_flag, tile_group));
+    if constexpr (PAIR) {
+        // clusters of two blocks, one pair of SMs each
+        const int tiles = ceil_div(N, BN) * ceil_div(M, 2 * BM) * splits;
+        const int pairs = tiles < NUM_SMS / 2 ? tiles : NUM_SMS / 2;
+        LLMK_CHECK_LAUNCH_RC("gemm_tc", llmk_launch_clusters(kernel, dim3(2 * pairs), dim3(THREADS), L::TOTAL, s, pdl != 0,
+                                                             dim3(2, 1, 1), ma, mw, mc, store_by_tma, splits, (TC*)C, M, N, K,
+                                                             ldc, error_flag, tile_group));
+    } else {
+        const int tiles = ceil_div(N, BN) * ceil_div(M, MB * BM) * splits;
+        LLMK_CHECK_LAUNCH_RC("gemm_tc", llmk_launch(kernel, dim3(tiles < NUM_SMS ? tiles : NUM_SMS), dim3(THREADS), L::TOTAL, s,
+                                                    pdl != 0, ma, mw, mc, store_by_tma, splits, (TC*)C, M, N, K, ldc,
+                                                    error_flag, tile_group));
+    }
     return LLMK_OK;
 }
 
-// 0: lone blocks only.  1: pairs of blocks where they are the faster ones.
-// 2, 3: pairs always, with tiles of two widths or all 128 columns wide (for measurements and tests).
+// 0: lone blocks only.  1: pairs of blocks (`cta_group::2`) where the product has rows for them.
+// 2, 3: pairs always, with tiles 256 or 128 columns wide (for measurements).
 int g_pair_mode = 1;
-
-// Nanoseconds that a launch takes besides its rounds of tiles, and that a tile of `width` columns takes for 64 along K, by a pair of blocks and by lone
-// ones.  Measured on products of 300 to 2,048 rows (K 1,024 to 12,288; graphs of 20 launches): a pair's tile of 128 / 160 / 192 / 224 / 256 columns
-// 206-220 / 224-250 / 240-297 / 299-305 / 305-342, a lone block's of 128 / 256 200-215 / 352-400.
-constexpr long long PAIR_LAUNCH = 5300, LONE_LAUNCH = 4300;
-inline long long pair_time(int width) { return 115 + 82 * width / 100; }
-inline long long lone_time(int width) { return width == 256 ? 370 : 205; }
-
-// The plan of the least time over the SM pairs, and that time.
-PairPlan pair_plan(int M, int N, int pairs, long long* time) {
-    PairPlan best{};
-    *time = -1;
-    const int panels = ceil_div(M, 2 * BM), per_panel = ceil_div(N, PAIR_BN);
-    auto consider = [&](int wide_items, int narrow) {
-        PairPlan p{};
-        p.panels = panels;
-        p.wide_items = wide_items;
-        const int lo = wide_items / panels, extra = wide_items % panels;
-        p.panels_hi = extra ? extra : panels;
-        p.wide_hi = extra ? lo + 1 : lo;
-        p.narrow = narrow;
-        p.total = wide_items;
-        if (narrow) {
-            const int rest_hi = N - p.wide_hi * PAIR_BN, rest_lo = N - lo * PAIR_BN;
-            p.narrow_hi = rest_hi > 0 ? ceil_div(rest_hi, narrow) : 0;
-            p.total += p.panels_hi * p.narrow_hi + (panels - p.panels_hi) * (rest_lo > 0 ? ceil_div(rest_lo, narrow) : 0);
-        }
-        const long long t = (long long)ceil_div(wide_items, pairs) * pair_time(PAIR_BN) +
-                            (narrow ? (long long)ceil_div(p.total - wide_items, pairs) * pair_time(narrow) : 0);
-        if (*time < 0 || t < *time) {
-            *time = t;
-            best = p;
-        }
-    };
-    if (g_pair_mode == 3) {
-        consider(0, 128);
-        return best;
-    }
-    const int all = panels * per_panel;
-    consider(all, 0);
-    for (int k = 0; k * pairs < all; ++k)
-        for (int w = 32; w < PAIR_BN; w += 32) consider(k * pairs, w);
-    return best;
-}
-
-template <typename TC, int ACT>
-int launch_pair(const PairPlan& plan, const void* A, const void* W, void* C, int M, int N, int K, long long lda, long long ldw,
-                long long ldc, int* error_flag, int pdl, cudaStream_t s) {
-    using L = Smem<PAIR_BN / 2, PAIR_STAGES, PAIR_KS>;
-    auto kernel = gemm_pair_kernel<TC, ACT>;
-    static bool configured = false;   // per instantiation
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-        if (e != cudaSuccess) LLMK_FAIL("gemm_tc: cannot raise shared memory to %d: %s", L::TOTAL, cudaGetErrorString(e));
-        configured = true;
-    }
-    CUtensorMap ma, mw, mn, mc{};
-    const int narrow = plan.narrow ? plan.narrow : PAIR_BN;
-    if (!get_map(&ma, A, M, K, lda, BM) || !get_map(&mw, W, N, K, ldw, PAIR_BN / 2) || !get_map(&mn, W, N, K, ldw, narrow / 2))
-        LLMK_FAIL("gemm_tc: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%lld ldw=%lld)", M, N, K, lda, ldw);
-    const int store_by_tma = store_map<TC, ACT>(&mc, C, M, N, ldc, 1);
-    const int pairs = std::min(plan.total, device_sm_count() / 2);
-    LLMK_CHECK_LAUNCH_RC("gemm_tc", llmk_launch_clusters(kernel, dim3(2 * pairs), dim3(THREADS), L::TOTAL, s, pdl != 0, dim3(2, 1, 1), ma, mw, mn,
-                                                         mc, store_by_tma, plan, (TC*)C, M, N, K, ldc, error_flag));
-    return LLMK_OK;
-}
 
 // ring depth of the narrower tiles (3, 4 and 6 were measured on a prompt's products: no difference
 // beyond 4, the MMA instructions set the pace)
@@ -829,33 +608,42 @@ constexpr int STAGES_128 = 3, KS_128 = 2, STAGES_64 = 4;      // 128-wide tiles:
 template <typename TC, int GATED>
 int dispatch_tile(const void* A, const void* W, void* C, int M, int N, int K, long long lda, long long ldw,
                   long long ldc, int* error_flag, int pdl, cudaStream_t s) {
-    // The tiles that take the least time in rounds over the SMs, lone blocks' or pairs'.  What the pairs gain (us, lone / pairs): 2,048 rows on 8,192 x 2,048
-    // 55.5 / 48.1, 2,048 x 6,144 40.3 / 36.8, gated 6,144 x 1,024 21.7 / 20.1; 1,501 rows on 4,096 x 12,288 180 / 120, gated 24,576 x 4,096 212 / 192;
-    // 700 rows on 4,096 x 4,096 28.9 / 23.5.  What stays with lone blocks: 2,048 rows on 1,024 x 2,048 10.7 / 11.5, 300 rows on 6,144 x 1,024 12.4 / 14.5.
-    // (64 columns take as long as 128; they are for W of few rows.)
+    // Tile width: the one whose tiles take the least time in rounds over the SMs.  The relative times
+    // of a tile were measured on the products of a 2,048-token prompt.  (Tiles of two row blocks,
+    // MB = 2, were measured too: 256 x 256 is no faster than 128 x 256 with its epilogue overlapped,
+    // so they are not used.)
     const int NUM_SMS = device_sm_count();
-    const long long steps = ceil_div(K, BK);
+    struct Shape { int bn; long long time; };
+    const Shape shapes[] = {{256, 528}, {128, 348}, {64, 264}};
     int bn = GATED ? 128 : 64;
     long long best = -1;
-    for (const int width : {256, 128, 64}) {
-        if (GATED && width == 64) continue;          // the gated epilogue is built for the wider tiles only
-        const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, width);
-        const long long cost = LONE_LAUNCH + (tiles + NUM_SMS - 1) / NUM_SMS * steps * lone_time(width);
+    for (const Shape& sh : shapes) {
+        if (GATED && sh.bn == 64) continue;          // the gated epilogue is built for the wider tiles only
+        const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, sh.bn);
+        const long long cost = ((tiles + NUM_SMS - 1) / NUM_SMS) * sh.time;
         if (best < 0 || cost < best) {
             best = cost;
-            bn = width;
+            bn = sh.bn;
         }
     }
-    if (g_pair_mode != 0) {
-        long long pair = -1;
-        const PairPlan plan = pair_plan(M, N, NUM_SMS / 2, &pair);
-        if (g_pair_mode >= 2 || PAIR_LAUNCH + pair * steps < best)
-            return launch_pair<TC, GATED>(plan, A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s);
+    int pair_bn = 0;
+    if (g_pair_mode >= 2) pair_bn = g_pair_mode == 2 ? 256 : 128;
+    else if (g_pair_mode == 1 && M >= 4096 && (long long)ceil_div(M, 2 * BM) * ceil_div(N, 256) >= 2 * (NUM_SMS / 2))
+        pair_bn = 256;      // measured: pairs win from about 4,096 rows, with two rounds of 256 x 256 tiles for the 74 SM pairs
+    if (pair_bn) {
+        CUtensorMap pa, pw;
+        if (!get_map(&pa, A, M, K, lda, BM) || !get_map(&pw, W, N, K, ldw, pair_bn / 2))
+            LLMK_FAIL("gemm_tc: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%lld ldw=%lld)", M, N, K, lda, ldw);
+        if (pair_bn == 256) return launch<TC, 256, 6, GATED, 1, true>(pa, pw, C, M, N, K, ldc, error_flag, pdl, s);
+        return launch<TC, 128, 4, GATED, 1, true, 2>(pa, pw, C, M, N, K, ldc, error_flag, pdl, s);
     }
+    CUtensorMap ma, mw;
+    if (!get_map(&ma, A, M, K, lda, BM) || !get_map(&mw, W, N, K, ldw, bn))
+        LLMK_FAIL("gemm_tc: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%lld ldw=%lld)", M, N, K, lda, ldw);
     switch (bn) {
-        case 256: return launch<TC, 256, 4, GATED>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, N);
-        case 128: return launch<TC, 128, STAGES_128, GATED, KS_128>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, N);
-        default: return launch<TC, 64, STAGES_64, GATE_NONE>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, N);
+        case 256: return launch<TC, 256, 4, GATED, 1>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s);
+        case 128: return launch<TC, 128, STAGES_128, GATED, 1, false, KS_128>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s);
+        default: return launch<TC, 64, STAGES_64, false, 1>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s);
     }
 }
 
@@ -897,7 +685,10 @@ LLMK_EXPORT int llmk_gemm_tc_sliced(float* C, const void* A, const void* W, int 
     if ((splits - 1) * (ceil_div(ceil_div(num_kb, splits), KS_128) * KS_128) >= num_kb)
         LLMK_FAIL("gemm_tc: %d slices of K=%d would leave one empty (slices are multiples of %d columns)", splits, K, KS_128 * BK);
     if (ldc < N) LLMK_FAIL("gemm_tc: ldc=%lld too small", ldc);
-    return launch<float, 128, STAGES_128, false, KS_128>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, (cudaStream_t)stream, N, splits);
+    CUtensorMap ma, mw;
+    if (!get_map(&ma, A, M, K, lda, BM) || !get_map(&mw, W, N, K, ldw, 128))
+        LLMK_FAIL("gemm_tc: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d lda=%lld ldw=%lld)", M, N, K, lda, ldw);
+    return launch<float, 128, STAGES_128, false, 1, false, KS_128>(ma, mw, C, M, N, K, ldc, error_flag, pdl, (cudaStream_t)stream, splits);
 }
 
 // Grouped product: the rows of A come in tiles of 128 that belong to one group each (`tile_group[i]` for rows
@@ -914,23 +705,25 @@ LLMK_EXPORT int llmk_gemm_tc_grouped(void* C, const void* A, const void* W, int 
     if (M % BM != 0 || !tile_group) LLMK_FAIL("gemm_tc_grouped: %d rows are not whole tiles of %d with a group each", M, BM);
     if (ldc < N) LLMK_FAIL("gemm_tc_grouped: ldc=%lld too small", ldc);
     const int bn = N >= 256 ? 256 : N > 64 ? 128 : 64;
-    const uint64_t w_rows = (uint64_t)groups * N;
+    CUtensorMap ma, mw;
+    if (!get_map(&ma, A, M, K, lda, BM) || !get_map(&mw, W, (uint64_t)groups * N, K, ldw, bn))
+        LLMK_FAIL("gemm_tc_grouped: cuTensorMapEncodeTiled failed (M=%d N=%d K=%d groups=%d)", M, N, K, groups);
     cudaStream_t s = (cudaStream_t)stream;
     if (relu2) {
         if (out_dtype != LLMK_BF16) LLMK_FAIL("gemm_tc_grouped: the squared relu is built for bfloat16 results");
-        if (bn == 256) return launch<bf16, 256, 4, ACT_RELU2>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, w_rows, 1, tile_group);
-        if (bn == 128) return launch<bf16, 128, STAGES_128, ACT_RELU2, KS_128>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, w_rows, 1, tile_group);
-        return launch<bf16, 64, STAGES_64, ACT_RELU2>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, w_rows, 1, tile_group);
+        if (bn == 256) return launch<bf16, 256, 4, ACT_RELU2, 1>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s, 1, tile_group);
+        if (bn == 128) return launch<bf16, 128, STAGES_128, ACT_RELU2, 1, false, KS_128>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s, 1, tile_group);
+        return launch<bf16, 64, STAGES_64, ACT_RELU2, 1>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s, 1, tile_group);
     }
     if (out_dtype == LLMK_BF16) {
-        if (bn == 256) return launch<bf16, 256, 4, false>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, w_rows, 1, tile_group);
-        if (bn == 128) return launch<bf16, 128, STAGES_128, false, KS_128>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, w_rows, 1, tile_group);
-        return launch<bf16, 64, STAGES_64, false>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, w_rows, 1, tile_group);
+        if (bn == 256) return launch<bf16, 256, 4, false, 1>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s, 1, tile_group);
+        if (bn == 128) return launch<bf16, 128, STAGES_128, false, 1, false, KS_128>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s, 1, tile_group);
+        return launch<bf16, 64, STAGES_64, false, 1>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s, 1, tile_group);
     }
     if (out_dtype == LLMK_F32) {
-        if (bn == 256) return launch<float, 256, 4, false>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, w_rows, 1, tile_group);
-        if (bn == 128) return launch<float, 128, STAGES_128, false, KS_128>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, w_rows, 1, tile_group);
-        return launch<float, 64, STAGES_64, false>(A, W, C, M, N, K, lda, ldw, ldc, error_flag, pdl, s, w_rows, 1, tile_group);
+        if (bn == 256) return launch<float, 256, 4, false, 1>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s, 1, tile_group);
+        if (bn == 128) return launch<float, 128, STAGES_128, false, 1, false, KS_128>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s, 1, tile_group);
+        return launch<float, 64, STAGES_64, false, 1>(ma, mw, C, M, N, K, ldc, error_flag, pdl, s, 1, tile_group);
     }
     LLMK_FAIL("gemm_tc_grouped: unknown output dtype %d", out_dtype);
 }
