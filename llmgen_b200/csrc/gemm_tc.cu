@@ -231,6 +231,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 }
             }
+            if constexpr (PAIR) {
+                // The MMA's last arrivals on `empty` come from the other block and have to land while this block's memory is still its own.
+                for (uint32_t k = it > (uint32_t)STAGES ? it - STAGES : 0; k < it && ok; ++k)
+                    ok = tc::mbar_wait(tc::smem_u32(&empty[k % STAGES]), (k / STAGES) & 1, abort_flag);
+            }
             if (*abort_flag && rank == 0) {
                 // Let the copies that are in flight land before the block's memory is given up (rank 0's
                 // barriers count the other block's copies too, and that block leaves only after rank 0).
