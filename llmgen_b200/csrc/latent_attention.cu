@@ -1099,12 +1099,45 @@ __global__ void latent_gate_kernel(T* __restrict__ out, const float* __restrict_
     }
 }
 
+// The same for bfloat16 rows in whole vectors of eight (vdim and the gate's row stride multiples of eight, 16-byte boundaries), a token's heads side by
+// side over the threads.  Bound by its traffic, 4 + 2 + 2 bytes a value: 2,048 tokens of 16 heads of 128 22.1 us value by value.
+__global__ void __launch_bounds__(256) latent_gate_vec_kernel(bf16* __restrict__ out, const float* __restrict__ o, const bf16* __restrict__ g, long long ldg,
+                                                              int n_tokens, int heads, int vdim, int t_pad) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int per_head = vdim / 8, per_row = heads * per_head;
+    for (int v = threadIdx.x; v < per_row; v += blockDim.x) {
+        const int h = v / per_head, j = v % per_head * 8;
+        for (int t = blockIdx.x; t < n_tokens; t += gridDim.x) {
+            const float4* src = reinterpret_cast<const float4*>(o + ((size_t)h * t_pad + t) * vdim + j);
+            const float4 a = src[0], b = src[1];
+            float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            Vec16<bf16> pk;
+            if (g) {
+                float gv[8];
+                pk.raw = *reinterpret_cast<const uint4*>(g + (size_t)t * ldg + v * 8);
+                pk.unpack(gv);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) x[i] *= 1.0f / (1.0f + expf(-gv[i]));
+            }
+            pk.pack(x);
+            *reinterpret_cast<uint4*>(out + (size_t)t * per_row * 8 + v * 8) = pk.raw;
+        }
+    }
+}
+
 LLMK_EXPORT int llmk_latent_gate(void* out, const float* o, const void* g, long long ldg, int n_tokens, int heads, int vdim, int t_pad,
                                  int dtype, void* stream) {
     if (n_tokens <= 0) return LLMK_OK;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (dtype == LLMK_BF16 && vdim % 8 == 0 && (!g || ldg % 8 == 0) && host_aligned16(out) && host_aligned16(o) && host_aligned16(g)) {
+        const int most = device_sm_count() * 8;         // blocks of 256 threads that are resident at once
+        LLMK_CHECK_LAUNCH_RC("latent_gate", llmk_launch(latent_gate_vec_kernel, dim3(n_tokens < most ? n_tokens : most), dim3(256), 0, s, true, (bf16*)out, o,
+                                                        (const bf16*)g, ldg, n_tokens, heads, vdim, t_pad));
+        return LLMK_OK;
+    }
     long long blocks = ((long long)n_tokens * heads * vdim + 255) / 256;
     if (blocks > device_sm_count() * 16) blocks = device_sm_count() * 16;
-    cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e;
     if (dtype == LLMK_F32)
         e = llmk_launch(latent_gate_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, s, true, (float*)out, o, (const float*)g, ldg, n_tokens,

@@ -53,6 +53,7 @@ MODULES: Dict[str, List[str]] = {
     "rowwise": [],
     "linear_attention": [],
     "latent_attention": [],
+    "latent_attention_tc": [],
     "moe": [],
     "recurrent": [],
     "memory_scan": [],

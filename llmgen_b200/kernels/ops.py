@@ -1577,18 +1577,8 @@ def latent_attention_on_tensor_cores(dtype: torch.dtype, rank: int, rot: int) ->
     return bool(build.load("latent_attention").llmk_latent_attention_on_tensor_cores(c_int(rank), c_int(rot), c_int(dtype_code(dtype))))
 
 
-def latent_attention(out: Optional[torch.Tensor], qa: Optional[torch.Tensor], cache: torch.Tensor, block_tables: torch.Tensor, max_blocks: int,
-                     ctx_len: torch.Tensor, cu_q: torch.Tensor, tile_seq: torch.Tensor, tile_q0: torch.Tensor, n_tokens: int,
-                     heads: int, rank: int, rot: int, page_size: int, scale: float, parts: int = 1,
-                     scratch: Optional[torch.Tensor] = None, out_head_major: Optional[torch.Tensor] = None, window: int = 0,
-                     q_head_major: Optional[torch.Tensor] = None, rows: int = 32) -> None:
-    """out float32 [n, heads, rank] = causal softmax attention of qa over the cached vectors (one shared kv head whose
-    values are the first `rank` entries of the cached vector).  With `out_head_major` (bfloat16 [heads, t_pad, rank]; the
-    tensor-core form only) the result goes there instead, rounded, for the grouped product that follows.  `q_head_major`
-    (bfloat16 [heads, t_pad, rank + rot]; the tensor-core form only): the queries, in place of float32 `qa`.  `window` > 0: a
-    query sees the last `window` positions up to its own.  `rows`: rows of a block (`latent_attention_rows`); the tiles hold
-    `latent_attention_tile_queries(heads, rows)` queries."""
-    lib = build.load("latent_attention")
+def _latent_attention_arrays(out, qa, out_head_major, q_head_major, heads: int, rank: int, rot: int):
+    """Looks the queries and the result of `latent_attention` over: (token rows a head of the head-major result, of the head-major queries)."""
     t_pad = 0
     if out_head_major is not None:
         if out_head_major.dtype != torch.bfloat16 or out_head_major.dim() != 3 or out_head_major.shape[0] != heads \
@@ -1605,6 +1595,22 @@ def latent_attention(out: Optional[torch.Tensor], qa: Optional[torch.Tensor], ca
         tq_pad = q_head_major.shape[1]
     elif qa is None or qa.dtype != torch.float32:
         raise KernelError("latent_attention: queries are float32")
+    return t_pad, tq_pad
+
+
+def latent_attention(out: Optional[torch.Tensor], qa: Optional[torch.Tensor], cache: torch.Tensor, block_tables: torch.Tensor, max_blocks: int,
+                     ctx_len: torch.Tensor, cu_q: torch.Tensor, tile_seq: torch.Tensor, tile_q0: torch.Tensor, n_tokens: int,
+                     heads: int, rank: int, rot: int, page_size: int, scale: float, parts: int = 1,
+                     scratch: Optional[torch.Tensor] = None, out_head_major: Optional[torch.Tensor] = None, window: int = 0,
+                     q_head_major: Optional[torch.Tensor] = None, rows: int = 32) -> None:
+    """out float32 [n, heads, rank] = causal softmax attention of qa over the cached vectors (one shared kv head whose
+    values are the first `rank` entries of the cached vector).  With `out_head_major` (bfloat16 [heads, t_pad, rank]; the
+    tensor-core form only) the result goes there instead, rounded, for the grouped product that follows.  `q_head_major`
+    (bfloat16 [heads, t_pad, rank + rot]; the tensor-core form only): the queries, in place of float32 `qa`.  `window` > 0: a
+    query sees the last `window` positions up to its own.  `rows`: rows of a block (`latent_attention_rows`); the tiles hold
+    `latent_attention_tile_queries(heads, rows)` queries."""
+    lib = build.load("latent_attention")
+    t_pad, tq_pad = _latent_attention_arrays(out, qa, out_head_major, q_head_major, heads, rank, rot)
     if parts > 1 and (scratch is None or scratch.numel() < latent_attention_scratch_floats(n_tokens, heads, rank, parts)):
         raise KernelError("latent_attention: scratch too small")
     _check(lib, lib.llmk_latent_attention(_ptr(out), _ptr(qa), _ptr(cache), _ptr(block_tables), c_int(max_blocks), _ptr(ctx_len),
@@ -1613,6 +1619,30 @@ def latent_attention(out: Optional[torch.Tensor], qa: Optional[torch.Tensor], ca
                                           _ptr(scratch), _ptr(out_head_major), c_int(t_pad), _ptr(q_head_major), c_int(tq_pad),
                                           c_int(rows), c_int(dtype_code(cache.dtype)), _stream()),
            2 if parts > 1 else 1)
+
+
+def latent_attention_tc_tile_queries(dtype: torch.dtype, heads: int, rank: int, rot: int, page_size: int) -> int:
+    """Queries per tile of `latent_attention_tc`; 0: it does not take these sizes."""
+    return int(build.load("latent_attention_tc").llmk_latent_attention_tc_tile_queries(c_int(heads), c_int(rank), c_int(rot), c_int(page_size),
+                                                                                       c_int(dtype_code(dtype))))
+
+
+def latent_attention_tc(out: Optional[torch.Tensor], qa: Optional[torch.Tensor], cache: torch.Tensor, block_tables: torch.Tensor, max_blocks: int,
+                        ctx_len: torch.Tensor, cu_q: torch.Tensor, tile_seq: torch.Tensor, tile_q0: torch.Tensor, n_tokens: int,
+                        heads: int, rank: int, rot: int, page_size: int, scale: float, out_head_major: Optional[torch.Tensor] = None,
+                        window: int = 0, q_head_major: Optional[torch.Tensor] = None) -> None:
+    """`latent_attention` of portions of prompts on tcgen05 (csrc/latent_attention_tc.cu): bfloat16 caches, no key parts, tiles of
+    `latent_attention_tc_tile_queries` queries."""
+    lib = build.load("latent_attention_tc")
+    t_pad, tq_pad = _latent_attention_arrays(out, qa, out_head_major, q_head_major, heads, rank, rot)
+    if cache.dtype != torch.bfloat16 or not cache.is_contiguous():
+        raise KernelError("latent_attention_tc: the cache is contiguous bfloat16")
+    _check(lib, lib.llmk_latent_attention_tc(_ptr(None if out_head_major is not None else out), _ptr(None if q_head_major is not None else qa),
+                                             _ptr(cache), c_longlong(cache.numel() // (rank + rot)), _ptr(block_tables), c_int(max_blocks),
+                                             _ptr(ctx_len), _ptr(cu_q), _ptr(tile_seq), _ptr(tile_q0), c_int(tile_seq.numel()), c_int(n_tokens),
+                                             c_int(heads), c_int(rank), c_int(rot), c_int(page_size), c_float(scale), c_int(window),
+                                             _ptr(out_head_major), c_int(t_pad), _ptr(q_head_major), c_int(tq_pad),
+                                             _ptr(tc_error_flag(cache.device)), _stream()))
 
 
 def latent_gate(out: torch.Tensor, o: torch.Tensor, gate: Optional[torch.Tensor], heads: int, vdim: int, t_pad: int) -> None:

@@ -60,7 +60,7 @@ class LatentAttention(Mixer):
 
     @staticmethod
     def kernel_modules(spec):
-        return ("latent_attention", "rowwise") + GEMM_MODULES
+        return ("latent_attention", "latent_attention_tc", "rowwise") + GEMM_MODULES
 
     def __init__(self, spec: LatentAttentionSpec, weights, dtype, device):
         self.direct = bool(spec.q_proj)            # queries straight from the stream
@@ -119,6 +119,7 @@ class LatentAttention(Mixer):
         self.grouped_query = (self.direct and on_tensor_cores and self.nope % 8 == 0 and self.rope % 8 == 0 and self.w_in.shape[0] % 8 == 0)
         self.w_uk_t = (self.w_uk.view(self.heads, self.nope, self.kv_rank).transpose(1, 2).contiguous() if self.grouped_query else None)
         self._head_of_tile = {}
+        self._tc_bq = {}
         self.device = device
 
     def cache_request(self) -> KVRequest:
@@ -128,10 +129,21 @@ class LatentAttention(Mixer):
         return self.position.max_positions if self.position is not None else None
 
     def step_arrays_key(self):
-        return ("attention_tiles", self.bq, self.bq_single)
+        return ("attention_tiles", self.bq, self.bq_single, self.heads, self.kv_rank, self.rope, self.window, float(self.spec.scale) > 0.0)
+
+    def tc_tile_queries(self, page_size: int) -> int:
+        """Queries per tile of the kernel on tcgen05 (0: steps other than single tokens stay on `mma.sync` or the CUDA cores)."""
+        if page_size not in self._tc_bq:
+            self._tc_bq[page_size] = (ops.latent_attention_tc_tile_queries(self.dtype, self.heads, self.kv_rank, self.rope, page_size)
+                                      if float(self.spec.scale) > 0.0 else 0)
+        return self._tc_bq[page_size]
 
     def prepare_step(self, builder) -> None:
-        add_query_tiles(builder, self.bq_single if builder.pure_decode else self.bq)
+        tc_bq = self.tc_tile_queries(builder.page_size) if builder.page_size and not builder.pure_decode else 0
+        if tc_bq:
+            add_query_tiles(builder, tc_bq, self.window, heaviest_first=True)
+        else:
+            add_query_tiles(builder, self.bq_single if builder.pure_decode else self.bq)
 
     def workspace_bytes(self, tokens: int) -> int:
         elem = 2 if self.dtype == torch.bfloat16 else 4
@@ -201,7 +213,8 @@ class LatentAttention(Mixer):
         cos, sin = self.position.tables() if self.position is not None else (None, None)
         packed = linear(x, self.w_in, ws.buffer("latent_in", T, self.w_in.shape[0], self.dtype))
         qa, qa_hm = (self._direct_query if self.direct else self._latent_query)(ctx, packed, cache, group, cos, sin)
-        bq, rows = (self.bq_single, self.rows_single) if ctx.pure_decode else (self.bq, self.rows)
+        tc_bq = 0 if ctx.pure_decode else self.tc_tile_queries(cache.page_size)
+        bq, rows = (self.bq_single, self.rows_single) if ctx.pure_decode else (tc_bq or self.bq, self.rows)
         name = f"attention_tiles_bq{bq}"
         parts = self._parts(ctx)
         scratch = None
@@ -209,21 +222,23 @@ class LatentAttention(Mixer):
             scratch = ws.flat("latent_split", ops.latent_attention_scratch_floats(T, n, self.kv_rank, parts), torch.float32)
         gate = packed[:, self.g_off:] if self.spec.gate_proj else None
         y = ws.buffer("latent_y", T, n * self.vd, self.dtype)
-        attend = dict(window=self.window, q_head_major=qa_hm, rows=rows)
+        attention = ops.latent_attention_tc if tc_bq else ops.latent_attention
+        attend = dict(window=self.window, q_head_major=qa_hm)
+        if not tc_bq:
+            attend.update(parts=parts, scratch=scratch, rows=rows)
         if self.grouped_expand:
             t_pad, cap = self._padded(ws, T)
             oa_hm = ws.buffer("latent_oa_hm", n * t_pad, self.kv_rank, self.dtype, capacity_rows=cap)
-            ops.latent_attention(None, qa, cache.k, group.block_tables, group.max_blocks, ctx.ctx_len, ctx.cu_q, ctx.array(name + "_seq"),
-                                 ctx.array(name + "_q0"), T, n, self.kv_rank, self.rope, cache.page_size, float(self.spec.scale), parts,
-                                 scratch, out_head_major=oa_hm.view(n, t_pad, self.kv_rank), **attend)
+            attention(None, qa, cache.k, group.block_tables, group.max_blocks, ctx.ctx_len, ctx.cu_q, ctx.array(name + "_seq"),
+                      ctx.array(name + "_q0"), T, n, self.kv_rank, self.rope, cache.page_size, float(self.spec.scale),
+                      out_head_major=oa_hm.view(n, t_pad, self.kv_rank), **attend)
             o_hm = ws.buffer("latent_o_hm", n * t_pad, self.vd, torch.float32, capacity_rows=cap)
             ops.gemm_tc_grouped(o_hm, oa_hm, self.w_uv.view(n, self.vd, self.kv_rank), self._tile_heads(t_pad), real_rows=n * T)
             ops.latent_gate(y, o_hm, gate, n, self.vd, t_pad)
         else:
             oa = ws.buffer("latent_oa", T, n * self.kv_rank, torch.float32)
-            ops.latent_attention(oa, qa, cache.k, group.block_tables, group.max_blocks, ctx.ctx_len, ctx.cu_q, ctx.array(name + "_seq"),
-                                 ctx.array(name + "_q0"), T, n, self.kv_rank, self.rope, cache.page_size, float(self.spec.scale), parts,
-                                 scratch, **attend)
+            attention(oa, qa, cache.k, group.block_tables, group.max_blocks, ctx.ctx_len, ctx.cu_q, ctx.array(name + "_seq"),
+                      ctx.array(name + "_q0"), T, n, self.kv_rank, self.rope, cache.page_size, float(self.spec.scale), **attend)
             ops.latent_expand(y, oa, self.w_uv, gate, n, self.kv_rank, self.vd)
         return linear_sliced(ws, "mixer_out", y, self.w_o, self.dtype)
 
