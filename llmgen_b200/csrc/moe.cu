@@ -26,6 +26,7 @@
 LLMK_DEFINE_LAST_ERROR()
 
 constexpr int MOE_TT = 16;      // rows per tile
+constexpr int MOE_SPAN = 256;      // most rows of a run of one expert's rows (csrc/gemm_grouped.cu)
 constexpr int MOE_KC = 256;     // input values per pass through shared memory
 
 // ---------------------------------------------------------------------------------------------- route
@@ -359,7 +360,7 @@ LLMK_EXPORT int llmk_moe_route(const void* h, long long ldh, const float* wr, co
 // order[pos] is then -1 where a tile has no row.
 __global__ void moe_plan_kernel(const int* __restrict__ slot_expert, int n_slots, int E, int max_tiles, int tt, int padded,
                                 int* __restrict__ order, int* __restrict__ pos_of_slot, int* __restrict__ tile_expert,
-                                int* __restrict__ tile_start, int* __restrict__ tile_rows) {
+                                int* __restrict__ tile_start, int* __restrict__ tile_rows, int4* __restrict__ spans) {
     extern __shared__ int sh[];     // counts [E], first tiles [E], cursors [E]
     int* count = sh;
     int* first = sh + E;
@@ -388,25 +389,33 @@ __global__ void moe_plan_kernel(const int* __restrict__ slot_expert, int n_slots
     __syncthreads();
     if (threadIdx.x < 32) {         // where each expert's rows and tiles start: sums over the lanes, 32 experts at a time
         const int lane = threadIdx.x;
-        int at = 0, tile = 0;
+        int at = 0, tile = 0, span = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const int e = e0 + lane, c = e < E ? count[e] : 0, tiles = ceil_div(c, tt), rows = padded ? tiles * tt : c;
-            int r = rows, q = tiles;
+            const int runs = ceil_div(c, MOE_SPAN);
+            int r = rows, q = tiles, u = runs;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const int pr = __shfl_up_sync(0xffffffffu, r, o), pq = __shfl_up_sync(0xffffffffu, q, o);
+                const int pr = __shfl_up_sync(0xffffffffu, r, o), pq = __shfl_up_sync(0xffffffffu, q, o), pu = __shfl_up_sync(0xffffffffu, u, o);
                 if (lane >= o) {
                     r += pr;
                     q += pq;
+                    u += pu;
                 }
             }
             if (e < E) {
                 cursor[e] = at + r - rows;
                 first[e] = tile + q - tiles;
             }
+            if (spans) {            // an expert's rows in even runs of at most MOE_SPAN, their length a multiple of 32
+                const int width = runs ? (ceil_div(c, runs) + 31) / 32 * 32 : 0;
+                for (int k = 0; k < runs; ++k) spans[1 + span + u - runs + k] = make_int4(e, at + r - rows + k * width, min(width, c - k * width), width);
+            }
             at += __shfl_sync(0xffffffffu, r, 31);
             tile += __shfl_sync(0xffffffffu, q, 31);
+            span += __shfl_sync(0xffffffffu, u, 31);
         }
+        if (spans && lane == 0) spans[0] = make_int4(span, 0, 0, 0);
     }
     __syncthreads();
     const int used = first[E - 1] + ceil_div(count[E - 1], tt);
@@ -454,17 +463,21 @@ LLMK_EXPORT int llmk_moe_max_tiles(int n_slots, int E, int tile) {
     return n_slots / tt + (E < n_slots ? E : n_slots);
 }
 
+// The most runs of at most 256 rows of one expert that `n_slots` slots can need (entries of `spans` behind its first).
+LLMK_EXPORT int llmk_moe_max_spans(int n_slots, int E) { return n_slots / MOE_SPAN + (E < n_slots ? E : n_slots); }
+
 // tile: rows per tile (0: 16, what `moe_experts` takes); padded != 0: experts' rows start on tile boundaries and `order`
-// has max_tiles * tile entries.
+// has max_tiles * tile entries.  spans (optional, 16-byte aligned): how many runs, then (expert, first row, rows, rows rounded up to 32) of each.
 LLMK_EXPORT int llmk_moe_plan(const int* slot_expert, int n_slots, int E, int tile, int padded, int* order, int* pos_of_slot,
-                              int* tile_expert, int* tile_start, int* tile_rows, void* stream) {
+                              int* tile_expert, int* tile_start, int* tile_rows, void* spans, void* stream) {
     if (n_slots <= 0) return LLMK_OK;
     const int tt = tile > 0 ? tile : MOE_TT;
     const size_t smem = (size_t)3 * E * sizeof(int);
     if (smem > 48 * 1024) LLMK_FAIL("moe_plan: %d experts are too many", E);
+    if (!host_aligned16(spans)) LLMK_FAIL("moe_plan: spans must start on a 16-byte boundary");
     LLMK_CHECK_LAUNCH_RC("moe_plan", llmk_launch(moe_plan_kernel, dim3(1), dim3(1024), smem, (cudaStream_t)stream, true, slot_expert, n_slots, E,
                                                  llmk_moe_max_tiles(n_slots, E, tile), tt, padded, order, pos_of_slot, tile_expert, tile_start,
-                                                 tile_rows));
+                                                 tile_rows, static_cast<int4*>(spans)));
     return LLMK_OK;
 }
 

@@ -571,7 +571,7 @@ def _cost_grouped_product(a, info: PassInfo) -> Tuple[int, int]:
     G, N, K = (int(v) for v in a["w"].shape)
     rows = int(a.get("real_rows") or a["a"].shape[0])
     touched = min(G, rows)
-    return 2 * rows * N * K, touched * N * K * a["w"].element_size() + rows * (K * a["a"].element_size() + N * a["out"].element_size())
+    return 2 * rows * N * K, touched * N * K * a["w"].element_size() + rows * (K * a["a"].element_size() + a["out"].shape[1] * a["out"].element_size())
 
 
 # kernel bindings of `ops` that launch work, and how each one's FLOPs and bytes are counted

@@ -43,6 +43,7 @@ MODULES: Dict[str, List[str]] = {
     "gemm_simt": [],
     "gemv": [],
     "gemm_tc": [],
+    "gemm_grouped": [],
     "gemm_skinny": [],
     "gemm_rows8": [],
     "attention": [],

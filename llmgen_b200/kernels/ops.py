@@ -1704,15 +1704,24 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, slot_expert: torch.Tensor, 
 
 
 def moe_plan(slot_expert: torch.Tensor, n_slots: int, experts: int, order: torch.Tensor, pos_of_slot: torch.Tensor,
-             tile_expert: torch.Tensor, tile_start: torch.Tensor, tile_rows: torch.Tensor, tile: int = 0, padded: bool = False) -> None:
+             tile_expert: torch.Tensor, tile_start: torch.Tensor, tile_rows: torch.Tensor, tile: int = 0, padded: bool = False,
+             spans: Optional[torch.Tensor] = None) -> None:
     """Groups the slots by expert into tiles of `tile` rows (0: 16).  `padded`: every expert's rows start on a tile, `order`
-    has moe_max_tiles(...) * tile entries (-1 where a tile has no row) and tile i is rows [i * tile, (i + 1) * tile)."""
+    has moe_max_tiles(...) * tile entries (-1 where a tile has no row) and tile i is rows [i * tile, (i + 1) * tile).  `spans`
+    (int32 [moe_max_spans(...) + 1, 4]): the runs of rows that `gemm_grouped` takes."""
     lib = build.load("moe")
     need = moe_max_tiles(n_slots, experts, tile) * tile if padded else n_slots
     if order.numel() < need or tile_expert.numel() < moe_max_tiles(n_slots, experts, tile):
         raise KernelError("moe_plan: arrays too small")
+    if spans is not None and (spans.dtype != torch.int32 or spans.numel() < 4 * (moe_max_spans(n_slots, experts) + 1)):
+        raise KernelError("moe_plan: spans are int32, four for every run and four in front")
     _check(lib, lib.llmk_moe_plan(_ptr(slot_expert), c_int(n_slots), c_int(experts), c_int(tile), c_int(1 if padded else 0), _ptr(order),
-                                  _ptr(pos_of_slot), _ptr(tile_expert), _ptr(tile_start), _ptr(tile_rows), _stream()))
+                                  _ptr(pos_of_slot), _ptr(tile_expert), _ptr(tile_start), _ptr(tile_rows), _ptr(spans), _stream()))
+
+
+def moe_max_spans(n_slots: int, experts: int) -> int:
+    """The most runs of at most 256 rows of one expert that `n_slots` rows grouped by expert can need."""
+    return int(build.load("moe").llmk_moe_max_spans(c_int(n_slots), c_int(experts)))
 
 
 def moe_gather(out: torch.Tensor, h: torch.Tensor, order: torch.Tensor, slot_weight: torch.Tensor, top: int, scale_rows: bool) -> None:
@@ -1742,6 +1751,28 @@ def gemm_tc_grouped(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, tile_gr
     _check(lib, lib.llmk_gemm_tc_grouped(_ptr(out), _ptr(a), _ptr(w), c_int(M), c_int(N), c_int(K), c_longlong(_row_stride(a)),
                                          c_longlong(K), c_longlong(_row_stride(out)), c_int(G), _ptr(tile_group),
                                          c_int(1 if activation == "relu2" else 0), c_int(dtype_code(out.dtype)), _ptr(tc_error_flag(a.device)), c_int(1), _stream()))
+
+
+GROUPED_ACTIVATIONS = {None: 0, "relu2": 1, "silu_glu": 2, "clamped_glu": 3}
+
+
+def gemm_grouped(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, spans: torch.Tensor, activation: Optional[str] = None,
+                 alpha: float = 1.0, limit: float = 0.0, real_rows: int = 0) -> None:
+    """out[m] = act(a[m] @ w[e]^T) for the rows of a [n, K] that `spans` (`moe_plan`) gives to expert e; w [experts, N, K] contiguous, both
+    bfloat16 (csrc/gemm_grouped.cu).  No activation: out [n, N] float32 or bfloat16.  "relu2", or a gated unit ("silu_glu", "clamped_glu" with
+    `alpha` and `limit`; w interleaves gate and up rows in groups of 16, out [n, N / 2]): bfloat16.  `real_rows`: how many rows hold data (for
+    the profiler's count of the work)."""
+    lib = build.load("gemm_grouped")
+    n, K = a.shape
+    E, N, Kw = w.shape
+    if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or Kw != K or not w.is_contiguous() or spans.dtype != torch.int32 \
+            or tuple(out.shape) != (n, N // 2 if activation in ("silu_glu", "clamped_glu") else N):
+        raise KernelError(f"gemm_grouped: a{list(a.shape)} w{list(w.shape)} out{list(out.shape)} do not fit")
+    if activation not in GROUPED_ACTIVATIONS:
+        raise KernelError(f"gemm_grouped: activation {activation!r} is not built")
+    _check(lib, lib.llmk_gemm_grouped(_ptr(out), _ptr(a), _ptr(w), _ptr(spans), c_int(spans.numel() // 4 - 1), c_int(n), c_int(E), c_int(N), c_int(K),
+                                      c_longlong(_row_stride(a)), c_longlong(_row_stride(out)), c_int(GROUPED_ACTIVATIONS[activation]),
+                                      c_float(alpha), c_float(limit), c_int(dtype_code(out.dtype)), _ptr(tc_error_flag(a.device)), _stream()))
 
 
 def moe_experts(out: torch.Tensor, x: torch.Tensor, w0: torch.Tensor, w1: Optional[torch.Tensor], order: torch.Tensor,

@@ -6,6 +6,7 @@ import torch
 from ..kernels import ops
 from .base import FeedForward
 from .linear import GEMM_MODULES, linear, linear_sliced
+from .mlp import GATE_UP_GROUP, interleave_gate_up
 from .registry import register_feed_forward
 from .spec import VECTOR, ClampedExpertSpec, DenseMLPSpec, GatedExpertSpec, GatedMLPSpec, PlainExpertSpec, RoutedMLPSpec, WeightDecl
 
@@ -70,11 +71,11 @@ class RoutedMLP(FeedForward):
     in slot order to the shared expert's output.  The experts' matrices are stacked [experts, ...] at load.  Between
     plan and sum:
 
-      bfloat16   tiles of 128 rows, every expert's rows starting on a tile: `moe_gather` copies the rows (times their
-                 weights, where the weight is on the expert's input; else `moe_combine` applies it) into that order, and the grouped tensor-core product (`gemm_tc_grouped`: TMA, tcgen05.mma,
-                 the expert of each tile read from the device) runs gate/up of all experts in one launch, the clamped
-                 gated activation follows row-wise (experts without a gate: relu squared in the product's epilogue), and a
-                 second grouped launch runs down
+      bfloat16   `moe_gather` copies the rows (times their
+                 weights, where the weight is on the expert's input; else `moe_combine` applies it) into the experts' order, and the grouped tensor-core product (`gemm_grouped`: TMA, tcgen05.mma,
+                 the runs of rows of one expert read from the device) runs gate/up of all experts in one launch, with the
+                 activation in its epilogue (gate and up rows interleaved in groups of 16 at load; expert widths that are no multiple of
+                 16: row-wise behind the product), and a second grouped launch runs down
       float32    (and operands TMA refuses) tiles of 16 rows through `moe_experts`, float32 sums on the CUDA cores
 
     A caller that adds the experts' rows up itself (`forward(..., combine=False)`) gets them as an `ops.RoutedRows`; one that has
@@ -108,7 +109,7 @@ class RoutedMLP(FeedForward):
 
     @staticmethod
     def kernel_modules(spec):
-        return ("moe", "rowwise", "elementwise") + GEMM_MODULES
+        return ("moe", "gemm_grouped", "rowwise", "elementwise") + GEMM_MODULES
 
     def __init__(self, spec: RoutedMLPSpec, weights, dtype, device):
         first = spec.experts[0]
@@ -141,11 +142,16 @@ class RoutedMLP(FeedForward):
         self.w_gate = None if self.gateless else stack([e.gate_proj for e in spec.experts])     # [E, F, H]
         self.w_up = stack([e.up_proj for e in spec.experts])         # [E, F, H]
         self.w_down = stack([e.down_proj for e in spec.experts])     # [E, H, F]
-        # the tensor-core path reads gate and up as one matrix per expert, [E, 2F, H]: gate rows, then up rows
+        # the tensor-core path reads gate and up as one matrix per expert, [E, 2F, H]: in turn, 16 rows each, or gate rows, then up rows
         H = spec.hidden_size
         self.grouped = dtype == torch.bfloat16 and H % 8 == 0 and self.F % 8 == 0
+        self.fused = self.grouped and not self.gateless and self.F % GATE_UP_GROUP == 0
         if self.grouped and not self.gateless:
-            self.w_gate_up = torch.cat([self.w_gate, self.w_up], dim=1).contiguous()
+            if self.fused:
+                # (one interleaving of all experts' rows, as `interleave_gate_up` does it for one matrix)
+                self.w_gate_up = interleave_gate_up(self.w_gate.view(-1, H), self.w_up.view(-1, H)).view(self.E, 2 * self.F, H)
+            else:
+                self.w_gate_up = torch.cat([self.w_gate, self.w_up], dim=1).contiguous()
             self.w_gate = self.w_up = None
         self.shared_gate_up = self.shared_down = self.shared_mlp = None
         if isinstance(spec.shared, GatedExpertSpec):
@@ -184,7 +190,9 @@ class RoutedMLP(FeedForward):
         ops.moe_route(x, self.router, slot_expert, slot_weight, top, spec.scoring, spec.renormalize, bias=self.router_bias,
                       choice_bias=self.choice_bias, weight_scale=float(spec.weight_scale), sum_eps=float(spec.sum_eps), pdl=pdl,
                       groups=spec.groups, keep_groups=spec.keep_groups, gate_out=shared_gate)
-        ops.moe_plan(slot_expert, n_slots, self.E, order, pos_of_slot, tile_expert, tile_start, tile_rows, tile=tile, padded=self.grouped)
+        spans = ws.flat("moe_spans", 4 * (ops.moe_max_spans(n_slots, self.E) + 1), torch.int32) if self.grouped else None
+        ops.moe_plan(slot_expert, n_slots, self.E, order, pos_of_slot, tile_expert, tile_start, tile_rows, tile=tile, padded=self.grouped,
+                     spans=spans)
         cap = (ws.default_rows * top // 128 + self.E) * 128 if self.grouped else ws.default_rows * top
         rows = ws.buffer("moe_rows", n_rows, H, torch.float32, capacity_rows=cap)
         if self.grouped:
@@ -192,12 +200,14 @@ class RoutedMLP(FeedForward):
             ops.moe_gather(xs, x, order, slot_weight, top, scale_rows=spec.weight_on_input)
             y = ws.buffer("moe_act", n_rows, self.F, self.dtype, capacity_rows=cap)
             if self.gateless:
-                ops.gemm_tc_grouped(y, xs, self.w_up, tile_expert, real_rows=n_slots, activation="relu2")
+                ops.gemm_grouped(y, xs, self.w_up, spans, "relu2", real_rows=n_slots)
+            elif self.fused:
+                ops.gemm_grouped(y, xs, self.w_gate_up, spans, self.act, alpha=self.alpha, limit=self.limit, real_rows=n_slots)
             else:
                 gate_up = ws.buffer("moe_gate_up", n_rows, 2 * self.F, self.dtype, capacity_rows=cap)
-                ops.gemm_tc_grouped(gate_up, xs, self.w_gate_up, tile_expert, real_rows=n_slots)
+                ops.gemm_grouped(gate_up, xs, self.w_gate_up, spans, real_rows=n_slots)
                 ops.act_rows(y, gate_up, self.act, alpha=self.alpha, limit=self.limit)
-            ops.gemm_tc_grouped(rows, y, self.w_down, tile_expert, real_rows=n_slots)
+            ops.gemm_grouped(rows, y, self.w_down, spans, real_rows=n_slots)
         else:
             y = ws.buffer("moe_act", n_rows, self.F, torch.float32, capacity_rows=cap)
             first = (self.w_up, None) if self.gateless else (self.w_gate, self.w_up)
