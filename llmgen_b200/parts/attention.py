@@ -19,23 +19,33 @@ def add_query_tiles(builder, bq: int, window: int = 0, heaviest_first: bool = Fa
     name = f"attention_tiles_bq{bq}"
     if builder.has(name + "_seq"):
         return name
-    tiles = []
+    # (a sequence's run of tiles at a time: tile by tile the list took 94 us of a step with prompts of 666 and 1,333 tokens in tiles of 8,
+    # 23 so; whole arrays of numpy cost a list of a dozen tiles 12 us more)
+    seq, start, keys = [], [], []
     bound = getattr(builder, "token_bound", 0)
     for s, n in enumerate(builder.q_lens):
         if bound and n == 0:
             continue
-        for start in range(0, max(n, 1), bq):
-            keys = builder.starts[s] + min(start + bq, max(n, 1))
-            tiles.append((min(keys, window + bq) if window else keys, s, start))
+        rows = max(n, 1)
+        firsts = range(0, rows, bq)
+        seq += [s] * len(firsts)
+        start += firsts
+        if heaviest_first:
+            before = builder.starts[s]
+            reads = list(range(before + bq, before + bq * len(firsts), bq))
+            reads.append(before + rows)
+            keys += [min(k, window + bq) for k in reads] if window else reads
     if heaviest_first:
-        tiles.sort(key=lambda t: -t[0])
+        order = sorted(range(len(seq)), key=keys.__getitem__, reverse=True)
+        seq, start = [seq[i] for i in order], [start[i] for i in order]
     if bound:
         # a list of fixed length for the step's shape: no more tiles than this exist for `bound` tokens in
         # `n_seqs` sequences; the rest is padding (sequence -1), which the kernels skip
-        most = bound // bq + builder.n_seqs
-        tiles += [(0, -1, 0)] * (most - len(tiles))
-    builder.add(name + "_seq", [t[1] for t in tiles])
-    builder.add(name + "_q0", [t[2] for t in tiles])
+        pad = bound // bq + builder.n_seqs - len(seq)
+        seq += [-1] * pad
+        start += [0] * pad
+    builder.add(name + "_seq", seq)
+    builder.add(name + "_q0", start)
     return name
 
 
