@@ -258,14 +258,15 @@ __device__ __forceinline__ float from_start(const Weights& w, int i) {
 // COLS columns of a chunk's rows on their way into shared memory: `ask` sends for a thread's 16-byte vectors, all at once, and `put` writes them
 // as NT terms, times `scale` per row (null: 1), zeros beyond the chunk's n tokens.
 // `odd`: whether one of the thread's values is none that terms can be made of.
-template <typename T, int NT, int COLS>
+template <typename T, int NT, int COLS, int NTHREADS = THREADS>
 struct Rows {
-    static constexpr int VN = Vec16<T>::N, LD = COLS + 8, EACH = C * COLS / VN / THREADS;
+    static constexpr int VN = Vec16<T>::N, LD = COLS + 8, EACH = C * COLS / VN / NTHREADS;
+    static_assert(EACH * VN * NTHREADS == C * COLS, "whole vectors a thread");
     Vec16<T> held[EACH];
     __device__ __forceinline__ void ask(const T* src, long long ld, int n) {
 #pragma unroll
         for (int i = 0; i < EACH; ++i) {
-            const int idx = threadIdx.x + i * THREADS, r = idx / (COLS / VN), c = idx % (COLS / VN) * VN;
+            const int idx = threadIdx.x + i * NTHREADS, r = idx / (COLS / VN), c = idx % (COLS / VN) * VN;
             if (r < n) held[i].raw = *reinterpret_cast<const decltype(held[i].raw)*>(src + (size_t)r * ld + c);
         }
     }
@@ -275,7 +276,7 @@ struct Rows {
         for (int i = 0; i < EACH; ++i) {
             float f[VN];
             held[i].unpack(f);
-            const bool row = (threadIdx.x + i * THREADS) / (COLS / VN) < n;
+            const bool row = (threadIdx.x + i * NTHREADS) / (COLS / VN) < n;
 #pragma unroll
             for (int u = 0; u < VN; ++u) any |= row && odd_value(f[u]);
         }
@@ -284,7 +285,7 @@ struct Rows {
     __device__ __forceinline__ void put(bf16* dst, int n, int silu, const float* scale) {
 #pragma unroll
         for (int i = 0; i < EACH; ++i) {
-            const int idx = threadIdx.x + i * THREADS, r = idx / (COLS / VN), c = idx % (COLS / VN) * VN;
+            const int idx = threadIdx.x + i * NTHREADS, r = idx / (COLS / VN), c = idx % (COLS / VN) * VN;
             float f[VN];
             if (r < n) {
                 if constexpr (NT == 1) {        // (bfloat16 as it is)
@@ -465,7 +466,12 @@ __global__ void __launch_bounds__(THREADS) chunk_memory_scan_kernel(Params p) {
 }
 
 // ------------------------------------------------------------------------------------------------------------------ out
-// Block (chunk, head): warp w has rows 16 (w % 4) of the chunk and half of the keys (scores) or of 64 value columns (outputs).
+// Block (chunk, head): warp w has rows 16 (w % 4) of the chunk and, as number w / 4 of `GROUPS`, that part of the keys (scores) or of 64 value columns
+// (outputs).  Sixteen warps an SM hide more of the MMAs' and loads' chains than eight: as two blocks of eight where the operands are one term and two
+// blocks' shared memory fits (a prompt of 2,048 under a running maximum, 8 heads: 28.4 -> 23.8 us; the layer's pass 296 -> 290, with one block of
+// sixteen 294), as one block of sixteen where they are three (constant decay, 16 heads: 70.1 -> 66.8 us, the pass 355 -> 350).  What holds the second
+// form is not its warps: the MMAs of its terms take 19 us at the rate `mma.sync` reaches alone.
+template <typename T, int FORM> constexpr int out_warps() { return input_terms<T, FORM>() == 1 ? 8 : 16; }
 template <typename T, int FORM, int D>
 struct OutLayout {
     static constexpr int NT = input_terms<T, FORM>(), LDD = D + 8;
@@ -473,16 +479,16 @@ struct OutLayout {
     static constexpr size_t bytes() { return (size_t)(Q + KS + P + V) * sizeof(bf16); }
 };
 template <typename T, int FORM, int D>
-__global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) {
+__global__ void __launch_bounds__(32 * out_warps<T, FORM>(), 16 / out_warps<T, FORM>()) chunk_memory_out_kernel(Params p) {
     using L = OutLayout<T, FORM, D>;
-    constexpr int NT = L::NT, LDD = L::LDD;
+    constexpr int NT = L::NT, LDD = L::LDD, WARPS = out_warps<T, FORM>(), NTHREADS = 32 * WARPS, GROUPS = WARPS / 4, N8 = 8 / GROUPS;
     extern __shared__ __align__(16) bf16 smem[];
     bf16* Qs = smem;                            // [NT][C][LDD]
     bf16* Ks = Qs + L::Q;                       // [NT][C][LDD], then the state's columns [3][D][LDE]
     bf16* Ps = Ks + L::KS;                      // [3][C][LDP]: the weighted scores
     bf16* Vs = Ps + L::P;                       // [NT][C][LDE]
     __shared__ Weights w;
-    __shared__ float start[C], sums[2][C], n_dot[C];
+    __shared__ float start[C], sums[GROUPS][C], n_dot[C];
     const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_launch_dependents();
     pdl_wait();
@@ -492,19 +498,19 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
     const int q_beg = p.cu_q[at.s], t0 = q_beg + at.chunk * C, n = min(C, p.cu_q[at.s + 1] - t0);
     const float* before = p.scratch + ((size_t)blockIdx.x * p.H + h) * p.entries;
     // the state's entries of 64 columns, float4 a thread and turn: asked for early, put down where the keys were
-    constexpr int SV = D * EB / 4 / THREADS;
+    constexpr int SV = D * EB / 4 / NTHREADS;
     float4 held[SV];
     auto ask = [&](int e0) {
 #pragma unroll
         for (int i = 0; i < SV; ++i) {
-            const int idx = tid + i * THREADS, d = idx / (EB / 4), c = idx % (EB / 4) * 4;
+            const int idx = tid + i * NTHREADS, d = idx / (EB / 4), c = idx % (EB / 4) * 4;
             held[i] = *reinterpret_cast<const float4*>(before + (size_t)d * p.E + e0 + c);
         }
     };
     const T* vp = static_cast<const T*>(p.v) + (size_t)t0 * p.ldv + (size_t)h * p.E;
-    Rows<T, NT, EB> values;
+    Rows<T, NT, EB, NTHREADS> values;
     {
-        Rows<T, NT, D> queries, keys;
+        Rows<T, NT, D, NTHREADS> queries, keys;
         queries.ask(static_cast<const T*>(p.q) + (size_t)t0 * p.ldq + (size_t)h * D, p.ldq, n);
         keys.ask(static_cast<const T*>(p.k) + (size_t)t0 * p.ldk + (size_t)h * D, p.ldk, n);
         values.ask(vp, p.ldv, n);
@@ -516,12 +522,12 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
     }
     __syncthreads();
     if (tid < C) start[tid] = tid < n ? from_start<FORM>(w, tid) * p.q_scale : 0.f;
-    const int r0 = 16 * (warp & 3), half = warp >> 2;
-    // scores of 16 rows and 32 keys, those of keys behind all rows left out
+    const int r0 = 16 * (warp & 3), group = warp >> 2;
+    // scores of 16 rows and the group's keys, those of keys behind all rows left out
     {
-        Sums<4> s;
+        Sums<N8> s;
         s.clear();
-        const int j0 = 32 * half;
+        const int j0 = 8 * N8 * group;
         if (j0 <= r0 + 15) {
 #pragma unroll 2
             for (int d = 0; d < D; d += 16) {
@@ -529,7 +535,7 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
 #pragma unroll
                 for (int t = 0; t < NT; ++t) ldsm4(a[t], Qs + (t * C + r0 + (lane & 15)) * LDD + d + (lane >> 4) * 8);
 #pragma unroll
-                for (int n8 = 0; n8 < 4; n8 += 2) {
+                for (int n8 = 0; n8 < N8; n8 += 2) {
                     if (j0 + 8 * n8 > r0 + 15) continue;
                     uint32_t b[NT][4];
 #pragma unroll
@@ -541,7 +547,7 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
         }
         float row_sum[2] = {0.f, 0.f};
 #pragma unroll
-        for (int n8 = 0; n8 < 4; ++n8)
+        for (int n8 = 0; n8 < N8; ++n8)
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int i = r0 + lane / 4 + 8 * u, j = j0 + 8 * n8 + 2 * (lane & 3);
@@ -559,11 +565,11 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
             for (int u = 0; u < 2; ++u) {
                 row_sum[u] += __shfl_xor_sync(0xffffffffu, row_sum[u], 1);
                 row_sum[u] += __shfl_xor_sync(0xffffffffu, row_sum[u], 2);
-                if ((lane & 3) == 0) sums[half][r0 + lane / 4 + 8 * u] = row_sum[u];
+                if ((lane & 3) == 0) sums[group][r0 + lane / 4 + 8 * u] = row_sum[u];
             }
-            // q . n of 8 rows a warp
+            // q . n, a row a warp in turn
             const float* nb = before + (size_t)D * p.E;
-            for (int i = warp; i < n; i += 8) {
+            for (int i = warp; i < n; i += WARPS) {
                 float x = 0.f;
 #pragma unroll
                 for (int d = lane; d < D; d += 32) {
@@ -581,7 +587,7 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
         __syncthreads();                        // the keys, or the columns before, are used
 #pragma unroll
         for (int i = 0; i < SV; ++i) {
-            const int idx = tid + i * THREADS, d = idx / (EB / 4), c = idx % (EB / 4) * 4;
+            const int idx = tid + i * NTHREADS, d = idx / (EB / 4), c = idx % (EB / 4) * 4;
             uint32_t a[3], b[3];
             terms<3>(a, held[i].x, held[i].y);
             terms<3>(b, held[i].z, held[i].w);
@@ -594,7 +600,7 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
             ask(e0 + EB);
             values.ask(vp + e0 + EB, p.ldv, n);
         }
-        Sums<4> o;
+        Sums<N8> o;
         o.clear();
 #pragma unroll 2
         for (int d = 0; d < D; d += 16) {
@@ -602,17 +608,17 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
 #pragma unroll
             for (int t = 0; t < NT; ++t) ldsm4(a[t], Qs + (t * C + r0 + (lane & 15)) * LDD + d + (lane >> 4) * 8);
 #pragma unroll
-            for (int n8 = 0; n8 < 4; n8 += 2) {
+            for (int n8 = 0; n8 < N8; n8 += 2) {
                 uint32_t b[3][4];
 #pragma unroll
                 for (int t = 0; t < 3; ++t)
-                    ldsm4t(b[t], Ks + (t * D + d + (lane & 7) + ((lane >> 3) & 1) * 8) * LDE + 32 * half + 8 * n8 + (lane >> 4) * 8);
+                    ldsm4t(b[t], Ks + (t * D + d + (lane & 7) + ((lane >> 3) & 1) * 8) * LDE + 8 * N8 * group + 8 * n8 + (lane >> 4) * 8);
                 mma_terms(o, n8, a, b);
             }
         }
         const float g[2] = {start[r0 + lane / 4], start[r0 + lane / 4 + 8]};
 #pragma unroll
-        for (int n8 = 0; n8 < 4; ++n8)
+        for (int n8 = 0; n8 < N8; ++n8)
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 o.main[n8][u] *= g[u / 2];
@@ -623,11 +629,11 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
 #pragma unroll
             for (int t = 0; t < 3; ++t) ldsm4(a[t], Ps + (t * C + r0 + (lane & 15)) * LDP + j + (lane >> 4) * 8);
 #pragma unroll
-            for (int n8 = 0; n8 < 4; n8 += 2) {
+            for (int n8 = 0; n8 < N8; n8 += 2) {
                 uint32_t b[NT][4];
 #pragma unroll
                 for (int t = 0; t < NT; ++t)
-                    ldsm4t(b[t], Vs + (t * C + j + (lane & 7) + ((lane >> 3) & 1) * 8) * LDE + 32 * half + 8 * n8 + (lane >> 4) * 8);
+                    ldsm4t(b[t], Vs + (t * C + j + (lane & 7) + ((lane >> 3) & 1) * 8) * LDE + 8 * N8 * group + 8 * n8 + (lane >> 4) * 8);
                 mma_terms(o, n8, a, b);
             }
         }
@@ -637,12 +643,15 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_memory_out_kernel(Params p) 
             if (i >= n) continue;
             float inv = 1.f;
             if (FORM == CM_MAX) {
-                const float dot = fmaf(start[i], n_dot[i], sums[0][i] + sums[1][i]);
+                float keys_sum = sums[0][i];
+#pragma unroll
+                for (int k = 1; k < GROUPS; ++k) keys_sum += sums[k][i];
+                const float dot = fmaf(start[i], n_dot[i], keys_sum);
                 inv = 1.0f / (fmaxf(fabsf(dot), expf(-w.top[i])) + p.den_eps);
             }
-            float* to = p.out + (size_t)(t0 + i) * ((size_t)p.H * p.E) + (size_t)h * p.E + e0 + 32 * half + 2 * (lane & 3);
+            float* to = p.out + (size_t)(t0 + i) * ((size_t)p.H * p.E) + (size_t)h * p.E + e0 + 8 * N8 * group + 2 * (lane & 3);
 #pragma unroll
-            for (int n8 = 0; n8 < 4; ++n8) *reinterpret_cast<float2*>(to + 8 * n8) = make_float2(o.at(n8, 2 * u) * inv, o.at(n8, 2 * u + 1) * inv);
+            for (int n8 = 0; n8 < N8; ++n8) *reinterpret_cast<float2*>(to + 8 * n8) = make_float2(o.at(n8, 2 * u) * inv, o.at(n8, 2 * u + 1) * inv);
         }
     }
 }
@@ -672,7 +681,7 @@ static int launch_width(const Params& p, cudaStream_t s) {
     const dim3 scan((unsigned)std::min<long long>(items, 8 * device_sm_count()));
     LLMK_CHECK_LAUNCH_RC("chunk_memory_local", llmk_launch(k1, grid, dim3(THREADS), local, s, true, p));
     LLMK_CHECK_LAUNCH_RC("chunk_memory_scan", llmk_launch(chunk_memory_scan_kernel<FORM>, scan, dim3(THREADS), 0, s, true, p));
-    LLMK_CHECK_LAUNCH_RC("chunk_memory_out", llmk_launch(k3, grid, dim3(THREADS), out, s, true, p));
+    LLMK_CHECK_LAUNCH_RC("chunk_memory_out", llmk_launch(k3, grid, dim3(32 * out_warps<T, FORM>()), out, s, true, p));
     return LLMK_OK;
 }
 template <typename T, int FORM>
