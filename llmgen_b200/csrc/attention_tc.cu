@@ -91,7 +91,7 @@ struct Smem {
     static constexpr int P_OFF = V_OFF + BUFFERS * KV_BYTES;   // BUFFERS x TERMS
     static constexpr int XCHG_OFF = P_OFF + BUFFERS * TERMS * P_BYTES;   // float [2][2][BM]: row maxima (and at the end sums) of the two halves
     static constexpr int BAR_OFF = XCHG_OFF + 2 * 2 * BM * 4;
-    static constexpr int NUM_BARS = 14;
+    static constexpr int NUM_BARS = 15, P_FULL = 11;     // (P_FULL, P_FULL + 1: an arrival from every softmax thread)
     // No slack for aligning the base: the kernel has no static shared memory, so the dynamic part
     // starts on a 1024-byte boundary; the kernel checks that and reports an error otherwise.
     static constexpr int TOTAL = BAR_OFF + NUM_BARS * 8 + 16;
@@ -169,8 +169,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     uint64_t* k_empty = bars + 5;       // 2
     uint64_t* v_empty = bars + 7;       // 2
     uint64_t* s_full = bars + 9;        // 2
-    uint64_t* p_full = bars + 11;       // 1, 256 arrivals
-    uint64_t* o_full = bars + 12;       // 2
+    // Two, for the tiles in turn, 256 arrivals each.  (One for all tiles is too few: the scores of tile j + 1 are there as soon as tile j - 1
+    // has been multiplied, so a warp may be done with tile j + 1 while another still writes its P of tile j, and its 32 arrivals would
+    // stand in for the missing ones: P V then read 32 rows that were not written yet.  An arrival for tile j + 2 comes after P V of tile j.)
+    uint64_t* p_full = bars + L::P_FULL;
+    uint64_t* o_full = bars + 13;       // 2
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NUM_BARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -183,7 +186,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < L::NUM_BARS; ++i) tc::mbar_init(tc::smem_u32(&bars[i]), i == 11 ? 256 : 1);
+        for (int i = 0; i < L::NUM_BARS; ++i) tc::mbar_init(tc::smem_u32(&bars[i]), i == L::P_FULL || i == L::P_FULL + 1 ? 256 : 1);
         tc::fence_barrier_init();
         tc::prefetch_tensormap(&map_q);
         tc::prefetch_tensormap(&map_k);
@@ -294,7 +297,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (ok && n_tiles > 1) ok = issue_qk(1);
             for (int j = 0; j < n_tiles && ok; ++j) {
                 const int st = j & 1;
-                ok = tc::mbar_wait_warp(tc::smem_u32(p_full), j & 1, abort_flag) &&
+                ok = tc::mbar_wait_warp(tc::smem_u32(&p_full[st]), (j >> 1) & 1, abort_flag) &&
                      tc::mbar_wait_warp(tc::smem_u32(&v_full[st & LAST]), (j / L::BUFFERS) & 1, abort_flag);
                 if (!ok) break;
                 tc::tc_fence_after_sync();
@@ -456,7 +459,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 l = l * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
                 tc::fence_proxy_async();
                 tc::tc_fence_before_sync();
-                if (TERMS == 1 || ok) tc::mbar_arrive(tc::smem_u32(p_full));
+                if (TERMS == 1 || ok) tc::mbar_arrive(tc::smem_u32(&p_full[st]));
             }
         }
         if (ok && n_tiles > 0) {
