@@ -358,11 +358,11 @@ __global__ void __launch_bounds__(NWARPS * 32) paged_attention_kernel(AttnParams
 
 // One warp per (token, head): merge the partial results of the key parts.
 template <typename T>
-__global__ void attention_reduce_kernel(T* __restrict__ out, long long o_stride, const float* __restrict__ part_o,
-                                        const float* __restrict__ part_ml, int n_rows, int nq, int hd,
-                                        int num_parts, int sink, const float* __restrict__ sink_values, const T* __restrict__ gate, long long gate_stride,
-                                        int gate_heads, const float* __restrict__ turn_cos, const float* __restrict__ turn_sin,
-                                        const int* __restrict__ positions) {
+__global__ void attention_reduce_kernel(T* out, long long o_stride, const float* part_o,
+                                        const float* part_ml, int n_rows, int nq, int hd,
+                                        int num_parts, int sink, const float* sink_values, const T* gate, long long gate_stride,
+                                        int gate_heads, const float* turn_cos, const float* turn_sin,
+                                        const int* positions) {
     const int lane = threadIdx.x & 31;
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     pdl_launch_dependents();

@@ -40,14 +40,14 @@ struct PackedRow {
 };
 
 template <typename T>
-__global__ void attn_prep_kernel(const void* __restrict__ qkv, long long row_stride, int splits, long long split_stride,
-                                 T* __restrict__ q_out, long long q_stride, T* __restrict__ kcache,
-                                 T* __restrict__ vcache, const int* __restrict__ positions,
-                                 const int* __restrict__ slots, const float* __restrict__ cos_tab,
-                                 const float* __restrict__ sin_tab, const float* __restrict__ q_gain,
-                                 const float* __restrict__ k_gain, int n_tokens, int nq, int nk, int nkv_cache,
+__global__ void attn_prep_kernel(const void* qkv, long long row_stride, int splits, long long split_stride,
+                                 T* q_out, long long q_stride, T* kcache,
+                                 T* vcache, const int* positions,
+                                 const int* slots, const float* cos_tab,
+                                 const float* sin_tab, const float* q_gain,
+                                 const float* k_gain, int n_tokens, int nq, int nk, int nkv_cache,
                                  int hd, int rot, int page_size, float eps, float q_off, float k_off,
-                                 const float* __restrict__ bias, int vd, int interleaved, int norm_after) {
+                                 const float* bias, int vd, int interleaved, int norm_after) {
     const int lane = threadIdx.x & 31;
     const int warps_per_block = blockDim.x >> 5;
     const int heads = nq + 2 * nk;
@@ -236,11 +236,11 @@ __global__ void attn_prep_kernel(const void* __restrict__ qkv, long long row_str
 // partial sums, and everything is 16-byte aligned.
 template <typename T, int LPR>
 __global__ void __launch_bounds__(256)
-attn_prep_vec_kernel(const T* __restrict__ qkv, long long row_stride, T* __restrict__ q_out, long long q_stride,
-                     T* __restrict__ kcache, T* __restrict__ vcache, const int* __restrict__ positions,
-                     const int* __restrict__ slots, const float* __restrict__ cos_tab,
-                     const float* __restrict__ sin_tab, const float* __restrict__ q_gain,
-                     const float* __restrict__ k_gain, int n_tokens, int nq, int nk, int nkv_cache, int hd,
+attn_prep_vec_kernel(const T* qkv, long long row_stride, T* q_out, long long q_stride,
+                     T* kcache, T* vcache, const int* positions,
+                     const int* slots, const float* cos_tab,
+                     const float* sin_tab, const float* q_gain,
+                     const float* k_gain, int n_tokens, int nq, int nk, int nkv_cache, int hd,
                      int page_size, float eps, float q_off, float k_off) {
     constexpr int EPL = Vec16<T>::N;            // elements per lane
     constexpr int RPW = 32 / LPR;               // rows per warp
@@ -369,11 +369,11 @@ __device__ __forceinline__ void load_floats(float* f, const float* src) {
 // of 128; with a lane's values in one piece and eight rounds 700 / 2,048 / 8,000 tokens took 5.8 / 10.7 / 43.2 us).
 template <typename T, int LPR, int U>
 __global__ void __launch_bounds__(256, 3)
-attn_prep_token_kernel(const T* __restrict__ qkv, long long row_stride, T* __restrict__ q_out, long long q_stride,
-                       T* __restrict__ kcache, T* __restrict__ vcache, const int* __restrict__ positions,
-                       const int* __restrict__ slots, const float* __restrict__ cos_tab,
-                       const float* __restrict__ sin_tab, const float* __restrict__ q_gain,
-                       const float* __restrict__ k_gain, int n_tokens, int nq, int nk, int nkv_cache, int hd,
+attn_prep_token_kernel(const T* qkv, long long row_stride, T* q_out, long long q_stride,
+                       T* kcache, T* vcache, const int* positions,
+                       const int* slots, const float* cos_tab,
+                       const float* sin_tab, const float* q_gain,
+                       const float* k_gain, int n_tokens, int nq, int nk, int nkv_cache, int hd,
                        int page_size, float eps, float q_off, float k_off) {
     constexpr int EPL = Vec16<T>::N, HALF = EPL / 2;       // elements per lane
     constexpr int RPW = 32 / LPR;               // rows per round
@@ -527,11 +527,11 @@ static bool launch_vec(const void* qkv, long long row_stride, void* q_out, long 
 // (token, head) row.
 template <typename T, int LPR>
 __global__ void __launch_bounds__(256)
-attn_prep_pairs_kernel(const T* __restrict__ qkv, long long row_stride, T* __restrict__ q_out, long long q_stride, T* __restrict__ kcache,
-                       T* __restrict__ vcache, const int* __restrict__ positions, const int* __restrict__ slots,
-                       const float* __restrict__ cos_tab, const float* __restrict__ sin_tab, const float* __restrict__ q_gain,
-                       const float* __restrict__ k_gain, int n_tokens, int nq, int nk, int nkv_cache, int hd, int rot, int page_size,
-                       float eps, float q_off, float k_off, const float* __restrict__ bias, int vd) {
+attn_prep_pairs_kernel(const T* qkv, long long row_stride, T* q_out, long long q_stride, T* kcache,
+                       T* vcache, const int* positions, const int* slots,
+                       const float* cos_tab, const float* sin_tab, const float* q_gain,
+                       const float* k_gain, int n_tokens, int nq, int nk, int nkv_cache, int hd, int rot, int page_size,
+                       float eps, float q_off, float k_off, const float* bias, int vd) {
     constexpr int EPL = Vec16<T>::N;
     const unsigned heads = (unsigned)(nq + 2 * nk);
     const unsigned row = (blockIdx.x * blockDim.x + threadIdx.x) / LPR;
@@ -713,12 +713,12 @@ LLMK_EXPORT int llmk_attn_prep(const void* qkv, long long row_stride, int splits
 // its vd values in pairs (m, m + vd / 2) by angles of its own table (vcos / vsin [max_positions, vd / 2]; none: v as it is).
 // q goes to q_out, k and v to the cache at the token's slot (slot < 0: not stored).  A block per token.
 template <typename T>
-__global__ void attn_prep_rows_kernel(const float* __restrict__ x, long long ld, T* __restrict__ q_out, long long q_stride,
-                                      T* __restrict__ kcache, T* __restrict__ vcache, const int* __restrict__ positions,
-                                      const int* __restrict__ slots, const float* __restrict__ cos_tab,
-                                      const float* __restrict__ sin_tab, const float* __restrict__ vcos,
-                                      const float* __restrict__ vsin, const float* __restrict__ q_gain,
-                                      const float* __restrict__ k_gain, int nq, int nk, int nkv_cache, int hd, int vd, int rot,
+__global__ void attn_prep_rows_kernel(const float* x, long long ld, T* q_out, long long q_stride,
+                                      T* kcache, T* vcache, const int* positions,
+                                      const int* slots, const float* cos_tab,
+                                      const float* sin_tab, const float* vcos,
+                                      const float* vsin, const float* q_gain,
+                                      const float* k_gain, int nq, int nk, int nkv_cache, int hd, int vd, int rot,
                                       int page_size, float eps) {
     __shared__ float scratch[33];
     const size_t t = blockIdx.x;
@@ -818,11 +818,11 @@ __device__ __forceinline__ float packed_sum(const void* x, size_t at, int splits
 }
 
 template <typename T>
-__global__ void __launch_bounds__(512) attn_prep_shared_rows_kernel(const void* __restrict__ x, long long ld, int splits, long long split_stride,
-                                                                    const float* __restrict__ bias, T* __restrict__ q_out, long long q_stride,
-                                                                    T* __restrict__ cache, float* __restrict__ k_scale,
-                                                                    const int* __restrict__ positions, const int* __restrict__ slots,
-                                                                    const float* __restrict__ gains, int nq, int nk, int nkv_cache, int hd,
+__global__ void __launch_bounds__(512) attn_prep_shared_rows_kernel(const void* x, long long ld, int splits, long long split_stride,
+                                                                    const float* bias, T* q_out, long long q_stride,
+                                                                    T* cache, float* k_scale,
+                                                                    const int* positions, const int* slots,
+                                                                    const float* gains, int nq, int nk, int nkv_cache, int hd,
                                                                     int page_size, float eps, float coef, float every) {
     extern __shared__ __align__(16) float prow[];     // nQ + nK floats, 33 scratch
     const int nQ = nq * hd, nK = nk * hd, n = nQ + nK;
@@ -933,9 +933,9 @@ LLMK_EXPORT int llmk_attn_prep_shared_rows(const void* x, long long ld, int spli
 // minus the position's angles (vcos / vsin [max_positions, vd / 2]; none: as they are), then multiplied by sigmoid(gate[t, h]),
 // one number per head (gate rows `gate_stride` apart; none: no gate).  In place; a thread per pair.
 template <typename T>
-__global__ void unrotate_gate_kernel(T* __restrict__ o, long long o_stride, const T* __restrict__ gate, long long gate_stride,
-                                     const int* __restrict__ positions, const float* __restrict__ vcos,
-                                     const float* __restrict__ vsin, long long n, int nq, int vd) {
+__global__ void unrotate_gate_kernel(T* o, long long o_stride, const T* gate, long long gate_stride,
+                                     const int* positions, const float* vcos,
+                                     const float* vsin, long long n, int nq, int vd) {
     pdl_launch_dependents();
     pdl_wait();
     const int vhalf = vd / 2;

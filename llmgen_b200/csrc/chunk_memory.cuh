@@ -77,7 +77,7 @@ inline long long scratch_floats(int form, int n_tokens, int n_seqs, int H, int D
 }
 // What the walk behind the chunks skips: head h of sequence s.  odd: Params::odd(), null where no chunks were launched.
 template <int FORM>
-__device__ __forceinline__ bool taken(const int* __restrict__ odd, int n_tokens, int s, int h, int H) {
+__device__ __forceinline__ bool taken(const int* odd, int n_tokens, int s, int h, int H) {
     return odd && n_tokens > few_of(FORM) && !odd[(size_t)s * H + h];
 }
 
@@ -155,12 +155,12 @@ struct Place {
     int s, chunk, base;         // base: number of the sequence's first chunk
 };
 template <int FORM>
-__device__ __forceinline__ int chunks_of(const int* __restrict__ cu_q, int s) {
+__device__ __forceinline__ int chunks_of(const int* cu_q, int s) {
     const int tokens = cu_q[s + 1] - cu_q[s];
     return tokens > few_of(FORM) ? ceil_div(tokens, C) : 0;
 }
 template <int FORM, bool BY_SEQUENCE>
-__device__ __forceinline__ Place place_of(const int* __restrict__ cu_q, int n_seqs, int c) {
+__device__ __forceinline__ Place place_of(const int* cu_q, int n_seqs, int c) {
     const int lane = threadIdx.x & 31, each = ceil_div(n_seqs, 32), s0 = lane * each, s1 = min(n_seqs, s0 + each);      // a run of sequences a lane
     int count = 0, found = 0;                   // their chunks, and what is counted: chunks, or sequences that have any
 #pragma unroll 4

@@ -140,7 +140,9 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // A kernel launched with `llmk_launch(..., pdl = true)` may start while the kernel before it in
 // the stream is still draining.  Such a kernel must call `pdl_wait()` before it reads anything an
 // earlier kernel wrote or writes anything an earlier kernel may still read; what comes before the
-// wait (barrier set-up, loads of weights) overlaps the predecessor's tail.  `pdl_launch_dependents()`
+// wait (barrier set-up, loads of weights) overlaps the predecessor's tail.  No pointer is `__restrict__` and no activation is read
+// through the read-only path: the kernel before writes these arrays while this grid is already resident, some calls give
+// the same array twice (q, k, v prepared in place), and such loads may be moved in front of the wait.  `pdl_launch_dependents()`
 // lets the next kernel begin its own prologue.  Both are no-ops in a plain launch.  LLMGEN_PDL=0 in
 // the environment turns the attribute off everywhere.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

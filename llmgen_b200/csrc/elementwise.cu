@@ -19,10 +19,10 @@ LLMK_DEFINE_LAST_ERROR()
 // sampled[ids_from[t]] instead: the token that the step before sampled for that row and that
 // the host has not read yet.
 template <typename T>
-__global__ void embed_rows_kernel(float* __restrict__ out, const T* __restrict__ table,
-                                  const int* __restrict__ ids, const int* __restrict__ ids_from,
-                                  const int* __restrict__ sampled, int H, int V, int* bad, float scale,
-                                  const T* __restrict__ pos_table, const int* __restrict__ positions, int n_pos) {
+__global__ void embed_rows_kernel(float* out, const T* table,
+                                  const int* ids, const int* ids_from,
+                                  const int* sampled, int H, int V, int* bad, float scale,
+                                  const T* pos_table, const int* positions, int n_pos) {
     const int t = blockIdx.x;
     pdl_launch_dependents();
     pdl_wait();
@@ -44,9 +44,9 @@ __global__ void embed_rows_kernel(float* __restrict__ out, const T* __restrict__
 
 // The same over whole 16-byte vectors of the table (2,048 rows of 2,048 bfloat16: 12.8 -> 8.3 us).
 template <typename T>
-__global__ void embed_rows_vec_kernel(float* __restrict__ out, const T* __restrict__ table, const int* __restrict__ ids, const int* __restrict__ ids_from,
-                                      const int* __restrict__ sampled, int H, int V, int* bad, float scale, const T* __restrict__ pos_table,
-                                      const int* __restrict__ positions, int n_pos) {
+__global__ void embed_rows_vec_kernel(float* out, const T* table, const int* ids, const int* ids_from,
+                                      const int* sampled, int H, int V, int* bad, float scale, const T* pos_table,
+                                      const int* positions, int n_pos) {
     constexpr int N = Vec16<T>::N;
     const int t = blockIdx.x;
     pdl_launch_dependents();
@@ -113,7 +113,7 @@ LLMK_EXPORT int llmk_embed_rows(float* out, const void* table, const int* ids, c
 
 // x = scale * x, then (cap > 0) x = cap * tanh(x / cap), on float32 logits in place: an architecture's factor on its
 // logits and its bound on them (`ModelSpec.logit_scale`, `ModelSpec.logit_cap`).
-__global__ void logit_cap_kernel(float* __restrict__ x, long long n, float scale, float cap) {
+__global__ void logit_cap_kernel(float* x, long long n, float scale, float cap) {
     pdl_launch_dependents();
     pdl_wait();
     const float inv = cap > 0.f ? 1.0f / cap : 0.f;
@@ -142,9 +142,9 @@ LLMK_EXPORT int llmk_logit_cap(float* x, long long n, float scale, float cap, vo
 //   out[r, :]   = v * (1 / sqrt(mean(v^2) + eps)) * (w + w_offset)      rounded once to T
 // The row is kept in shared memory between the two passes.
 template <typename T>
-__global__ void add_rmsnorm_kernel(float* __restrict__ resid, const void* __restrict__ delta,
-                                   const float* __restrict__ w, T* __restrict__ out,
-                                   const int* __restrict__ rows, int H, float eps, float w_offset,
+__global__ void add_rmsnorm_kernel(float* resid, const void* delta,
+                                   const float* w, T* out,
+                                   const int* rows, int H, float eps, float w_offset,
                                    int write_resid, int splits, long long split_stride) {
     extern __shared__ float srow[];  // H floats + 33 scratch
     float* scratch = srow + H;
@@ -219,9 +219,9 @@ __device__ __forceinline__ void store4(bf16* p, float4 v) {
 }
 
 template <typename T, int VPT>
-__global__ void add_rmsnorm_vec_kernel(float* __restrict__ resid, const void* __restrict__ delta,
-                                       const float* __restrict__ w, T* __restrict__ out,
-                                       const int* __restrict__ rows, int H, float eps, float w_offset,
+__global__ void add_rmsnorm_vec_kernel(float* resid, const void* delta,
+                                       const float* w, T* out,
+                                       const int* rows, int H, float eps, float w_offset,
                                        int write_resid, int splits, long long split_stride) {
     __shared__ float scratch[33];
     const int r = blockIdx.x;
@@ -288,8 +288,8 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ resid, const void* __
 // in T or absent.  (A block per row with one float4 per thread ran at 2.5 TB/s on 2,048 rows of 1,024.)
 template <typename T, int LPT>
 __global__ void __launch_bounds__(128)
-add_rmsnorm_warp_kernel(float* __restrict__ resid, const T* __restrict__ delta, const float* __restrict__ w,
-                        T* __restrict__ out, int n_rows, int H, float eps, float w_offset, int write_resid) {
+add_rmsnorm_warp_kernel(float* resid, const T* delta, const float* w,
+                        T* out, int n_rows, int H, float eps, float w_offset, int write_resid) {
     pdl_launch_dependents();
     pdl_wait();
     const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -410,7 +410,7 @@ LLMK_EXPORT int llmk_add_rmsnorm(float* resid, const void* delta, const float* w
 // rounded once.  Output column j reads gate column 2 * group * (j / group) + j % group and the up
 // column `group` further.
 template <typename T>
-__global__ void silu_mul_kernel(T* __restrict__ out, const T* __restrict__ in, int n, int F, int ld_in, int group) {
+__global__ void silu_mul_kernel(T* out, const T* in, int n, int F, int ld_in, int group) {
     const size_t total = (size_t)n * F;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
@@ -423,7 +423,7 @@ __global__ void silu_mul_kernel(T* __restrict__ out, const T* __restrict__ in, i
 }
 
 template <typename T>
-__global__ void silu_mul_vec_kernel(T* __restrict__ out, const T* __restrict__ in, int n, int F, int ld_in, int group) {
+__global__ void silu_mul_vec_kernel(T* out, const T* in, int n, int F, int ld_in, int group) {
     constexpr int N = Vec16<T>::N;
     const int fv = F / N;
     const size_t total = (size_t)n * fv;
@@ -448,7 +448,7 @@ __global__ void silu_mul_vec_kernel(T* __restrict__ out, const T* __restrict__ i
 // The same from the float32 partial sums of a product cut along K: in is [splits][n][ld_in] with
 // slices `split_stride` floats apart, added in slice order before the activation.
 template <typename T>
-__global__ void silu_mul_partials_kernel(T* __restrict__ out, const float* __restrict__ in, int n, int F, int ld_in,
+__global__ void silu_mul_partials_kernel(T* out, const float* in, int n, int F, int ld_in,
                                          int group, int splits, long long split_stride) {
     pdl_launch_dependents();
     pdl_wait();
@@ -518,7 +518,7 @@ LLMK_EXPORT int llmk_silu_mul(void* out, const void* in, int n_rows, int F, int 
 // --------------------------------------------------------- convert rows to float32
 // out[n, W] float32 = in[n, W] of type T (used to hand bfloat16 logits out as float32).
 template <typename T>
-__global__ void widen_kernel(float* __restrict__ out, const T* __restrict__ in, size_t total) {
+__global__ void widen_kernel(float* out, const T* in, size_t total) {
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x)
         out[idx] = to_float(in[idx]);

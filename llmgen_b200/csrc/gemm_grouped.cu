@@ -59,7 +59,7 @@ __device__ __forceinline__ float glu(float g, float u, float alpha, float limit)
 template <typename TC, int ACT>
 __global__ void __launch_bounds__(THREADS)
 gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x128, const __grid_constant__ CUtensorMap map_x64,
-                    const __grid_constant__ CUtensorMap map_x32, const __grid_constant__ CUtensorMap map_x16, TC* __restrict__ C, const Params p) {
+                    const __grid_constant__ CUtensorMap map_x32, const __grid_constant__ CUtensorMap map_x16, TC* C, const Params p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + BAR_OFF);

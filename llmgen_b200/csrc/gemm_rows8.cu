@@ -48,7 +48,7 @@ __device__ __forceinline__ uint4 load_weight16(const bf16* p) {
 // KB: 32-wide blocks of K per slice (the last slice may hold fewer values: what lies beyond K is zero)
 template <int KB>
 __global__ void __launch_bounds__(WARPS * 32)
-gemm_rows8_kernel(float* __restrict__ out, const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ W,
+gemm_rows8_kernel(float* out, const bf16* x, long long ldx, const bf16* W,
                   long long ldw, int M, int N, int K, int pre) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;          // the MMA's row group and thread in the group
@@ -121,8 +121,8 @@ __device__ __forceinline__ float silu(float g) { return __fdividef(g, 1.0f + __e
 // before it, whose own loads grow with the sequences), so the engine uses it there (`ops.ROWS8_GATED_BEST_ROWS`).
 template <int KB>
 __global__ void __launch_bounds__(WARPS * 32)
-gemm_rows8_gated_kernel(bf16* __restrict__ out, long long ldo, const bf16* __restrict__ x, long long ldx,
-                        const bf16* __restrict__ W, long long ldw, int M, int N, int K, int pre) {
+gemm_rows8_gated_kernel(bf16* out, long long ldo, const bf16* x, long long ldx,
+                        const bf16* W, long long ldw, int M, int N, int K, int pre) {
     __shared__ float part[WARPS][2][16][8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;

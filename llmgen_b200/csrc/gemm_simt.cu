@@ -24,7 +24,7 @@ constexpr int BN = 64, BK = 16, THREADS = 256;      // gemm_simt_kernel
 // Tile BM x BN per block, 16 x 16 threads, each thread TM x 4 outputs (BM = 16 * TM).
 template <typename TA, typename TW, typename TC, int TM>
 __global__ void __launch_bounds__(THREADS)
-gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restrict__ W, int M, int N, int K,
+gemm_simt_kernel(TC* C, const TA* A, const TW* W, int M, int N, int K,
                  long long lda, long long ldw, long long ldc, int accumulate) {
     constexpr int BM = 16 * TM;
     __shared__ float As[BK][BM + 4];

@@ -62,7 +62,7 @@ __device__ __forceinline__ float silu(float g) { return __fdividef(g, 1.0f + __e
 template <typename TC, int MPAD, int STAGES, int MODE>
 __global__ void __launch_bounds__(THREADS)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                   TC* __restrict__ C, int M, int N, int K, long long ldc, int kb_per_split, int* error_flag) {
+                   TC* C, int M, int N, int K, long long ldc, int kb_per_split, int* error_flag) {
     using L = Smem<MPAD, STAGES>;
     constexpr int TMEM_COLS = MPAD < 32 ? 32 : MPAD;
     extern __shared__ uint8_t smem_raw[];

@@ -101,8 +101,8 @@ template <typename TC, int BN, int STAGES, int ACT, int MB, bool PAIR = false, i
 __global__ void __launch_bounds__(THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ CUtensorMap map_c, int store_by_tma, int splits,
-               TC* __restrict__ C, int M, int N, int K, long long ldc, int* error_flag,
-               const int* __restrict__ tile_group) {
+               TC* C, int M, int N, int K, long long ldc, int* error_flag,
+               const int* tile_group) {
     static_assert(!PAIR || MB == 1, "a pair of blocks takes one block of rows each");
     constexpr bool GATED = is_glu(ACT);
     using L = Smem<BN, STAGES, MB, PAIR, KS>;

@@ -14,7 +14,7 @@ constexpr int WARPS = 8;
 
 template <int M, typename TC>
 __global__ void __launch_bounds__(WARPS * 32)
-gemv_bf16_kernel(TC* __restrict__ C, const bf16* __restrict__ A, const bf16* __restrict__ W, int N, int K,
+gemv_bf16_kernel(TC* C, const bf16* A, const bf16* W, int N, int K,
                  long long lda, long long ldw, long long ldc, int accumulate) {
     const int lane = threadIdx.x & 31;
     const int n = blockIdx.x * WARPS + (threadIdx.x >> 5);
@@ -42,7 +42,7 @@ gemv_bf16_kernel(TC* __restrict__ C, const bf16* __restrict__ A, const bf16* __r
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 Vec16<bf16> a;
-                a.raw = __ldg(reinterpret_cast<const uint4*>(A + (size_t)m * lda) + v);
+                a.raw = reinterpret_cast<const uint4*>(A + (size_t)m * lda)[v];
                 float af[8];
                 a.unpack(af);
 #pragma unroll

@@ -25,7 +25,7 @@ LLMK_DEFINE_LAST_ERROR()
 
 constexpr int MAX_TAPS = 8;
 
-__device__ __forceinline__ int seq_of_row(const int* __restrict__ cu_q, int n_seqs, int t) {
+__device__ __forceinline__ int seq_of_row(const int* cu_q, int n_seqs, int t) {
     if (t >= cu_q[n_seqs]) return -1;
     int lo = 0, hi = n_seqs;
     while (hi - lo > 1) {

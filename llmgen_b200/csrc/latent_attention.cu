@@ -41,8 +41,8 @@ __device__ __forceinline__ void rotate_into(float* dst, const float* src, int ro
 // A token's cached vector z = [rmsnorm(c~) * gain | rotate(kr)] from its projected row [c~ | kr], by the whole block.
 // `sm`: 33 + 2 rot floats of shared memory.
 template <typename T>
-__device__ __forceinline__ void latent_entry(T* __restrict__ z, const T* __restrict__ src, int rank, int rot, const float* __restrict__ gain,
-                                             float eps, int pos, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+__device__ __forceinline__ void latent_entry(T* z, const T* src, int rank, int rot, const float* gain,
+                                             float eps, int pos, const float* cos_t, const float* sin_t,
                                              int pairing, float* sm) {
     float* scratch = sm;
     float* kr_in = sm + 33;
@@ -65,10 +65,10 @@ __device__ __forceinline__ void latent_entry(T* __restrict__ z, const T* __restr
 // ---------------------------------------------------------------------------------------------- prep
 // One block per token.  `dq` [q_rank] and `dkv` [rank + rot] are read from the packed projection row.
 template <typename T>
-__global__ void latent_prep_kernel(const T* __restrict__ packed, long long ld, int dq_off, int dkv_off, int q_rank, int rank, int rot,
-                                   const float* __restrict__ q_gain, const float* __restrict__ kv_gain, float eps,
-                                   T* __restrict__ cq_out, T* __restrict__ cache, const int* __restrict__ positions,
-                                   const int* __restrict__ slots, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+__global__ void latent_prep_kernel(const T* packed, long long ld, int dq_off, int dkv_off, int q_rank, int rank, int rot,
+                                   const float* q_gain, const float* kv_gain, float eps,
+                                   T* cq_out, T* cache, const int* positions,
+                                   const int* slots, const float* cos_t, const float* sin_t,
                                    int pairing) {
     extern __shared__ float sm[];   // 33 scratch, rot floats in, rot floats out
     float* scratch = sm;
@@ -132,9 +132,9 @@ struct LatentEntries {
 // QS: into how many shares of the key dimension a block's threads are cut (128 / QS latent columns a block); steps of a few tokens
 // take 4, so that there are blocks for the SMs, and add the shares up in their order.
 template <typename T, int QS>
-__global__ void __launch_bounds__(128) latent_absorb_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ wuk,
-                                                            float* __restrict__ qa, const int* __restrict__ positions,
-                                                            const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+__global__ void __launch_bounds__(128) latent_absorb_kernel(const T* q, long long ldq, const T* wuk,
+                                                            float* qa, const int* positions,
+                                                            const float* cos_t, const float* sin_t,
                                                             int n_tokens, int heads, int dim, int rot, int rank, int pairing,
                                                             LatentEntries en) {
     extern __shared__ float sm[];   // [TT][dim] unrotated parts, [TT][rot] rotated parts in, [TT][rot] out
@@ -262,9 +262,9 @@ LLMK_EXPORT int llmk_latent_absorb(float* qa, const void* q, long long ldq, cons
 // qn [heads, t_pad, dim] (the operand of the grouped product with Wuk, whose result is columns [0, rank) of qa_hm), their rotated
 // parts turned to columns [rank, rank + rot) of qa_hm [heads, t_pad, rank + rot], and, with `cache`, the token's cached vector to
 // its slot.  One block per token.
-__global__ void __launch_bounds__(256) latent_split_kernel(const bf16* __restrict__ packed, long long ld, bf16* __restrict__ qn,
-                                                           bf16* __restrict__ qa_hm, const int* __restrict__ positions,
-                                                           const float* __restrict__ cos_t, const float* __restrict__ sin_t, int heads,
+__global__ void __launch_bounds__(256) latent_split_kernel(const bf16* packed, long long ld, bf16* qn,
+                                                           bf16* qa_hm, const int* positions,
+                                                           const float* cos_t, const float* sin_t, int heads,
                                                            int dim, int rot, int rank, int t_pad, int pairing, int dkv_off, LatentEntries en) {
     extern __shared__ float sm[];
     const size_t t = blockIdx.x;
@@ -314,8 +314,8 @@ LLMK_EXPORT int llmk_latent_split(const void* packed, long long ld, void* qn, vo
 // -------------------------------------------------------------------------------------------- rotate
 // For queries that were projected straight into the latent space (Wuk folded into Wuq when the model was loaded):
 // the rotated part of every head of qa [tokens, heads, rank + rot] is turned in place.  One block per token.
-__global__ void latent_rotate_kernel(float* __restrict__ qa, const int* __restrict__ positions, const float* __restrict__ cos_t,
-                                     const float* __restrict__ sin_t, int heads, int rank, int rot, int pairing) {
+__global__ void latent_rotate_kernel(float* qa, const int* positions, const float* cos_t,
+                                     const float* sin_t, int heads, int rank, int rot, int pairing) {
     const size_t t = blockIdx.x;
     pdl_launch_dependents();
     pdl_wait();
@@ -919,9 +919,9 @@ __global__ void __launch_bounds__(128 * RG) latent_attention_mma_kernel(LatentAt
 
 // One block per (token, head): merge the key parts in part order.  The parts' weights e^(m_p - M) are computed once,
 // then every thread adds up its values of the latent over the parts.
-__global__ void __launch_bounds__(128) latent_reduce_kernel(float* __restrict__ out, const float* __restrict__ part_o,
-                                                            const float* __restrict__ part_ml, int rank, int num_parts,
-                                                            bf16* __restrict__ out_hm, int heads, int t_pad) {
+__global__ void __launch_bounds__(128) latent_reduce_kernel(float* out, const float* part_o,
+                                                            const float* part_ml, int rank, int num_parts,
+                                                            bf16* out_hm, int heads, int t_pad) {
     extern __shared__ float wgt[];     // [num_parts] weights, then 1 / denominator
     const size_t row = blockIdx.x;
     pdl_launch_dependents();
@@ -1084,7 +1084,7 @@ LLMK_EXPORT int llmk_latent_attention(float* out, const float* qa, const void* c
 // After the grouped product Wuv_h oa_h: out[t, h * vdim + j] = (T)(o[(h * t_pad + t) * vdim + j] * sigmoid(g[t, h * vdim + j])),
 // o float32 head-major.
 template <typename T>
-__global__ void latent_gate_kernel(T* __restrict__ out, const float* __restrict__ o, const T* __restrict__ g, long long ldg, int n_tokens,
+__global__ void latent_gate_kernel(T* out, const float* o, const T* g, long long ldg, int n_tokens,
                                    int heads, int vdim, int t_pad) {
     pdl_launch_dependents();
     pdl_wait();
@@ -1101,7 +1101,7 @@ __global__ void latent_gate_kernel(T* __restrict__ out, const float* __restrict_
 
 // The same for bfloat16 rows in whole vectors of eight (vdim and the gate's row stride multiples of eight, 16-byte boundaries), a token's heads side by
 // side over the threads.  Bound by its traffic, 4 + 2 + 2 bytes a value: 2,048 tokens of 16 heads of 128 22.1 us value by value.
-__global__ void __launch_bounds__(256) latent_gate_vec_kernel(bf16* __restrict__ out, const float* __restrict__ o, const bf16* __restrict__ g, long long ldg,
+__global__ void __launch_bounds__(256) latent_gate_vec_kernel(bf16* out, const float* o, const bf16* g, long long ldg,
                                                               int n_tokens, int heads, int vdim, int t_pad) {
     pdl_launch_dependents();
     pdl_wait();
@@ -1157,8 +1157,8 @@ LLMK_EXPORT int llmk_latent_gate(void* out, const float* o, const void* g, long 
 // outputs are cut into slices of 32 so that there are blocks for the SMs; with many, one block takes the whole head and
 // reads its rows of oa once.
 template <typename T>
-__global__ void __launch_bounds__(256) latent_expand_kernel(T* __restrict__ out, const float* __restrict__ oa, const T* __restrict__ wuv,
-                                                            const T* __restrict__ g, long long ldg, int n_tokens, int heads, int rank,
+__global__ void __launch_bounds__(256) latent_expand_kernel(T* out, const float* oa, const T* wuv,
+                                                            const T* g, long long ldg, int n_tokens, int heads, int rank,
                                                             int vdim, int cols) {
     extern __shared__ float os[];   // [TT][rank]
     const int t0 = blockIdx.x * LT_TT, h = blockIdx.y;

@@ -40,9 +40,9 @@ __device__ __forceinline__ float logsigmoidf_(float x) { return x < -20.f ? x : 
 // ------------------------------------------------------------------------------------------------------- min_gru
 // A thread per (sequence, channel) walks the sequence's tokens.  zxg [n, 3C] float32: z, u and g side by side.
 template <typename T>
-__global__ void min_gru_kernel(T* __restrict__ out, const float* __restrict__ zxg, long long ld, const float* __restrict__ bz,
-                               const float* __restrict__ bx, float* __restrict__ state, long long state_ld,
-                               const int* __restrict__ cu_q, const int* __restrict__ state_slots, int C) {
+__global__ void min_gru_kernel(T* out, const float* zxg, long long ld, const float* bz,
+                               const float* bx, float* state, long long state_ld,
+                               const int* cu_q, const int* state_slots, int C) {
     const int s = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_launch_dependents();
@@ -72,10 +72,10 @@ __global__ void min_gru_kernel(T* __restrict__ out, const float* __restrict__ zx
 // lanes; then token w's row goes out.  The sums of a token are regrouped, not changed, against the walk above.
 constexpr int GT = 32;
 template <typename T>
-__global__ void __launch_bounds__(GT* GT) min_gru_tile_kernel(T* __restrict__ out, const float* __restrict__ zxg, long long ld,
-                                                              const float* __restrict__ bz, const float* __restrict__ bx,
-                                                              float* __restrict__ state, long long state_ld,
-                                                              const int* __restrict__ cu_q, const int* __restrict__ state_slots, int C) {
+__global__ void __launch_bounds__(GT* GT) min_gru_tile_kernel(T* out, const float* zxg, long long ld,
+                                                              const float* bz, const float* bx,
+                                                              float* state, long long state_ld,
+                                                              const int* cu_q, const int* state_slots, int C) {
     __shared__ float sa[GT][GT + 1], sb[GT][GT + 1];
     const int s = blockIdx.y, cb = blockIdx.x * GT;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -126,9 +126,9 @@ __global__ void __launch_bounds__(GT* GT) min_gru_tile_kernel(T* __restrict__ ou
 // ------------------------------------------------------------------------------------------------------- mlstm gates
 // A warp per (token, head): gates[t, h] = (i, f, (q . k) q_scale, -).
 template <typename T>
-__global__ void mlstm_gates_kernel(float* __restrict__ gates, const T* __restrict__ q, long long ldq, const T* __restrict__ k,
-                                   long long ldk, const T* __restrict__ gi, long long ldi, const T* __restrict__ gf, long long ldf,
-                                   const float* __restrict__ bi, const float* __restrict__ bf, const int* __restrict__ cu_q,
+__global__ void mlstm_gates_kernel(float* gates, const T* q, long long ldq, const T* k,
+                                   long long ldk, const T* gi, long long ldi, const T* gf, long long ldf,
+                                   const float* bi, const float* bf, const int* cu_q,
                                    int n_seqs, int n_rows, int H, int D, float cap, float q_scale) {
     const int lane = threadIdx.x & 31;
     const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -158,7 +158,7 @@ __global__ void mlstm_gates_kernel(float* __restrict__ gates, const T* __restric
 // step m -> max(f + m, i) composes with the next, (f1, i1) then (f2, i2) = (f1 + f2, max(i1 + f2, i2)), so five rounds over the
 // lanes give every token's maximum.  What the memory's step needs follows from (i, f, m_(t-1)) alone, m_t = max(f + m_(t-1), i),
 // keep = exp(f + m_(t-1) - m_t), take = exp(i - m_t), exp(-m_t), and is made where it is used.
-__device__ __forceinline__ void maxima_by_warp(float* __restrict__ gates, float* __restrict__ m_state, long long state_ld, int q_beg, int n, int slot,
+__device__ __forceinline__ void maxima_by_warp(float* gates, float* m_state, long long state_ld, int q_beg, int n, int slot,
                                                int h, int H) {
     const int lane = threadIdx.x & 31;
     float m = slot >= 0 ? m_state[(size_t)slot * state_ld + h] : 0.f;
@@ -188,8 +188,8 @@ __device__ __forceinline__ void maxima_by_warp(float* __restrict__ gates, float*
     }
     if (slot >= 0 && lane == 0) m_state[(size_t)slot * state_ld + h] = m;
 }
-__global__ void mlstm_maxima_kernel(float* __restrict__ gates, float* __restrict__ m_state, long long state_ld,
-                                    const int* __restrict__ cu_q, const int* __restrict__ state_slots, int n_seqs, int H) {
+__global__ void mlstm_maxima_kernel(float* gates, float* m_state, long long state_ld,
+                                    const int* cu_q, const int* state_slots, int n_seqs, int H) {
     const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     pdl_launch_dependents();
     pdl_wait();
@@ -203,8 +203,8 @@ __global__ void mlstm_maxima_kernel(float* __restrict__ gates, float* __restrict
 // Sequences of up to MAXIMA_FEW_TOKENS are a warp's here too: how a token's sums are grouped follows from its own sequence.
 constexpr int MAXIMA_FEW_TOKENS = 64;
 constexpr int MX_THREADS = 256, MX_EACH = 8;
-__global__ void __launch_bounds__(MX_THREADS) mlstm_maxima_block_kernel(float* __restrict__ gates, float* __restrict__ m_state, long long state_ld,
-                                                                        const int* __restrict__ cu_q, const int* __restrict__ state_slots, int H) {
+__global__ void __launch_bounds__(MX_THREADS) mlstm_maxima_block_kernel(float* gates, float* m_state, long long state_ld,
+                                                                        const int* cu_q, const int* state_slots, int H) {
     __shared__ float2 warps[MX_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int s = blockIdx.y, h = blockIdx.x;
@@ -261,10 +261,10 @@ __global__ void __launch_bounds__(MX_THREADS) mlstm_maxima_block_kernel(float* _
 // ------------------------------------------------------------------------------------------------------- delta rule prep
 // A block per token, a warp per head in turn.  aux[t] = [w | b | u] (H D each), dots[t, h] = (b . r, k . r).
 template <typename T>
-__global__ void delta_rule_prep_kernel(float* __restrict__ aux, float* __restrict__ dots, const T* __restrict__ r, long long ldr,
-                                       const T* __restrict__ k, long long ldk, const T* __restrict__ a, long long lda,
-                                       const float* __restrict__ decay, long long ldd, const float* __restrict__ a_bias,
-                                       const float* __restrict__ w_bias, const int* __restrict__ cu_q, int n_seqs, int H, int D,
+__global__ void delta_rule_prep_kernel(float* aux, float* dots, const T* r, long long ldr,
+                                       const T* k, long long ldk, const T* a, long long lda,
+                                       const float* decay, long long ldd, const float* a_bias,
+                                       const float* w_bias, const int* cu_q, int n_seqs, int H, int D,
                                        float decay_scale, float unit_eps) {
     const int t = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -332,12 +332,12 @@ struct ScanParams {
 // The loads are volatile asm so that they are issued where they stand, a chunk ahead of their use, and not moved down to it.
 __device__ __forceinline__ uint32_t load_bits(const float* p) {
     uint32_t v;
-    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ uint32_t load_bits(const bf16* p) {
     unsigned short v;
-    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
     return v;
 }
 template <typename T> __device__ __forceinline__ float bits_value(uint32_t b);
@@ -346,7 +346,7 @@ template <> __device__ __forceinline__ float bits_value<bf16>(uint32_t b) { retu
 
 // A lane's DPL rows of one of a token's vectors (rows l DPL ..), zeros beyond D; sixteen bytes at a time where the sizes allow.
 template <int DPL>
-__device__ __forceinline__ void lane_rows(float (&dst)[DPL], const float* __restrict__ src, int l, int D, bool vec4) {
+__device__ __forceinline__ void lane_rows(float (&dst)[DPL], const float* src, int l, int D, bool vec4) {
     if (DPL % 4 == 0 && vec4) {
 #pragma unroll
         for (int i4 = 0; i4 < DPL / 4; ++i4) {

@@ -32,10 +32,10 @@ constexpr int MOE_KC = 256;     // input values per pass through shared memory
 // ---------------------------------------------------------------------------------------------- route
 // A warp scores token t's products s [E] (with `gate_out` one more) and picks its experts; `by` [E]: what chooses (s itself where that is the
 // same), gm [groups]: room for the groups' largest.
-__device__ __forceinline__ void score_and_pick(size_t t, float* s, float* by, float* gm, bool apart, int lane, int* __restrict__ slot_expert,
-                                               float* __restrict__ slot_weight, int E, int top, int scoring, int renorm,
-                                               const float* __restrict__ choice_bias, float weight_scale, float sum_eps, int groups, int keep,
-                                               float* __restrict__ gate_out) {
+__device__ __forceinline__ void score_and_pick(size_t t, float* s, float* by, float* gm, bool apart, int lane, int* slot_expert,
+                                               float* slot_weight, int E, int top, int scoring, int renorm,
+                                               const float* choice_bias, float weight_scale, float sum_eps, int groups, int keep,
+                                               float* gate_out) {
     if (gate_out && lane == 0) gate_out[t] = 1.0f / (1.0f + expf(-s[E]));
     if (scoring == 2) {
         // the logits choose
@@ -116,11 +116,11 @@ __device__ __forceinline__ void score_and_pick(size_t t, float* s, float* by, fl
 // TOK tokens per block: a prompt's rows share what a block reads of the router; steps of a few tokens take a token a block
 // with a warp per expert.
 template <typename T, int TOK>
-__global__ void __launch_bounds__(TOK > 1 ? 256 : 1024) moe_route_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ wr,
-                                                        const float* __restrict__ bias, int* __restrict__ slot_expert,
-                                                        float* __restrict__ slot_weight, int n_tokens, int K, int E, int top, int scoring,
-                                                        int renorm, const float* __restrict__ choice_bias, float weight_scale,
-                                                        float sum_eps, int groups, int keep, float* __restrict__ gate_out) {
+__global__ void __launch_bounds__(TOK > 1 ? 256 : 1024) moe_route_kernel(const T* h, long long ldh, const float* wr,
+                                                        const float* bias, int* slot_expert,
+                                                        float* slot_weight, int n_tokens, int K, int E, int top, int scoring,
+                                                        int renorm, const float* choice_bias, float weight_scale,
+                                                        float sum_eps, int groups, int keep, float* gate_out) {
     // [TOK][K] the rows in float32, [TOK][NE] scores (the gate's row last), [TOK][NE] what chooses (with `choice_bias` or
     // groups), [TOK][groups] the groups' largest
     extern __shared__ float sm[];
@@ -201,11 +201,11 @@ __device__ __forceinline__ float4 four_values(const bf16* p) {
     return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
 }
 template <typename T>
-__global__ void __launch_bounds__(RT_WARPS * 32) moe_route_rows_kernel(const T* __restrict__ h, long long ldh, const float* __restrict__ wr,
-                                                                       const float* __restrict__ bias, int* __restrict__ slot_expert,
-                                                                       float* __restrict__ slot_weight, int n_tokens, int K, int E, int top, int scoring,
-                                                                       int renorm, const float* __restrict__ choice_bias, float weight_scale,
-                                                                       float sum_eps, int groups, int keep, float* __restrict__ gate_out) {
+__global__ void __launch_bounds__(RT_WARPS * 32) moe_route_rows_kernel(const T* h, long long ldh, const float* wr,
+                                                                       const float* bias, int* slot_expert,
+                                                                       float* slot_weight, int n_tokens, int K, int E, int top, int scoring,
+                                                                       int renorm, const float* choice_bias, float weight_scale,
+                                                                       float sum_eps, int groups, int keep, float* gate_out) {
     // [RT_STAGES] of router [RT_EXP][RT_KC] and rows [RT_TOK][RT_KC], [RT_TOK][NE] scores, [RT_TOK][NE] what chooses, [RT_TOK][groups]
     extern __shared__ __align__(16) float sm[];
     constexpr int STAGE = (int)(rt_stage_bytes(sizeof(T)) / sizeof(float)), VN = Vec16<T>::N;
@@ -358,9 +358,9 @@ LLMK_EXPORT int llmk_moe_route(const void* h, long long ldh, const float* wr, co
 // is computed by itself).  tile_expert[i], tile_start[i], tile_rows[i] for i < max_tiles; expert -1 pads.
 // `padded`: every expert's rows begin on a multiple of `tt` (whole tiles per expert, for the grouped tensor-core product);
 // order[pos] is then -1 where a tile has no row.
-__global__ void moe_plan_kernel(const int* __restrict__ slot_expert, int n_slots, int E, int max_tiles, int tt, int padded,
-                                int* __restrict__ order, int* __restrict__ pos_of_slot, int* __restrict__ tile_expert,
-                                int* __restrict__ tile_start, int* __restrict__ tile_rows, int4* __restrict__ spans) {
+__global__ void moe_plan_kernel(const int* slot_expert, int n_slots, int E, int max_tiles, int tt, int padded,
+                                int* order, int* pos_of_slot, int* tile_expert,
+                                int* tile_start, int* tile_rows, int4* spans) {
     extern __shared__ int sh[];     // counts [E], first tiles [E], cursors [E]
     int* count = sh;
     int* first = sh + E;
@@ -485,8 +485,8 @@ LLMK_EXPORT int llmk_moe_plan(const int* slot_expert, int n_slots, int E, int ti
 // xs[pos, :] = (T)(weight * h[token of order[pos], :]) for the rows a padded plan filled; rows of padding stay as they are: the
 // products that follow compute them like any other and nobody reads the result.
 template <typename T>
-__global__ void moe_gather_kernel(T* __restrict__ xs, const T* __restrict__ h, long long ldh, const int* __restrict__ order,
-                                  const float* __restrict__ slot_weight, int top, int K, int scale_rows) {
+__global__ void moe_gather_kernel(T* xs, const T* h, long long ldh, const int* order,
+                                  const float* slot_weight, int top, int K, int scale_rows) {
     const size_t pos = blockIdx.x;
     pdl_launch_dependents();
     pdl_wait();
@@ -500,8 +500,8 @@ __global__ void moe_gather_kernel(T* __restrict__ xs, const T* __restrict__ h, l
 
 // The same with a warp a row and whole 16-byte vectors (12,288 rows of 2,048 bfloat16, 8,192 of them filled: 26.9 -> 9.8 us).
 template <typename T>
-__global__ void __launch_bounds__(256) moe_gather_vec_kernel(T* __restrict__ xs, const T* __restrict__ h, long long ldh, const int* __restrict__ order,
-                                                             const float* __restrict__ slot_weight, int n_rows, int top, int K, int scale_rows) {
+__global__ void __launch_bounds__(256) moe_gather_vec_kernel(T* xs, const T* h, long long ldh, const int* order,
+                                                             const float* slot_weight, int n_rows, int top, int K, int scale_rows) {
     constexpr int N = Vec16<T>::N;
     const size_t pos = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -557,11 +557,11 @@ LLMK_EXPORT int llmk_moe_gather(void* xs, const void* h, long long ldh, const in
 // FIRST: x = weight * h[token] (or h[token]), K = width, N = ff; y[pos, f] = act(x . Wgate[e, f], x . Wup[e, f])   float32
 // else:  x = y[pos], K = ff, N = width; out[pos, c] = (x . Wdown[e, c]) (* weight)                                  float32
 template <typename T, bool FIRST>
-__global__ void __launch_bounds__(128) moe_experts_kernel(float* __restrict__ out, const void* __restrict__ in, long long ld_in,
-                                                          const T* __restrict__ w0, const T* __restrict__ w1,
-                                                          const int* __restrict__ order, const float* __restrict__ slot_weight,
-                                                          const int* __restrict__ tile_expert, const int* __restrict__ tile_start,
-                                                          const int* __restrict__ tile_rows, int top, int K, int N, int scale_rows,
+__global__ void __launch_bounds__(128) moe_experts_kernel(float* out, const void* in, long long ld_in,
+                                                          const T* w0, const T* w1,
+                                                          const int* order, const float* slot_weight,
+                                                          const int* tile_expert, const int* tile_start,
+                                                          const int* tile_rows, int top, int K, int N, int scale_rows,
                                                           float alpha, float limit, int plain) {
     __shared__ float xs[MOE_TT][MOE_KC];
     __shared__ int src_row[MOE_TT];

@@ -28,7 +28,7 @@ LLMK_DEFINE_LAST_ERROR()
 
 constexpr int MAX_TAPS = 8;
 
-__device__ __forceinline__ int seq_of_row(const int* __restrict__ cu_q, int n_seqs, int t) {
+__device__ __forceinline__ int seq_of_row(const int* cu_q, int n_seqs, int t) {
     if (t >= cu_q[n_seqs]) return -1;
     int lo = 0, hi = n_seqs;
     while (hi - lo > 1) {
@@ -48,10 +48,10 @@ __device__ __forceinline__ float gelu_tanhf_(float z) {
 // out[t, c] = act( sum_i taps[c, i] in(j - (K-1) + i, c) + conv_bias[c] ), j the token's index in its portion;
 // in(r, c) = x[row of r, c] + in_bias[c] for r >= 0, else the state's row K - 1 + r (zeros for a fresh request).
 template <typename T>
-__global__ void short_conv_kernel(float* __restrict__ out, long long out_ld, const T* __restrict__ x, long long x_ld,
-                                  const float* __restrict__ in_bias, const float* __restrict__ taps,
-                                  const float* __restrict__ conv_bias, const float* __restrict__ state, long long state_ld,
-                                  const int* __restrict__ cu_q, const int* __restrict__ state_slots, int n_seqs, int C, int K,
+__global__ void short_conv_kernel(float* out, long long out_ld, const T* x, long long x_ld,
+                                  const float* in_bias, const float* taps,
+                                  const float* conv_bias, const float* state, long long state_ld,
+                                  const int* cu_q, const int* state_slots, int n_seqs, int C, int K,
                                   int act) {
     const int t = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -76,9 +76,9 @@ __global__ void short_conv_kernel(float* __restrict__ out, long long out_ld, con
 }
 
 template <typename T>
-__global__ void conv_state_update_kernel(float* __restrict__ state, long long state_ld, const T* __restrict__ x, long long x_ld,
-                                         const float* __restrict__ in_bias, const int* __restrict__ cu_q,
-                                         const int* __restrict__ state_slots, int C, int K) {
+__global__ void conv_state_update_kernel(float* state, long long state_ld, const T* x, long long x_ld,
+                                         const float* in_bias, const int* cu_q,
+                                         const int* state_slots, int C, int K) {
     const int s = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_launch_dependents();
@@ -109,10 +109,10 @@ __global__ void conv_state_update_kernel(float* __restrict__ state, long long st
 constexpr int SHORT_CONV_FEW_TOKENS = 64;
 
 template <typename T>
-__global__ void short_conv_few_kernel(float* __restrict__ out, long long out_ld, const T* __restrict__ x, long long x_ld,
-                                      const float* __restrict__ in_bias, const float* __restrict__ taps,
-                                      const float* __restrict__ conv_bias, float* __restrict__ state, long long state_ld,
-                                      const int* __restrict__ cu_q, const int* __restrict__ state_slots, int C, int K, int act,
+__global__ void short_conv_few_kernel(float* out, long long out_ld, const T* x, long long x_ld,
+                                      const float* in_bias, const float* taps,
+                                      const float* conv_bias, float* state, long long state_ld,
+                                      const int* cu_q, const int* state_slots, int C, int K, int act,
                                       int update_state) {
     const int s = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -201,10 +201,10 @@ LLMK_EXPORT int llmk_short_conv(float* out, long long out_ld, const void* x, lon
 constexpr int GATE_OUT = 128;
 
 template <typename T, int TT>
-__global__ void __launch_bounds__(GATE_OUT) rglru_gates_kernel(float* __restrict__ a_out, float* __restrict__ b_out,
-                                                               const float* __restrict__ u, const T* __restrict__ Wa,
-                                                               const T* __restrict__ Wi, const float* __restrict__ ba,
-                                                               const float* __restrict__ bi, const float* __restrict__ lam,
+__global__ void __launch_bounds__(GATE_OUT) rglru_gates_kernel(float* a_out, float* b_out,
+                                                               const float* u, const T* Wa,
+                                                               const T* Wi, const float* ba,
+                                                               const float* bi, const float* lam,
                                                                int n_tokens, int C, int n, float decay_scale, int vec_ok) {
     extern __shared__ __align__(16) float Us[];   // [TT][n]
     const int b = blockIdx.y, t0 = blockIdx.z * TT;
@@ -278,10 +278,10 @@ __global__ void __launch_bounds__(GATE_OUT) rglru_gates_kernel(float* __restrict
 // Thread (sequence, channel): S = a S + b = (S - c S) + b over the sequence's new tokens (c = 1 - a, see above),
 // out = S * gelu_tanh(y + y_bias).
 template <typename T>
-__global__ void rglru_scan_kernel(T* __restrict__ out, long long out_ld, const float* __restrict__ a, const float* __restrict__ bx,
-                                  const T* __restrict__ y, long long y_ld, const float* __restrict__ y_bias,
-                                  float* __restrict__ state, long long state_ld, const int* __restrict__ cu_q,
-                                  const int* __restrict__ state_slots, int C) {
+__global__ void rglru_scan_kernel(T* out, long long out_ld, const float* a, const float* bx,
+                                  const T* y, long long y_ld, const float* y_bias,
+                                  float* state, long long state_ld, const int* cu_q,
+                                  const int* state_slots, int C) {
     const int s = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_launch_dependents();
@@ -321,7 +321,7 @@ __global__ void rglru_scan_kernel(T* __restrict__ out, long long out_ld, const f
 // is the k-th of the first sequence s with j < sum of ceil(n_s' / SCAN_SEG) over s' <= s.
 constexpr int SCAN_SEG = 64;
 
-__device__ __forceinline__ bool find_segment(const int* __restrict__ cu_q, int n_seqs, int j, int* t0, int* t1) {
+__device__ __forceinline__ bool find_segment(const int* cu_q, int n_seqs, int j, int* t0, int* t1) {
     for (int s = 0; s < n_seqs; ++s) {
         const int beg = cu_q[s], n = cu_q[s + 1] - beg;
         const int segs = (n + SCAN_SEG - 1) / SCAN_SEG;
@@ -335,8 +335,8 @@ __device__ __forceinline__ bool find_segment(const int* __restrict__ cu_q, int n
     return false;
 }
 
-__global__ void rglru_segment_local_kernel(const float* __restrict__ a, float* __restrict__ bx, float* __restrict__ seg_p,
-                                           float* __restrict__ seg_f, const int* __restrict__ cu_q, int n_seqs, int C) {
+__global__ void rglru_segment_local_kernel(const float* a, float* bx, float* seg_p,
+                                           float* seg_f, const int* cu_q, int n_seqs, int C) {
     const int j = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_launch_dependents();
@@ -373,8 +373,8 @@ __global__ void rglru_segment_local_kernel(const float* __restrict__ a, float* _
 }
 
 // seg_f[j] becomes the state segment j is entered with
-__global__ void rglru_segment_carry_kernel(const float* __restrict__ seg_p, float* __restrict__ seg_f, float* __restrict__ state,
-                                           long long state_ld, const int* __restrict__ cu_q, const int* __restrict__ state_slots,
+__global__ void rglru_segment_carry_kernel(const float* seg_p, float* seg_f, float* state,
+                                           long long state_ld, const int* cu_q, const int* state_slots,
                                            int C) {
     const int s = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -397,10 +397,10 @@ __global__ void rglru_segment_carry_kernel(const float* __restrict__ seg_p, floa
 }
 
 template <typename T>
-__global__ void rglru_segment_finish_kernel(T* __restrict__ out, long long out_ld, const float* __restrict__ a,
-                                            const float* __restrict__ local, const float* __restrict__ seg_in,
-                                            const T* __restrict__ y, long long y_ld, const float* __restrict__ y_bias,
-                                            const int* __restrict__ cu_q, int n_seqs, int C) {
+__global__ void rglru_segment_finish_kernel(T* out, long long out_ld, const float* a,
+                                            const float* local, const float* seg_in,
+                                            const T* y, long long y_ld, const float* y_bias,
+                                            const int* cu_q, int n_seqs, int C) {
     const int j = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_launch_dependents();
@@ -534,9 +534,9 @@ constexpr int DELTA_CHUNK = 16;
 constexpr int DELTA_THREADS = 128;
 
 template <typename T>
-__global__ void __launch_bounds__(256) delta_prep_kernel(float* __restrict__ qkv, long long qkv_ld, float* __restrict__ decay,
-                                                         float* __restrict__ beta_out, const T* __restrict__ beta, long long beta_ld,
-                                                         const float* __restrict__ dt_bias, const float* __restrict__ a_log,
+__global__ void __launch_bounds__(256) delta_prep_kernel(float* qkv, long long qkv_ld, float* decay,
+                                                         float* beta_out, const T* beta, long long beta_ld,
+                                                         const float* dt_bias, const float* a_log,
                                                          int H, int G, int D, float unit_eps, float q_scale) {
     const size_t t = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -825,9 +825,9 @@ LLMK_EXPORT int llmk_delta_scan_heads(float* out, const float* qkv, long long qk
 // that reads a sequence's state row also leaves the sequence's last row there, after reading, so that no other thread's
 // read meets the write.
 template <typename T>
-__global__ void token_shift_mix_kernel(T* __restrict__ out, long long out_plane, const T* __restrict__ x, long long x_ld,
-                                       const float* __restrict__ mu, float* __restrict__ state, long long state_ld,
-                                       const int* __restrict__ cu_q, const int* __restrict__ state_slots, int n_seqs, int W,
+__global__ void token_shift_mix_kernel(T* out, long long out_plane, const T* x, long long x_ld,
+                                       const float* mu, float* state, long long state_ld,
+                                       const int* cu_q, const int* state_slots, int n_seqs, int W,
                                        int n_mix) {
     const int t = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -891,10 +891,10 @@ LLMK_EXPORT int llmk_token_shift_mix(void* out, long long out_plane, const void*
 enum { DECAY_SIGMOID_POW = 0, DECAY_EXP_EXP = 1 };
 
 template <typename T>
-__global__ void __launch_bounds__(256) decay_prep_kernel(float* __restrict__ qkv, long long qkv_ld, float* __restrict__ decay,
-                                                         float* __restrict__ dots, const T* __restrict__ q, long long q_ld,
-                                                         const T* __restrict__ k, long long k_ld, const T* __restrict__ v,
-                                                         long long v_ld, const float* __restrict__ bias, const float* __restrict__ bonus,
+__global__ void __launch_bounds__(256) decay_prep_kernel(float* qkv, long long qkv_ld, float* decay,
+                                                         float* dots, const T* q, long long q_ld,
+                                                         const T* k, long long k_ld, const T* v,
+                                                         long long v_ld, const float* bias, const float* bonus,
                                                          int H, int D, int E, int mode, float inv_tau, float q_scale) {
     const size_t t = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -1107,11 +1107,11 @@ static cudaError_t launch_decay(const DeltaParams& p, const DecaySegments& g, in
 constexpr int DECAY_STEP_MAX_TOKENS = 32;
 
 template <typename T, bool READ_FIRST, int NR>
-__global__ void __launch_bounds__(256) decay_step_kernel(float* __restrict__ out, const T* __restrict__ q, long long q_ld,
-                                                         const T* __restrict__ k, long long k_ld, const T* __restrict__ v, long long v_ld,
-                                                         const float* __restrict__ z, const float* __restrict__ bias,
-                                                         const float* __restrict__ bonus, float* __restrict__ state, long long state_ld,
-                                                         const int* __restrict__ cu_q, const int* __restrict__ state_slots, int H, int D,
+__global__ void __launch_bounds__(256) decay_step_kernel(float* out, const T* q, long long q_ld,
+                                                         const T* k, long long k_ld, const T* v, long long v_ld,
+                                                         const float* z, const float* bias,
+                                                         const float* bonus, float* state, long long state_ld,
+                                                         const int* cu_q, const int* state_slots, int H, int D,
                                                          int E, int mode, float inv_tau, float q_scale) {
     __shared__ float sq[4 * NR], sk[4 * NR], sc[4 * NR];
     __shared__ float partial[4][64];

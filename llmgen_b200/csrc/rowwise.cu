@@ -88,10 +88,10 @@ __device__ __forceinline__ void store_four(T* p, float a, float b, float c, floa
 static bool four_ok(const void* p, int elem) { return (reinterpret_cast<uintptr_t>(p) & (size_t)(4 * elem - 1)) == 0; }
 
 template <typename T>
-__global__ void norm_add_kernel(float* __restrict__ resid, const void* __restrict__ y, const float* __restrict__ w,
-                                T* __restrict__ copy, int H, float eps, int splits, long long split_stride,
-                                const void* __restrict__ y2, int splits2, long long split_stride2, float a, float b,
-                                const float* __restrict__ w_next, float eps_next) {
+__global__ void norm_add_kernel(float* resid, const void* y, const float* w,
+                                T* copy, int H, float eps, int splits, long long split_stride,
+                                const void* y2, int splits2, long long split_stride2, float a, float b,
+                                const float* w_next, float eps_next) {
     extern __shared__ float srow[];  // H floats + 33 scratch
     float* scratch = srow + H;
     const size_t r = blockIdx.x;
@@ -130,10 +130,10 @@ __global__ void norm_add_kernel(float* __restrict__ resid, const void* __restric
 // The same with four neighbouring values a thread, which holds them from the products' rows to the new row: rows of up to 4,096 values, a
 // multiple of four, on 16-byte boundaries (8 for bfloat16).  2,048 rows of 2,048: 21.9 -> 14.3 us, 50 MB.
 template <typename T>
-__global__ void __launch_bounds__(1024) norm_add_vec_kernel(float* __restrict__ resid, const void* __restrict__ y, const float* __restrict__ w,
-                                                            T* __restrict__ copy, int H, float eps, int splits, long long split_stride,
-                                                            const void* __restrict__ y2, int splits2, long long split_stride2, float a, float b,
-                                                            const float* __restrict__ w_next, float eps_next) {
+__global__ void __launch_bounds__(1024) norm_add_vec_kernel(float* resid, const void* y, const float* w,
+                                                            T* copy, int H, float eps, int splits, long long split_stride,
+                                                            const void* y2, int splits2, long long split_stride2, float a, float b,
+                                                            const float* w_next, float eps_next) {
     __shared__ float scratch[33];
     const size_t r = blockIdx.x, at = r * H + 4 * threadIdx.x;
     const int i = 4 * threadIdx.x;
@@ -369,8 +369,8 @@ LLMK_EXPORT int llmk_parallel_add(float* resid, const void* y1, int splits1, lon
 
 // out[i] (float32) = a * y[i] + b * y2[i]; y and y2 arrays of T or float32 slices.
 template <typename T>
-__global__ void scaled_sum_kernel(float* __restrict__ out, const void* __restrict__ y, int splits, long long split_stride,
-                                  const void* __restrict__ y2, int splits2, long long split_stride2, float a, float b, long long n) {
+__global__ void scaled_sum_kernel(float* out, const void* y, int splits, long long split_stride,
+                                  const void* y2, int splits2, long long split_stride2, float a, float b, long long n) {
     pdl_launch_dependents();
     pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -396,7 +396,7 @@ LLMK_EXPORT int llmk_scaled_sum(float* out, const void* y, int splits, long long
 }
 
 template <typename T>
-__global__ void cast_rows_kernel(T* __restrict__ out, const float* __restrict__ in, long long n) {
+__global__ void cast_rows_kernel(T* out, const float* in, long long n) {
     pdl_launch_dependents();
     pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -405,7 +405,7 @@ __global__ void cast_rows_kernel(T* __restrict__ out, const float* __restrict__ 
 
 // Eight values at a time.
 template <typename T>
-__global__ void __launch_bounds__(256) cast_rows_vec_kernel(T* __restrict__ out, const float* __restrict__ in, long long vecs) {
+__global__ void __launch_bounds__(256) cast_rows_vec_kernel(T* out, const float* in, long long vecs) {
     pdl_launch_dependents();
     pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += (long long)gridDim.x * blockDim.x) {
@@ -461,7 +461,7 @@ __device__ __forceinline__ float gelu_tanh(float z) {
 }
 
 template <typename T>
-__global__ void act_rows_kernel(T* __restrict__ out, const void* __restrict__ x, int n, int F, long long ld, int mode,
+__global__ void act_rows_kernel(T* out, const void* x, int n, int F, long long ld, int mode,
                                 float alpha, float limit, int splits, long long split_stride, int group) {
     pdl_launch_dependents();
     pdl_wait();
@@ -495,7 +495,7 @@ __global__ void act_rows_kernel(T* __restrict__ out, const void* __restrict__ x,
 // one vector (rows that are no partial sums, column counts and strides in whole vectors).  The arithmetic is the scalar
 // kernel's.  relu2 of 2,048 rows of 6,144: 40.1 -> 11.2 us, 50 MB.
 template <typename T>
-__global__ void __launch_bounds__(256) act_rows_vec_kernel(T* __restrict__ out, const T* __restrict__ x, int n, int F, long long ld,
+__global__ void __launch_bounds__(256) act_rows_vec_kernel(T* out, const T* x, int n, int F, long long ld,
                                                            int mode, float alpha, float limit, int group) {
     constexpr int N = Vec16<T>::N;
     pdl_launch_dependents();
@@ -591,8 +591,8 @@ LLMK_EXPORT int llmk_act_rows(void* out, const void* x, int n, int F, long long 
 // its own, w [heads, H] (w_rows = 1: one vector for all).
 enum { GATE_SIGMOID = 0, GATE_SILU = 1, GATE_PLAIN = 2 };
 template <typename T>
-__global__ void gated_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ o, const T* __restrict__ g,
-                                     const float* __restrict__ w, int H, long long ldg, float eps, int gate_act, int w_rows,
+__global__ void gated_rmsnorm_kernel(T* out, const float* o, const T* g,
+                                     const float* w, int H, long long ldg, float eps, int gate_act, int w_rows,
                                      int heads, long long ldo) {
     __shared__ float scratch[33];
     const size_t r = blockIdx.x;
@@ -622,8 +622,8 @@ __global__ void gated_rmsnorm_kernel(T* __restrict__ out, const float* __restric
 
 // The same for short rows (a head's values): a warp a row, eight rows a block, no block-wide sum.
 template <typename T>
-__global__ void __launch_bounds__(256) gated_rmsnorm_warp_kernel(T* __restrict__ out, const float* __restrict__ o, const T* __restrict__ g,
-                                                                 const float* __restrict__ w, int n_rows, int H, long long ldg, float eps,
+__global__ void __launch_bounds__(256) gated_rmsnorm_warp_kernel(T* out, const float* o, const T* g,
+                                                                 const float* w, int n_rows, int H, long long ldg, float eps,
                                                                  int gate_act, int w_rows, int heads, long long ldo) {
     const size_t r = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -656,8 +656,8 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_warp_kernel(T* __restrict__
 // holding its four from the sum of squares to the row that goes out.  Rows, gains, gates and outputs on boundaries of four values.
 // 2,048 rows of 2,048: 27.4 -> 14.0 us, 34 MB.
 template <typename T, bool WARP>
-__global__ void __launch_bounds__(WARP ? 256 : 1024) gated_rmsnorm_vec_kernel(T* __restrict__ out, const float* __restrict__ o, const T* __restrict__ g,
-                                                                              const float* __restrict__ w, int n_rows, int H, long long ldg, float eps,
+__global__ void __launch_bounds__(WARP ? 256 : 1024) gated_rmsnorm_vec_kernel(T* out, const float* o, const T* g,
+                                                                              const float* w, int n_rows, int H, long long ldg, float eps,
                                                                               int gate_act, int w_rows, int heads, long long ldo) {
     __shared__ float scratch[33];
     const size_t r = WARP ? (size_t)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;
@@ -736,7 +736,7 @@ LLMK_EXPORT int llmk_gated_rmsnorm(void* out, const float* o, const void* g, con
 
 // y[r, i] += b[i].  y is [n, H] of T (rows `ld` apart), or float32 (dtype of the ARRAY, which may differ from the engine's).
 template <typename T>
-__global__ void add_bias_kernel(T* __restrict__ y, const float* __restrict__ b, int n, int H, long long ld) {
+__global__ void add_bias_kernel(T* y, const float* b, int n, int H, long long ld) {
     pdl_launch_dependents();
     pdl_wait();
     const long long total = (long long)n * H;
@@ -764,8 +764,8 @@ LLMK_EXPORT int llmk_add_bias(void* y, const float* b, int n, int H, long long l
 }
 
 template <typename T>
-__global__ void concat_stream_kernel(T* __restrict__ out, const float* __restrict__ resid, const void* __restrict__ delta,
-                                     const float* __restrict__ x0, int n, int H, int splits, long long split_stride) {
+__global__ void concat_stream_kernel(T* out, const float* resid, const void* delta,
+                                     const float* x0, int n, int H, int splits, long long split_stride) {
     pdl_launch_dependents();
     pdl_wait();
     const long long total = (long long)n * H;
@@ -808,11 +808,11 @@ constexpr int MAX_STREAMS = 16;
 
 // MS: the most streams this instance takes (4, 8 or 16); the loops over streams are unrolled to it, except the outer one of 16.
 template <typename T, int MS>
-__global__ void __launch_bounds__(512) stream_step_kernel(float* __restrict__ streams, const void* __restrict__ y, int splits, long long split_stride,
-                                   const void* __restrict__ y2, int splits2, long long split_stride2, float a, float b,
-                                   const float* __restrict__ mix, const float* __restrict__ out_coef,
-                                   const float* __restrict__ next_in, const float* __restrict__ next_gain, float eps,
-                                   T* __restrict__ normed, int S, int H, const float* one, float* sum) {
+__global__ void __launch_bounds__(512) stream_step_kernel(float* streams, const void* y, int splits, long long split_stride,
+                                   const void* y2, int splits2, long long split_stride2, float a, float b,
+                                   const float* mix, const float* out_coef,
+                                   const float* next_in, const float* next_gain, float eps,
+                                   T* normed, int S, int H, const float* one, float* sum) {
     extern __shared__ float srow[];  // H floats + 33 scratch + S * S + 2 * S coefficients
     float* scratch = srow + H;
     float* coef = scratch + 33;      // mix [S, S], out [S], in [S]
@@ -891,11 +891,11 @@ __device__ __forceinline__ float4 load_sum4(const void* y, size_t at, int splits
 // The same with four neighbouring values a thread, which holds them from the streams to the normed row: rows of up to 4,096
 // values, a multiple of four, on 16-byte boundaries; up to 8 streams.
 template <typename T, int MS>
-__global__ void __launch_bounds__(1024) stream_step_vec_kernel(float* __restrict__ streams, const void* __restrict__ y, int splits, long long split_stride,
-                                   const void* __restrict__ y2, int splits2, long long split_stride2, float a, float b,
-                                   const float* __restrict__ mix, const float* __restrict__ out_coef,
-                                   const float* __restrict__ next_in, const float* __restrict__ next_gain, float eps,
-                                   T* __restrict__ normed, int S, int H, const float* one, float* sum) {
+__global__ void __launch_bounds__(1024) stream_step_vec_kernel(float* streams, const void* y, int splits, long long split_stride,
+                                   const void* y2, int splits2, long long split_stride2, float a, float b,
+                                   const float* mix, const float* out_coef,
+                                   const float* next_in, const float* next_gain, float eps,
+                                   T* normed, int S, int H, const float* one, float* sum) {
     __shared__ float scratch[33];
     __shared__ float coef[MS * MS + 2 * MS];      // mix [S, S], out [S], in [S]
     const size_t r = blockIdx.x;
@@ -1031,7 +1031,7 @@ LLMK_EXPORT int llmk_stream_step(float* streams, const void* y, int splits, long
 }
 
 // collapse == 0: streams[r, s, :] = row[r, :] for every s.  collapse != 0: row[r, :] = sum_s streams[r, s, :].
-__global__ void stream_spread_kernel(float* __restrict__ streams, float* __restrict__ row, long long n, int S, int H, int collapse) {
+__global__ void stream_spread_kernel(float* streams, float* row, long long n, int S, int H, int collapse) {
     pdl_launch_dependents();
     pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n * H; i += (long long)gridDim.x * blockDim.x) {
@@ -1050,7 +1050,7 @@ __global__ void stream_spread_kernel(float* __restrict__ streams, float* __restr
 }
 
 // The same four values at a time (2,048 rows of 2,048, four streams: 21.2 -> 12.4 us, 84 MB).
-__global__ void __launch_bounds__(256) stream_spread_vec_kernel(float4* __restrict__ streams, float4* __restrict__ row, long long n, int S, int H4, int collapse) {
+__global__ void __launch_bounds__(256) stream_spread_vec_kernel(float4* streams, float4* row, long long n, int S, int H4, int collapse) {
     pdl_launch_dependents();
     pdl_wait();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n * H4; i += (long long)gridDim.x * blockDim.x) {

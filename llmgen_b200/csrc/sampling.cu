@@ -59,9 +59,9 @@ __device__ __forceinline__ float gumbel_score(float logit, float temp, unsigned 
 }
 
 __global__ void __launch_bounds__(THREADS)
-sample_kernel(int* __restrict__ out, unsigned long long* __restrict__ cand, unsigned* __restrict__ tickets,
-              const float* __restrict__ logits, long long ld, const float* __restrict__ temps,
-              const unsigned long long* seed_ptr, const unsigned long long* __restrict__ row_keys, int V) {
+sample_kernel(int* out, unsigned long long* cand, unsigned* tickets,
+              const float* logits, long long ld, const float* temps,
+              const unsigned long long* seed_ptr, const unsigned long long* row_keys, int V) {
     const int share = blockIdx.x, row = blockIdx.y;
     const float* x = logits + (size_t)row * ld;
     const float temp = temps[row];
