@@ -191,7 +191,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tc::prefetch_tensormap(&map_q);
         tc::prefetch_tensormap(&map_k);
         tc::prefetch_tensormap(&map_v);
-        pdl_launch_dependents();
     }
     if (warp == 1) {
         tc::tmem_alloc(tc::smem_u32(tmem_slot), TMEM_COLS);
@@ -201,6 +200,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __syncthreads();
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    if (threadIdx.x == 0) pdl_launch_dependents();      // (behind the allocation: the next kernel's blocks must not get their tensor memory first)
     pdl_wait();   // q, the cache and the step's arrays come from earlier work of the stream
 
     const int s = p.tile_seq[blockIdx.y];
