@@ -10,7 +10,7 @@
 //                       e^(L_n) S + sum_j e^(L_n - L_j) k_j u_j^T.  What does not need the state (the two triangular systems' solutions
 //                       W = (I + M)^-1 diag(beta e^L) K and (I + M)^-1 diag(beta) V, the matrix of the read-out) is made for all chunks
 //                       side by side; the walk over the chunks then touches the state once a chunk instead of once a token, and leaves it for
-//                       the outputs, again of all chunks side by side
+//                       the outputs, again of all chunks side by side (in steps of few chunks the walk makes the outputs itself)
 //   head_delta_step     steps of a few tokens (single decoded tokens above all) in one launch: all of the preparation, the
 //                       recurrence, each head's RMSNorm and the gate silu(z)
 //
@@ -955,15 +955,215 @@ __global__ void __launch_bounds__(OTHREADS) chunk_out_kernel(ChunkParams p) {
     }
 }
 
+// The walk that makes the outputs too, for steps of few chunks (`few_chunks`): block (sequence, head, COLS value columns), the state's columns in
+// shared memory.  A chunk takes three steps:
+//   1  rows of W and of Q times S: a thread has 4 rows, all columns, and one of 8 slices of the key channels; warps 0 .. 3 hold W's rows
+//      and leave U, warps 4 .. 7 hold Q's
+//   2  S <- e^(L_n) S + K^T (U scaled): a thread has 4 key channels, all columns, and one slice of the chunk's tokens
+//   3  (warps 4 .. 7) the outputs: e^(L_i) times the rows of step 1 + P U
+// Operands of W, Q, K and P are used by one thread each and go from global memory straight into registers, asked for a step ahead.
+template <int DP, int COLS>
+__global__ void __launch_bounds__(CTHREADS) chunk_walk_kernel(ChunkParams p) {
+    constexpr int KR = DP / 32;                    // runs of four key channels a thread has in step 1
+    constexpr int TS = CTHREADS / (DP / 4);        // slices of tokens in step 2
+    constexpr int TR = CHUNK / TS;                 // tokens of one
+    constexpr int SQ = 4 * COLS + 4;               // four rows of S side by side, padded: slices read different banks
+    constexpr int UL = COLS + 4;                   // a row of U
+    constexpr int NV = 4 * COLS;                   // outputs of a thread before the slices are summed up
+    __shared__ __align__(16) float S[DP / 4 * SQ];
+    __shared__ __align__(16) float U[2][CHUNK / 4 * SQ];   // as the outputs read it (four rows side by side), two chunks in turn
+    __shared__ __align__(16) float Ud[CHUNK * UL];         // times e^(L_n - L_j)
+    const int s = blockIdx.x, h = blockIdx.y, e0 = blockIdx.z * COLS, tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    const int kvh = h / (p.H / p.G);
+    const int ks = lane & 7, rt = warp * 4 + (lane >> 3);  // slice of key channels, row tile (0 .. 15: W, 16 .. 31: Q)
+    const bool reads_out = rt >= 16;
+    const int row0 = (reads_out ? rt - 16 : rt) * 4;
+    const int ts = tid & (TS - 1), d0 = tid / TS * 4;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int q_beg = p.cu_q[s], n = p.cu_q[s + 1] - q_beg;
+    if (n <= 0) return;
+    const int slot = p.state_slots[s], D = p.D, E = p.E;
+    float* st = slot >= 0 ? p.state + (size_t)slot * p.state_ld + (size_t)h * D * E : nullptr;
+    for (int idx = tid; idx < DP * COLS; idx += CTHREADS) {
+        const int d = idx / COLS, c = idx % COLS;
+        S[(d >> 2) * SQ + (d & 3) * COLS + c] = (st && d < D && e0 + c < E) ? st[(size_t)d * E + e0 + c] : 0.f;
+    }
+    const int place0 = q_beg / CHUNK + s, chunks = ceil_div(n, CHUNK);
+    float4 a4[4][KR], k4[TR], p4[4][2];
+    auto load_rows = [&](int c) {
+        const size_t place = place0 + c;
+        const float* src = reads_out ? p.qs + ((place * p.G + kvh) * CHUNK + row0) * DP : p.w + ((place * p.H + h) * CHUNK + row0) * DP;
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int i = 0; i < KR; ++i) a4[r][i] = *reinterpret_cast<const float4*>(src + r * DP + i * 32 + ks * 4);
+    };
+    auto load_keys = [&](int c) {
+        const float* src = p.ks + ((size_t)(place0 + c) * p.G + kvh) * CHUNK * DP + tid * 4;
+#pragma unroll
+        for (int j = 0; j < TR; ++j) k4[j] = *reinterpret_cast<const float4*>(src + j * CTHREADS * 4);
+    };
+    load_rows(0);
+    load_keys(0);
+    __syncthreads();
+    for (int c = 0; c < chunks; ++c) {
+        const size_t ph = (size_t)(place0 + c) * p.H + h;
+        const float* dec = p.dec + ph * 2 * CHUNK;
+        float v[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = 0.f;
+#pragma unroll
+        for (int i = 0; i < KR; ++i) {
+            const float* sr = S + (i * 8 + ks) * SQ;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float4 sv[COLS / 4];
+#pragma unroll
+                for (int u = 0; u < COLS / 4; ++u) sv[u] = *reinterpret_cast<const float4*>(sr + q * COLS + 4 * u);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float w = q == 0 ? a4[r][i].x : q == 1 ? a4[r][i].y : q == 2 ? a4[r][i].z : a4[r][i].w;
+#pragma unroll
+                    for (int u = 0; u < COLS / 4; ++u) {
+                        v[r * COLS + 4 * u] = fmaf(w, sv[u].x, v[r * COLS + 4 * u]);
+                        v[r * COLS + 4 * u + 1] = fmaf(w, sv[u].y, v[r * COLS + 4 * u + 1]);
+                        v[r * COLS + 4 * u + 2] = fmaf(w, sv[u].z, v[r * COLS + 4 * u + 2]);
+                        v[r * COLS + 4 * u + 3] = fmaf(w, sv[u].w, v[r * COLS + 4 * u + 3]);
+                    }
+                }
+            }
+        }
+        // what the slices add up to: this lane keeps NV / 8 values of one row
+        constexpr int KEEP = NV / 8;
+        const int at = ks * KEEP, row = row0 + at / COLS, col = at % COLS;
+        float4 uv[KEEP / 4];
+        if (!reads_out) {
+#pragma unroll
+            for (int u = 0; u < KEEP / 4; ++u) uv[u] = *reinterpret_cast<const float4*>(p.uv + (ph * CHUNK + row) * p.EP + e0 + col + 4 * u);
+        }
+        const float scale = reads_out ? dec[row] : dec[CHUNK + row], keep = dec[CHUNK - 1];
+        reduce_scatter<NV, 8>(v, ks);
+        float* ur = U[c & 1];
+        if (!reads_out) {
+#pragma unroll
+            for (int u = 0; u < KEEP / 4; ++u) {
+                const float4 x = make_float4(uv[u].x - v[4 * u], uv[u].y - v[4 * u + 1], uv[u].z - v[4 * u + 2], uv[u].w - v[4 * u + 3]);
+                *reinterpret_cast<float4*>(ur + (row >> 2) * SQ + (row & 3) * COLS + col + 4 * u) = x;
+                *reinterpret_cast<float4*>(Ud + row * UL + col + 4 * u) = make_float4(scale * x.x, scale * x.y, scale * x.z, scale * x.w);
+            }
+        }
+        float o[KEEP];
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i) o[i] = scale * v[i];
+        __syncthreads();                     // U is there, and S has been read
+        if (c + 1 < chunks) load_rows(c + 1);
+        if (reads_out) {
+            const float* src = p.p + (ph * CHUNK + row0) * CHUNK;
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) p4[r][i] = *reinterpret_cast<const float4*>(src + r * CHUNK + i * 32 + ks * 4);
+        }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < TR; ++j) {
+            float4 u4[COLS / 4];
+#pragma unroll
+            for (int u = 0; u < COLS / 4; ++u) u4[u] = *reinterpret_cast<const float4*>(Ud + (j * TS + ts) * UL + 4 * u);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float k = r == 0 ? k4[j].x : r == 1 ? k4[j].y : r == 2 ? k4[j].z : k4[j].w;
+#pragma unroll
+                for (int u = 0; u < COLS / 4; ++u) {
+                    v[r * COLS + 4 * u] = fmaf(k, u4[u].x, v[r * COLS + 4 * u]);
+                    v[r * COLS + 4 * u + 1] = fmaf(k, u4[u].y, v[r * COLS + 4 * u + 1]);
+                    v[r * COLS + 4 * u + 2] = fmaf(k, u4[u].z, v[r * COLS + 4 * u + 2]);
+                    v[r * COLS + 4 * u + 3] = fmaf(k, u4[u].w, v[r * COLS + 4 * u + 3]);
+                }
+            }
+        }
+        if (c + 1 < chunks) load_keys(c + 1);
+        reduce_scatter<NV, TS>(v, ts);
+        {
+            constexpr int KEEP2 = NV / TS;
+            float* sr = S + (d0 >> 2) * SQ + ts * KEEP2;
+            if (KEEP2 % 4 == 0) {
+#pragma unroll
+                for (int u = 0; u < KEEP2 / 4; ++u) {
+                    float4 x = *reinterpret_cast<float4*>(sr + 4 * u);
+                    x.x = fmaf(keep, x.x, v[4 * u]);
+                    x.y = fmaf(keep, x.y, v[4 * u + 1]);
+                    x.z = fmaf(keep, x.z, v[4 * u + 2]);
+                    x.w = fmaf(keep, x.w, v[4 * u + 3]);
+                    *reinterpret_cast<float4*>(sr + 4 * u) = x;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < KEEP2; ++i) sr[i] = fmaf(keep, sr[i], v[i]);
+            }
+        }
+        __syncthreads();                     // S is the state after the chunk
+        if (reads_out) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) v[i] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float* uj = ur + (i * 8 + ks) * SQ + q * COLS;
+                    float4 u4[COLS / 4];
+#pragma unroll
+                    for (int u = 0; u < COLS / 4; ++u) u4[u] = *reinterpret_cast<const float4*>(uj + 4 * u);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const float w = q == 0 ? p4[r][i].x : q == 1 ? p4[r][i].y : q == 2 ? p4[r][i].z : p4[r][i].w;
+#pragma unroll
+                        for (int u = 0; u < COLS / 4; ++u) {
+                            v[r * COLS + 4 * u] = fmaf(w, u4[u].x, v[r * COLS + 4 * u]);
+                            v[r * COLS + 4 * u + 1] = fmaf(w, u4[u].y, v[r * COLS + 4 * u + 1]);
+                            v[r * COLS + 4 * u + 2] = fmaf(w, u4[u].z, v[r * COLS + 4 * u + 2]);
+                            v[r * COLS + 4 * u + 3] = fmaf(w, u4[u].w, v[r * COLS + 4 * u + 3]);
+                        }
+                    }
+                }
+            }
+            reduce_scatter<NV, 8>(v, ks);
+            if (c * CHUNK + row < n) {
+                float* dst = p.out + (size_t)(q_beg + c * CHUNK + row) * ((size_t)p.H * E) + (size_t)h * E + e0 + col;
+#pragma unroll
+                for (int i = 0; i < KEEP; ++i)
+                    if (e0 + col + i < E) dst[i] = o[i] + v[i];
+            }
+        }
+    }
+    if (st) {
+        for (int idx = tid; idx < DP * COLS; idx += CTHREADS) {
+            const int d = idx / COLS, c = idx % COLS;
+            if (d < D && e0 + c < E) st[(size_t)d * E + e0 + c] = S[(d >> 2) * SQ + (d & 3) * COLS + c];
+        }
+    }
+}
+
 static int chunk_width(int D) { return D <= 32 ? 32 : D <= 64 ? 64 : 128; }
 static int chunk_places(int n_tokens, int n_seqs) { return n_tokens / CHUNK + std::min(n_seqs, n_tokens); }
+
+// Whether the outputs of a step are made in the walk along each sequence or, side by side, behind it: a block of the outputs alone takes some 30 us,
+// which pays once its blocks, one a place and head, fill the SMs twice.  One sequence, 16 heads of 128 x 128, all launches, us in the walk / behind
+// it: 256 tokens 64 / 97, 600 98 / 117, 1,000 136 / 143, 2,048 284 / 240; four of 512 297 / 247, 64 single tokens beside 256 858 / 769.
+static bool few_chunks(int places, int H) { return (long long)places * H < 2LL * device_sm_count(); }
 
 // Floats of scratch for a step of n_tokens rows in n_seqs sequences; 0: the kernels do not take these sizes.
 LLMK_EXPORT long long llmk_head_delta_chunk_floats(int n_tokens, int n_seqs, int H, int G, int D, int E) {
     if (n_tokens <= 0 || n_seqs <= 0 || D <= 0 || D > 128 || E <= 0 || H <= 0 || G <= 0) return 0;
     const long long dp = chunk_width(D), ep = ceil_div(E, 16) * 16;
-    return (long long)chunk_places(n_tokens, n_seqs) * (CHUNK * (2 * G * dp + H * (dp + ep + CHUNK + 2)) + H * dp * ep);
+    const long long places = chunk_places(n_tokens, n_seqs);
+    return places * (CHUNK * (2 * G * dp + H * (dp + ep + CHUNK + 2)) + (few_chunks((int)places, H) ? 0 : H * dp * ep));
 }
+// How many kernels `llmk_head_delta_chunks` launches.
+LLMK_EXPORT int llmk_head_delta_chunk_launches(int n_tokens, int n_seqs, int H) { return few_chunks(chunk_places(n_tokens, n_seqs), H) ? 2 : 3; }
 
 template <int DP>
 static cudaError_t launch_chunks(const ChunkParams& p, int places, cudaStream_t s) {
@@ -978,7 +1178,11 @@ static cudaError_t launch_chunks(const ChunkParams& p, int places, cudaStream_t 
     cudaError_t e = llmk_launch(chunk_prep_kernel<DP>, dim3(places, p.H), dim3(CTHREADS), smem, s, true, p);
     if (e != cudaSuccess) return e;
     // sixteen columns a block where eight would not fit the SMs side by side
-    e = p.H * ceil_div(p.E, 8) <= device_sm_count()
+    const bool narrow = p.H * ceil_div(p.E, 8) <= device_sm_count();
+    if (few_chunks(places, p.H))
+        return narrow ? llmk_launch(chunk_walk_kernel<DP, 8>, dim3(p.n_seqs, p.H, ceil_div(p.E, 8)), dim3(CTHREADS), 0, s, true, p)
+                      : llmk_launch(chunk_walk_kernel<DP, 16>, dim3(p.n_seqs, p.H, ceil_div(p.E, 16)), dim3(CTHREADS), 0, s, true, p);
+    e = narrow
             ? llmk_launch(chunk_scan_kernel<DP, 8>, dim3(p.n_seqs, p.H, p.EP / 8), dim3(CTHREADS), 0, s, true, p)
             : llmk_launch(chunk_scan_kernel<DP, 16>, dim3(p.n_seqs, p.H, p.EP / 16), dim3(CTHREADS), 0, s, true, p);
     if (e != cudaSuccess) return e;

@@ -1360,7 +1360,8 @@ def head_delta_chunks(out: torch.Tensor, qkv: torch.Tensor, gates: torch.Tensor,
         raise KernelError("head_delta_chunks: the scratch is too small")
     _check(lib, lib.llmk_head_delta_chunks(_ptr(out), _ptr(qkv), _ptr(gates), _ptr(state), c_longlong(_row_stride(state)), _ptr(cu_q),
                                            _ptr(state_slots), _ptr(scratch), c_int(n_seqs), c_int(out.shape[0]), c_int(heads), c_int(kv_heads),
-                                           c_int(dim), c_int(vdim), _stream()), 3)
+                                           c_int(dim), c_int(vdim), _stream()),
+           lib.llmk_head_delta_chunk_launches(c_int(out.shape[0]), c_int(n_seqs), c_int(heads)))
 
 
 def head_delta_step_usable(heads: int, kv_heads: int, dim: int, vdim: int) -> bool:
