@@ -216,7 +216,7 @@ class Executor:
     def _activation_reserve(self) -> int:
         """Device memory to leave beside the cache pages for a step's activations: what the widest layer says it
         keeps in the workspace (`workspace_bytes(tokens)`; a layer that does not say is counted by its hidden
-        width alone), the float32 residual, and the logits of a batch of decoded tokens."""
+        width alone), what its mixers' scratch takes more for as many sequences as a step can have, the float32 residual, and the logits of a batch of decoded tokens."""
         spec = self.model.spec
         tokens = self.limits.max_step_tokens
         elem = 2 if self.dtype == torch.bfloat16 else 4
@@ -224,6 +224,10 @@ class Executor:
         for layer in self.model.layers:
             ask = getattr(layer, "workspace_bytes", None)
             widest = max(widest, ask(tokens) if ask is not None else 6 * tokens * spec.hidden_size * elem)
+        # scratch that follows the sequences: as many of them as a step can have
+        seqs = min(self.limits.max_num_seqs, tokens)
+        asks = [getattr(m, "sequence_bytes", None) for m in self.model.mixers()]
+        widest += max([f(tokens, seqs) for f in asks if f is not None] + [0])
         rows = max(64, self.limits.max_num_seqs)
         return widest + tokens * spec.hidden_size * 4 + 2 * rows * spec.vocab_size * 4 + (64 << 20)
 

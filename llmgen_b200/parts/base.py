@@ -49,6 +49,9 @@ Mixer, feed-forward and block, optional:
     workspace_bytes(tokens) -> int            bytes of activations a step of `tokens` rows keeps in
                                               the workspace for this part; the engine leaves that
                                               much device memory beside the cache pages
+Mixer, optional:
+    sequence_bytes(tokens, seqs) -> int       what scratch that grows with the sequences of a step takes more (or
+                                              less) for `seqs` of them than `workspace_bytes` counts
 Block:
     mixer                                     the block's mixer (the engine asks it for cache)
     forward(ctx, resid, delta, cache) -> delta_out

@@ -164,6 +164,10 @@ class HeadDecayDelta(Mixer):
         return chunks + tokens * ((self.decay_off + self.H) * elem + self.qkv * 4 + (2 * self.H + self.G) * 4 + he * (4 + elem)
                          + self.spec.hidden_size * elem) + ops.SLICED_PRODUCT_BYTES
 
+    def sequence_bytes(self, tokens: int, seqs: int) -> int:
+        return 4 * (ops.head_delta_chunk_floats(tokens, max(seqs, 1), self.H, self.G, self.D, self.E)
+                    - ops.head_delta_chunk_floats(tokens, max(1, tokens // 32), self.H, self.G, self.D, self.E))
+
     # -- what a parallel mixer asks that multiplies with several branches' matrices at once (see `parts.parallel`)
     def shared_projections(self):
         return SharedProjections(self.w_in, self.w_o)
@@ -195,9 +199,10 @@ class HeadDecayDelta(Mixer):
                             cache.state[:, self.s_size:] if self.spec.conv.taps > 1 else None, ctx.cu_q, ctx.state_slots, ctx.n_seqs,
                             H, G, D, E, float(self.spec.unit_eps))
         o = ws.buffer("hdelta_o", T, H * E, torch.float32)
-        floats = ops.head_delta_chunk_floats(T, ctx.n_seqs, H, G, D, E) if T >= self.CHUNKED_ROWS else 0
-        if floats:
-            scratch = ws.flat("hdelta_chunks", floats, torch.float32)
+        if T >= self.CHUNKED_ROWS and ops.head_delta_chunk_floats(T, ctx.n_seqs, H, G, D, E):
+            # (one array for all steps, as long as the largest step of the engine asks for)
+            most = ops.head_delta_chunk_floats(max(T, ws.default_rows), max(ctx.n_seqs, ctx.max_seqs_bound), H, G, D, E)
+            scratch = ws.flat("hdelta_chunks", most, torch.float32)
             ops.head_delta_chunks(o, qkv, gates, cache.state, ctx.cu_q, ctx.state_slots, scratch, ctx.n_seqs, H, G, D, E)
         else:
             ops.delta_scan_heads(o, qkv, gates, cache.state, ctx.cu_q, ctx.state_slots, ctx.n_seqs, H, G, D, E)

@@ -118,6 +118,10 @@ class ParallelMixer(Mixer):
         shared = tokens * (self.w_in.shape[0] + self.w_out.shape[1]) * self.w_in.element_size() if self.w_in is not None else 0
         return sum(f(tokens) for f in asks if f is not None) + tokens * self.cols_hint() * 4 + shared
 
+    def sequence_bytes(self, tokens: int, seqs: int) -> int:
+        asks = [getattr(b, "sequence_bytes", None) for b in self.branches]
+        return sum(f(tokens, seqs) for f in asks if f is not None)
+
     def cols_hint(self) -> int:
         return int(getattr(self.spec.branches[0], "hidden_size", 0))
 
