@@ -4,7 +4,7 @@
 //
 // X's rows are sorted by expert; `spans` (csrc/moe.cu, on the device: the launch has the same shape whatever the experts' counts are) lists
 // runs of at most 256 rows of one expert, an expert's rows cut evenly.  A pair of blocks (a cluster of two, `tcgen05.mma.cta_group::2`) computes
-// 256 rows of W by one span, one such tile after the other; 192 threads a block:
+// 256 rows of W by one span, one such tile after the other; 320 threads a block:
 //   warp 0     TMA producer: per step of 64 along K this block's 128 rows of W and its half of the span's rows (boxes of 128, 64, 32 and
 //              16 rows), in a ring of six stages; no multicast, every block loads what it holds.
 //   warp 1     of rank 0 issues the MMAs (columns: the span's rows rounded up to 32), two accumulators of 256 columns in turn

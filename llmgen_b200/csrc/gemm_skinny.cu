@@ -302,8 +302,8 @@ int dispatch_rows(const CUtensorMap& mw, const void* X, void* C, int M, int N, i
 }
 
 // Into how many slices of K, a cluster's blocks, a product written directly is cut: W of fewer rows than keep half of the SMs busy is
-// pulled by few of them at some 40 GB/s each.  At most 8 slices, of four steps of 64 at least; from N and K alone, so that
-// a row's sum does not depend on M.
+// pulled by few of them at some 40 GB/s each.  At most 8 slices, of four steps of 64 at least; from N, K and the device's SMs, so that
+// a row's sum is the same for any M up to 64, the most rows that a cluster's shared memory holds (above, K is not cut).
 int direct_splits(int N, int K) {
     const int tiles = ceil_div(N, BW), num_kb = ceil_div(K, BK);
     int splits = std::min(std::min(device_sm_count() / tiles, num_kb / 4), 8);

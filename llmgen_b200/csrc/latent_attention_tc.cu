@@ -57,7 +57,7 @@ struct Params {
     const int* tile_seq;
     const int* tile_q0;
     int* error_flag;
-    int tq_pad, t_pad, max_blocks, heads, rank, window, gc, bq, halves, page_shift;
+    int tq_pad, t_pad, max_blocks, heads, rank, window, bq, halves, page_shift;
     float scale_log2;
 };
 
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attention_tc_kernel(const _
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // (the same for all lanes, and known to be)
-    const int half = blockIdx.x % p.halves, chunk = blockIdx.x / p.halves;
+    const int half = blockIdx.x;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
@@ -314,8 +314,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attention_tc_kernel(const _
         // index of this lane's row among the queries and among the results (tokens x heads in either layout); -1: nobody's row
         int source = -1, place = -1;
         {
-            const int qi = r / p.gc, hh = chunk * p.gc + r % p.gc, tok = q_beg + q0 + qi;
-            if (r < p.bq * p.gc && qi < nq_tile && hh < p.heads) {
+            const int qi = r / p.heads, hh = r % p.heads, tok = q_beg + q0 + qi;
+            if (r < p.bq * p.heads && qi < nq_tile) {
                 source = p.qa_hm ? hh * p.tq_pad + tok : tok * p.heads + hh;
                 place = p.out_hm ? hh * p.t_pad + tok : tok * p.heads + hh;
             }
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attention_tc_kernel(const _
             tc::tc_fence_before_sync();
             tc::mbar_arrive(tc::smem_u32(q_full));
         }
-        const int qpos = first_pos + r / p.gc;
+        const int qpos = first_pos + r / p.heads;
         const int lo = p.window > 0 ? qpos - p.window : -1;      // keys at positions > lo are seen
         const uint32_t s_addr = tmem_base + lane_addr + L::S_COL + (uint32_t)(side * 32);
         const uint32_t p_addr = tmem_base + lane_addr + L::P_COL + (uint32_t)(side * 16);
@@ -603,7 +603,7 @@ LLMK_EXPORT int llmk_latent_attention_tc(float* out, const float* qa, const void
     p.qa = qa; p.qa_hm = static_cast<const bf16*>(qa_hm); p.out = out; p.out_hm = static_cast<bf16*>(out_hm);
     p.block_tables = block_tables; p.ctx_len = ctx_len; p.cu_q = cu_q; p.tile_seq = tile_seq; p.tile_q0 = tile_q0; p.error_flag = error_flag;
     p.tq_pad = tq_pad; p.t_pad = t_pad; p.max_blocks = max_blocks; p.heads = heads; p.rank = rank; p.window = window > 0 ? window : 0;
-    p.gc = heads; p.bq = bq; p.halves = rank / NV;
+    p.bq = bq; p.halves = rank / NV;
     p.page_shift = page_size == 16 ? 4 : page_size == 32 ? 5 : page_size == 64 ? 6 : 7;
     p.scale_log2 = scale * 1.4426950408889634f;
     // the cache as [blocks of 64 entries][tokens][64]

@@ -482,8 +482,8 @@ LLMK_EXPORT int llmk_moe_plan(const int* slot_expert, int n_slots, int E, int ti
 }
 
 // --------------------------------------------------------------------------------------------- gather
-// xs[pos, :] = (T)(weight * h[token of order[pos], :]) for the rows a padded plan filled; rows of padding stay as they are: the
-// products that follow compute them like any other and nobody reads the result.
+// xs[pos, :] = (T)(weight * h[token of order[pos], :]) for the rows a padded plan filled; rows of padding stay as they are: no
+// span of the products that follow has them.
 template <typename T>
 __global__ void moe_gather_kernel(T* xs, const T* h, long long ldh, const int* order,
                                   const float* slot_weight, int top, int K, int scale_rows) {

@@ -503,7 +503,8 @@ def gemm_skinny(out: torch.Tensor, a: torch.Tensor, w: torch.Tensor, mode: int =
     SKINNY_DIRECT: out[M, N]; SKINNY_GATED: out[M, N/2] = silu(gate) * up; SKINNY_PARTIAL: out is
     float32 [splits, M, N] and receives the partial sums of `splits` slices of K;
     SKINNY_CLUSTER_GATED: out[M, N/2] = silu(gate) * up from `splits` slices of K (2 or 4) added up
-    inside a thread-block cluster (M <= 64)."""
+    inside a thread-block cluster (M <= 64).  SKINNY_DIRECT with M <= 64 and a W of few rows is cut along K too: a row's sum is the same for
+    any M up to 64 on one kind of device, and in another order above."""
     lib = build.load("gemm_skinny")
     M, K = a.shape
     N = w.shape[0]

@@ -132,7 +132,11 @@ class LatentAttention(Mixer):
         return ("attention_tiles", self.bq, self.bq_single, self.heads, self.kv_rank, self.rope, self.window, float(self.spec.scale) > 0.0)
 
     def tc_tile_queries(self, page_size: int) -> int:
-        """Queries per tile of the kernel on tcgen05 (0: steps other than single tokens stay on `mma.sync` or the CUDA cores)."""
+        """Queries per tile of the kernel on tcgen05 (0: steps other than single tokens stay on `mma.sync` or the CUDA cores).  Every step that is
+        not single tokens alone takes it, its single tokens too, which fill 16 of a tile's 128 rows: a block's walk along the keys is what such a
+        step waits for, and a tile of 64 keys takes a third of the time (us, `mma.sync` / tcgen05, 16 heads of rank 512: 8 single tokens at
+        3,500 keys beside a portion of 300 295 / 110, 64 at 2,000 beside 500 178 / 96, 64 at 500 beside 64 49 / 27, 200 at 500 99 / 83, a portion of 16
+        alone 15.6 / 14.2, of 64 20.7 / 14.3; steps of single tokens have their keys in parts on `mma.sync`)."""
         if page_size not in self._tc_bq:
             self._tc_bq[page_size] = (ops.latent_attention_tc_tile_queries(self.dtype, self.heads, self.kv_rank, self.rope, page_size)
                                       if float(self.spec.scale) > 0.0 else 0)

@@ -5,8 +5,9 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# two to eight slices, a last one shorter than the others, tails in N and M, one tile of W
-@pytest.mark.parametrize("N,K", [(2048, 2048), (2048, 4096), (1000, 520), (130, 3072), (8, 776), (9000, 512)])
+# clusters of two to eight slices (8, 8, 2, 8, 3, 2, then 4, 5, 6, 7), a last one shorter than the others, tails in N and M, one tile of W
+@pytest.mark.parametrize("N,K", [(2048, 2048), (2048, 4096), (1000, 520), (130, 3072), (8, 776), (9000, 512), (4700, 1024), (3712, 1280), (3000, 1536),
+                                 (2600, 1792)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 def test_rows_and_their_independence(N, K, out_dtype):
     from llmgen_b200.kernels import ops
@@ -20,7 +21,7 @@ def test_rows_and_their_independence(N, K, out_dtype):
     ops.gemm_skinny(full[:64, :N], ad, wd)
     torch.cuda.synchronize()
     ops.check_tc_errors(full.device)
-    # float32 sums of K products, in slices; a bfloat16 result is rounded once (2^-9 of it)
+    # float32 sums of K products, in slices; a bfloat16 result is rounded once (up to 2^-8 of it)
     assert float((full[:64, :N].double().cpu() - ref).abs().max()) < (2e-5 if out_dtype == torch.float32 else 4e-3) * float(ref.abs().max())
     assert bool((full[64] == 7.0).all()) and bool((full[:, N:] == 7.0).all())
     for rows in (slice(0, 1), slice(5, 8), slice(11, 28), slice(40, 64)):        # a row's sum does not depend on how many there are

@@ -16,7 +16,8 @@ def _exact(q, z, rank, scale, positions, window):
 
 
 # sequences: (tokens in the cache after the step, tokens of the step).  Tiles are 128 // heads queries by 64 keys: one token alone, whole
-# tiles, one more and one less, a portion deep into its context, heads that leave rows over, one query a tile
+# tiles, one more and one less, a portion deep into its context, heads that leave rows over, one query a tile, single tokens deep into theirs
+# beside a portion
 @pytest.mark.parametrize("heads,rank,page,window,seqs", [
     (16, 512, 16, 0, [(1, 1), (64, 64), (65, 65), (63, 9), (200, 7)]),
     (16, 512, 32, 0, [(321, 130), (128, 128)]),
@@ -25,6 +26,8 @@ def _exact(q, z, rank, scale, positions, window):
     (128, 256, 128, 0, [(130, 5), (3, 3)]),
     (16, 512, 16, 50, [(300, 60), (40, 40)]),
     (5, 256, 128, 64, [(260, 100)]),
+    (16, 512, 16, 0, [(700, 1), (515, 1), (300, 77), (1100, 1), (64, 1)]),
+    (8, 256, 64, 100, [(1000, 1), (333, 33), (129, 1)]),
 ])
 def test_against_float64(heads, rank, page, window, seqs):
     from llmgen_b200.kernels import ops
