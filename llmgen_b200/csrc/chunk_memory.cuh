@@ -471,6 +471,10 @@ __global__ void __launch_bounds__(THREADS) chunk_memory_scan_kernel(Params p) {
 // blocks' shared memory fits (a prompt of 2,048 under a running maximum, 8 heads: 28.4 -> 23.8 us; the layer's pass 296 -> 290, with one block of
 // sixteen 294), as one block of sixteen where they are three (constant decay, 16 heads: 70.1 -> 66.8 us, the pass 355 -> 350).  What holds the second
 // form is not its warps: the MMAs of its terms take 19 us at the rate `mma.sync` reaches alone.
+// BLOCKS: blocks an SM has to have room for.  Room for two takes half of the registers from a block's chain, so where the SMs have a chunk and head each at the most
+// a block has its SM for itself (`lone_blocks`): under a running maximum, the three launches, us with room for two / for one: 8 heads of 128 x 128, 100 tokens
+// 33.3 / 27.8, 600 35.5 / 31.1, 1,200 40.0 / 43.1, eight of 100 53.9 / 47.8; 16 heads, 300 tokens 35.5 / 33.0, 600 41.7 / 44.0, 64 single tokens beside
+// 300 143 / 127.
 template <typename T, int FORM> constexpr int out_warps() { return input_terms<T, FORM>() == 1 ? 8 : 16; }
 template <typename T, int FORM, int D>
 struct OutLayout {
@@ -478,8 +482,8 @@ struct OutLayout {
     static constexpr int Q = NT * C * LDD, KS = (NT * C * LDD > 3 * D * LDE ? NT * C * LDD : 3 * D * LDE), P = 3 * C * LDP, V = NT * C * LDE;
     static constexpr size_t bytes() { return (size_t)(Q + KS + P + V) * sizeof(bf16); }
 };
-template <typename T, int FORM, int D>
-__global__ void __launch_bounds__(32 * out_warps<T, FORM>(), 16 / out_warps<T, FORM>()) chunk_memory_out_kernel(Params p) {
+template <typename T, int FORM, int D, int BLOCKS>
+__global__ void __launch_bounds__(32 * out_warps<T, FORM>(), BLOCKS) chunk_memory_out_kernel(Params p) {
     using L = OutLayout<T, FORM, D>;
     constexpr int NT = L::NT, LDD = L::LDD, WARPS = out_warps<T, FORM>(), NTHREADS = 32 * WARPS, GROUPS = WARPS / 4, N8 = 8 / GROUPS;
     extern __shared__ __align__(16) bf16 smem[];
@@ -663,16 +667,23 @@ inline bool usable(const Params& p, int elem) {
            host_aligned16(p.v) && host_aligned16(p.out) && host_aligned16(p.scratch);
 }
 
+// Whether a step's chunks and heads, with half a chunk more for every sequence that may be long, are no more than the SMs.
+inline bool lone_blocks(const Params& p, int n_tokens) {
+    return (2LL * n_tokens + (long long)p.longs * C) * p.H <= 2LL * C * device_sm_count();
+}
 template <typename T, int FORM, int D>
-static int launch_width(const Params& p, cudaStream_t s) {
+static int launch_width(const Params& p, int n_tokens, cudaStream_t s) {
     constexpr int NT = input_terms<T, FORM>();
     const size_t local = (size_t)(NT * C * (D + 8) + 3 * C * LDE) * sizeof(bf16), out = OutLayout<T, FORM, D>::bytes();
     auto k1 = chunk_memory_local_kernel<T, FORM, D>;
-    auto k3 = chunk_memory_out_kernel<T, FORM, D>;
+    constexpr int MOST = 16 / out_warps<T, FORM>();
+    auto k3 = chunk_memory_out_kernel<T, FORM, D, MOST>;
+    auto k3_lone = chunk_memory_out_kernel<T, FORM, D, 1>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)local);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k3_lone, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
         if (e != cudaSuccess) LLMK_FAIL("chunk_memory: cannot raise shared memory: %s", cudaGetErrorString(e));
         configured = true;
     }
@@ -681,12 +692,12 @@ static int launch_width(const Params& p, cudaStream_t s) {
     const dim3 scan((unsigned)std::min<long long>(items, 8 * device_sm_count()));
     LLMK_CHECK_LAUNCH_RC("chunk_memory_local", llmk_launch(k1, grid, dim3(THREADS), local, s, true, p));
     LLMK_CHECK_LAUNCH_RC("chunk_memory_scan", llmk_launch(chunk_memory_scan_kernel<FORM>, scan, dim3(THREADS), 0, s, true, p));
-    LLMK_CHECK_LAUNCH_RC("chunk_memory_out", llmk_launch(k3, grid, dim3(32 * out_warps<T, FORM>()), out, s, true, p));
+    LLMK_CHECK_LAUNCH_RC("chunk_memory_out", llmk_launch(lone_blocks(p, n_tokens) ? k3_lone : k3, grid, dim3(32 * out_warps<T, FORM>()), out, s, true, p));
     return LLMK_OK;
 }
 template <typename T, int FORM>
-static int launch(const Params& p, cudaStream_t s) {
-    return p.D == 64 ? launch_width<T, FORM, 64>(p, s) : launch_width<T, FORM, 128>(p, s);
+static int launch(const Params& p, int n_tokens, cudaStream_t s) {
+    return p.D == 64 ? launch_width<T, FORM, 64>(p, n_tokens, s) : launch_width<T, FORM, 128>(p, n_tokens, s);
 }
 
 }  // namespace chunk_memory

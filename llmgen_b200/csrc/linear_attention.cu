@@ -456,8 +456,8 @@ LLMK_EXPORT int llmk_linear_attention(float* out, const void* q, const void* k, 
         c.n_seqs = n_seqs; c.silu = silu; c.q_scale = 1.f;
         chunk_memory::shape(c, chunk_memory::CM_CONST, n_tokens);
         if (chunk_memory::usable(c, dtype == LLMK_F32 ? 4 : 2)) {
-            const int rc = dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_CONST>(c, (cudaStream_t)stream)
-                                             : chunk_memory::launch<bf16, chunk_memory::CM_CONST>(c, (cudaStream_t)stream);
+            const int rc = dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_CONST>(c, n_tokens, (cudaStream_t)stream)
+                                             : chunk_memory::launch<bf16, chunk_memory::CM_CONST>(c, n_tokens, (cudaStream_t)stream);
             if (rc != LLMK_OK) return rc;
             *launches = 3;
             p.odd = c.odd();

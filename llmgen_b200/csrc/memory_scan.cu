@@ -685,7 +685,7 @@ LLMK_EXPORT int llmk_memory_scan(float* out, const void* r, long long ldr, const
         c.n_seqs = n_seqs; c.q_scale = r_scale; c.den_eps = den_eps;
         chunk_memory::shape(c, chunk_memory::CM_MAX, n_tokens);
         if (chunk_memory::usable(c, dtype == LLMK_F32 ? 4 : 2) && host_aligned16(dots)) {
-            const int rc = dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_MAX>(c, st) : chunk_memory::launch<bf16, chunk_memory::CM_MAX>(c, st);
+            const int rc = dtype == LLMK_F32 ? chunk_memory::launch<float, chunk_memory::CM_MAX>(c, n_tokens, st) : chunk_memory::launch<bf16, chunk_memory::CM_MAX>(c, n_tokens, st);
             if (rc != LLMK_OK) return rc;
             *launches = 3;
             p.odd = c.odd();

@@ -80,6 +80,20 @@ def test_a_sequence_gives_what_it_gives_alone(form, dtype):
     assert torch.equal(state[100], before[100])
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("form", [linear, mlstm])
+def test_a_sequence_among_more_chunks_than_the_sms_take_at_once(form, dtype):
+    """60 sequences of 100 tokens and 2 heads: 240 blocks of outputs, two an SM; alone a sequence's blocks have an SM each."""
+    lens = [100] * 60
+    x, state = rows(sum(lens), dtype), fresh(form, len(lens))
+    before = state.clone()
+    out = form(x, state, lens)
+    for s in (0, 31, 59):
+        alone = before[s:s + 1].clone()
+        assert torch.equal(form(x[100 * s:100 * (s + 1)].contiguous(), alone, [100]), out[100 * s:100 * (s + 1)])
+        assert torch.equal(alone, state[s:s + 1])
+
+
 @pytest.mark.parametrize("form", [linear, mlstm])
 def test_scratch_follows_what_long_sequences_can_be_there(form):
     entries = D * E + (D if form is mlstm else 0)
