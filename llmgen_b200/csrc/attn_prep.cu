@@ -328,43 +328,46 @@ attn_prep_vec_kernel(const T* qkv, long long row_stride, T* q_out, long long q_s
     }
 }
 
-// Eight bytes from each half of a row: two float32 or four bfloat16 values twice.
-template <typename T>
-struct Halves {
-    uint2 lo, hi;
+// Four values from each half of a row: 16 bytes twice of float32, 8 bytes twice of bfloat16.
+template <typename T> struct Halves;
+template <> struct Halves<float> {
+    typedef float4 Part;
+    Part lo, hi;
     __device__ __forceinline__ void unpack(float* f) const {
-        Vec16<T> v;
-        if constexpr (sizeof(T) == 4) v.raw = make_float4(__uint_as_float(lo.x), __uint_as_float(lo.y), __uint_as_float(hi.x), __uint_as_float(hi.y));
-        else v.raw = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w;
+        f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
+    }
+    __device__ __forceinline__ void pack(const float* f) {
+        lo = make_float4(f[0], f[1], f[2], f[3]);
+        hi = make_float4(f[4], f[5], f[6], f[7]);
+    }
+    __device__ __forceinline__ void clear() { lo = hi = make_float4(0.f, 0.f, 0.f, 0.f); }
+};
+template <> struct Halves<bf16> {
+    typedef uint2 Part;
+    Part lo, hi;
+    __device__ __forceinline__ void unpack(float* f) const {
+        Vec16<bf16> v;
+        v.raw = make_uint4(lo.x, lo.y, hi.x, hi.y);
         v.unpack(f);
     }
     __device__ __forceinline__ void pack(const float* f) {
-        Vec16<T> v;
+        Vec16<bf16> v;
         v.pack(f);
-        if constexpr (sizeof(T) == 4) {
-            lo = make_uint2(__float_as_uint(v.raw.x), __float_as_uint(v.raw.y));
-            hi = make_uint2(__float_as_uint(v.raw.z), __float_as_uint(v.raw.w));
-        } else {
-            lo = make_uint2(v.raw.x, v.raw.y);
-            hi = make_uint2(v.raw.z, v.raw.w);
-        }
+        lo = make_uint2(v.raw.x, v.raw.y);
+        hi = make_uint2(v.raw.z, v.raw.w);
     }
+    __device__ __forceinline__ void clear() { lo = hi = make_uint2(0u, 0u); }
 };
-template <int N>
 __device__ __forceinline__ void load_floats(float* f, const float* src) {
-    if constexpr (N == 4) {
-        const float4 v = *reinterpret_cast<const float4*>(src);
-        f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
-    } else {
-        const float2 v = *reinterpret_cast<const float2*>(src);
-        f[0] = v.x; f[1] = v.y;
-    }
+    const float4 v = *reinterpret_cast<const float4*>(src);
+    f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
 }
 
 // The same, a warp taking `U` rounds of rows of ONE token at a time: position, slot, the lane's cos and
 // sin values and its gains are read once for U * 32 / LPR rows (16 heads of 128 in bfloat16) instead of
 // once a row, and the U loads of the rows are in flight together.  A lane holds EPL / 2 neighbouring values of a row's low half and the
-// same of its high half, so the pairs that the rotation mixes lie in one lane: 8-byte accesses, but no exchange of
+// same of its high half, so the pairs that the rotation mixes lie in one lane: 8-byte accesses in bfloat16, but no exchange of
 // every value and half the cos and sin values a lane, and registers for more warps (bound by the loads in flight: 34 MB for 2,048 tokens of 32 heads
 // of 128; with a lane's values in one piece and eight rounds 700 / 2,048 / 8,000 tokens took 5.8 / 10.7 / 43.2 us).
 template <typename T, int LPR, int U>
@@ -375,7 +378,8 @@ attn_prep_token_kernel(const T* qkv, long long row_stride, T* q_out, long long q
                        const float* sin_tab, const float* q_gain,
                        const float* k_gain, int n_tokens, int nq, int nk, int nkv_cache, int hd,
                        int page_size, float eps, float q_off, float k_off) {
-    constexpr int EPL = Vec16<T>::N, HALF = EPL / 2;       // elements per lane
+    constexpr int HALF = 4, EPL = 2 * HALF;     // elements per lane
+    typedef typename Halves<T>::Part Part;
     constexpr int RPW = 32 / LPR;               // rows per round
     constexpr int RC = U * RPW;                 // rows per item
     pdl_launch_dependents();
@@ -406,18 +410,18 @@ attn_prep_token_kernel(const T* qkv, long long row_stride, T* q_out, long long q
         for (int u = 0; u < U; ++u) {
             const int h = h0 + u * RPW;
             if (h < heads) {
-                x[u].lo = *reinterpret_cast<const uint2*>(src + (size_t)h * hd + low);
-                x[u].hi = *reinterpret_cast<const uint2*>(src + (size_t)h * hd + high);
+                x[u].lo = *reinterpret_cast<const Part*>(src + (size_t)h * hd + low);
+                x[u].hi = *reinterpret_cast<const Part*>(src + (size_t)h * hd + high);
             } else {
-                x[u].lo = x[u].hi = make_uint2(0u, 0u);
+                x[u].clear();
             }
         }
         const int slot = slots ? slots[t] : -1;
         float cv[HALF], sv[HALF];
         if (cos_tab) {
             const size_t at = (size_t)positions[t] * (hd / 2) + low;
-            load_floats<HALF>(cv, cos_tab + at);
-            load_floats<HALF>(sv, sin_tab + at);
+            load_floats(cv, cos_tab + at);
+            load_floats(sv, sin_tab + at);
         }
         const int page = slot >= 0 ? slot / page_size : 0;
         const int in_page = slot - page * page_size;
@@ -462,8 +466,8 @@ attn_prep_token_kernel(const T* qkv, long long row_stride, T* q_out, long long q
                     }
                     x[u].pack(f);
                 }
-                *reinterpret_cast<uint2*>(dst + low) = x[u].lo;
-                *reinterpret_cast<uint2*>(dst + high) = x[u].hi;
+                *reinterpret_cast<Part*>(dst + low) = x[u].lo;
+                *reinterpret_cast<Part*>(dst + high) = x[u].hi;
             }
         }
     }
@@ -494,7 +498,8 @@ static bool launch_vec(const void* qkv, long long row_stride, void* q_out, long 
     if (g_prep_by_token) {
 #define LAUNCH_TOKEN(L, U)                                                                                                  \
     do {                                                                                                                    \
-        const int chunks = (nq + 2 * nk + U * rpw - 1) / (U * rpw);                                                         \
+        constexpr int rows_item = U * 32 / (L);                                                                             \
+        const int chunks = (nq + 2 * nk + rows_item - 1) / rows_item;                                                       \
         long long tblocks = ((long long)n_tokens * chunks + 7) / 8;                                                         \
         if (tblocks > device_sm_count() * 8) tblocks = device_sm_count() * 8;                                                                           \
         *err = llmk_launch(attn_prep_token_kernel<T, L, U>, dim3((unsigned)tblocks), dim3(256), 0, s, true, (const T*)qkv,  \
@@ -503,9 +508,19 @@ static bool launch_vec(const void* qkv, long long row_stride, void* q_out, long 
     } while (0)
         // four rounds of rows in flight a warp, three blocks an SM: 700 / 2,048 / 8,000 tokens of 32 heads of 128 in bfloat16 4.1 / 9.9 / 34.3 us;
         // eight rounds at two blocks 5.5 / 10.5 / 42.7, four at four blocks (registers to memory) 5.8 / 9.8 / 34.8, two at five 5.8 / 12.7 / 43.3
-        if (lpr == 8) LAUNCH_TOKEN(8, 4);
-        else if (lpr == 16) LAUNCH_TOKEN(16, 4);
-        else LAUNCH_TOKEN(32, 4);
+        // float32, 8 lanes' 16 bytes twice a row: two rounds while there are few warps (16 for each SM's 128 lanes): 48 / 300 / 500 tokens of 32 heads 2.8 / 4.4 / 5.5 us,
+        // with four 4.0 / 4.9 / 5.1; 2,048 / 8,000 tokens 16.0 / 74.2 (8 bytes twice a row 22.5 / 96.8, a row's 16 bytes in one piece and eight rounds 22.1 / 89.7)
+        const int lanes = hd / 8;
+        if constexpr (sizeof(T) == 4) {
+            const bool few = (long long)n_tokens * (nq + 2 * nk) * lanes <= 128LL * 16 * device_sm_count();
+            if (lanes == 4) { if (few) LAUNCH_TOKEN(4, 2); else LAUNCH_TOKEN(4, 4); }
+            else if (lanes == 8) { if (few) LAUNCH_TOKEN(8, 2); else LAUNCH_TOKEN(8, 4); }
+            else { if (few) LAUNCH_TOKEN(16, 2); else LAUNCH_TOKEN(16, 4); }
+        } else {
+            if (lanes == 8) LAUNCH_TOKEN(8, 4);
+            else if (lanes == 16) LAUNCH_TOKEN(16, 4);
+            else LAUNCH_TOKEN(32, 4);
+        }
 #undef LAUNCH_TOKEN
         return true;
     }
